@@ -12,6 +12,7 @@ namespace {
 
 constexpr int FWD_WARPS = 4;
 constexpr int FWD_BATCH = 32;
+static_assert(FWD_BATCH == 1 << SEG_SHIFT_MIN, "a segment of the backward is a whole number of batches");
 #ifndef B2K_FWD_GROUP
 #define B2K_FWD_GROUP 4
 #endif
@@ -25,12 +26,16 @@ constexpr int FWD_GROUP = B2K_FWD_GROUP;                 // fragments whose stat
 // whether any pixel of the tile can still take a fragment.
 constexpr uint32_t DONE_BIT = 0x80000000u;
 
-template <bool BWD, bool DEPTH, bool CHUNKED, bool FEAT>
+// What the forward leaves for the backward (common.cuh): nothing, checkpoints of the running sums, or of each segment's sums.
+enum Checkpoints { NONE = 0, RUNNING = 1, PER_SEGMENT = 2 };
+
+template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
 __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, uint32_t* __restrict__ alive,
-    const float2* __restrict__ proj3, float4* __restrict__ ckpt, float4* __restrict__ feat_acc) {
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc) {
+  constexpr bool BWD = CKPT != NONE;
   // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
   // pixel travel in feat_acc and move into out_feat.xyz when the last chunk, which then visits every pixel, is done.
   static_assert(!(FEAT && CHUNKED && BWD), "the chunked backward reads the colour sums from out_feat.xyz");
@@ -66,11 +71,20 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     }
   }
   // Checkpoints for the backward's segmented replay (see common.cuh): the state a later chunk starts a tile with, and
-  // the state before every SEG_LEN-th fragment of the list.
+  // the state before every (1 << seg_shift)-th fragment of the list.
   const int q = CHUNKED ? chunk * n_tiles + tile : tile;
+  float sr[2] = {0.f, 0.f}, sg[2] = {0.f, 0.f}, sb[2] = {0.f, 0.f};   // PER_SEGMENT: colour sums of the segment at hand
+  uint32_t seg_now = 0;
   auto checkpoint = [&](uint32_t seg) {
-    float4* dst = ckpt + (size_t)ckpt_slot(range.x, q, seg) * RT_PX + lane * 2;
-    dst[0] = make_float4(r[0], g[0], b[0], T[0]); dst[1] = make_float4(r[1], g[1], b[1], T[1]);
+    float4* dst = ckpt + (size_t)ckpt_slot(range.x, q, seg, seg_shift) * RT_PX + lane * 2;
+    if constexpr (CKPT == PER_SEGMENT) {   // the sums of the segment before the boundary
+      dst[0] = make_float4(sr[0], sg[0], sb[0], T[0]); dst[1] = make_float4(sr[1], sg[1], sb[1], T[1]);
+#pragma unroll
+      for (int p = 0; p < 2; p++) { sr[p] = 0.f; sg[p] = 0.f; sb[p] = 0.f; }
+      seg_now = seg;
+    } else {
+      dst[0] = make_float4(r[0], g[0], b[0], T[0]); dst[1] = make_float4(r[1], g[1], b[1], T[1]);
+    }
   };
   if (BWD && CHUNKED && !first && range.y > range.x) checkpoint(0u);
   // The records of a batch are gathered one batch ahead, into registers: the two dependent loads (list entry, then the
@@ -87,7 +101,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   gather(range.x);
   for (uint32_t start = range.x; start < range.y; start += FWD_BATCH) {
     if (__all_sync(0xffffffffu, done[0] && done[1])) break;
-    if (BWD && start != range.x && ((start - range.x) & (uint32_t)(SEG_LEN - 1)) == 0u) checkpoint((start - range.x) >> SEG_SHIFT);
+    if (BWD && start != range.x && ((start - range.x) & ((1u << seg_shift) - 1u)) == 0u) checkpoint((start - range.x) >> seg_shift);
     const uint32_t remaining = min((uint32_t)FWD_BATCH, range.y - start);
     __syncwarp();
     if ((uint32_t)lane < remaining) {
@@ -132,6 +146,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
           if (hit[p]) {
             const float vis = alpha[u][p] * T[p];
             r[p] += cr * vis; g[p] += cg * vis; b[p] += cb * vis;
+            if constexpr (CKPT == PER_SEGMENT) { sr[p] += cr * vis; sg[p] += cg * vis; sb[p] += cb * vis; }
             if constexpr (DEPTH) zs[p] += vis * cz;
             if constexpr (FEAT) { const float2 fz = s3[warp][t]; f0[p] += col.w * vis; f1[p] += fz.x * vis; f2[p] += fz.y * vis; }
             T[p] = next_T;
@@ -169,7 +184,20 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     uint32_t m = max(last[0], last[1]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) tile_ranges[tile].y = CHUNKED ? min(max(m, range.x), range.y) : m;
+    if constexpr (CHUNKED) m = min(max(m, range.x), range.y);
+    if (lane == 0) tile_ranges[tile].y = m;
+    if (CKPT == PER_SEGMENT && m > range.x) {
+      // Slot 0 has no segment before it: its colour takes the sums of the range's last segment (which is the one at hand
+      // unless nothing after its boundary was seen).
+      const uint32_t segs = (m - range.x + (1u << seg_shift) - 1u) >> seg_shift;
+      float* dst = reinterpret_cast<float*>(ckpt + (size_t)ckpt_slot(range.x, q, 0u, seg_shift) * RT_PX + lane * 2);
+      const float4* src = ckpt + (size_t)ckpt_slot(range.x, q, segs, seg_shift) * RT_PX + lane * 2;
+#pragma unroll
+      for (int p = 0; p < 2; p++) {
+        const float4 v = segs - 1u == seg_now ? make_float4(sr[p], sg[p], sb[p], 0.f) : src[p];
+        dst[p * 4] = v.x; dst[p * 4 + 1] = v.y; dst[p * 4 + 2] = v.z;
+      }
+    }
   }
 }
 
@@ -185,19 +213,16 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
   uint2* ranges = (uint2*)c->tile_ranges + (n_chunks > 1 ? (size_t)chunk * c->n_tiles : 0);
 #define L(B, D, C, F) raster_fwd_kernel<B, D, C, F><<<div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, s>>>(ranges, c->vals_sorted, (const float4*)c->proj0, \
     (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, \
-    chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, (n_chunks > 1 && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr)
+    chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(c->n_tiles), (n_chunks > 1 && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr)
+#define LB(B) do { if (n_chunks > 1) { if (c->out_depth) L(B, true, true, false); else L(B, false, true, false); } \
+    else if (o->feat_mode != 0) { if (c->out_depth) L(B, true, false, true); else L(B, false, false, true); } \
+    else { if (c->out_depth) L(B, true, false, false); else L(B, false, false, false); } } while (0)
   if (n_chunks > 1 && o->feat_mode != 0) {   // forward only (checked by the caller): the scratch of the backward carries the feature sums
-    if (c->out_depth) L(false, true, true, true); else L(false, false, true, true);
-  } else if (n_chunks > 1) {
-    if (o->bwd_info) { if (c->out_depth) L(true, true, true, false); else L(true, false, true, false); }
-    else { if (c->out_depth) L(false, true, true, false); else L(false, false, true, false); }
-  } else if (o->feat_mode != 0) {
-    if (o->bwd_info) { if (c->out_depth) L(true, true, false, true); else L(true, false, false, true); }
-    else { if (c->out_depth) L(false, true, false, true); else L(false, false, false, true); }
-  } else {
-    if (o->bwd_info) { if (c->out_depth) L(true, true, false, false); else L(true, false, false, false); }
-    else { if (c->out_depth) L(false, true, false, false); else L(false, false, false, false); }
-  }
+    if (c->out_depth) L(NONE, true, true, true); else L(NONE, false, true, true);
+  } else if (!o->bwd_info) LB(NONE);
+  else if (short_segments(c->n_tiles)) LB(PER_SEGMENT);
+  else LB(RUNNING);
+#undef LB
 #undef L
   return check_launch();
 }

@@ -98,7 +98,7 @@ typedef struct {
                               and counts, one "some pixel can still take a fragment" flag per tile, the summed-area table
                               of those flags), or NULL when n_chunks <= 1 */
   void* bwd_scratch;       /* b2k_bwd_scratch_bytes() bytes, needed when the forward runs with bwd_info: per-pixel (colour
-                              sums, transmittance) checkpoints the forward leaves every 128 fragments of a tile's list, and
+                              sums, transmittance) checkpoints the forward leaves at every segment boundary of a tile's list, and
                               the work list of the backward, which replays the segments between checkpoints independently.
                               Takes the place of nothing in the reference (its backward walks a tile's list in one CTA) */
   uint64_t bwd_scratch_bytes;
@@ -222,7 +222,7 @@ uint64_t b2k_bwd_scratch_bytes(int32_t W, int32_t H, int32_t n_chunks, uint64_t 
 
 /* ---- backward ---- */
 /* rasterize_backward, src/gpu/render.h:106 (raster_bwd_kernel, src/gpu/raster_bwd.cu:11-143). Same gradients; the
- * tile lists are replayed in segments of 128 fragments from the forward's checkpoints in ctx->bwd_scratch. */
+ * tile lists are replayed in segments of 32 or 64 fragments from the forward's checkpoints in ctx->bwd_scratch. */
 int b2k_raster_bwd(const B2kCtx* ctx, const B2kModel* m, const B2kRenderOpts* opts, b2k_stream_t s);
 /* rasterize_backward_tc, src/gpu/render.h:107-109 (raster_bwd_tc_kernel, src/gpu/raster_bwd_tc.cu:30-225), as far as its
  * contract goes: the pixel gradients in v_out were produced with LossParams::grad_scale applied and the per-splat
