@@ -1,0 +1,667 @@
+// From depth-ordered splats to per-tile fragment lists, in two levels. Reference semantics: the emission, the tile sort and
+// the ranges of bin_and_sort (src/gpu/binning.cu:16-105,117-145): every (tile, splat) pair the exact ellipse test keeps,
+// grouped by tile, in depth order inside a tile.
+//
+// A splat touches tens of tiles, and sorting its (tile, splat) pairs moves 48 bytes a pair and needs one place to do the
+// ellipse tests, whose number varies from 1 to thousands a splat. Here the image is divided into BINS of 8x8 tiles. Level 1
+// distributes the splats over the bins their boxes overlap (two to five pairs a splat), in depth order; level 2 takes the
+// pairs of a bin 256 at a time, tests each splat against the at most 64 tiles of the bin, and writes the hits straight to
+// their places. Both levels are a stable counting distribution: count, scan, write; no block ever waits for another, and
+// all counts stay on the device.
+//   level 1  bin_count    a block per run of depth ranks counts its pairs per bin
+//            bin_rows     per bin: scan over the blocks; the last block to finish lays out the bins and cuts them into items
+//            bin_scatter  the same blocks write their pairs (splat indices) to their places
+//   level 2  item_count   ellipse tests of an item's pairs -> 64-bit hit words, hits per tile
+//            item_columns per bin and tile: scan over the bin's items
+//            tile_scan    scan over the tiles, row-major -> ranges
+//            item_emit    the item's hits to their tiles' lists
+// A box that lies in one depth chunk of a view (b2k_render_chunked) skips tiles whose pixels have all saturated: the
+// compositing kernel clears their bits in one 64-bit word per bin.
+//
+// Bound by instruction issue (ellipse tests, bit work) and by launch latency in small views. Against emission of expanded
+// pairs and two radix passes over them, sum of the stage's kernels per view: 4K, 6M splats, 37.5M hits 2,660 -> 960 us;
+// 1080p, 500k splats, 4.4M hits 330 -> 150; 1024x1024, 1M splats of which a tenth cover hundreds of tiles 1,350 -> 390.
+// Inside that, the tests of a warp's 32 pairs shared out by tile row (not a pair per lane): 455 -> 286 us at 4K.
+#include "common.cuh"
+#include <algorithm>
+
+namespace b2k {
+namespace {
+
+constexpr int BIN_W = 8;                      // tiles along a bin's edge
+constexpr int BIN_TILES = BIN_W * BIN_W;
+constexpr int MAX_BINS = 2048;                // bins of one band: what a block's tables in shared memory hold; larger images take several bands of bin rows
+constexpr int MAX_ITEMS = 8192;               // items of one band: BINS_TABLE_WORDS / 64
+constexpr int L1_THREADS = 256, L1_WARPS = L1_THREADS / 32;
+constexpr int L2_THREADS = 256, L2_WARPS = L2_THREADS / 32;
+constexpr int SERIAL_BINS = 12;               // a splat over more bins is spread by its whole warp (4K view: 8 -> 12 takes 360 + 338 to 264 + 204 us)
+constexpr int SCAN_TILES = 1024;              // tiles per block of tile_scan
+constexpr unsigned FULL = 0xffffffffu;
+static_assert((size_t)MAX_ITEMS * BIN_TILES <= BINS_TABLE_WORDS, "the counts of the items take the place of level 1's table");
+static_assert(MAX_BINS * BIN_TILES / SCAN_TILES <= BINS_SEGMENTS, "one sum per tile_scan block");
+
+// The bins and tiles of one band.
+struct Band { int tiles_x, tiles_y, bins_x, bin_row0, bin_rows; };
+__device__ __forceinline__ int band_bins(const Band& g) { return g.bins_x * g.bin_rows; }
+
+// What a call works on. words == nullptr: the whole view, from exact hit masks; else depth chunk `chunk` of a chunked view.
+struct View {
+  const uint32_t* order; const uint4* hit_info; const uint32_t* tile_count; const float4* proj0; const float4* proj1;
+  int n; uint32_t* words; int chunk, lo_num, hi_num; const unsigned long long* alive; int first_band, last_band;
+};
+
+struct Tables {
+  uint32_t* cells;       // [bin][block] of level 1, then [item][64] of level 2
+  uint32_t* totals;      // [MAX_BINS] pairs per bin
+  uint32_t* base;        // [MAX_BINS + 1] first pair of each bin
+  uint32_t* first_item;  // [MAX_BINS + 1]
+  uint32_t* item_bin;    // [MAX_ITEMS]
+  uint32_t* block_sums;  // [1024] tile counts of level 1's blocks (whole view)
+  uint32_t* segments;    // [BINS_SEGMENTS] hits per tile_scan block
+  uint32_t* st;          // [16] see S_*
+};
+enum { S_PAIRS = 0, S_ITEMS, S_ITEM_LEN, S_DONE_ROWS, S_DONE_TILES, S_SLOT, S_OVER, S_TOTAL };
+
+__device__ __forceinline__ void view_ranks(const View& v, uint32_t& r0, uint32_t& r1) {
+  if (!v.words) { r0 = 0u; r1 = (uint32_t)v.n; return; }
+  const uint64_t V = v.words[CW_V];
+  r0 = (uint32_t)((V * (uint64_t)v.lo_num) >> 8);
+  r1 = (uint32_t)((V * (uint64_t)v.hi_num) >> 8);
+}
+__device__ __forceinline__ uint32_t run_len(uint32_t n, uint32_t blocks) {
+  const uint32_t per = (n + blocks - 1) / blocks;
+  return (per + L1_THREADS - 1) / L1_THREADS * L1_THREADS;
+}
+
+// A splat's tile box, half open; empty when x1 == x0.
+struct Box { int x0, y0, x1, y1; };
+__device__ __forceinline__ Box box_of(const uint4& hi) {
+  Box b;
+  if (hi.z == 0xFFFFFFFFu) {
+    b.x0 = (int)(hi.x & 0xFFFFu); b.y0 = (int)(hi.x >> 16);
+    b.x1 = b.x0 + (int)(hi.y & 0xFFFFu); b.y1 = b.y0 + (int)(hi.y >> 16);
+  } else {
+    b.x0 = (int)(hi.z & 0xFFFu); b.y0 = (int)((hi.z >> 12) & 0xFFFu);
+    b.x1 = b.x0 + (int)(hi.z >> 24); b.y1 = b.y0 + (int)hi.w;
+  }
+  return b;
+}
+// The box's tiles inside bin (bx, by), bit = row * 8 + column.
+__device__ __forceinline__ unsigned long long rect_bits(const Box& b, int bx, int by) {
+  const int lx0 = max(b.x0 - bx * BIN_W, 0), lx1 = min(b.x1 - bx * BIN_W, BIN_W), ly0 = max(b.y0 - by * BIN_W, 0), ly1 = min(b.y1 - by * BIN_W, BIN_W);
+  const unsigned long long row = ((1u << (lx1 - lx0)) - 1u) << lx0;
+  return (row * 0x0101010101010101ull) & ((~0ull >> (64 - BIN_W * (ly1 - ly0))) << (BIN_W * ly0));
+}
+// The same from the exact hit mask of a box of at most 64 tiles (row-major inside the box).
+__device__ __forceinline__ unsigned long long mask_bits(const uint4& hi, const Box& b, int bx, int by) {
+  const unsigned long long mask = ((unsigned long long)hi.y << 32) | hi.x;
+  const int xs = max(b.x0, bx * BIN_W), xe = min(b.x1, bx * BIN_W + BIN_W), ys = max(b.y0, by * BIN_W), ye = min(b.y1, by * BIN_W + BIN_W), bw = b.x1 - b.x0;
+  unsigned long long out = 0ull;
+  for (int y = ys; y < ye; y++)
+    out |= ((mask >> ((y - b.y0) * bw + (xs - b.x0))) & ((1ull << (xe - xs)) - 1ull)) << ((y - by * BIN_W) * BIN_W + (xs - bx * BIN_W));
+  return out;
+}
+
+// The bins a splat's box overlaps, inside the band.
+struct BinSpan { int bx0, by0, w, count; };
+__device__ __forceinline__ BinSpan span_of(const Box& b, const Band& g) {
+  BinSpan s{0, 0, 0, 0};
+  if (b.x1 <= b.x0 || b.y1 <= b.y0) return s;
+  const int by0 = max(b.y0 / BIN_W, g.bin_row0), by1 = min((b.y1 - 1) / BIN_W + 1, g.bin_row0 + g.bin_rows);
+  s.bx0 = b.x0 / BIN_W; s.by0 = by0; s.w = (b.x1 - 1) / BIN_W + 1 - s.bx0;
+  s.count = by1 > by0 ? s.w * (by1 - by0) : 0;
+  return s;
+}
+
+// One rank's splat as level 1 sees it.
+struct Rank { uint32_t splat, tiles; uint4 hi; Box box; BinSpan span; };
+// Walks a list of splats in rounds of blockDim.x, the dependent loads (list entry, then the splat's record) one and two rounds
+// ahead of their use.
+template <bool WHOLE>
+struct RankReader {
+  const View& v; const Band& g; const uint32_t* list; uint64_t at, end;
+  uint32_t i1 = 0u, i2 = 0u, t1 = 0u;
+  uint4 h1 = make_uint4(0u, 0u, 0u, 0u);
+  __device__ __forceinline__ RankReader(const View& v_, const Band& g_, const uint32_t* list_, uint64_t begin, uint64_t end_) : v(v_), g(g_), list(list_), at(begin + threadIdx.x), end(end_) {
+    i1 = entry(at); i2 = entry(at + blockDim.x);
+    record(at);
+  }
+  __device__ __forceinline__ uint32_t entry(uint64_t p) const { return p < end ? list[p] : 0u; }
+  __device__ __forceinline__ void record(uint64_t p) {
+    const bool valid = p < end;
+    h1 = valid ? v.hit_info[i1] : make_uint4(0u, 0u, 0u, 0u);
+    if (WHOLE) t1 = valid ? v.tile_count[i1] : 0u;
+  }
+  __device__ __forceinline__ Rank next() {
+    Rank k;
+    k.splat = i1; k.tiles = t1; k.hi = h1;
+    at += blockDim.x;
+    i1 = i2;
+    record(at);
+    i2 = entry(at + blockDim.x);
+    if (WHOLE && k.tiles == 0u) k.hi = make_uint4(0u, 0u, 0u, 0u);
+    k.box = box_of(k.hi);
+    k.span = span_of(k.box, g);
+    return k;
+  }
+};
+// Whether a splat goes into bin (bx, by): a chunk asks for a tile of the box that is still alive; the whole view for a hit
+// tile, except that a large box takes every bin it overlaps (level 2 finds out) and a box inside one bin has a hit there.
+template <bool WHOLE>
+__device__ __forceinline__ bool takes_bin(const unsigned long long* s_alive, const uint4& hi, const Box& b, int bx, int by, int bin, int count) {
+  if constexpr (WHOLE) return count == 1 || hi.z == 0xFFFFFFFFu || mask_bits(hi, b, bx, by) != 0ull;
+  else return (s_alive[bin] & rect_bits(b, bx, by)) != 0ull;   // (looking for all-alive and all-dead bins first measured slower: 204 -> 238 us)
+}
+// The band's alive words, in shared memory.
+__device__ __forceinline__ void load_alive(const View& v, const Band& g, unsigned long long* s_alive) {
+  for (int i = threadIdx.x; i < band_bins(g); i += blockDim.x) s_alive[i] = v.alive ? v.alive[g.bin_row0 * g.bins_x + i] : ~0ull;
+}
+// The few bins of a lane's own splat that it goes into, as bits in the order of its span; zero for a wide splat.
+template <bool WHOLE>
+__device__ __forceinline__ uint32_t own_bins(const unsigned long long* s_alive, const Band& g, const Rank& k) {
+  uint32_t take = 0u;
+  if (k.span.count <= SERIAL_BINS) {
+    int bx = k.span.bx0, by = k.span.by0;
+    for (int c = 0; c < k.span.count; c++) {
+      if (takes_bin<WHOLE>(s_alive, k.hi, k.box, bx, by, (by - g.bin_row0) * g.bins_x + bx, k.span.count)) take |= 1u << c;
+      if (++bx == k.span.bx0 + k.span.w) { bx = k.span.bx0; by++; }
+    }
+  }
+  return take;
+}
+__device__ __forceinline__ int own_bin(const Band& g, const Rank& k, int c) {
+  const int dy = c / k.span.w;
+  return (k.span.by0 + dy - g.bin_row0) * g.bins_x + k.span.bx0 + c - dy * k.span.w;
+}
+// Splats over many bins are spread by the whole warp, one after the other: f(lane of the splat, splat, local bin) for every
+// bin. All lanes call this together; returns whether this lane's own splat is wide and went into any bin.
+template <bool WHOLE, class F>
+__device__ __forceinline__ bool wide_bins(const unsigned long long* s_alive, const Band& g, const Rank& k, F f) {
+  const int lane = threadIdx.x & 31;
+  bool took = false;
+  for (uint32_t wide = __ballot_sync(FULL, k.span.count > SERIAL_BINS); wide; wide &= wide - 1u) {
+    const int src = __ffs(wide) - 1;
+    uint4 hi;
+    hi.x = __shfl_sync(FULL, k.hi.x, src); hi.y = __shfl_sync(FULL, k.hi.y, src); hi.z = __shfl_sync(FULL, k.hi.z, src); hi.w = __shfl_sync(FULL, k.hi.w, src);
+    const uint32_t splat = __shfl_sync(FULL, k.splat, src);
+    const Box b = box_of(hi);
+    const BinSpan s = span_of(b, g);
+    bool any = false;
+    for (int c = lane; c < s.count; c += 32) {
+      const int dy = c / s.w, bx = s.bx0 + c - dy * s.w, by = s.by0 + dy, bin = (by - g.bin_row0) * g.bins_x + bx;
+      if (takes_bin<WHOLE>(s_alive, hi, b, bx, by, bin, s.count)) { any = true; f(src, splat, bin); }
+    }
+    any = __any_sync(FULL, any);
+    if (lane == src) took = any;
+  }
+  return took;
+}
+
+// Inclusive scan over the block of one value per thread (at most 1024 threads); s_warp holds 32 words. Synchronises.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(FULL, v, o); if (lane >= o) v += u; }
+  __syncthreads();
+  if (lane == 31) s_warp[warp] = v;
+  __syncthreads();
+  uint32_t pre = 0, all = 0;
+  for (int w = 0; w < warps; w++) { const uint32_t t = s_warp[w]; if (w < warp) pre += t; all += t; }
+  total = all;
+  return v + pre;
+}
+
+// ---- level 1 -----------------------------------------------------------------------------------------------------------
+
+// Pairs per bin of each block's run of ranks. A chunk also leaves the run's splats that go anywhere, in order, at the run's
+// place in `live`: in the later chunks most splats lie behind saturated tiles, and the write pass never looks at them. The
+// whole view leaves the run's tile count instead (tile_off is its running sum).
+constexpr int COUNT_THREADS = 512;
+template <bool WHOLE>
+__global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g, Tables t, uint32_t* __restrict__ live) {
+  extern __shared__ __align__(16) unsigned long long s_alive[];   // [bins], then [bins] counts
+  const int bins = band_bins(g), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_alive + (WHOLE ? 0 : bins));
+  __shared__ uint32_t s_live[2][COUNT_THREADS / 32], s_warp[32];
+  for (int i = tid; i < bins; i += COUNT_THREADS) s_cnt[i] = 0u;
+  if (!WHOLE) load_alive(v, g, s_alive);
+  if (blockIdx.x == 0 && tid == 0) {    // this band's counters; the view's with its first band
+    t.st[S_DONE_ROWS] = 0u; t.st[S_DONE_TILES] = 0u;
+    if (v.first_band) { t.st[S_SLOT] = v.words ? v.words[CW_BASE + v.chunk] : 0u; if (!v.words || v.chunk == 0) t.st[S_OVER] = 0u; }
+  }
+  __syncthreads();
+  uint32_t r0, r1;
+  view_ranks(v, r0, r1);
+  const uint32_t len = run_len(r1 - r0, gridDim.x);
+  const uint64_t begin = (uint64_t)r0 + (uint64_t)blockIdx.x * len, end = begin + len < (uint64_t)r1 ? begin + len : (uint64_t)r1;
+  uint32_t tiles = 0, n_live = 0;
+  int parity = 0;
+  RankReader<WHOLE> ranks(v, g, v.order, begin, end);
+  for (uint64_t at = begin; at < end; at += COUNT_THREADS, parity ^= 1) {
+    const Rank k = ranks.next();
+    tiles += k.tiles;
+    const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
+    for (uint32_t b = take; b; b &= b - 1u) atomicAdd(&s_cnt[own_bin(g, k, __ffs(b) - 1)], 1u);
+    const bool wide = wide_bins<WHOLE>(s_alive, g, k, [&](int, uint32_t, int bin) { atomicAdd(&s_cnt[bin], 1u); });
+    if constexpr (!WHOLE) {
+      const uint32_t on = __ballot_sync(FULL, take != 0u || wide);
+      if (lane == 0) s_live[parity][warp] = (uint32_t)__popc(on);
+      __syncthreads();
+      uint32_t pre = 0, all = 0;
+#pragma unroll
+      for (int w = 0; w < COUNT_THREADS / 32; w++) { const uint32_t c = s_live[parity][w]; pre += w < warp ? c : 0u; all += c; }
+      if ((on >> lane) & 1u) live[begin + n_live + pre + __popc(on & ((1u << lane) - 1u))] = k.splat;
+      n_live += all;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < bins; i += COUNT_THREADS) t.cells[(size_t)i * gridDim.x + blockIdx.x] = s_cnt[i];
+  if (!WHOLE) {
+    if (tid == 0) t.block_sums[blockIdx.x] = n_live;
+  } else if (v.first_band) {
+    uint32_t total;
+    block_scan(tiles, s_warp, total);
+    if (tid == 0) t.block_sums[blockIdx.x] = total;
+  }
+}
+
+// A warp per bin turns the bin's counts into offsets. The last block to finish lays out the band: first pair of every bin,
+// and the items (runs of pairs of one bin) that level 2 works on. An item is 256 pairs unless that made too many.
+constexpr int ROWS_THREADS = 512, ROWS_BINS = ROWS_THREADS / 32, ROWS_PER = 16;   // at most 32 * ROWS_PER blocks of level 1
+__global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int bins, uint32_t cap, Tables t) {
+  __shared__ uint32_t s_warp[32];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x, lane = tid & 31, bin = blockIdx.x * ROWS_BINS + (tid >> 5);
+  if (bin < bins) {
+    uint32_t* row = t.cells + (size_t)bin * blocks;
+    uint32_t c[ROWS_PER], at = 0;
+#pragma unroll
+    for (int u = 0; u < ROWS_PER; u++) { const int k = u * 32 + lane; c[u] = k < blocks ? row[k] : 0u; }
+#pragma unroll
+    for (int u = 0; u < ROWS_PER; u++) {
+      if (u * 32 >= blocks) break;
+      uint32_t incl = c[u];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const uint32_t x = __shfl_up_sync(FULL, incl, o); if (lane >= o) incl += x; }
+      if (u * 32 + lane < blocks) row[u * 32 + lane] = at + incl - c[u];
+      at += __shfl_sync(FULL, incl, 31);
+    }
+    if (lane == 0) t.totals[bin] = at;
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(t.st + S_DONE_ROWS, 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  constexpr int PER = MAX_BINS / ROWS_THREADS;
+  uint32_t tot[PER], sum = 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) { const int b = tid * PER + u; tot[u] = b < bins ? __ldcg(t.totals + b) : 0u; sum += tot[u]; }
+  uint32_t pairs;
+  uint32_t at = block_scan(sum, s_warp, pairs) - sum;
+  const uint32_t room = MAX_ITEMS - (uint32_t)bins, len = 256u * (pairs / (256u * room) + 1u);   // items <= pairs / len + bins <= MAX_ITEMS
+  uint32_t items = 0, n_items;
+#pragma unroll
+  for (int u = 0; u < PER; u++) items += (tot[u] + len - 1u) / len;
+  uint32_t it = block_scan(items, s_warp, n_items) - items;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const int b = tid * PER + u;
+    if (b < bins) { t.base[b] = at; t.first_item[b] = it; }
+    at += tot[u]; it += (tot[u] + len - 1u) / len;
+  }
+  if (tid == 0) {
+    t.base[bins] = pairs; t.first_item[bins] = n_items;
+    t.st[S_PAIRS] = pairs; t.st[S_ITEMS] = n_items; t.st[S_ITEM_LEN] = len;
+    if (pairs > cap && pairs > t.st[S_OVER]) t.st[S_OVER] = pairs;   // level 1's own pairs did not fit: the caller grows the buffers
+  }
+  if (tid < BINS_SEGMENTS) t.segments[tid] = 0u;
+}
+
+// The pairs to their places, stable: bit l of s_bits[bin][w] says that lane l of warp w adds a pair to the bin in this round.
+// The splat that adds a bin's first pair of the round afterwards moves the bin's place on and clears its bits.
+template <bool WHOLE>
+__global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ live, uint32_t* __restrict__ pairs,
+                                                                 uint32_t* __restrict__ tile_off) {
+  extern __shared__ __align__(16) uint32_t s_bits[];   // [bins][8], then [bins] alive words, then [bins] next free place
+  const int bins = band_bins(g), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned long long* s_alive = reinterpret_cast<unsigned long long*>(s_bits + (size_t)bins * L1_WARPS);
+  uint32_t* s_next = reinterpret_cast<uint32_t*>(s_alive + (WHOLE ? 0 : bins));
+  __shared__ uint32_t s_warp[32];
+  uint32_t r0, r1;
+  view_ranks(v, r0, r1);
+  const uint32_t len = run_len(r1 - r0, gridDim.x);
+  const uint64_t begin = (uint64_t)r0 + (uint64_t)blockIdx.x * len;
+  const uint64_t end = WHOLE ? (begin + len < (uint64_t)r1 ? begin + len : (uint64_t)r1) : begin + t.block_sums[blockIdx.x];
+  const bool offsets = WHOLE && v.first_band;
+  for (int b = blockIdx.x * L1_WARPS + warp; b < bins; b += gridDim.x * L1_WARPS) {   // the items' bins, a warp per bin
+    const uint32_t e = t.first_item[b + 1];
+    for (uint32_t k = t.first_item[b] + (uint32_t)lane; k < e; k += 32) t.item_bin[k] = (uint32_t)b;
+  }
+  if (begin >= end && !(offsets && blockIdx.x == gridDim.x - 1)) return;
+  for (int i = tid; i < bins * L1_WARPS; i += L1_THREADS) s_bits[i] = 0u;
+  for (int i = tid; i < bins; i += L1_THREADS) s_next[i] = t.base[i] + t.cells[(size_t)i * gridDim.x + blockIdx.x];
+  if (!WHOLE) load_alive(v, g, s_alive);
+  uint32_t tiles_before = 0;
+  if (offsets) {
+    uint32_t mine = 0, total;
+    for (int b = tid; b < (int)blockIdx.x; b += L1_THREADS) mine += t.block_sums[b];
+    block_scan(mine, s_warp, total);
+    tiles_before = total;
+  }
+  __syncthreads();
+  auto earlier = [&](int bin, int l) {   // pairs of this round before lane l of this warp
+    const uint4* b4 = reinterpret_cast<const uint4*>(s_bits + bin * L1_WARPS);
+    const uint4 a = b4[0], b = b4[1];
+    const uint32_t w[L1_WARPS] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t n = 0;
+#pragma unroll
+    for (int k = 0; k < L1_WARPS; k++) n += (uint32_t)__popc(k < warp ? w[k] : k == warp ? w[k] & ((1u << l) - 1u) : 0u);
+    return n;
+  };
+  auto move_on = [&](int bin) {
+    uint4* b4 = reinterpret_cast<uint4*>(s_bits + bin * L1_WARPS);
+    const uint4 a = b4[0], b = b4[1];
+    const uint32_t added = __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w) + __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
+    if (added) { s_next[bin] += added; b4[0] = make_uint4(0u, 0u, 0u, 0u); b4[1] = make_uint4(0u, 0u, 0u, 0u); }
+  };
+  RankReader<WHOLE> ranks(v, g, WHOLE ? v.order : live, begin, end);
+  for (uint64_t at = begin; at < end; at += L1_THREADS) {
+    const Rank k = ranks.next();
+    const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
+    for (uint32_t b = take; b; b &= b - 1u) atomicOr(&s_bits[own_bin(g, k, __ffs(b) - 1) * L1_WARPS + warp], 1u << lane);
+    wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t, int bin) { atomicOr(&s_bits[bin * L1_WARPS + warp], 1u << l); });
+    if (offsets) {
+      uint32_t total;
+      const uint32_t incl = block_scan(k.tiles, s_warp, total);
+      if (at + tid < end) tile_off[at + tid] = tiles_before + incl;
+      tiles_before += total;
+    }
+    const bool any_wide = __syncthreads_or(k.span.count > SERIAL_BINS);
+    uint32_t first = 0u;
+    for (uint32_t b = take; b; b &= b - 1u) {
+      const int bin = own_bin(g, k, __ffs(b) - 1);
+      const uint32_t n = earlier(bin, lane), pos = s_next[bin] + n;
+      if (pos < cap) pairs[pos] = k.splat;
+      if (n == 0u) first |= b & (0u - b);
+    }
+    wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t splat, int bin) { const uint32_t pos = s_next[bin] + earlier(bin, l); if (pos < cap) pairs[pos] = splat; });
+    __syncthreads();
+    if (any_wide) { for (int i = tid; i < bins; i += L1_THREADS) move_on(i); }
+    else { for (uint32_t b = first; b; b &= b - 1u) move_on(own_bin(g, k, __ffs(b) - 1)); }
+    __syncthreads();
+  }
+  if (offsets && blockIdx.x == gridDim.x - 1 && tid == 0) t.st[S_TOTAL] = tiles_before;   // the view's hits, also when the pairs did not fit
+}
+
+// ---- level 2 -----------------------------------------------------------------------------------------------------------
+
+// Transposes the 32x32 bit matrix whose row i is lane i's word.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const uint32_t m = o == 16 ? 0x0000FFFFu : o == 8 ? 0x00FF00FFu : o == 4 ? 0x0F0F0F0Fu : o == 2 ? 0x33333333u : 0x55555555u;   // columns without bit o
+    const uint32_t y = __shfl_xor_sync(FULL, x, o);
+    x = (lane & o) ? (x & ~m) | ((y >> o) & m) : (x & m) | ((y & m) << o);
+  }
+  return x;
+}
+
+// The pairs of one item and the bin's corner.
+struct Item { uint32_t first, end; int bx, by; };
+__device__ __forceinline__ Item item_of(const Tables& t, const Band& g, uint32_t it, uint32_t cap) {
+  const uint32_t bin = t.item_bin[it], len = t.st[S_ITEM_LEN];
+  Item m;
+  m.first = t.base[bin] + (it - t.first_item[bin]) * len;
+  m.end = min(min(m.first + len, t.base[bin + 1]), cap);
+  m.bx = (int)bin % g.bins_x; m.by = g.bin_row0 + (int)bin / g.bins_x;
+  return m;
+}
+
+// Hit word of every pair of an item (bit = row * 8 + column of the tile in its bin), and the item's hits per tile.
+template <bool WHOLE>
+__global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ pairs, uint32_t* __restrict__ hit_lo,
+                                                                uint32_t* __restrict__ hit_hi) {
+  struct WarpShare { float4 rec[64]; unsigned long long hits[32]; uint32_t unit[32 * BIN_W]; };   // unit: pair | row << 5 | columns << 8
+  __shared__ WarpShare s_share[L2_WARPS];
+  __shared__ uint32_t s_cnt[L2_WARPS][BIN_TILES];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  WarpShare& ws = s_share[warp];
+  const uint32_t n_items = t.st[S_ITEMS];
+  for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
+    const Item m = item_of(t, g, it, cap);
+    const unsigned long long alive = !WHOLE && v.alive ? v.alive[m.by * g.bins_x + m.bx] : ~0ull;
+    uint32_t c_lo = 0, c_hi = 0;   // this warp's hits on tiles `lane` and `lane + 32`
+    for (uint32_t p0 = m.first; p0 < m.end; p0 += L2_THREADS) {
+      const uint32_t p = p0 + tid;
+      unsigned long long hits = 0ull, todo = 0ull;   // todo: tiles to test
+      if (p < m.end) {
+        const uint32_t i = pairs[p];
+        const uint4 hi = v.hit_info[i];
+        const Box b = box_of(hi);
+        if (WHOLE && hi.z != 0xFFFFFFFFu) {
+          hits = mask_bits(hi, b, m.bx, m.by);   // the projection has tested this box
+        } else {
+          todo = rect_bits(b, m.bx, m.by) & alive;
+          const float4 q0 = v.proj0[i], q1 = v.proj1[i];
+          const TileRec rec = make_tile_rec(q0.x, q0.y, q0.z, q0.w, q1.x, q1.w);
+          ws.rec[lane * 2] = make_float4(rec.mx, rec.my, rec.c00, rec.c01);
+          ws.rec[lane * 2 + 1] = make_float4(rec.c11, rec.power, rec.ia, rec.ib);
+        }
+      }
+      // The tests of the warp's pairs are shared out by tile row: boxes hold one to 64 tiles of the bin, and with a pair per
+      // lane most lanes wait for the largest.
+      uint32_t rows = 0u;
+#pragma unroll
+      for (int r = 0; r < BIN_W; r++) rows |= ((uint32_t)(todo >> (8 * r)) & 0xFFu) ? 1u << r : 0u;
+      uint32_t at = __popc(rows);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(FULL, at, o); if (lane >= o) at += u; }
+      const uint32_t units = __shfl_sync(FULL, at, 31);
+      if (units) {
+        at -= __popc(rows);
+        for (uint32_t b = rows; b; b &= b - 1u, at++) {
+          const int r = __ffs(b) - 1;
+          ws.unit[at] = (uint32_t)lane | ((uint32_t)r << 5) | (((uint32_t)(todo >> (8 * r)) & 0xFFu) << 8);
+        }
+        ws.hits[lane] = 0ull;
+        __syncwarp();
+        for (uint32_t u = lane; u < units; u += 32) {
+          const uint32_t e = ws.unit[u], owner = e & 31u, r = (e >> 5) & 7u;
+          const float4 a = ws.rec[owner * 2], b = ws.rec[owner * 2 + 1];
+          const TileRec rec{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          const TileRow row = tile_row(m.by * BIN_W + (int)r, rec);
+          uint32_t out = 0u;
+          for (uint32_t cols = e >> 8; cols; cols &= cols - 1u) {
+            const int c = __ffs(cols) - 1;
+            if (tile_hit(m.bx * BIN_W + c, row, rec)) out |= 1u << c;
+          }
+          reinterpret_cast<unsigned char*>(ws.hits + owner)[r] = (unsigned char)out;
+        }
+        __syncwarp();
+        hits |= ws.hits[lane];
+        __syncwarp();
+      }
+      if (p < m.end) { hit_lo[p] = (uint32_t)hits; hit_hi[p] = (uint32_t)(hits >> 32); }
+      c_lo += __popc(transpose_bits((uint32_t)hits)); c_hi += __popc(transpose_bits((uint32_t)(hits >> 32)));
+    }
+    s_cnt[warp][lane] = c_lo; s_cnt[warp][lane + 32] = c_hi;
+    __syncthreads();
+    if (tid < BIN_TILES) {
+      uint32_t sum = 0;
+#pragma unroll
+      for (int w = 0; w < L2_WARPS; w++) sum += s_cnt[w][tid];
+      t.cells[(size_t)it * BIN_TILES + tid] = sum;
+    }
+    __syncthreads();
+  }
+}
+
+// A block per bin: the counts of its items become offsets inside each tile, the totals go to the tiles (ranges[tile].x until
+// tile_scan has run) and to the sums of tile_scan's blocks. Groups of 64 threads share a column: sixteen where few bins have long ones,
+// four where there are bins enough to fill the GPU (74 -> 29 us over the five chunks of a 4K view).
+template <int COL_GROUPS>
+__global__ void __launch_bounds__(COL_GROUPS * BIN_TILES) item_columns_kernel(Band g, Tables t, uint2* __restrict__ ranges) {
+  __shared__ uint32_t s_sum[COL_GROUPS][BIN_TILES];
+  const int bin = blockIdx.x, tile = threadIdx.x % BIN_TILES, group = threadIdx.x / BIN_TILES;
+  const uint32_t i0 = t.first_item[bin], i1 = t.first_item[bin + 1], per = (i1 - i0 + COL_GROUPS - 1) / COL_GROUPS;
+  const uint32_t a = min(i0 + group * per, i1), b = min(a + per, i1);
+  uint32_t* col = t.cells + tile;
+  uint32_t sum = 0;
+#pragma unroll 8
+  for (uint32_t k = a; k < b; k++) sum += col[(size_t)k * BIN_TILES];
+  s_sum[group][tile] = sum;
+  __syncthreads();
+  uint32_t at = 0, total = 0;
+#pragma unroll
+  for (int k = 0; k < COL_GROUPS; k++) { const uint32_t s = s_sum[k][tile]; if (k < group) at += s; total += s; }
+#pragma unroll 8
+  for (uint32_t k = a; k < b; k++) { const uint32_t c = col[(size_t)k * BIN_TILES]; col[(size_t)k * BIN_TILES] = at; at += c; }
+  const int bx = bin % g.bins_x, by = g.bin_row0 + bin / g.bins_x, x = bx * BIN_W + (tile & 7), y = by * BIN_W + (tile >> 3);
+  if (group == 0 && x < g.tiles_x && y < g.tiles_y) {
+    const int id = y * g.tiles_x + x;
+    ranges[id] = make_uint2(total, 0u);
+    if (total) atomicAdd(t.segments + (id - g.bin_row0 * BIN_W * g.tiles_x) / SCAN_TILES, total);
+  }
+}
+
+// Ranges of the band's tiles, row-major: block b starts behind the hits of the blocks before it. Empty tiles get (0, 0);
+// ranges end with the buffers. The last block to finish moves the view's slot on.
+__global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, Tables t, uint32_t cap, uint2* __restrict__ ranges, uint32_t* __restrict__ num_isect) {
+  __shared__ uint32_t s_warp[32];
+  const int tid = threadIdx.x;
+  const int tile0 = g.bin_row0 * BIN_W * g.tiles_x, tiles = (min((g.bin_row0 + g.bin_rows) * BIN_W, g.tiles_y) - g.bin_row0 * BIN_W) * g.tiles_x;
+  const int mine = blockIdx.x * SCAN_TILES + tid;
+  uint32_t all, before;
+  {
+    const uint32_t seg = tid < (int)gridDim.x ? t.segments[tid] : 0u;
+    const uint32_t incl = block_scan(seg, s_warp, all);
+    __shared__ uint32_t s_before;
+    if (tid == (int)blockIdx.x) s_before = incl - seg;
+    __syncthreads();
+    before = s_before;
+  }
+  const uint32_t slot = t.st[S_SLOT];
+  const uint32_t c = mine < tiles ? ranges[tile0 + mine].x : 0u;
+  uint32_t total;
+  const uint32_t start = slot + before + block_scan(c, s_warp, total) - c;
+  if (mine < tiles) ranges[tile0 + mine] = c ? make_uint2(min(start, cap), min(start + c, cap)) : make_uint2(0u, 0u);
+  __threadfence();
+  __syncthreads();
+  if (tid == 0 && atomicAdd(t.st + S_DONE_TILES, 1u) == gridDim.x - 1u) {   // every block has read the slot
+    uint32_t end = slot + all;
+    if (v.last_band) {
+      if (v.words) { v.words[CW_COUNT + v.chunk] = end - v.words[CW_BASE + v.chunk]; v.words[CW_BASE + v.chunk + 1] = (end + 31u) & ~31u; }
+      *num_isect = max(v.words ? end : t.st[S_TOTAL], t.st[S_OVER]);
+    }
+    t.st[S_SLOT] = end;
+  }
+}
+
+// The hits of an item to their tiles' lists, in the order of the pairs: for each tile the warp takes the 32 pairs of one hit
+// word at a time, and the lanes with a hit write side by side.
+__global__ void __launch_bounds__(L2_THREADS) item_emit_kernel(Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ pairs, const uint32_t* __restrict__ hit_lo,
+                                                               const uint32_t* __restrict__ hit_hi, const uint2* __restrict__ ranges, uint32_t* __restrict__ vals) {
+  __shared__ uint32_t s_splat[L2_THREADS], s_word[L2_WARPS][BIN_TILES];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lane_lt = (1u << lane) - 1u, n_items = t.st[S_ITEMS];
+  constexpr int TPW = BIN_TILES / L2_WARPS;   // tiles a warp writes
+  for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
+    const Item m = item_of(t, g, it, cap);
+    uint32_t next = 0;   // lane k < TPW: next place of the warp's k-th tile
+    if (lane < TPW) {
+      const int tile = warp * TPW + lane, x = m.bx * BIN_W + (tile & 7), y = m.by * BIN_W + (tile >> 3);
+      if (x < g.tiles_x && y < g.tiles_y) next = ranges[y * g.tiles_x + x].x + t.cells[(size_t)it * BIN_TILES + tile];
+    }
+    for (uint32_t p0 = m.first; p0 < m.end; p0 += L2_THREADS) {
+      const uint32_t p = p0 + tid;
+      const bool valid = p < m.end;
+      s_splat[tid] = valid ? pairs[p] : 0u;
+      s_word[warp][lane] = transpose_bits(valid ? hit_lo[p] : 0u);
+      s_word[warp][lane + 32] = transpose_bits(valid ? hit_hi[p] : 0u);
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < TPW; k++) {
+        uint32_t pos = __shfl_sync(FULL, next, k);
+#pragma unroll
+        for (int w = 0; w < L2_WARPS; w++) {
+          const uint32_t word = s_word[w][warp * TPW + k];
+          if (word == 0u) continue;
+          const uint32_t at = pos + __popc(word & lane_lt);
+          if (((word >> lane) & 1u) && at < cap) vals[at] = s_splat[w * 32 + lane];
+          pos += __popc(word);
+        }
+        if (lane == k) next = pos;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Tile ids of the sorted list, for callers of the whole-view binning: a warp per tile.
+__global__ void __launch_bounds__(256) fill_keys_kernel(int n_tiles, const uint2* __restrict__ ranges, uint32_t* __restrict__ keys) {
+  const int lane = threadIdx.x & 31;
+  for (int tile = blockIdx.x * 8 + (threadIdx.x >> 5); tile < n_tiles; tile += gridDim.x * 8) {
+    const uint2 r = ranges[tile];
+    for (uint32_t p = r.x + lane; p < r.y; p += 32) keys[p] = (uint32_t)tile;
+  }
+}
+
+}  // namespace
+
+// Bins the ranks of one depth chunk (words != nullptr) or of the whole view into vals_sorted and `ranges`. Level 1's pairs
+// take ctx->keys, the hit words ctx->vals and ctx->keys_sorted, a chunk's live splats the scratch of the depth sort.
+int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, int hi_num, const unsigned long long* alive, uint32_t* tables, cudaStream_t s) {
+  Tables t;
+  t.cells = tables;
+  t.totals = t.cells + BINS_TABLE_WORDS; t.base = t.totals + MAX_BINS; t.first_item = t.base + MAX_BINS + 1; t.item_bin = t.first_item + MAX_BINS + 1;
+  t.block_sums = t.item_bin + MAX_ITEMS; t.segments = t.block_sums + 1024; t.st = t.segments + BINS_SEGMENTS;
+  static_assert(MAX_BINS + 2 * (MAX_BINS + 1) + MAX_ITEMS + 1024 + BINS_SEGMENTS + 16 <= BINS_EXTRA_WORDS, "scratch");
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  constexpr int smem_max = MAX_BINS * ((L1_WARPS + 1) * (int)sizeof(uint32_t) + 8);
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !attr_set[dev]) {
+    B2K_CUDA(cudaFuncSetAttribute(bin_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    B2K_CUDA(cudaFuncSetAttribute(bin_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    attr_set[dev] = true;
+  }
+  const uint32_t cap = (uint32_t)c->isect_cap;
+  uint2* ranges = (uint2*)c->tile_ranges + (words ? (size_t)chunk * c->n_tiles : 0);
+  const int bins_x = div_up(c->tiles_x, BIN_W), bin_rows = div_up(c->tiles_y, BIN_W);
+  if (bins_x > MAX_BINS) return B2K_ERR_UNSUPPORTED;   // tile boxes hold twelve bits of a tile's column: the caller's own limit is lower
+  const int rows_per_band = MAX_BINS / bins_x;
+  View v{c->order, (const uint4*)c->hit_info, c->tile_count, (const float4*)c->proj0, (const float4*)c->proj1, n, words, chunk, lo_num, hi_num, alive, 0, 0};
+  for (int row = 0; row < bin_rows; row += rows_per_band) {
+    Band g{c->tiles_x, c->tiles_y, bins_x, row, std::min(rows_per_band, bin_rows - row)};
+    v.first_band = row == 0; v.last_band = row + g.bin_rows == bin_rows;
+    const int bins = g.bins_x * g.bin_rows;
+    // Blocks of level 1: two per SM, no more than the table holds rows for, none without a rank.
+    const long long ranks = words ? (long long)n * (hi_num - lo_num) / 256 + 1 : n;
+    const int blocks = (int)std::max<long long>(1, std::min<long long>({2LL * sm_count(), 32LL * ROWS_PER, (long long)(BINS_TABLE_WORDS / bins), (ranks + L1_THREADS - 1) / L1_THREADS}));
+    // Items are read on the device: a grid that fills the GPU, or what few splats can make at most.
+    const int item_blocks = (int)std::min<long long>(sm_count() * 8LL, bins + ranks * std::min(bins, 64) / L2_THREADS);
+    const int tiles = (std::min((row + g.bin_rows) * BIN_W, c->tiles_y) - row * BIN_W) * c->tiles_x, scan_blocks = div_up(tiles, SCAN_TILES);
+#define L(WHOLE) do { \
+    const size_t alive_bytes = WHOLE ? 0 : bins * sizeof(unsigned long long); \
+    bin_count_kernel<WHOLE><<<blocks, COUNT_THREADS, alive_bytes + bins * sizeof(uint32_t), s>>>(v, g, t, c->depth_keys); \
+    bin_rows_kernel<<<div_up(bins, ROWS_BINS), ROWS_THREADS, 0, s>>>(blocks, bins, cap, t); \
+    bin_scatter_kernel<WHOLE><<<blocks, L1_THREADS, alive_bytes + bins * (L1_WARPS + 1) * sizeof(uint32_t), s>>>(v, g, t, cap, c->depth_keys, c->keys, c->tile_off); \
+    item_count_kernel<WHOLE><<<item_blocks, L2_THREADS, 0, s>>>(v, g, t, cap, c->keys, c->vals, c->keys_sorted); } while (0)
+    if (words) L(false); else L(true);
+#undef L
+    if (bins >= 2 * sm_count()) item_columns_kernel<4><<<bins, 4 * BIN_TILES, 0, s>>>(g, t, ranges);
+    else item_columns_kernel<16><<<bins, 16 * BIN_TILES, 0, s>>>(g, t, ranges);
+    tile_scan_kernel<<<scan_blocks, SCAN_TILES, 0, s>>>(v, g, t, cap, ranges, c->num_isect);
+    item_emit_kernel<<<item_blocks, L2_THREADS, 0, s>>>(g, t, cap, c->keys, c->vals, c->keys_sorted, ranges, c->vals_sorted);
+  }
+  return check_launch();
+}
+
+int launch_fill_keys(const B2kCtx* c, cudaStream_t s) {
+  fill_keys_kernel<<<std::min(div_up(c->n_tiles, 8), sm_count() * 8), 256, 0, s>>>(c->n_tiles, (const uint2*)c->tile_ranges, c->keys_sorted);
+  return check_launch();
+}
+
+}  // namespace b2k

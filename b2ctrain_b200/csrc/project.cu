@@ -69,16 +69,18 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
   if (i >= n) return;
   const float4 po = pos_op[i], q = quat[i], ls = lscale[i];
   Proj pr;
-  uint32_t hits = 0, mask_lo = 0, mask_hi = 0, box = 0;
+  uint32_t hits = 0, mask_lo = 0, mask_hi = 0, box = 0, height = 0;
   bool shade = false, big = false;
   if (project_one(po, q, ls, cam, pr)) {
     const TileRec rec = make_tile_rec(pr.mx, pr.my, pr.c00, pr.c01, pr.c11, pr.power);
     TileBox bb;
     if (tile_box(rec, cam.W, cam.H, tiles_x, tiles_y, bb)) {
       const int bw = bb.max_x - bb.min_x, bh = bb.max_y - bb.min_y;
+      height = (uint32_t)bh;
       if (bw * bh > MASK_TILES) {
         big = true; shade = true;
         box = 0xFFFFFFFFu;
+        mask_lo = (uint32_t)bb.min_x | ((uint32_t)bb.min_y << 16); mask_hi = (uint32_t)bw | ((uint32_t)bh << 16);   // no mask: the box itself
         big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
       } else if (bw > 0 && bh > 0) {
         int bit = 0;
@@ -106,7 +108,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
   } else {
     proj1[i] = make_float4(0.f, 0.f, 0.f, -1.f);   // no record
   }
-  hit_info[i] = make_uint4(mask_lo, mask_hi, box, 0u);
+  hit_info[i] = make_uint4(mask_lo, mask_hi, box, height);
   order_in[i] = (uint32_t)i;
   if (!big) {   // big splats get their count and key from count_big_kernel
     tile_count[i] = hits;
@@ -207,15 +209,17 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 a = proj0[i], b = proj1[i];
-  uint32_t hits = 0, mask_lo = 0, mask_hi = 0, box = 0;
+  uint32_t hits = 0, mask_lo = 0, mask_hi = 0, box = 0, height = 0;
   bool big = false;
   if (b.w > -0.5f) {
     const TileRec rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
     TileBox bb;
     if (tile_box(rec, W, H, tiles_x, tiles_y, bb)) {
       const int bw = bb.max_x - bb.min_x, bh = bb.max_y - bb.min_y;
+      height = (uint32_t)bh;
       if (bw * bh > MASK_TILES) {
         big = true; box = 0xFFFFFFFFu;
+        mask_lo = (uint32_t)bb.min_x | ((uint32_t)bb.min_y << 16); mask_hi = (uint32_t)bw | ((uint32_t)bh << 16);
         big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
       } else if (bw > 0 && bh > 0) {
         int bit = 0;
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
       }
     }
   }
-  hit_info[i] = make_uint4(mask_lo, mask_hi, box, 0u);
+  hit_info[i] = make_uint4(mask_lo, mask_hi, box, height);
   order_in[i] = (uint32_t)i;
   if (!big) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
 }

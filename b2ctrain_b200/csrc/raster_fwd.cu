@@ -22,8 +22,8 @@ constexpr int FWD_GROUP = B2K_FWD_GROUP;                 // fragments whose stat
 // launches a pixel's state lives in the output buffers: the colour sums in out_feat.xyz, the transmittance in
 // out_feat.w, and last_idx with bit 31 set once the pixel has reached the cutoff; out_rgba holds the finished pixel
 // after every chunk, so a launch only touches tiles that received fragments. With DEPTH the depth sum travels in
-// out_depth and the last chunk visits every pixel to divide it out. alive[tile] tells the binning of the next chunk
-// whether any pixel of the tile can still take a fragment.
+// out_depth and the last chunk visits every pixel to divide it out. The tile's bit in `alive` tells the binning of the next
+// chunk whether any pixel of the tile can still take a fragment.
 constexpr uint32_t DONE_BIT = 0x80000000u;
 
 // What the forward leaves for the backward (common.cuh): nothing, checkpoints of the running sums, or of each segment's sums.
@@ -33,7 +33,7 @@ template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
 __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
-    float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, uint32_t* __restrict__ alive,
+    float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
     const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc) {
   constexpr bool BWD = CKPT != NONE;
   // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   }
   if (CHUNKED && !final) {
     const bool open = __any_sync(0xffffffffu, !done[0] || !done[1]);
-    if (lane == 0) alive[tile] = open ? 1u : 0u;
+    if (lane == 0 && !open) atomicAnd(alive + (size_t)(ty >> 3) * ((tiles_x + 7) >> 3) + (tx >> 3), ~(1ull << ((ty & 7) * 8 + (tx & 7))));
   }
   if constexpr (BWD) {
     // The backward never needs to look past the last fragment any pixel used. (A pixel whose last fragment lies in an
@@ -208,7 +208,7 @@ using namespace b2k;
 
 namespace b2k {
 // One chunk of a chunked view (n_chunks > 1), or the whole view (n_chunks <= 1).
-int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_chunks, uint32_t* alive, cudaStream_t s) {
+int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_chunks, unsigned long long* alive, cudaStream_t s) {
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
   uint2* ranges = (uint2*)c->tile_ranges + (n_chunks > 1 ? (size_t)chunk * c->n_tiles : 0);
 #define L(B, D, C, F) raster_fwd_kernel<B, D, C, F><<<div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, s>>>(ranges, c->vals_sorted, (const float4*)c->proj0, \

@@ -63,14 +63,15 @@ typedef struct {
   float* proj2;            /* [n][4] r, g, b, feature x (0 without a feature mode) */
   uint32_t* tile_count;    /* [n] tiles hit */
   uint32_t* hit_info;      /* [n][4] bit mask (lo, hi) of the hit tiles inside the splat's tile box, row-major; packed box
-                              min_x | min_y << 12 | width << 24; unused. Boxes above 64 tiles carry box = 0xFFFFFFFF and are
-                              re-tested when emitted (the reference keeps a 32-tile mask, src/gpu/project.cu:33-43) */
+                              min_x | min_y << 12 | width << 24; height. Boxes above 64 tiles carry (min_x | min_y << 16,
+                              width | height << 16, 0xFFFFFFFF, height) and are tested when binned (the reference keeps a 32-tile
+                              mask, src/gpu/project.cu:33-43) */
   uint32_t* depth_keys;    /* [n] scratch of the depth sort */
   uint32_t* depth_keys_sorted; /* [n] b2k_project leaves the unsorted keys here; b2k_bin_sort sorts them in place */
   uint32_t* order_in;      /* [n] scratch of the depth sort */
   uint32_t* order;         /* [n] after b2k_project: identity; after b2k_bin_sort: splat index by depth rank (culled last) */
   uint32_t* tile_off;      /* [n] inclusive scan of tile counts in depth order */
-  uint32_t *keys, *vals, *keys_sorted, *vals_sorted; /* [isect_cap] tile id / splat index before and after the tile sort */
+  uint32_t *keys, *vals, *keys_sorted, *vals_sorted; /* [isect_cap] scratch, scratch; tile id / splat index by tile, then depth */
   uint64_t isect_cap;
   uint32_t* num_isect;     /* [4] device words: [0] intersections of this view (may exceed isect_cap: overflow);
                               [1] entries of vis_list; [2] largest [0] since the caller cleared it (b2k_loss_accumulate) */
@@ -95,8 +96,8 @@ typedef struct {
                               range per chunk and tile, indices into vals_sorted) and b2k_raster_bwd walks them all */
   float* proj3;            /* [n][2] feature lanes y, z (x rides in proj2.w), render.h:70; NULL unless a feature mode is used */
   uint32_t* chunk_words;   /* [32 + n_tiles + (tiles_x + 1)(tiles_y + 1)] device scratch of b2k_render_chunked (chunk windows
-                              and counts, one "some pixel can still take a fragment" flag per tile, the summed-area table
-                              of those flags), or NULL when n_chunks <= 1 */
+                              and counts, one "some pixel can still take a fragment" flag per tile), or NULL when
+                              n_chunks <= 1 */
   void* bwd_scratch;       /* b2k_bwd_scratch_bytes() bytes, needed when the forward runs with bwd_info: per-pixel (colour
                               sums, transmittance) checkpoints the forward leaves at every segment boundary of a tile's list, and
                               the work list of the backward, which replays the segments between checkpoints independently.
@@ -160,8 +161,7 @@ int b2k_count_tiles(const B2kCtx* ctx, int32_t n, b2k_stream_t s);
  * total stays on the device in ctx->num_isect and the later stages read it there. */
 int b2k_bin_sort(const B2kCtx* ctx, int32_t n, b2k_stream_t s);
 /* b2k_bin_sort with CUDA events between its phases (measurement aid; waits for the stream). ms[10]: [0] depth sort,
- * [1] scan + emit, [2],[3] / [4],[5] / [6],[7] count+row-scan and scatter of tile-sort passes 0 / 1 / 2, [8] tile
- * ranges, [9] whole call. The role of the reference's StageTimer (src/train/trainer.cpp:57-73) at kernel granularity. */
+ * [1] distribution to the tiles (hits, ranges, list), [2]..[7] 0, [8] tile ids of the list, [9] whole call. The role of the reference's StageTimer (src/train/trainer.cpp:57-73) at kernel granularity. */
 int b2k_bin_sort_profile(const B2kCtx* ctx, int32_t n, b2k_stream_t s, float* ms);
 /* The 4-byte count readback of binning.cu:125-127 as its own call: waits for the stream, returns the total and
  * B2K_ERR_OVERFLOW when it exceeds ctx->isect_cap (the caller grows the four buffers and redoes the view). */
@@ -186,9 +186,9 @@ int b2k_raster_fwd(const B2kCtx* ctx, const B2kRenderOpts* opts, b2k_stream_t s)
  * increasing depth (the nearest 1/4^(C-1) of the visible splats first, each chunk four times the one before). A
  * tile whose pixels have all reached the transmittance cutoff emits no intersections in later chunks, so most of a
  * dense view is never sorted. out_rgba, out_feat.w, out_depth and every gradient of the backward are bit-identical to
- * b2k_project + b2k_bin_sort + b2k_raster_fwd; what differs is the bookkeeping a caller can see: vals_sorted /
- * keys_sorted hold one sorted window per chunk (without the intersections that were skipped), tile_ranges one range
- * per chunk and tile, last_idx an index into that layout with bit 31 set on pixels that reached the cutoff,
+ * b2k_project + b2k_bin_sort + b2k_raster_fwd; what differs is the bookkeeping a caller can see: vals_sorted
+ * holds one sorted window per chunk (without the intersections that were skipped; keys_sorted is scratch), tile_ranges one
+ * range per chunk and tile, last_idx an index into that layout with bit 31 set on pixels that reached the cutoff,
  * out_feat.xyz the colour sums without the background (with a feature mode, forward only: the feature lanes, as in the
  * whole-view path; their running sums travel in ctx->bwd_scratch between chunks), num_isect[0] the slots used. Needs last_idx and chunk_words;
  * tile_off and depth_keys are scratch; tile_count holds each splat's

@@ -46,3 +46,59 @@ def test_backward_segments_and_odd_batches(n, W, H):
         assert rel_l2(got[:, lane], want[:, lane]) <= 5e-5, lane
     assert np.all(got[:, 10:] == 0)
     assert rel_l2(h.model.vis_weight[:n].cpu().numpy(), visw) <= 1e-5
+
+
+def bin_scene(n, W, H, wide, seed=5):
+    scene = scenes.make_splats(n, 0, seed, log_scale=(-3.5, 0.6))
+    scene["lscale"][::max(1, n // max(1, wide)), :3] = -0.7 if wide else -3.5      # splats over most of the image
+    cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 25.0, 10.0), W, H, float(max(W, H)))
+    return scenes.floor_for_cameras(scene, [cam]), cam
+
+
+@pytest.mark.parametrize("W,H,n,wide", [(8, 8, 40, 3),             # one tile
+                                        (64, 64, 300, 3),          # one bin of 8x8 tiles
+                                        (65, 63, 300, 3),          # a ragged second column of bins
+                                        (1040, 72, 5000, 200),     # 17x2 bins: splats over more bins than a lane walks alone
+                                        (3848, 2312, 600, 40)])    # 61x37 bins: two bands of bin rows
+def test_binning_at_the_edges_of_bins_and_bands(W, H, n, wide):
+    """Tile sets, list order and ranges are bit-exact functions of the records; a chunked view composites the same image."""
+    import torch
+    scene, cam = bin_scene(n, W, H, wide)
+    h = Harness(scene, cam, isect_cap=1 << 23)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    h.api.bin_and_sort(h.ctx, h.model)
+    tc_o, vals_o, keys_o, ranges_o = orc.bin_sort(h.ctx.proj0[:n].cpu().numpy(), h.ctx.proj1[:n].cpu().numpy(), W, H)
+    tc = h.u32(h.ctx.tile_count, n)
+    assert np.array_equal(tc, tc_o)
+    assert h.ctx.num_isect == len(vals_o) > n // 2
+    assert np.array_equal(h.u32(h.ctx.vals_sorted, len(vals_o)), vals_o)
+    assert np.array_equal(h.u32(h.ctx.keys_sorted, len(vals_o)), keys_o)
+    assert np.array_equal(h.u32(h.ctx.tile_ranges).reshape(-1, 2), ranges_o)
+    assert np.array_equal(h.u32(h.ctx.tile_off, n), np.cumsum(tc[h.u32(h.ctx.order, n)], dtype=np.uint32))
+    h.api.rasterize_forward(h.ctx, h.rp)
+    chunked = h.api.RenderCtx("cuda:0")
+    chunked.setup(W, H, h.model.cap, n_chunks=3, isect_cap=1 << 23)
+    h.api.render_forward(chunked, h.model, h.rp)
+    assert torch.equal(chunked.out_rgba, h.ctx.out_rgba)
+
+
+def test_binning_with_more_pairs_than_items_of_256_hold():
+    """Two and a half million (bin, splat) pairs: level 2 works on longer items. Every splat appears tile_count times, each
+    tile's list is in depth order, and the lists fill the ranges."""
+    import torch
+    W, H, n = 1024, 1024, 60_000
+    scene, cam = bin_scene(n, W, H, 0)
+    scene["lscale"][:, :3] = -2.2
+    h = Harness(scene, cam, isect_cap=1 << 26)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    counts = h.ctx.tile_count[:n].clone()
+    h.api.bin_and_sort(h.ctx, h.model)
+    total = h.ctx.num_isect
+    assert total == int(counts.to(torch.int64).sum()) and total > 20_000_000
+    vals, keys = h.ctx.vals_sorted[:total].to(torch.int64), h.ctx.keys_sorted[:total].to(torch.int64)
+    assert torch.equal(torch.bincount(vals, minlength=n).to(torch.int32), counts)
+    rank = torch.empty(n, dtype=torch.int64, device="cuda:0")
+    rank[h.ctx.order[:n].to(torch.int64)] = torch.arange(n, device="cuda:0")
+    assert bool((torch.diff(keys * n + rank[vals]) > 0).all())
+    r = h.ctx.tile_ranges.view(-1, 2).to(torch.int64)
+    assert torch.equal(r[:, 1] - r[:, 0], torch.bincount(keys, minlength=h.ctx.n_tiles))
