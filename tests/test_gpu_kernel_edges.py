@@ -102,3 +102,26 @@ def test_binning_with_more_pairs_than_items_of_256_hold():
     assert bool((torch.diff(keys * n + rank[vals]) > 0).all())
     r = h.ctx.tile_ranges.view(-1, 2).to(torch.int64)
     assert torch.equal(r[:, 1] - r[:, 0], torch.bincount(keys, minlength=h.ctx.n_tiles))
+
+
+@pytest.mark.parametrize("kind", ["uniform", "wide", "same", "culled", "all_culled", "any_bits"])
+@pytest.mark.parametrize("n", [1, 33, 2048, 2049, 8192, 8193, 100_003, 1_300_001])   # one block, then small, middle and large tiles
+def test_depth_sort_is_stable_at_every_size(n, kind):
+    import ctypes as C
+    import torch
+    from b2ctrain_b200 import api
+    g = torch.Generator(device="cuda:0"); g.manual_seed(n)
+    u = torch.rand(n, device="cuda:0", generator=g)
+    z = {"wide": torch.exp(u * 27.6 - 4.6).clamp(0.01, 1e10), "same": torch.full_like(u, 2.5)}.get(kind, 3 + 2 * u)
+    keys = z.view(torch.int32).clone()
+    if kind == "any_bits":   # a caller's own keys
+        keys = torch.randint(-2 ** 31, 2 ** 31, (n,), device="cuda:0", generator=g, dtype=torch.int64).to(torch.int32)
+    if kind in ("culled", "all_culled"):
+        keys[u < (0.5 if kind == "culled" else 2.0)] = -1
+    ctx = api.RenderCtx("cuda:0"); ctx.setup(64, 64, n)
+    ctx.depth_keys_sorted.copy_(keys); ctx.order.copy_(torch.arange(n, dtype=torch.int32)); ctx.tile_count.zero_(); ctx.hit_info.zero_()
+    cs = ctx.struct()
+    assert api.lib().b2k_bin_sort(C.byref(cs), n, api._stream(None)) == api.B2K_OK
+    wide = keys.to(torch.int64) & 0xFFFFFFFF
+    want = torch.argsort(wide, stable=True)
+    assert torch.equal(ctx.order.to(torch.int64), want) and torch.equal(ctx.depth_keys_sorted.to(torch.int64) & 0xFFFFFFFF, wide[want])
