@@ -46,237 +46,317 @@ __device__ __forceinline__ void load16(const float* p, float (&v)[16]) {
 }
 
 // ---- The loss kernel --------------------------------------------------------------------------------------------------
-// One CTA owns a strip of STRIP_W output columns, a segment of rows and one colour channel, and walks the segment four
-// rows at a time. Both blurs are separable, so only the horizontal direction pays for a halo: the row-blurred moments
-// and the derivative maps of the last RING rows live in shared-memory rings, and the four stages of the chain run
-// side by side as a pipeline, each on its own warps and on its own rows, with one barrier per four rows:
-//   A (2 warps)  rows a..a+3      : effective target and prediction -> five moments blurred along the row
-//   B (4 warps)  rows a-9..a-6    : blurred down the column -> SSIM -> derivative maps (three: the two that the chain
+// One CTA owns a strip of STRIP_W output columns and a segment of rows, all three channels, and walks the segment four rows at
+// a time. Both blurs are separable, so only the horizontal direction pays for a halo: the row-blurred moments and the
+// derivative maps of the last RING rows live in shared-memory rings, and the four stages of the chain run side by side as a
+// pipeline, each on its own warps (six to a channel) and on its own rows, with one barrier per four rows:
+//   A (1 warp)   rows a..a+3      : prediction and effective target -> five moments blurred along the row
+//   B (2 warps)  rows a-9..a-6    : blurred down the column -> SSIM -> derivative maps (three: the two that the chain
 //                                   rule multiplies by p and by the target, and the sum of the three it does not)
-//   C (2 warps)  rows a-18..a-15  : derivative maps blurred down the column
-//   D (2 warps)  rows a-22..a-19  : blurred along the row, chain rule, L1 term, one component of v_out per pixel
-// Every thread also fetches one element of the next four input rows while it works. Against one CTA per 16x16 tile (a 36x36 footprint
-// blurred for 256 outputs, the reference's shape) this spends about a quarter of the warp instructions per pixel:
-// measured 0.41 -> 0.20 ms for a 1920x1080 view.
+//   C (1 warp)   rows a-18..a-15  : derivative maps blurred down the column
+//   D (2 warps)  rows a-22..a-19  : blurred along the row, chain rule, L1 term
+// While they work, all threads fetch the next four input rows, a whole pixel each, and write the gradient rows of the step
+// before, a whole pixel each: with a CTA per channel every 32-byte sector crossed the L2 three times in both directions. A
+// pixel's values also wait in a ring for stage D, so that no stage waits for global memory.
+//
+// Bound by instruction issue: 176 multiply-adds per pixel and channel in the four blurs. They run two to an instruction
+// (fp32x2) with operands that lie in pairs as they are stored: prediction and target side by side, and so their means, their
+// squares, and the two maps with a per-pixel factor; the product moment and the third map are paired over two rows (A) or two
+// columns (C). A thread makes four or eight outputs from one window, so that a value read from shared memory feeds eleven to
+// forty-four multiply-adds. Measured against the same pipeline with scalar multiply-adds and a CTA per channel: 187 -> 125 us on
+// a 1920x1080 view, 101 -> 95 us on a masked 1024x1024 one, 26 -> 21 us on 333x217. Other arrangements on 1920x1080: packed,
+// a CTA per channel 133 to 147; channels of one CTA with a barrier each 130; the pairs in plain order (two-way bank conflicts in
+// stages A and D) 139; two columns per thread in stage B 142.
 constexpr int STRIP_W = 54;                   // output columns of a strip
 constexpr int STRIP_ST = STRIP_W + 2 * HALO;  // 64 statistics columns
-constexpr int STRIP_IN = 76;                  // input columns staged: STRIP_W + 4 * HALO = 74, padded to whole 16-byte words
+constexpr int STRIP_IN = 80;                  // input columns staged: STRIP_W + 4 * HALO = 74, padded to whole groups of eight 16-byte chunks
 constexpr int STRIP_ROWS = 4;                 // rows per pipeline step
 constexpr int RING = 18;                      // rows of a ring: the 14 a column window of four outputs reads + the 4 being written
-constexpr int BV_S = STRIP_ST + 4;            // row stride of stage C's output: the last row window overruns into zero padding
-constexpr int STRIP_THREADS = 320;
-constexpr int STRIP_CTAS_PER_SM = 4;         // 48 registers per thread; measured faster than 2 or 3 CTAs with more registers
+constexpr int BV_S = STRIP_ST + 16;           // row stride of stage C's output: the last row window overruns into zero padding
+constexpr int PX_RING = 32;                   // rows of the ring that keeps pixels for stage D: a + 7 down to a - 22 are in use
+constexpr int PX_S = 64;                      // its columns: STRIP_W, padded likewise
+constexpr int CH_WARPS = 6, STRIP_THREADS = 3 * CH_WARPS * 32;
+constexpr int STRIP_CTAS_PER_SM = 1;
 static_assert(STRIP_ST == 64 && STRIP_IN >= STRIP_W + 4 * HALO && STRIP_IN % 4 == 0, "strip geometry");
 
-__device__ __forceinline__ int ring_slot(int row) { return (row + RING * 256) % RING; }
+struct Gauss2 { float2 w[11]; };   // every weight twice, as an operand of packed arithmetic
 
+// One ring row of row-blurred moments, and one of derivative maps: everything of a row behind one address.
+struct MomentRow { float2 mean[STRIP_ST], square[STRIP_ST]; float cross[STRIP_ST]; };   // (prediction, target) twice; their product
+struct MapRow { float2 e12[STRIP_ST]; float e0[STRIP_ST]; };                            // the maps multiplied by p and by the target; the sum of the others
+// Rows of pairs are kept as 16-byte chunks of two columns in a slightly permuted order: threads that read or write every other
+// chunk (four columns each) then meet all banks, and runs of chunks still do.
+__device__ __forceinline__ int chunk_at(int chunk) { return chunk ^ ((chunk >> 3) & 1); }
+__device__ __forceinline__ int pair_at(int col) { return chunk_at(col >> 1) * 2 + (col & 1); }   // place of one column's pair
+
+struct ChannelShare {
+  float2 in[2][STRIP_ROWS][STRIP_IN];     // [buffer][row][column]: prediction, effective target
+  float2 px[PX_RING][PX_S];               // the strip's own columns of the same, until stage D has used them
+  MomentRow moments[RING];
+  MapRow maps[RING];
+  float2 b12[2][STRIP_ROWS][BV_S];        // [buffer] the maps blurred down the column
+  float b0[2][STRIP_ROWS][BV_S];
+};
+struct StripShare {
+  ChannelShare ch[3];
+  float out[2][STRIP_ROWS][PX_S][4];      // [buffer] gradient of the step's pixels
+  float red[20];
+};
+static_assert(sizeof(StripShare) % 16 == 0 && sizeof(StripShare) <= 227 * 1024 && STRIP_THREADS / 32 <= 20, "one CTA per SM");
+
+__device__ __forceinline__ int ring_slot(int row) { return (row + RING * 256) % RING; }
+template <class ROW>
+__device__ __forceinline__ ROW* ring_next(ROW* row, ROW* ring) { return row == ring + (RING - 1) ? ring : row + 1; }
+__device__ __forceinline__ float fast_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+// Byte c of a packed pixel as 0 .. 1: the byte under the exponent of 2^23, less 2^23 (an integer conversion runs at a quarter
+// of the rate of these).
+__device__ __forceinline__ float byte_unit(uint32_t p, int c) { return (__uint_as_float(__byte_perm(p, 0x4B000000u, 0x7440u | (uint32_t)c)) - 8388608.f) * (1.f / 255.f); }
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+
+// MASKED: per-pixel weights or the target's alpha scale the loss, or there is an alpha lane.
+template <bool MASKED>
 __global__ void __launch_bounds__(STRIP_THREADS, STRIP_CTAS_PER_SM) photometric_strip_kernel(const float4* __restrict__ pred, const uint32_t* __restrict__ gt,
                                                                           const uint8_t* __restrict__ weights, int W, int H, int seg_rows, LossArgs lp,
-                                                                          Gauss gauss, float4* __restrict__ v_out, float* __restrict__ loss_accum) {
-  __shared__ __align__(16) float s_in[2][2][STRIP_ROWS][STRIP_IN];   // [buffer][prediction, target][row][column]
-  __shared__ __align__(16) float s_hb[5][RING][STRIP_ST];            // row-blurred moments
-  __shared__ __align__(16) float s_dv[3][RING][STRIP_ST];            // derivative maps
-  __shared__ __align__(16) float s_bv[2][3][STRIP_ROWS][BV_S];       // [buffer] derivative maps blurred down the column
-  __shared__ float s_red[STRIP_THREADS / 32];
-  const int tid = threadIdx.x, warp = tid >> 5, c = blockIdx.z;
+                                                                          Gauss2 gauss, float4* __restrict__ v_out, float* __restrict__ loss_accum) {
+  extern __shared__ __align__(16) unsigned char s_bytes[];
+  StripShare& all = *reinterpret_cast<StripShare*>(s_bytes);
+  const int tid = threadIdx.x, lane = tid & 31, c = (tid >> 5) / CH_WARPS, warp = (tid >> 5) % CH_WARPS;   // channel, role
+  ChannelShare& sh = all.ch[c];
   const int x0 = blockIdx.x * STRIP_W, y0 = blockIdx.y * seg_rows, y1 = min(y0 + seg_rows, H);
   const int x_end = min(x0 + STRIP_W, W);
   const float norm = lp.scale / (3.f * (float)W * (float)H);
-  const float bg_c = lp.composite ? lp.bg[c] : 0.f;
   const float alpha_norm = lp.match_alpha_weight * lp.scale / ((float)W * (float)H);
-  const float* pred_c = reinterpret_cast<const float*>(pred) + c;
-  float* out_c = reinterpret_cast<float*>(v_out) + c;
 
-  for (int i = tid; i < 5 * RING * STRIP_ST; i += STRIP_THREADS) (&s_hb[0][0][0])[i] = 0.f;
-  for (int i = tid; i < 3 * RING * STRIP_ST; i += STRIP_THREADS) (&s_dv[0][0][0])[i] = 0.f;
-  for (int i = tid; i < 2 * 3 * STRIP_ROWS * BV_S; i += STRIP_THREADS) (&s_bv[0][0][0][0])[i] = 0.f;
-  // One input element (prediction and effective target, zero outside the image and in the row pad).
-  auto fetch = [&](int row0, int e, float& px, float& ty) {
-    const int row = e / STRIP_IN, col = e - row * STRIP_IN;
-    const int y = row0 + row, x = x0 - 2 * HALO + col;
-    px = 0.f; ty = 0.f;
-    if (col < STRIP_W + 4 * HALO && y >= 0 && y < H && x >= 0 && x < W) {
-      const size_t q = (size_t)y * W + x;
-      const uint32_t gp = gt[q];
-      px = pred_c[q * 4];
-      ty = unpack(gp, c) + (1.f - unpack(gp, 3)) * bg_c;
+  for (int i = tid; i < (int)(sizeof(StripShare) / 16); i += STRIP_THREADS) reinterpret_cast<float4*>(s_bytes)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  // The input pixel a thread fetches (zero outside the image and in the row pad): which one, and whether its column is inside
+  // the image, does not change from step to step.
+  const int f_row = tid / STRIP_IN, f_col = tid - f_row * STRIP_IN, f_x = x0 - 2 * HALO + f_col;
+  const bool f_thread = tid < STRIP_ROWS * STRIP_IN;
+  const bool f_ok = f_thread && f_col < STRIP_W + 4 * HALO && f_x >= 0 && f_x < W;
+  static_assert(STRIP_ROWS * STRIP_IN <= STRIP_THREADS, "one pixel a thread");
+  float3 f_p = make_float3(0.f, 0.f, 0.f);
+  uint32_t f_t = 0xFF000000u;
+  auto fetch = [&](int row0) {
+    const int y = row0 + f_row;
+    f_p = make_float3(0.f, 0.f, 0.f); f_t = 0xFF000000u;   // an opaque black target is zero with any background
+    if (f_ok && y >= 0 && y < H) { const size_t q = (size_t)y * W + f_x; f_t = gt[q]; const float4 v = pred[q]; f_p = make_float3(v.x, v.y, v.z); }
+  };
+  auto store = [&](int buf, int row0) {
+    if (!f_thread) return;
+    const float p[3] = {f_p.x, f_p.y, f_p.z};
+    const float behind = lp.composite ? 1.f - byte_unit(f_t, 3) : 0.f;
+    const int px = f_col - 2 * HALO, slot = (row0 + f_row) & (PX_RING - 1);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const float2 v = make_float2(p[k], byte_unit(f_t, k) + behind * lp.bg[k]);
+      all.ch[k].in[buf][f_row][pair_at(f_col)] = v;
+      if (px >= 0 && px < PX_S) all.ch[k].px[slot][pair_at(px)] = v;
     }
   };
-  for (int e = tid; e < STRIP_ROWS * STRIP_IN; e += STRIP_THREADS) {
-    float px, ty;
-    fetch(y0 - 2 * HALO, e, px, ty);
-    (&s_in[0][0][0][0])[e] = px; (&s_in[0][1][0][0])[e] = ty;
-  }
+  fetch(y0 - 2 * HALO);
+  store(0, y0 - 2 * HALO);
   __syncthreads();
 
-  // Every thread fetches one element of the next four input rows while it does its stage's work (304 elements, 320
-  // threads): which element, and whether its column is inside the image, does not change from step to step.
-  const int st_row = tid / STRIP_IN, st_col = tid - st_row * STRIP_IN, st_x = x0 - 2 * HALO + st_col;
-  const bool st_slot = tid < STRIP_ROWS * STRIP_IN;
-  const bool st_ok = st_slot && st_col < STRIP_W + 4 * HALO && st_x >= 0 && st_x < W;
   float loss_local = 0.f;
   const int steps = 8 + (y1 - y0 + STRIP_ROWS - 1) / STRIP_ROWS;
-  for (int it = 0; it < steps; it++) {
+  for (int it = 0; it <= steps; it++) {   // the last round only writes what stage D left in the one before
     const int a = y0 - 2 * HALO + STRIP_ROWS * it, b = a - 9, cr = b - 9, d = cr - STRIP_ROWS;
     const int buf = it & 1;
     const bool more = a + STRIP_ROWS <= y1 - 1 + 2 * HALO;   // stage A has rows to blur in the next step
-    float nx = 0.f, ny = 0.f;
-    {
-      const int y = a + STRIP_ROWS + st_row;
-      if (more && st_ok && y >= 0 && y < H) {
-        const size_t q = (size_t)y * W + st_x;
-        const uint32_t gp = gt[q];
-        nx = pred_c[q * 4];
-        ny = unpack(gp, c) + (1.f - unpack(gp, 3)) * bg_c;
-      }
-    }
-    if (warp < 2) {
-      // A: rows a .. a+3, sixteen groups of four statistics columns each.
+    if (more) fetch(a + STRIP_ROWS);
+    if (warp == 0) {
+      // A: rows a .. a+3; a thread takes two rows and four statistics columns.
       if (a <= y1 - 1 + 2 * HALO) {
-        const int row = tid >> 4, g4 = (tid & 15) * 4;
-        float x[16], y[16], in[16], out[4];
-        load16(&s_in[buf][0][row][g4], x);
-        load16(&s_in[buf][1][row][g4], y);
-        const int slot = ring_slot(a + row);
-        window4(x, gauss, out); *reinterpret_cast<float4*>(&s_hb[0][slot][g4]) = make_float4(out[0], out[1], out[2], out[3]);
+        const int r2 = (lane >> 4) * 2, g4 = (lane & 15) * 4;
+        MomentRow *row_a = sh.moments + ring_slot(a + r2), *row_b = ring_next(row_a, sh.moments);
+        float2 cross_in[14], cross[4];
 #pragma unroll
-        for (int k = 0; k < 16; k++) in[k] = x[k] * x[k];
-        window4(in, gauss, out); *reinterpret_cast<float4*>(&s_hb[1][slot][g4]) = make_float4(out[0], out[1], out[2], out[3]);
-        window4(y, gauss, out); *reinterpret_cast<float4*>(&s_hb[2][slot][g4]) = make_float4(out[0], out[1], out[2], out[3]);
+        for (int r = 0; r < 2; r++) {
+          const float4* src = reinterpret_cast<const float4*>(sh.in[buf][r2 + r]);
+          float2 mean[4], square[4];
 #pragma unroll
-        for (int k = 0; k < 16; k++) in[k] = y[k] * y[k];
-        window4(in, gauss, out); *reinterpret_cast<float4*>(&s_hb[3][slot][g4]) = make_float4(out[0], out[1], out[2], out[3]);
+          for (int o = 0; o < 4; o++) { mean[o] = make_float2(0.f, 0.f); square[o] = make_float2(0.f, 0.f); }
 #pragma unroll
-        for (int k = 0; k < 16; k++) in[k] = x[k] * y[k];
-        window4(in, gauss, out); *reinterpret_cast<float4*>(&s_hb[4][slot][g4]) = make_float4(out[0], out[1], out[2], out[3]);
-      }
-    } else if (warp < 6) {
-      // B: statistics rows b .. b+3; a thread takes one column and two of the rows.
-      if (b + STRIP_ROWS - 1 >= y0 - HALO && b <= y1 - 1 + HALO) {
-        const int t = tid - 64, col = t & 63, r2 = (t >> 6) * 2;
-        int slots[12];
-        slots[0] = ring_slot(b + r2 - HALO);
+          for (int k2 = 0; k2 < 7; k2++) {
+            const float4 v4 = src[chunk_at(g4 / 2 + k2)];
 #pragma unroll
-        for (int k = 1; k < 12; k++) slots[k] = slots[k - 1] + 1 == RING ? 0 : slots[k - 1] + 1;
-        float st[5][2];
+            for (int h = 0; h < 2; h++) {
+              const int k = k2 * 2 + h;
+              const float2 v = h ? hi2(v4) : lo2(v4), vv = __fmul2_rn(v, v);
+              if (r == 0) cross_in[k].x = v.x * v.y; else cross_in[k].y = v.x * v.y;
 #pragma unroll
-        for (int m = 0; m < 5; m++) {
-          float in[12];
-#pragma unroll
-          for (int k = 0; k < 12; k++) in[k] = s_hb[m][slots[k]][col];
-          float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-          for (int dd = 0; dd < 11; dd++) { o0 += gauss.w[dd] * in[dd]; o1 += gauss.w[dd] * in[dd + 1]; }
-          st[m][0] = o0; st[m][1] = o1;
-        }
-        const int xg = x0 - HALO + col;
-        const bool x_in = xg >= 0 && xg < W, x_own = xg >= x0 && xg < x_end;
-#pragma unroll
-        for (int o = 0; o < 2; o++) {
-          const int y = b + r2 + o;
-          float E0 = 0.f, E1 = 0.f, E2 = 0.f;
-          if (x_in && y >= 0 && y < H) {
-            const size_t q = (size_t)y * W + xg;
-            const float wp = weights ? (float)weights[q] * (1.f / 255.f) : 1.f;
-            const float M = wp * (lp.mask ? unpack(gt[q], 3) : 1.f) * norm;
-            const float mu1 = st[0][o], mu2 = st[2][o];
-            const float mu1_sq = mu1 * mu1, mu2_sq = mu2 * mu2;
-            const float s1_raw = st[1][o] - mu1_sq, s2_raw = st[3][o] - mu2_sq;
-            const float sigma1_sq = fmaxf(0.f, s1_raw), sigma2_sq = fmaxf(0.f, s2_raw);
-            const float sigma12 = st[4][o] - mu1 * mu2;
-            const float A1 = 2.f * mu1 * mu2 + C1, A2 = 2.f * sigma12 + C2, B1 = mu1_sq + mu2_sq + C1, B2 = sigma1_sq + sigma2_sq + C2;
-            const float inv_BB = __fdividef(1.f, B1 * B2);   // approximate divisions, as in the reference's fast-math build
-            const float raw = A1 * A2 * inv_BB;
-            const float ssim = fminf(fmaxf(raw, -1.f), 1.f);
-            if (x_own && y >= y0 && y < y1) loss_local += M * lp.ssim_w * ssim;
-            if (raw > -1.f && raw < 1.f) {
-              const float k = M * lp.ssim_w;
-              const float d_mu1 = 2.f * mu2 * A2 * inv_BB - __fdividef(2.f * mu1 * ssim, B1);
-              const float d_s1 = s1_raw > 0.f ? -__fdividef(ssim, B2) : 0.f;
-              const float d_s12 = 2.f * A1 * inv_BB;
-              const float Am = k * d_mu1, Bv = k * d_s1, Cc = k * d_s12;
-              // gradient = blur(Am) + 2 p blur(Bv) - 2 blur(Bv mu1) + target blur(Cc) - blur(Cc mu2): the three maps
-              // without a per-pixel factor are blurred as one.
-              E0 = Am - 2.f * (Bv * mu1) - Cc * mu2; E1 = Bv; E2 = Cc;
+              for (int o = 0; o < 4; o++)
+                if (k - o >= 0 && k - o < 11) { mean[o] = __ffma2_rn(gauss.w[k - o], v, mean[o]); square[o] = __ffma2_rn(gauss.w[k - o], vv, square[o]); }
             }
           }
-          const int slot = slots[HALO + o];
-          s_dv[0][slot][col] = E0; s_dv[1][slot][col] = E1; s_dv[2][slot][col] = E2;
+          MomentRow* row = r == 0 ? row_a : row_b;
+          float4 *dm = reinterpret_cast<float4*>(row->mean), *dq = reinterpret_cast<float4*>(row->square);
+          const int c0 = chunk_at(g4 / 2), c1 = chunk_at(g4 / 2 + 1);
+          dm[c0] = make_float4(mean[0].x, mean[0].y, mean[1].x, mean[1].y); dm[c1] = make_float4(mean[2].x, mean[2].y, mean[3].x, mean[3].y);
+          dq[c0] = make_float4(square[0].x, square[0].y, square[1].x, square[1].y); dq[c1] = make_float4(square[2].x, square[2].y, square[3].x, square[3].y);
+        }
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          cross[o] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int k = 0; k < 11; k++) cross[o] = __ffma2_rn(gauss.w[k], cross_in[o + k], cross[o]);
+        }
+        *reinterpret_cast<float4*>(&row_a->cross[g4]) = make_float4(cross[0].x, cross[1].x, cross[2].x, cross[3].x);
+        *reinterpret_cast<float4*>(&row_b->cross[g4]) = make_float4(cross[0].y, cross[1].y, cross[2].y, cross[3].y);
+      }
+    } else if (warp < 3) {
+      // B: statistics rows b .. b+3; a thread takes one column.
+      if (b + STRIP_ROWS - 1 >= y0 - HALO && b <= y1 - 1 + HALO) {
+        const int col = (warp - 1) * 32 + lane, at = pair_at(col);
+        const MomentRow* row = sh.moments + ring_slot(b - HALO);
+        float2 mean[4], square[4];   // (prediction, target)
+        float cross[4];
+#pragma unroll
+        for (int o = 0; o < 4; o++) { mean[o] = square[o] = make_float2(0.f, 0.f); cross[o] = 0.f; }
+#pragma unroll
+        for (int k = 0; k < 14; k++) {
+          const float2 m2 = row->mean[at], q2 = row->square[at];
+          const float x = row->cross[col];
+          row = ring_next(row, const_cast<const MomentRow*>(sh.moments));
+#pragma unroll
+          for (int o = 0; o < 4; o++)
+            if (k - o >= 0 && k - o < 11) {
+              mean[o] = __ffma2_rn(gauss.w[k - o], m2, mean[o]); square[o] = __ffma2_rn(gauss.w[k - o], q2, square[o]);
+              cross[o] = fmaf(gauss.w[k - o].x, x, cross[o]);
+            }
+        }
+        const int xg = x0 - HALO + col;
+        const bool col_in = xg >= 0 && xg < W, col_own = xg >= x0 && xg < x_end;
+        MapRow* out = sh.maps + ring_slot(b);
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          // Outside the image the weight is zero; the expressions below stay finite there (both images are zero).
+          const int y = b + o;
+          const bool in = col_in && y >= 0 && y < H;
+          float M = in ? norm * lp.ssim_w : 0.f;
+          if constexpr (MASKED) {
+            if (in) {
+              const size_t q = (size_t)y * W + xg;
+              if (weights) M *= (float)weights[q] * (1.f / 255.f);
+              if (lp.mask) M *= byte_unit(gt[q], 3);
+            }
+          }
+          const float mu1 = mean[o].x, mu2 = mean[o].y, mu12 = mu1 * mu2;
+          const float2 mu_sq = __fmul2_rn(mean[o], mean[o]);
+          // The variances are small differences: one rounding each, not two.
+          const float2 raw_var = __ffma2_rn(make_float2(-mu1, -mu2), mean[o], square[o]);
+          const float s1_raw = raw_var.x, s2_raw = raw_var.y, sigma12 = fmaf(-mu1, mu2, cross[o]);
+          const float A1 = 2.f * mu12 + C1, A2 = 2.f * sigma12 + C2, B1 = mu_sq.x + mu_sq.y + C1, B2 = fmaxf(0.f, s1_raw) + fmaxf(0.f, s2_raw) + C2;
+          const float inv_BB = fast_rcp(B1 * B2);   // approximate division, as in the reference's fast-math build
+          const float raw = A1 * A2 * inv_BB;
+          const float ssim = fminf(fmaxf(raw, -1.f), 1.f);
+          if (col_own && y >= y0 && y < y1) loss_local += M * ssim;
+          const float k = raw > -1.f && raw < 1.f ? M : 0.f;   // the clamp has zero slope
+          const float d_mu1 = 2.f * inv_BB * (mu2 * A2 - mu1 * ssim * B2);
+          const float d_s1 = s1_raw > 0.f ? -ssim * (inv_BB * B1) : 0.f;
+          const float Bv = k * d_s1, Cc = k * (2.f * A1 * inv_BB);
+          // gradient = blur(Am) + 2 p blur(Bv) - 2 blur(Bv mu1) + target blur(Cc) - blur(Cc mu2): the three maps
+          // without a per-pixel factor are blurred as one.
+          out->e12[at] = make_float2(Bv, Cc);
+          out->e0[col] = k * d_mu1 - 2.f * (Bv * mu1) - Cc * mu2;
+          out = ring_next(out, sh.maps);
+        }
+      }
+    } else if (warp == 3) {
+      // C: rows cr .. cr+3 of the derivative maps blurred down the column, two columns per thread.
+      if (cr + STRIP_ROWS - 1 >= y0 && cr < y1) {
+        const int col = lane * 2, chunk = chunk_at(lane);
+        const MapRow* row = sh.maps + ring_slot(cr - HALO);
+        float2 b12[4][2], b0[4];
+#pragma unroll
+        for (int o = 0; o < 4; o++) b12[o][0] = b12[o][1] = b0[o] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 14; k++) {
+          const float4 e4 = reinterpret_cast<const float4*>(row->e12)[chunk];
+          const float2 z2 = *reinterpret_cast<const float2*>(&row->e0[col]);
+          row = ring_next(row, const_cast<const MapRow*>(sh.maps));
+#pragma unroll
+          for (int o = 0; o < 4; o++)
+            if (k - o >= 0 && k - o < 11) {
+              const float2 w = gauss.w[k - o];
+              b12[o][0] = __ffma2_rn(w, lo2(e4), b12[o][0]); b12[o][1] = __ffma2_rn(w, hi2(e4), b12[o][1]); b0[o] = __ffma2_rn(w, z2, b0[o]);
+            }
+        }
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          reinterpret_cast<float4*>(sh.b12[buf][o])[chunk] = make_float4(b12[o][0].x, b12[o][0].y, b12[o][1].x, b12[o][1].y);
+          *reinterpret_cast<float2*>(&sh.b0[buf][o][col]) = b0[o];
         }
       }
     } else {
-      const int t = tid - 192;   // 0 .. 127
-      if (warp < 8) {
-        // C: rows cr .. cr+3 of the three derivative maps blurred down the column, one column per thread.
-        if (cr + STRIP_ROWS - 1 >= y0 && cr < y1) {
-          const int col = t;
-          int slot = ring_slot(cr - HALO);
-          int slots[14];
+      // D: rows d .. d+3 (stage C wrote them in the step before), fourteen groups of four output columns.
+      const int row = (warp - 4) * 2 + (lane >> 4), g4 = (lane & 15) * 4, y = d + row;
+      if (g4 < STRIP_W && y >= y0 && y < y1) {
+        float2 b12[4];
+        float b0[4];
 #pragma unroll
-          for (int k = 0; k < 14; k++) { slots[k] = slot; slot = slot + 1 == RING ? 0 : slot + 1; }
+        for (int o = 0; o < 4; o++) { b12[o] = make_float2(0.f, 0.f); b0[o] = 0.f; }
+        const float4* s12 = reinterpret_cast<const float4*>(sh.b12[buf ^ 1][row]);
+        const float4* s0 = reinterpret_cast<const float4*>(&sh.b0[buf ^ 1][row][g4]);
 #pragma unroll
-          for (int m = 0; m < 3; m++) {
-            float in[16], out[4];
+        for (int k2 = 0; k2 < 7; k2++) {
+          const float4 v4 = s12[chunk_at(g4 / 2 + k2)];
 #pragma unroll
-            for (int k = 0; k < 14; k++) in[k] = s_dv[m][slots[k]][col];
-            in[14] = in[15] = 0.f;
-            window4(in, gauss, out);
+          for (int h = 0; h < 2; h++)
 #pragma unroll
-            for (int o = 0; o < 4; o++) s_bv[buf][m][o][col] = out[o];
-          }
+            for (int o = 0; o < 4; o++) { const int k = k2 * 2 + h - o; if (k >= 0 && k < 11) b12[o] = __ffma2_rn(gauss.w[k], h ? hi2(v4) : lo2(v4), b12[o]); }
         }
-      } else {
-        // D: rows d .. d+3 (stage C wrote them in the step before), fourteen groups of four output columns.
-        const int u = t - 64, row = u >> 4, g4 = (u & 15) * 4;
-        const int y = d + row;
-        if (g4 < STRIP_W && y >= y0 && y < y1) {
-          float bl[3][4];
 #pragma unroll
-          for (int m = 0; m < 3; m++) {
-            float in[16];
-            load16(&s_bv[buf ^ 1][m][row][g4], in);
-            window4(in, gauss, bl[m]);
-          }
+        for (int k4 = 0; k4 < 4; k4++) {
+          const float4 v4 = s0[k4];
+          const float v[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-          for (int o = 0; o < 4; o++) {
-            const int x = x0 + g4 + o;
-            if (x < x_end) {
+          for (int h = 0; h < 4; h++)
+#pragma unroll
+            for (int o = 0; o < 4; o++) { const int k = k4 * 4 + h - o; if (k >= 0 && k < 11) b0[o] = fmaf(gauss.w[k].x, v[h], b0[o]); }
+        }
+        const float4* own_row = reinterpret_cast<const float4*>(sh.px[y & (PX_RING - 1)]);
+        const float4 own[2] = {own_row[chunk_at(g4 / 2)], own_row[chunk_at(g4 / 2 + 1)]};
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          const int x = x0 + g4 + o;
+          if (x < x_end) {
+            const float2 pg = o & 1 ? hi2(own[o >> 1]) : lo2(own[o >> 1]);
+            float M = norm * lp.l1_w;
+            if constexpr (MASKED) {
               const size_t q = (size_t)y * W + x;
-              const uint32_t gp = gt[q];
-              const float ga = unpack(gp, 3);
-              const float wp = weights ? (float)weights[q] * (1.f / 255.f) : 1.f;
-              const float M = wp * (lp.mask ? ga : 1.f) * norm;
-              float p, pa = 0.f;
-              if (c == 0) { const float4 pv = pred[q]; p = pv.x; pa = pv.w; } else p = pred_c[q * 4];
-              const float g = unpack(gp, c) + (1.f - ga) * bg_c;
-              const float sgn = p > g ? 1.f : (p < g ? -1.f : 0.f);
-              loss_local += M * lp.l1_w * fabsf(p - g);
-              out_c[q * 4] = (M * lp.l1_w * sgn + bl[0][o] + 2.f * p * bl[1][o] + g * bl[2][o]) * lp.grad_scale;
-              if (c == 0) {   // the alpha lane travels with the first channel
-                float ga_grad = 0.f;
-                if (lp.alpha_lane) {
-                  const float da = pa - ga;
-                  const float sa = da > 0.f ? 1.f : (da < 0.f ? -1.f : 0.f);
-                  const float Ma = wp * alpha_norm;
-                  ga_grad = Ma * sa * lp.grad_scale;
-                  loss_local += Ma * fabsf(da);
-                }
-                out_c[q * 4 + 3] = ga_grad;
+              const float wp = weights ? (float)weights[q] * (1.f / 255.f) : 1.f, ga = byte_unit(gt[q], 3);
+              M *= wp * (lp.mask ? ga : 1.f);
+              if (c == 0 && lp.alpha_lane) {   // the alpha lane travels with the first channel
+                const float da = pred[q].w - ga, Ma = wp * alpha_norm;
+                all.out[buf][row][g4 + o][3] = (da > 0.f ? Ma : (da < 0.f ? -Ma : 0.f)) * lp.grad_scale;
+                loss_local += Ma * fabsf(da);
               }
             }
+            const float diff = pg.x - pg.y;
+            loss_local += M * fabsf(diff);
+            const float l1 = diff > 0.f ? M : (diff < 0.f ? -M : 0.f);
+            all.out[buf][row][g4 + o][c] = (l1 + b0[o] + 2.f * pg.x * b12[o].x + pg.y * b12[o].y) * lp.grad_scale;
           }
         }
       }
     }
-    if (more && st_slot) { (&s_in[buf ^ 1][0][0][0])[tid] = nx; (&s_in[buf ^ 1][1][0][0])[tid] = ny; }   // consumed by stage A in the next step
+    {
+      // The gradient rows that stage D left in the step before.
+      const int row = tid / PX_S, col = tid - row * PX_S, y = d - STRIP_ROWS + row, x = x0 + col;
+      if (row < STRIP_ROWS && col < STRIP_W && x < x_end && y >= y0 && y < y1) v_out[(size_t)y * W + x] = *reinterpret_cast<const float4*>(all.out[buf ^ 1][row][col]);
+    }
+    if (more) store(buf ^ 1, a + STRIP_ROWS);   // consumed by stage A in the next step
     __syncthreads();
   }
   const float s = warp_sum(loss_local);
-  if ((tid & 31) == 0) s_red[warp] = s;
+  if (lane == 0) all.red[tid >> 5] = s;
   __syncthreads();
   if (tid == 0) {
     float t = 0.f;
-    for (int i = 0; i < STRIP_THREADS / 32; i++) t += s_red[i];
+    for (int i = 0; i < STRIP_THREADS / 32; i++) t += all.red[i];
     if (t != 0.f) atomicAdd(loss_accum, t);
   }
 }
@@ -394,16 +474,27 @@ extern "C" int b2k_loss_photometric(const B2kCtx* c, const B2kLoss* lp, b2k_stre
   a.composite = lp->composite; a.mask = lp->mask; a.alpha_lane = lp->alpha_lane;
   a.match_alpha_weight = lp->match_alpha_weight; a.scale = lp->scale; a.grad_scale = lp->grad_scale;
   static const Gauss g = make_gauss();
+  Gauss2 g2;
+  for (int i = 0; i < 11; i++) g2.w[i] = make_float2(g.w[i], g.w[i]);
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !attr_set[dev]) {
+    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare)));
+    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare)));
+    attr_set[dev] = true;
+  }
   // Rows per segment: as many segments as fill the resident CTA slots once (a second, partial wave costs more than the
   // eight pipeline-fill steps a longer segment amortises), in whole steps of four rows.
   const int strips = div_up(c->W, STRIP_W), slots = sm_count() * STRIP_CTAS_PER_SM;
-  int segs = slots / (strips * 3);
+  int segs = slots / strips;
   segs = segs < 1 ? 1 : segs;
   int seg_rows = div_up(div_up(c->H, segs), STRIP_ROWS) * STRIP_ROWS;
-  if (seg_rows < 32) seg_rows = 32;
-  const dim3 grid(strips, div_up(c->H, seg_rows), 3);
-  photometric_strip_kernel<<<grid, STRIP_THREADS, 0, (cudaStream_t)stream>>>((const float4*)c->out_rgba, lp->rgba, lp->weights, c->W, c->H, seg_rows, a, g,
-                                                                            (float4*)c->v_out, c->loss_accum);
+  if (seg_rows < 8) seg_rows = 8;
+  const dim3 grid(strips, div_up(c->H, seg_rows));
+#define L(MASKED) photometric_strip_kernel<MASKED><<<grid, STRIP_THREADS, sizeof(StripShare), (cudaStream_t)stream>>>((const float4*)c->out_rgba, lp->rgba, lp->weights, c->W, c->H, \
+    seg_rows, a, g2, (float4*)c->v_out, c->loss_accum)
+  if (lp->weights || lp->mask || lp->alpha_lane) L(true); else L(false);
+#undef L
   return check_launch();
 }
 

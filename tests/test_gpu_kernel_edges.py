@@ -125,3 +125,24 @@ def test_depth_sort_is_stable_at_every_size(n, kind):
     wide = keys.to(torch.int64) & 0xFFFFFFFF
     want = torch.argsort(wide, stable=True)
     assert torch.equal(ctx.order.to(torch.int64), want) and torch.equal(ctx.depth_keys_sorted.to(torch.int64) & 0xFFFFFFFF, wide[want])
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("W,H", [(1, 1), (8, 5), (53, 4), (54, 9), (55, 12), (108, 3), (163, 37), (16100, 21)])   # one strip, its edge, many; segments of 8 rows and of the whole image
+def test_loss_strips(W, H, masked):
+    scene, cam = stack_scene(4, W, H)
+    rng = np.random.Generator(np.random.PCG64(W * 64 + H))
+    gt = rng.integers(0, 2 ** 32, W * H, dtype=np.uint64).astype(np.uint32)
+    wts = rng.integers(64, 256, W * H).astype(np.uint8) if masked else None
+    lp = dict(l1_w=0.8, ssim_w=-0.2, bg=(0.2, 0.1, 0.3), composite=not masked, mask=masked, alpha_lane=masked, match_alpha_weight=0.3, scale=1.7, grad_scale=1.0)
+    pred = rng.random((W * H, 4)).astype(np.float32)
+    h = Harness(scene, cam, gt, wts, lp)
+    h.ctx.out_rgba.copy_(h.torch.from_numpy(pred))
+    h.ctx.loss_accum.zero_(); h.ctx.v_out.fill_(1e9)
+    h.api.photometric_loss(h.ctx, h.view, h.lp)
+    f32 = {k: (np.float32(v) if isinstance(v, float) else v) for k, v in lp.items()}
+    f32["bg"] = tuple(np.float32(x) for x in lp["bg"])
+    want, v_out = orc.loss(W, H, pred, gt, wts, f32)
+    assert abs(float(h.ctx.loss_accum[0].item()) - want) <= 2e-5 * abs(want)
+    v = h.ctx.v_out.cpu().numpy()
+    assert rel_l2(v, v_out) <= 2e-4 and np.max(np.abs(v - v_out)) <= 2e-3 * np.max(np.abs(v_out))
