@@ -26,6 +26,7 @@ constexpr int MAX_CHUNKS = 5;
 // V = number of depth-sorted keys that are not the culled marker (they sort last); every tile is alive.
 __global__ void __launch_bounds__(256) chunk_prepare_kernel(const uint32_t* __restrict__ keys_sorted, int n, uint32_t* __restrict__ words, unsigned long long* __restrict__ alive,
                                                             int bins) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < bins) alive[i] = ~0ull;
   if (i >= 32) return;
@@ -126,7 +127,7 @@ extern "C" int b2k_render_chunked(const B2kModel* m, const B2kCamera* cam, const
   st = depth_sort(c, n, true, tables, s);
   if (st) return st;
   const int bins = div_up(c->tiles_x, 8) * div_up(c->tiles_y, 8);
-  chunk_prepare_kernel<<<div_up(bins, 256), 256, 0, s>>>(c->depth_keys_sorted, n, words, alive, bins);
+  launch_next(chunk_prepare_kernel, div_up(bins, 256), 256, 0, s, c->depth_keys_sorted, n, words, alive, bins);
   for (int ch = 0; ch < C; ch++) {
     const int lo = ch == 0 ? 0 : 256 >> (2 * (C - ch)), hi = 256 >> (2 * (C - 1 - ch));
     st = launch_bins(c, n, words, ch, lo, hi, ch == 0 ? nullptr : alive, tables, s);   // the first chunk meets only live tiles

@@ -219,6 +219,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uin
 constexpr int COUNT_THREADS = 512;
 template <bool WHOLE>
 __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g, Tables t, uint32_t* __restrict__ live) {
+  after_previous();
   extern __shared__ __align__(16) unsigned long long s_alive[];   // [bins], then [bins] counts
   const int bins = band_bins(g), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_alive + (WHOLE ? 0 : bins));
@@ -269,6 +270,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
 // and the items (runs of pairs of one bin) that level 2 works on. An item is 256 pairs unless that made too many.
 constexpr int ROWS_THREADS = 512, ROWS_BINS = ROWS_THREADS / 32, ROWS_PER = 16;   // at most 32 * ROWS_PER blocks of level 1
 __global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int bins, uint32_t cap, Tables t) {
+  after_previous();
   __shared__ uint32_t s_warp[32];
   __shared__ bool s_last;
   const int tid = threadIdx.x, lane = tid & 31, bin = blockIdx.x * ROWS_BINS + (tid >> 5);
@@ -324,6 +326,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int 
 template <bool WHOLE>
 __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ live, uint32_t* __restrict__ pairs,
                                                                  uint32_t* __restrict__ tile_off) {
+  after_previous();
   extern __shared__ __align__(16) uint32_t s_bits[];   // [bins][8], then [bins] alive words, then [bins] next free place
   const int bins = band_bins(g), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long* s_alive = reinterpret_cast<unsigned long long*>(s_bits + (size_t)bins * L1_WARPS);
@@ -424,6 +427,7 @@ __device__ __forceinline__ Item item_of(const Tables& t, const Band& g, uint32_t
 template <bool WHOLE>
 __global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ pairs, uint32_t* __restrict__ hit_lo,
                                                                 uint32_t* __restrict__ hit_hi) {
+  after_previous();
   struct WarpShare { float4 rec[64]; unsigned long long hits[32]; uint32_t unit[32 * BIN_W]; };   // unit: pair | row << 5 | columns << 8
   __shared__ WarpShare s_share[L2_WARPS];
   __shared__ uint32_t s_cnt[L2_WARPS][BIN_TILES];
@@ -504,6 +508,7 @@ __global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, 
 // four where there are bins enough to fill the GPU (74 -> 29 us over the five chunks of a 4K view).
 template <int COL_GROUPS>
 __global__ void __launch_bounds__(COL_GROUPS * BIN_TILES) item_columns_kernel(Band g, Tables t, uint2* __restrict__ ranges) {
+  after_previous();
   __shared__ uint32_t s_sum[COL_GROUPS][BIN_TILES];
   const int bin = blockIdx.x, tile = threadIdx.x % BIN_TILES, group = threadIdx.x / BIN_TILES;
   const uint32_t i0 = t.first_item[bin], i1 = t.first_item[bin + 1], per = (i1 - i0 + COL_GROUPS - 1) / COL_GROUPS;
@@ -530,6 +535,7 @@ __global__ void __launch_bounds__(COL_GROUPS * BIN_TILES) item_columns_kernel(Ba
 // Ranges of the band's tiles, row-major: block b starts behind the hits of the blocks before it. Empty tiles get (0, 0);
 // ranges end with the buffers. The last block to finish moves the view's slot on.
 __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, Tables t, uint32_t cap, uint2* __restrict__ ranges, uint32_t* __restrict__ num_isect) {
+  after_previous();
   __shared__ uint32_t s_warp[32];
   const int tid = threadIdx.x;
   const int tile0 = g.bin_row0 * BIN_W * g.tiles_x, tiles = (min((g.bin_row0 + g.bin_rows) * BIN_W, g.tiles_y) - g.bin_row0 * BIN_W) * g.tiles_x;
@@ -564,6 +570,7 @@ __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, T
 // word at a time, and the lanes with a hit write side by side.
 __global__ void __launch_bounds__(L2_THREADS) item_emit_kernel(Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ pairs, const uint32_t* __restrict__ hit_lo,
                                                                const uint32_t* __restrict__ hit_hi, const uint2* __restrict__ ranges, uint32_t* __restrict__ vals) {
+  after_previous();
   __shared__ uint32_t s_splat[L2_THREADS], s_word[L2_WARPS][BIN_TILES];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lane_lt = (1u << lane) - 1u, n_items = t.st[S_ITEMS];
@@ -602,6 +609,7 @@ __global__ void __launch_bounds__(L2_THREADS) item_emit_kernel(Band g, Tables t,
 
 // Tile ids of the sorted list, for callers of the whole-view binning: a warp per tile.
 __global__ void __launch_bounds__(256) fill_keys_kernel(int n_tiles, const uint2* __restrict__ ranges, uint32_t* __restrict__ keys) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   for (int tile = blockIdx.x * 8 + (threadIdx.x >> 5); tile < n_tiles; tile += gridDim.x * 8) {
     const uint2 r = ranges[tile];
@@ -645,22 +653,22 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
     const int tiles = (std::min((row + g.bin_rows) * BIN_W, c->tiles_y) - row * BIN_W) * c->tiles_x, scan_blocks = div_up(tiles, SCAN_TILES);
 #define L(WHOLE) do { \
     const size_t alive_bytes = WHOLE ? 0 : bins * sizeof(unsigned long long); \
-    bin_count_kernel<WHOLE><<<blocks, COUNT_THREADS, alive_bytes + bins * sizeof(uint32_t), s>>>(v, g, t, c->depth_keys); \
-    bin_rows_kernel<<<div_up(bins, ROWS_BINS), ROWS_THREADS, 0, s>>>(blocks, bins, cap, t); \
-    bin_scatter_kernel<WHOLE><<<blocks, L1_THREADS, alive_bytes + bins * (L1_WARPS + 1) * sizeof(uint32_t), s>>>(v, g, t, cap, c->depth_keys, c->keys, c->tile_off); \
-    item_count_kernel<WHOLE><<<item_blocks, L2_THREADS, 0, s>>>(v, g, t, cap, c->keys, c->vals, c->keys_sorted); } while (0)
+    launch_next(bin_count_kernel<WHOLE>, blocks, COUNT_THREADS, alive_bytes + bins * sizeof(uint32_t), s, v, g, t, c->depth_keys); \
+    launch_next(bin_rows_kernel, div_up(bins, ROWS_BINS), ROWS_THREADS, 0, s, blocks, bins, cap, t); \
+    launch_next(bin_scatter_kernel<WHOLE>, blocks, L1_THREADS, alive_bytes + bins * (L1_WARPS + 1) * sizeof(uint32_t), s, v, g, t, cap, c->depth_keys, c->keys, c->tile_off); \
+    launch_next(item_count_kernel<WHOLE>, item_blocks, L2_THREADS, 0, s, v, g, t, cap, c->keys, c->vals, c->keys_sorted); } while (0)
     if (words) L(false); else L(true);
 #undef L
-    if (bins >= 2 * sm_count()) item_columns_kernel<4><<<bins, 4 * BIN_TILES, 0, s>>>(g, t, ranges);
-    else item_columns_kernel<16><<<bins, 16 * BIN_TILES, 0, s>>>(g, t, ranges);
-    tile_scan_kernel<<<scan_blocks, SCAN_TILES, 0, s>>>(v, g, t, cap, ranges, c->num_isect);
-    item_emit_kernel<<<item_blocks, L2_THREADS, 0, s>>>(g, t, cap, c->keys, c->vals, c->keys_sorted, ranges, c->vals_sorted);
+    if (bins >= 2 * sm_count()) launch_next(item_columns_kernel<4>, bins, 4 * BIN_TILES, 0, s, g, t, ranges);
+    else launch_next(item_columns_kernel<16>, bins, 16 * BIN_TILES, 0, s, g, t, ranges);
+    launch_next(tile_scan_kernel, scan_blocks, SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect);
+    launch_next(item_emit_kernel, item_blocks, L2_THREADS, 0, s, g, t, cap, c->keys, c->vals, c->keys_sorted, ranges, c->vals_sorted);
   }
   return check_launch();
 }
 
 int launch_fill_keys(const B2kCtx* c, cudaStream_t s) {
-  fill_keys_kernel<<<std::min(div_up(c->n_tiles, 8), sm_count() * 8), 256, 0, s>>>(c->n_tiles, (const uint2*)c->tile_ranges, c->keys_sorted);
+  launch_next(fill_keys_kernel, std::min(div_up(c->n_tiles, 8), sm_count() * 8), 256, 0, s, c->n_tiles, (const uint2*)c->tile_ranges, c->keys_sorted);
   return check_launch();
 }
 

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(EV_WARPS * 32) evidence_kernel(
     const float4* __restrict__ out_rgba, const float4* __restrict__ out_feat, const uint32_t* __restrict__ last_idx, const uint32_t* __restrict__ gt,
     const uint32_t* __restrict__ gtn, const uint8_t* __restrict__ weights, int W, int H, int tiles_x, int n_tiles, int n_chunks, int masked_has_alpha,
     float normal_weight, float* __restrict__ acc) {
+  after_previous();
   __shared__ float4 s0[EV_WARPS][EV_BATCH], s1[EV_WARPS][EV_BATCH];
   __shared__ uint32_t s_gid[EV_WARPS][EV_BATCH];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(EV_WARPS * 32) evidence_kernel(
 
 // ev[i] += this view's (w_in, w_all, err), w_in^2 and the mass-weighted direction to the camera (evidence.cu:123-136).
 __global__ void evidence_fold_kernel(int n, const float* __restrict__ acc, const float4* __restrict__ pos, float3 cam, float* __restrict__ ev) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float w_in = acc[i * 3], err = acc[i * 3 + 1], w_all = acc[i * 3 + 2];
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(EV_WARPS * 32) label_vote_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const uint32_t* __restrict__ last_idx, const uint32_t* __restrict__ gt, const uint8_t* __restrict__ labels, const uint8_t* __restrict__ weights, int W, int H,
     int tiles_x, int n_tiles, int n_chunks, int masked_has_alpha, float* __restrict__ votes) {
+  after_previous();
   __shared__ float4 s0[EV_WARPS][EV_BATCH], s1[EV_WARPS][EV_BATCH];
   __shared__ uint32_t s_gid[EV_WARPS][EV_BATCH];
   __shared__ float s_votes[EV_WARPS][EV_BATCH][LABEL_BINS];
@@ -189,7 +192,7 @@ extern "C" int b2k_evidence_view(const B2kCtx* c, const uint32_t* rgba, const ui
   B2K_REQUIRE(!use_normals || c->out_feat);
   const int chunks = c->n_chunks > 1 ? c->n_chunks : 1;
   if (use_normals && chunks > 1) return B2K_ERR_UNSUPPORTED;   // a chunked view has no composited feature lanes
-#define L(N) evidence_kernel<N><<<div_up(c->n_tiles, EV_WARPS), EV_WARPS * 32, 0, (cudaStream_t)stream>>>( \
+#define L(N) launch_next(evidence_kernel<N>, div_up(c->n_tiles, EV_WARPS), EV_WARPS * 32, 0, (cudaStream_t)stream,  \
       (const uint2*)c->tile_ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, (const float4*)c->out_rgba, (const float4*)c->out_feat, c->last_idx, \
       rgba, normals, weights, c->W, c->H, c->tiles_x, c->n_tiles, chunks, masked_has_alpha, normal_weight, acc)
   if (use_normals) L(true); else L(false);
@@ -200,7 +203,7 @@ extern "C" int b2k_evidence_view(const B2kCtx* c, const uint32_t* rgba, const ui
 extern "C" int b2k_evidence_fold(const B2kModel* m, const float* acc, const float* cam_pos, float* evidence, b2k_stream_t stream) {
   B2K_REQUIRE(m && m->pos_op && acc && cam_pos && evidence && m->n >= 0);
   if (m->n == 0) return B2K_OK;
-  evidence_fold_kernel<<<div_up(m->n, 256), 256, 0, (cudaStream_t)stream>>>(m->n, acc, (const float4*)m->pos_op, make_float3(cam_pos[0], cam_pos[1], cam_pos[2]), evidence);
+  launch_next(evidence_fold_kernel, div_up(m->n, 256), 256, 0, (cudaStream_t)stream, m->n, acc, (const float4*)m->pos_op, make_float3(cam_pos[0], cam_pos[1], cam_pos[2]), evidence);
   return check_launch();
 }
 
@@ -210,7 +213,7 @@ extern "C" int b2k_label_vote(const B2kCtx* c, const uint32_t* rgba, const uint8
   if (st) return st;
   B2K_REQUIRE(rgba && labels && votes);
   const int chunks = c->n_chunks > 1 ? c->n_chunks : 1;
-  label_vote_kernel<<<div_up(c->n_tiles, EV_WARPS), EV_WARPS * 32, 0, (cudaStream_t)stream>>>(
+  launch_next(label_vote_kernel, div_up(c->n_tiles, EV_WARPS), EV_WARPS * 32, 0, (cudaStream_t)stream, 
       (const uint2*)c->tile_ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, c->last_idx, rgba, labels, weights, c->W, c->H, c->tiles_x, c->n_tiles,
       chunks, masked_has_alpha, votes);
   return check_launch();

@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(STRIP_THREADS, STRIP_CTAS_PER_SM) photometric_
   const float alpha_norm = lp.match_alpha_weight * lp.scale / ((float)W * (float)H);
 
   for (int i = tid; i < (int)(sizeof(StripShare) / 16); i += STRIP_THREADS) reinterpret_cast<float4*>(s_bytes)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  after_previous();
   __syncthreads();
   // The input pixel a thread fetches (zero outside the image and in the row pad): which one, and whether its column is inside
   // the image, does not change from step to step.
@@ -372,6 +373,7 @@ constexpr int EV_S = 28;                     // row stride of the footprint plan
 
 __global__ void __launch_bounds__(TILE_PX) eval_kernel(const float4* __restrict__ pred, const uint32_t* __restrict__ gt, int W, int H, int tiles_x, int mask_w,
                                                        Gauss gauss, float* __restrict__ accum) {
+  after_previous();
   __shared__ __align__(16) float s_q[3][EV_W * EV_S];          // quantised prediction per channel
   __shared__ __align__(16) float s_t[3][EV_W * EV_S];          // target per channel
   __shared__ __align__(16) float s_row[5][EV_W][LOSS_TILE];    // horizontally blurred moments of the current channel
@@ -456,11 +458,12 @@ __global__ void __launch_bounds__(TILE_PX) eval_kernel(const float4* __restrict_
 // Running loss sum and view count; also keeps the largest intersection total any view of the step produced, so that
 // one readback per step (instead of one per view) tells the host whether a view overflowed its buffers.
 __global__ void accumulate_kernel(float* a, uint32_t* num_isect) {
+  after_previous();
   a[2] += a[0] + a[1]; a[3] += 1.f;
   if (num_isect) num_isect[2] = max(num_isect[2], num_isect[0]);
 }
 // dst[2] += src[2], dst[3] += src[3]: folds the running loss of a second context (a view in flight on another stream).
-__global__ void fold_loss_kernel(float* dst, const float* src) { dst[2] += src[2]; dst[3] += src[3]; }
+__global__ void fold_loss_kernel(float* dst, const float* src) { after_previous(); dst[2] += src[2]; dst[3] += src[3]; }
 
 }  // namespace
 }  // namespace b2k
@@ -491,7 +494,7 @@ extern "C" int b2k_loss_photometric(const B2kCtx* c, const B2kLoss* lp, b2k_stre
   int seg_rows = div_up(div_up(c->H, segs), STRIP_ROWS) * STRIP_ROWS;
   if (seg_rows < 8) seg_rows = 8;
   const dim3 grid(strips, div_up(c->H, seg_rows));
-#define L(MASKED) photometric_strip_kernel<MASKED><<<grid, STRIP_THREADS, sizeof(StripShare), (cudaStream_t)stream>>>((const float4*)c->out_rgba, lp->rgba, lp->weights, c->W, c->H, \
+#define L(MASKED) launch_next(photometric_strip_kernel<MASKED>, grid, STRIP_THREADS, sizeof(StripShare), (cudaStream_t)stream, (const float4*)c->out_rgba, lp->rgba, lp->weights, c->W, c->H, \
     seg_rows, a, g2, (float4*)c->v_out, c->loss_accum)
   if (lp->weights || lp->mask || lp->alpha_lane) L(true); else L(false);
 #undef L
@@ -500,26 +503,25 @@ extern "C" int b2k_loss_photometric(const B2kCtx* c, const B2kLoss* lp, b2k_stre
 
 extern "C" int b2k_loss_accumulate(const B2kCtx* c, b2k_stream_t stream) {
   B2K_REQUIRE(c && c->loss_accum);
-  accumulate_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(c->loss_accum, c->num_isect);
+  launch_next(accumulate_kernel, 1, 1, 0, (cudaStream_t)stream, c->loss_accum, c->num_isect);
   return check_launch();
 }
 
 extern "C" int b2k_loss_zero(const B2kCtx* c, int32_t first, int32_t count, b2k_stream_t stream) {
   B2K_REQUIRE(c && c->loss_accum && first >= 0 && count >= 0 && first + count <= 16);
-  if (count) B2K_CUDA(cudaMemsetAsync(c->loss_accum + first, 0, (size_t)count * sizeof(float), (cudaStream_t)stream));
-  return B2K_OK;
+  if (count) launch_clear(c->loss_accum + first, count, nullptr, 0, (cudaStream_t)stream);
+  return check_launch();
 }
 
 extern "C" int b2k_step_begin(const B2kCtx* c, b2k_stream_t stream) {
   B2K_REQUIRE(c && c->loss_accum);
-  B2K_CUDA(cudaMemsetAsync(c->loss_accum, 0, 16 * sizeof(float), (cudaStream_t)stream));
-  if (c->num_isect) B2K_CUDA(cudaMemsetAsync(c->num_isect + 2, 0, sizeof(uint32_t), (cudaStream_t)stream));
-  return B2K_OK;
+  launch_clear(c->loss_accum, 16, c->num_isect ? c->num_isect + 2 : nullptr, c->num_isect ? 1 : 0, (cudaStream_t)stream);
+  return check_launch();
 }
 
 extern "C" int b2k_loss_fold(const B2kCtx* dst, const B2kCtx* src, b2k_stream_t stream) {
   B2K_REQUIRE(dst && src && dst->loss_accum && src->loss_accum && dst->loss_accum != src->loss_accum);
-  fold_loss_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(dst->loss_accum, src->loss_accum);
+  launch_next(fold_loss_kernel, 1, 1, 0, (cudaStream_t)stream, dst->loss_accum, src->loss_accum);
   return check_launch();
 }
 
@@ -527,6 +529,6 @@ extern "C" int b2k_eval_metrics(const B2kCtx* c, const uint32_t* rgba, int32_t m
   B2K_REQUIRE(c && rgba && c->out_rgba && c->loss_accum && c->W > 0 && c->H > 0);
   const int tiles_x = div_up(c->W, LOSS_TILE), tiles = tiles_x * div_up(c->H, LOSS_TILE);
   static const Gauss g = make_gauss();
-  eval_kernel<<<tiles, TILE_PX, 0, (cudaStream_t)stream>>>((const float4*)c->out_rgba, rgba, c->W, c->H, tiles_x, mask_weighted, g, c->loss_accum);
+  launch_next(eval_kernel, tiles, TILE_PX, 0, (cudaStream_t)stream, (const float4*)c->out_rgba, rgba, c->W, c->H, tiles_x, mask_weighted, g, c->loss_accum);
   return check_launch();
 }

@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
     float4* __restrict__ proj0, float4* __restrict__ proj1, float4* __restrict__ proj2, uint32_t* __restrict__ tile_count,
     uint4* __restrict__ hit_info, uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in, float* __restrict__ max_screen,
     uint32_t* __restrict__ big_list, uint32_t* __restrict__ big_count, int feat_mode, const float* __restrict__ feat_in, float2* __restrict__ proj3) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 po = pos_op[i], q = quat[i], ls = lscale[i];
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_lite_kernel(
     float4* __restrict__ proj0, float4* __restrict__ proj1, float4* __restrict__ proj2, uint32_t* __restrict__ tile_count, uint4* __restrict__ hit_info,
     uint32_t* __restrict__ depth_keys, float* __restrict__ max_screen, int feat_mode, const float* __restrict__ feat_in,
     float2* __restrict__ proj3) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 po = pos_op[i], q = quat[i], ls = lscale[i];
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_lite_kernel(
 __global__ void __launch_bounds__(256) count_big_kernel(const uint32_t* __restrict__ big_list, const uint32_t* __restrict__ big_count,
                                                         const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H, int tiles_x,
                                                         int tiles_y, uint32_t* __restrict__ tile_count, uint32_t* __restrict__ depth_keys) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5), count = *big_count;
   for (uint32_t e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); e < count; e += warps) {
@@ -205,6 +208,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
                                                                  int tiles_x, int tiles_y, uint32_t* __restrict__ tile_count, uint4* __restrict__ hit_info,
                                                                  uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in,
                                                                  uint32_t* __restrict__ big_list, uint32_t* __restrict__ big_count) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 a = proj0[i], b = proj1[i];
@@ -234,6 +238,13 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
   if (!big) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
 }
 
+// A few words to zero. (A memset node would break the chain of overlapped launches on both sides.)
+__global__ void clear_kernel(uint32_t* a, int words_a, uint32_t* b, int words_b) {
+  after_previous();
+  for (int i = threadIdx.x; i < words_a; i += 32) a[i] = 0u;
+  for (int i = threadIdx.x; i < words_b; i += 32) b[i] = 0u;
+}
+
 template <int DEG>
 int launch(const B2kModel* m, const CamDev& cam, const B2kRenderOpts* o, const B2kCtx* c, cudaStream_t s) {
   const float4* pos = (const float4*)(o->pos_override ? o->pos_override : m->pos_op);
@@ -242,17 +253,19 @@ int launch(const B2kModel* m, const CamDev& cam, const B2kRenderOpts* o, const B
   const int active = o->sh_degree < m->degree ? o->sh_degree : m->degree;
   uint32_t* big_count = big_count_ptr(c);
   uint32_t* big_list = big_list_ptr(c);
-  if (cudaMemsetAsync(big_count, 0, sizeof(uint32_t), s) != cudaSuccess) return check_launch();
-  project_kernel<DEG><<<div_up(m->n, PROJ_BLOCK), PROJ_BLOCK, 0, s>>>(
+  launch_clear(big_count, 1, nullptr, 0, s);
+  launch_next(project_kernel<DEG>, div_up(m->n, PROJ_BLOCK), PROJ_BLOCK, 0, s, 
       m->n, (size_t)m->cap, pos, quat, lscale, m->sh_dc, m->sh_hi, cam, active < 0 ? 0 : active, c->tiles_x, c->tiles_y,
       (float4*)c->proj0, (float4*)c->proj1, (float4*)c->proj2, c->tile_count, (uint4*)c->hit_info, c->depth_keys_sorted, c->order, m->max_screen,
       big_list, big_count, o->feat_mode, o->feat_buffer, (float2*)c->proj3);
-  count_big_kernel<<<sm_count() * 8, 256, 0, s>>>(big_list, big_count, (const float4*)c->proj0, (const float4*)c->proj1, cam.W, cam.H, c->tiles_x,
+  launch_next(count_big_kernel, sm_count() * 8, 256, 0, s, big_list, big_count, (const float4*)c->proj0, (const float4*)c->proj1, cam.W, cam.H, c->tiles_x,
                                                   c->tiles_y, c->tile_count, c->depth_keys_sorted);
   return check_launch();
 }
 
 }  // namespace
+
+void launch_clear(void* a, int words_a, void* b, int words_b, cudaStream_t s) { launch_next(clear_kernel, 1, 32, 0, s, (uint32_t*)a, words_a, (uint32_t*)b, words_b); }
 
 int launch_project_lite(const B2kModel* m, const B2kCamera* cam, const B2kRenderOpts* o, const B2kCtx* c, cudaStream_t s) {
   const float4* pos = (const float4*)(o->pos_override ? o->pos_override : m->pos_op);
@@ -260,7 +273,7 @@ int launch_project_lite(const B2kModel* m, const B2kCamera* cam, const B2kRender
   const float4* lscale = (const float4*)(o->lscale_override ? o->lscale_override : m->lscale);
   const int active = o->sh_degree < m->degree ? (o->sh_degree < 0 ? 0 : o->sh_degree) : m->degree;
   const CamDev cd = to_camdev(*cam);
-#define L(D) project_lite_kernel<D><<<div_up(m->n, PROJ_BLOCK), PROJ_BLOCK, 0, s>>>(m->n, (size_t)m->cap, pos, quat, lscale, m->sh_dc, m->sh_hi, active, cd, \
+#define L(D) launch_next(project_lite_kernel<D>, div_up(m->n, PROJ_BLOCK), PROJ_BLOCK, 0, s, m->n, (size_t)m->cap, pos, quat, lscale, m->sh_dc, m->sh_hi, active, cd, \
       c->tiles_x, c->tiles_y, (float4*)c->proj0, (float4*)c->proj1, (float4*)c->proj2, c->tile_count, (uint4*)c->hit_info, c->depth_keys_sorted, m->max_screen, \
       o->feat_mode, o->feat_buffer, (float2*)c->proj3)
   switch (m->degree) { case 0: L(0); break; case 1: L(1); break; case 2: L(2); break; case 3: L(3); break; default: L(4); break; }
@@ -301,10 +314,10 @@ extern "C" int b2k_count_tiles(const B2kCtx* c, int32_t n, b2k_stream_t stream) 
   cudaStream_t s = (cudaStream_t)stream;
   uint32_t* big_count = big_count_ptr(c);
   uint32_t* big_list = big_list_ptr(c);
-  B2K_CUDA(cudaMemsetAsync(big_count, 0, sizeof(uint32_t), s));
-  count_tiles_kernel<<<div_up(n, 256), 256, 0, s>>>(n, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y, c->tile_count,
+  launch_clear(big_count, 1, nullptr, 0, s);
+  launch_next(count_tiles_kernel, div_up(n, 256), 256, 0, s, n, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y, c->tile_count,
                                                    (uint4*)c->hit_info, c->depth_keys_sorted, c->order, big_list, big_count);
-  count_big_kernel<<<sm_count() * 8, 256, 0, s>>>(big_list, big_count, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y,
+  launch_next(count_big_kernel, sm_count() * 8, 256, 0, s, big_list, big_count, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y,
                                                   c->tile_count, c->depth_keys_sorted);
   return check_launch();
 }

@@ -79,6 +79,7 @@ __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z,
 // Work list of the replay: one item (range index = chunk * n_tiles + tile, segment) per segment of every
 // non-empty range the forward left. Order is irrelevant (items are independent); work[0] receives the count.
 __global__ void __launch_bounds__(256) bwd_items_kernel(const uint2* __restrict__ tile_ranges, int n_ranges, int seg_shift, uint2* __restrict__ items, uint32_t* __restrict__ work) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   for (int q0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; q0 < n_ranges; q0 += gridDim.x * blockDim.x) {
     const int q = q0 + lane;
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(256) bwd_items_kernel(const uint2* __restrict_
 // slot 0 those of the last one; afterwards slot j holds the colour from boundary j on.
 __global__ void __launch_bounds__(128) bwd_suffix_kernel(const uint2* __restrict__ tile_ranges, int n_tiles, int n_chunks, int seg_shift, uint2* __restrict__ items,
                                                          uint32_t* __restrict__ work, float4* __restrict__ ckpt) {
+  after_previous();
   const int lane = threadIdx.x & 31, tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (tile >= n_tiles) return;
   float3 acc[2] = {make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
@@ -148,6 +150,7 @@ __global__ void __launch_bounds__(BWD_WARPS * 32, BWD_CTAS_PER_SM) raster_bwd_ke
     const float4* __restrict__ v_out, int W, int H, int tiles_x, int n_tiles, float3 bg, float* __restrict__ v_splat, uint32_t* __restrict__ vis_flag,
     float* __restrict__ vis_weight, int n_chunks, const uint2* __restrict__ items, uint32_t* __restrict__ work, const float4* __restrict__ ckpt,
     int seg_shift, float out_scale) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char s_bytes[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpMem& sm = reinterpret_cast<WarpMem*>(s_bytes)[warp];
@@ -419,12 +422,12 @@ extern "C" int b2k_raster_bwd_scaled(const B2kCtx* c, const B2kModel* m, const B
   const int chunks = c->n_chunks > 1 ? c->n_chunks : 1;
   uint32_t* work = bwd_work_ptr(c);
   uint2* items = bwd_items_ptr(c);
-  B2K_CUDA(cudaMemsetAsync(work, 0, 2 * sizeof(uint32_t), s));
+  launch_clear(work, 2, nullptr, 0, s);
   const int n_ranges = chunks * c->n_tiles;
   const int seg_shift = seg_shift_of(c->n_tiles);
   const bool brief = short_segments(c->n_tiles);
-  if (brief) bwd_suffix_kernel<<<div_up(c->n_tiles, 4), 128, 0, s>>>((const uint2*)c->tile_ranges, c->n_tiles, chunks, seg_shift, items, work, bwd_ckpt_ptr(c));
-  else bwd_items_kernel<<<min(div_up(n_ranges, 256), sm_count() * 4), 256, 0, s>>>((const uint2*)c->tile_ranges, n_ranges, seg_shift, items, work);
+  if (brief) launch_next(bwd_suffix_kernel, div_up(c->n_tiles, 4), 128, 0, s, (const uint2*)c->tile_ranges, c->n_tiles, chunks, seg_shift, items, work, bwd_ckpt_ptr(c));
+  else launch_next(bwd_items_kernel, min(div_up(n_ranges, 256), sm_count() * 4), 256, 0, s, (const uint2*)c->tile_ranges, n_ranges, seg_shift, items, work);
   // Persistent grid: as many CTAs as an SM holds.
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -435,7 +438,7 @@ extern "C" int b2k_raster_bwd_scaled(const B2kCtx* c, const B2kModel* m, const B
     attr_set[dev] = true;
   }
   const int ctas = sm_count() * BWD_CTAS_PER_SM;
-#define L(CH) raster_bwd_kernel<CH><<<ctas, BWD_WARPS * 32, BWD_SMEM, s>>>( \
+#define L(CH) launch_next(raster_bwd_kernel<CH>, ctas, BWD_WARPS * 32, BWD_SMEM, s,  \
       (const uint2*)c->tile_ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, (const float4*)c->proj2, (const float4*)c->out_rgba, \
       (const float4*)c->out_feat, c->last_idx, (const float4*)c->v_out, c->W, c->H, c->tiles_x, c->n_tiles, bg, c->v_splat, c->vis_flag, m->vis_weight, chunks, \
       items, work, bwd_ckpt_ptr(c), seg_shift, 1.f / grad_scale)

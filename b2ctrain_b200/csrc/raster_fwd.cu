@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
     const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc) {
+  after_previous();
   constexpr bool BWD = CKPT != NONE;
   // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
   // pixel travel in feat_acc and move into out_feat.xyz when the last chunk, which then visits every pixel, is done.
@@ -211,7 +212,7 @@ namespace b2k {
 int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_chunks, unsigned long long* alive, cudaStream_t s) {
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
   uint2* ranges = (uint2*)c->tile_ranges + (n_chunks > 1 ? (size_t)chunk * c->n_tiles : 0);
-#define L(B, D, C, F) raster_fwd_kernel<B, D, C, F><<<div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, s>>>(ranges, c->vals_sorted, (const float4*)c->proj0, \
+#define L(B, D, C, F) launch_next(raster_fwd_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, \
     (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, \
     chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(c->n_tiles), (n_chunks > 1 && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr)
 #define LB(B) do { if (n_chunks > 1) { if (c->out_depth) L(B, true, true, false); else L(B, false, true, false); } \

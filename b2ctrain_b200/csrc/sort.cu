@@ -48,7 +48,7 @@ constexpr size_t small_smem(int items) { return (size_t)SMALL_THREADS * items * 
 // A warp owns a contiguous run of 32 * ITEMS pairs, held in registers from one pass to the write of the next; pair j * 32 + l
 // of the run is lane l's j-th.
 template <int ITEMS>
-__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* keys_out, uint32_t* vals_out) {   // may work in place
+__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* keys_out, uint32_t* vals_out) { after_previous();   // may work in place
   extern __shared__ __align__(16) uint32_t s_mem[];
   uint32_t* s_key = s_mem;
   uint32_t* s_val = s_key + SMALL_THREADS * ITEMS;
@@ -127,6 +127,7 @@ struct Range { uint32_t lo[MAX_BLOCKS], hi[MAX_BLOCKS]; Digits digits; };   // p
 __device__ __forceinline__ uint32_t run_of(uint32_t n, uint32_t blocks, uint32_t tile) { return ((n + blocks - 1) / blocks + tile - 1) / tile * tile; }
 
 __global__ void __launch_bounds__(CNT_THREADS) key_range_kernel(const uint32_t* __restrict__ keys, uint32_t n, Range* __restrict__ range) {
+  after_previous();
   __shared__ uint32_t s_lo[CNT_THREADS / 32], s_hi[CNT_THREADS / 32];
   uint32_t lo = CULLED, hi = 0u;
   auto see = [&](uint32_t k) { if (k != CULLED) { lo = min(lo, k); hi = max(hi, k); } };
@@ -173,6 +174,7 @@ __device__ __forceinline__ uint32_t digit_at(uint32_t key, const Digits& d, int 
 template <bool COMPRESS>
 __global__ void __launch_bounds__(CNT_THREADS) digit_count_kernel(const uint32_t* __restrict__ keys, uint32_t n, uint32_t tile, int pass, int passes, Range* __restrict__ range,
                                                                   int range_blocks, uint32_t* __restrict__ table) {
+  after_previous();
   __shared__ uint32_t s_hist[MAX_RADIX];
   const Digits d = load_digits<COMPRESS>(range, range_blocks, passes, pass == 0);
   const uint32_t radix = 1u << d.width, copies = min((uint32_t)(CNT_THREADS / 32), MAX_RADIX / radix);
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(CNT_THREADS) digit_count_kernel(const uint32_t
 constexpr int ROW_WARPS = 16;
 template <bool COMPRESS>
 __global__ void __launch_bounds__(ROW_WARPS * 32) digit_rows_kernel(uint32_t* __restrict__ table, int blocks, Range* __restrict__ range, uint32_t* __restrict__ totals) {
+  after_previous();
   const Digits d = load_digits<COMPRESS>(range, 0, 0, false);
   const int g = blockIdx.x * ROW_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (g >= 1 << d.width) return;
@@ -226,6 +229,7 @@ template <bool COMPRESS, int MOST, int SCAT_THREADS, int ITEMS>
 __global__ void __launch_bounds__(SCAT_THREADS, 2) digit_scatter_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
                                                                         uint32_t* __restrict__ vals_out, uint32_t n, int pass, Range* __restrict__ range,
                                                                         const uint32_t* __restrict__ table, const uint32_t* __restrict__ totals) {
+  after_previous();
   constexpr int SCAT_WARPS = SCAT_THREADS / 32, PER = MOST > SCAT_THREADS ? MOST / SCAT_THREADS : 1;
   constexpr uint32_t TILE = SCAT_THREADS * ITEMS;
   extern __shared__ __align__(16) uint32_t s_mem[];
@@ -360,14 +364,14 @@ int scatter(const uint32_t* ki, const uint32_t* vi, uint32_t* ko, uint32_t* vo, 
     B2K_CUDA(cudaFuncSetAttribute(digit_scatter_kernel<COMPRESS, MOST, THREADS, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[dev] = true;
   }
-  digit_scatter_kernel<COMPRESS, MOST, THREADS, ITEMS><<<blocks, THREADS, smem, s>>>(ki, vi, ko, vo, n, pass, range, table, totals);
+  launch_next(digit_scatter_kernel<COMPRESS, MOST, THREADS, ITEMS>, blocks, THREADS, smem, s, ki, vi, ko, vo, n, pass, range, table, totals);
   return check_launch();
 }
 template <bool COMPRESS, int MOST>
 int one_pass(const Shape& sh, const uint32_t* ki, const uint32_t* vi, uint32_t* ko, uint32_t* vo, uint32_t n, int pass, int passes, Range* range, int range_blocks, uint32_t* table,
              uint32_t* totals, cudaStream_t s) {
-  digit_count_kernel<COMPRESS><<<sh.blocks, CNT_THREADS, 0, s>>>(ki, n, (uint32_t)sh.tile, pass, passes, range, range_blocks, table);
-  digit_rows_kernel<COMPRESS><<<MOST / ROW_WARPS, ROW_WARPS * 32, 0, s>>>(table, sh.blocks, range, totals);
+  launch_next(digit_count_kernel<COMPRESS>, sh.blocks, CNT_THREADS, 0, s, ki, n, (uint32_t)sh.tile, pass, passes, range, range_blocks, table);
+  launch_next(digit_rows_kernel<COMPRESS>, MOST / ROW_WARPS, ROW_WARPS * 32, 0, s, table, sh.blocks, range, totals);
   switch (sh.tile) {
     case LARGE_TILE: return scatter<COMPRESS, MOST, 512, 8>(ki, vi, ko, vo, n, sh.blocks, pass, range, table, totals, s);
     case MIDDLE_TILE: return scatter<COMPRESS, MOST, 256, 8>(ki, vi, ko, vo, n, sh.blocks, pass, range, table, totals, s);
@@ -383,7 +387,7 @@ int small_sort(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* ko, 
     B2K_CUDA(cudaFuncSetAttribute(small_sort_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(ITEMS)));
     attr_set[dev] = true;
   }
-  small_sort_kernel<ITEMS><<<1, SMALL_THREADS, small_smem(ITEMS), s>>>(keys, vals, n, ko, vo);
+  launch_next(small_sort_kernel<ITEMS>, 1, SMALL_THREADS, small_smem(ITEMS), s, keys, vals, n, ko, vo);
   return check_launch();
 }
 
@@ -400,7 +404,7 @@ int depth_sort(const B2kCtx* c, int n, bool identity, uint32_t* tables, cudaStre
   static_assert(MAX_RADIX + sizeof(Range) / sizeof(uint32_t) <= BINS_EXTRA_WORDS, "scratch");
   const Shape sh = shape_of((uint32_t)n);
   const int range_blocks = std::min<int>(std::min(2 * sm_count(), MAX_BLOCKS), div_up(n, CNT_THREADS * 16));
-  key_range_kernel<<<range_blocks, CNT_THREADS, 0, s>>>(in, (uint32_t)n, range);
+  launch_next(key_range_kernel, range_blocks, CNT_THREADS, 0, s, in, (uint32_t)n, range);
   // Three passes by way of two scratch pairs (the second: tile_off and the projection's list, both free here).
   uint32_t* list = big_list_ptr(c);
   const uint32_t* ki[3] = {in, c->depth_keys, c->tile_off};
