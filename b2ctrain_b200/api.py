@@ -12,6 +12,8 @@ GPU raises.
 """
 import ctypes as C
 import os
+import struct as _st
+from operator import attrgetter, itemgetter
 
 import numpy as np
 import torch
@@ -67,6 +69,27 @@ class B2kOptim(C.Structure):
                 ("lr_sh_rest", C.c_float), ("noise_weight", C.c_float), ("noise_clamp", C.c_float), ("seed", C.c_uint32),
                 ("step", C.c_uint32), ("sparse", C.c_int32), ("pos_override", C.c_void_p), ("quat_override", C.c_void_p),
                 ("lscale_override", C.c_void_p), ("grad_out", C.c_void_p), ("touched_out", C.c_void_p)]
+
+
+# The records above are filled with one native-layout pack each (assigning field by field cost 2 to 7 us a record, as much as
+# the launches of a small step; packing takes about a third). Pads follow the C layout; the assertions hold the two together.
+_CAMERA_PACK, _OPTS_PACK = _st.Struct("19f2i4f"), _st.Struct("3f2i4x3Pi4xP")
+_MODEL_PACK, _LOSS_PACK = _st.Struct("3i4x%dP" % len(_MODEL_PTRS)), _st.Struct("2P5f3i3f4x")
+_OPTIM_PACK = _st.Struct("2i11f2Ii5P")
+_CTX_PACK = _st.Struct("7i4x14PQ2PQ10Pi4x3PQ")
+for _record, _pack in ((B2kCamera, _CAMERA_PACK), (B2kRenderOpts, _OPTS_PACK), (B2kModel, _MODEL_PACK), (B2kLoss, _LOSS_PACK), (B2kOptim, _OPTIM_PACK),
+                       (B2kCtx, _CTX_PACK)):
+    assert C.sizeof(_record) == _pack.size, _record
+
+
+def _floats(a, n):
+    """The first n entries of a list or an array, as what a pack accepts."""
+    a = a.tolist() if hasattr(a, "tolist") else a
+    return a if len(a) == n else [a[i] for i in range(n)]
+
+
+def _addr(t):
+    return 0 if t is None else t.data_ptr()
 
 
 # Every entry point include/b2k.h declares, with its argument types (the symbol-table test walks this list).
@@ -172,18 +195,14 @@ def _ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+_CAMERA_HEAD, _CAMERA_SIZE = itemgetter("fx", "fy", "cx", "cy"), itemgetter("W", "H")
+_CAMERA_LIMITS = itemgetter("lim_pos_x", "lim_pos_y", "lim_neg_x", "lim_neg_y")
+
+
 def camera_from(cam):
     """CameraGPU record from a camera dict of b2ctrain_b200.scenes (CameraGPU::from, src/gpu/render.h:15-24)."""
-    s = B2kCamera()
-    for i in range(9):
-        s.R[i] = float(cam["R"][i])
-    for i in range(3):
-        s.t[i] = float(cam["t"][i])
-        s.pos[i] = float(cam["pos"][i])
-    for k in ("fx", "fy", "cx", "cy", "lim_pos_x", "lim_pos_y", "lim_neg_x", "lim_neg_y"):
-        setattr(s, k, float(cam[k]))
-    s.W, s.H = int(cam["W"]), int(cam["H"])
-    return s
+    return B2kCamera.from_buffer_copy(_CAMERA_PACK.pack(*_floats(cam["R"], 9), *_floats(cam["t"], 3), *_floats(cam["pos"], 3), *_CAMERA_HEAD(cam),
+                                                        *map(int, _CAMERA_SIZE(cam)), *_CAMERA_LIMITS(cam)))
 
 
 def _capacity_for(n):
@@ -193,7 +212,41 @@ def _capacity_for(n):
     return cap
 
 
-class Model:
+def _fields(obj, names, get):
+    """The named attributes of an object, None where it has none (yet)."""
+    try:
+        return get(obj)
+    except AttributeError:
+        return [getattr(obj, k, None) for k in names]
+
+
+_MODEL_GET = attrgetter(*_MODEL_PTRS)
+
+
+class _Recorded:
+    """An object whose C record is kept until one of its attributes is set or deleted: a step passes the same context to six
+    calls and the same model to four, and reading forty-seven tensors' addresses each time cost more than the launches of a
+    small step. Tensors are swapped by setting the attribute; one whose storage is exchanged in place (Tensor.set_,
+    Tensor.resize_) has to be set again."""
+    _kept = None
+
+    def __setattr__(self, name, value):
+        self.__dict__["_kept"] = None
+        self.__dict__[name] = value
+
+    def __delattr__(self, name):
+        self.__dict__["_kept"] = None
+        object.__delattr__(self, name)
+
+    def struct(self):
+        """A record of its own for the caller, who may change it."""
+        s = self._kept
+        if s is None:
+            s = self.__dict__["_kept"] = self._record()
+        return type(s).from_buffer_copy(s)
+
+
+class Model(_Recorded):
     """Device splat model: parameters, Adam moments and refine statistics (src/model.h:14-40). Capacity doubles from
     1024 (src/model.cu:10-11); SH is planar with stride `cap`."""
 
@@ -286,16 +339,18 @@ class Model:
         n, K = self.n, self.K()
         return torch.cat([dc, hi], 0)[:, :n].t().reshape(n, K, 3).contiguous().cpu().numpy()
 
-    def struct(self):
-        s = B2kModel()
-        s.n, s.cap, s.degree = self.n, self.cap, self.degree
-        for k in _MODEL_PTRS:
-            t = getattr(self, k, None)
-            setattr(s, k, None if t is None or t.numel() == 0 else t.data_ptr())
-        return s
+    def _record(self):
+        return B2kModel.from_buffer_copy(_MODEL_PACK.pack(self.n, self.cap, self.degree, *map(_addr, _fields(self, _MODEL_PTRS, _MODEL_GET))))
 
 
-class RenderCtx:
+# The pointers of a context in the order of its record (num_isect, which is d_num_isect here, goes between vals_sorted and sort_tmp).
+_CTX_PTRS = ("proj0", "proj1", "proj2", "tile_count", "hit_info", "depth_keys", "depth_keys_sorted", "order_in", "order", "tile_off", "keys", "vals",
+             "keys_sorted", "vals_sorted", "sort_tmp", "tile_ranges", "out_rgba", "out_feat", "out_depth", "last_idx", "v_splat", "vis_flag", "vis_list",
+             "v_out", "loss_accum", "proj3", "chunk_words", "bwd_scratch")
+_CTX_GET = attrgetter(*_CTX_PTRS)
+
+
+class RenderCtx(_Recorded):
     """Per-view scratch (src/gpu/render.h:66-95); member names follow the reference. `setup` sizes everything; the
     intersection buffers start at 2^22 entries (src/gpu/render.cu:20) and double on overflow."""
 
@@ -355,21 +410,11 @@ class RenderCtx:
         self.bwd_scratch = torch.zeros(int(lib().b2k_bwd_scratch_bytes(self.W, self.H, self.n_chunks, self.isect_cap)), dtype=torch.uint8,
                                        device=self.device)
 
-    def struct(self):
-        s = B2kCtx()
-        for k in ("W", "H", "tiles_x", "tiles_y", "n_tiles", "tile_bits", "n_cap"):
-            setattr(s, k, getattr(self, k))
-        for k in ("proj0", "proj1", "proj2", "tile_count", "hit_info", "depth_keys", "depth_keys_sorted", "order_in", "order", "tile_off", "keys",
-                  "vals", "keys_sorted", "vals_sorted", "sort_tmp", "tile_ranges", "out_rgba", "out_feat", "out_depth", "last_idx",
-                  "v_splat", "vis_flag", "vis_list", "v_out", "loss_accum", "chunk_words", "proj3", "bwd_scratch"):
-            t = getattr(self, k, None)
-            setattr(s, k, None if t is None else t.data_ptr())
-        s.num_isect = self.d_num_isect.data_ptr()
-        s.isect_cap = self.isect_cap
-        s.sort_tmp_bytes = self.sort_tmp.numel()
-        s.bwd_scratch_bytes = self.bwd_scratch.numel()
-        s.n_chunks = self.n_chunks
-        return s
+    def _record(self):
+        p = [0 if t is None else t.data_ptr() for t in _fields(self, _CTX_PTRS, _CTX_GET)]
+        return B2kCtx.from_buffer_copy(_CTX_PACK.pack(
+            self.W, self.H, self.tiles_x, self.tiles_y, self.n_tiles, self.tile_bits, self.n_cap, *p[:14], self.isect_cap, self.d_num_isect.data_ptr(), p[14],
+            self.sort_tmp.numel(), *p[15:25], self.n_chunks, *p[25:], self.bwd_scratch.numel()))
 
 
 class RenderParams:
@@ -392,13 +437,9 @@ class RenderParams:
             raise RuntimeError("RenderParams: mip / warp / sh_frame / app / hollow lanes are not implemented (unsupported lane)")
         if self.feat not in self._FEAT or (self.feat == "Buffer") != (self.feat_buffer is not None):
             raise RuntimeError("RenderParams: feat is None, Normals or Buffer, and feat_buffer goes with Buffer")
-        s = B2kRenderOpts()
-        s.feat_mode, s.feat_buffer = self._FEAT[self.feat], _ptr(self.feat_buffer)
-        for i in range(3):
-            s.bg[i] = float(self.bg[i])
-        s.sh_degree, s.bwd_info = int(self.sh_degree), int(bool(self.bwd_info))
-        s.pos_override, s.quat_override, s.lscale_override = _ptr(self.pos_override), _ptr(self.quat_override), _ptr(self.lscale_override)
-        return s
+        return B2kRenderOpts.from_buffer_copy(_OPTS_PACK.pack(
+            *_floats(self.bg, 3), int(self.sh_degree), bool(self.bwd_info), _addr(self.pos_override), _addr(self.quat_override), _addr(self.lscale_override),
+            self._FEAT[self.feat], _addr(self.feat_buffer)))
 
     def camera(self):
         return self.cam if isinstance(self.cam, B2kCamera) else camera_from(self.cam)
@@ -428,14 +469,9 @@ class LossParams:
     def struct(self, view):
         if self.normal_scale != 0.0:
             raise RuntimeError("LossParams: the normal-supervision lane is not implemented (unsupported lane)")
-        s = B2kLoss()
-        s.rgba, s.weights = _ptr(view.rgba), _ptr(view.weights)
-        s.l1_w, s.ssim_w = self.l1_w, self.ssim_w
-        for i in range(3):
-            s.bg[i] = float(self.bg[i])
-        s.composite, s.mask, s.alpha_lane = int(self.composite), int(self.mask), int(self.alpha_lane)
-        s.match_alpha_weight, s.scale, s.grad_scale = self.match_alpha_weight, self.scale, self.grad_scale
-        return s
+        return B2kLoss.from_buffer_copy(_LOSS_PACK.pack(
+            _addr(view.rgba), _addr(view.weights), self.l1_w, self.ssim_w, *_floats(self.bg, 3), int(self.composite), int(self.mask), int(self.alpha_lane),
+            self.match_alpha_weight, self.scale, self.grad_scale))
 
 
 class OptimParams:
@@ -467,15 +503,10 @@ class OptimParams:
     def struct(self):
         if self.mip or self.frozen or any(getattr(self, k) is not None for k in self._UNSUPPORTED):
             raise RuntimeError("OptimParams: cage / deformation / sparsification lanes are not implemented (unsupported lane)")
-        s = B2kOptim()
-        for k in ("active_sh_degree", "t", "beta1", "beta2", "eps", "lr_mean", "lr_rot", "lr_scale", "lr_opac", "lr_dc", "lr_sh_rest",
-                  "noise_weight", "noise_clamp", "seed", "step"):
-            setattr(s, k, getattr(self, k))
-        s.sparse = int(bool(self.sparse))
-        s.pos_override, s.quat_override, s.lscale_override = _ptr(self.pos_override), _ptr(self.quat_override), _ptr(self.lscale_override)
-        s.grad_out = _ptr(self.grad_out)
-        s.touched_out = _ptr(self.touched_out)
-        return s
+        return B2kOptim.from_buffer_copy(_OPTIM_PACK.pack(
+            self.active_sh_degree, self.t, self.beta1, self.beta2, self.eps, self.lr_mean, self.lr_rot, self.lr_scale, self.lr_opac, self.lr_dc, self.lr_sh_rest,
+            self.noise_weight, self.noise_clamp, self.seed & 0xFFFFFFFF, self.step & 0xFFFFFFFF, bool(self.sparse), _addr(self.pos_override),
+            _addr(self.quat_override), _addr(self.lscale_override), _addr(self.grad_out), _addr(self.touched_out)))
 
     def camera(self):
         return self.cam if isinstance(self.cam, B2kCamera) else camera_from(self.cam)
@@ -497,22 +528,27 @@ def count_tiles(ctx, m, stream=None):
 def bin_and_sort(ctx, m, stream=None, sync=True):
     """With sync=True behaves like the reference (binning.cu:125-133): reads the intersection total back, and when it
     exceeds the buffers grows them by doubling and redoes the binning. sync=False leaves the total on the device."""
-    cs = ctx.struct()
-    _check(lib().b2k_bin_sort(C.byref(cs), m.n, _stream(stream)), "bin_and_sort")
+    _bin_and_sort(ctx, m, ctx.struct(), _stream(stream), sync)
+
+
+def _bin_and_sort(ctx, m, cs, stream, sync):
+    """bin_and_sort over the context's record; returns the record, which is another one when the buffers grew."""
+    _check(lib().b2k_bin_sort(C.byref(cs), m.n, stream), "bin_and_sort")
     if not sync:
-        return
+        return cs
     total = C.c_uint32(0)
-    st = lib().b2k_read_num_isect(C.byref(cs), _stream(stream), C.byref(total))
+    st = lib().b2k_read_num_isect(C.byref(cs), stream, C.byref(total))
     if st == B2K_ERR_OVERFLOW:
         cap = ctx.isect_cap
         while cap < total.value:
             cap *= 2
         ctx._alloc_isect(cap)
         cs = ctx.struct()
-        _check(lib().b2k_bin_sort(C.byref(cs), m.n, _stream(stream)), "bin_and_sort")
-        st = lib().b2k_read_num_isect(C.byref(cs), _stream(stream), C.byref(total))
+        _check(lib().b2k_bin_sort(C.byref(cs), m.n, stream), "bin_and_sort")
+        st = lib().b2k_read_num_isect(C.byref(cs), stream, C.byref(total))
     _check(st, "bin_and_sort")
     ctx.num_isect = int(total.value)
+    return cs
 
 
 def bin_and_sort_profile(ctx, m, stream=None):
@@ -534,9 +570,10 @@ def render_forward(ctx, m, p, stream=None, sync=True):
     (b2k_render_chunked: same image and gradients, intersections behind saturated pixels never sorted)."""
     if ctx.n_chunks > 1:
         return render_chunked(ctx, m, p, stream, sync=sync)
-    project_splats(ctx, m, p, stream)
-    bin_and_sort(ctx, m, stream, sync=sync)
-    rasterize_forward(ctx, p, stream)
+    cs, ms, os_, cam, st = ctx.struct(), m.struct(), p.struct(), p.camera(), _stream(stream)
+    _check(lib().b2k_project(C.byref(ms), C.byref(cam), C.byref(os_), C.byref(cs), st), "project_splats")
+    cs = _bin_and_sort(ctx, m, cs, st, sync)
+    _check(lib().b2k_raster_fwd(C.byref(cs), C.byref(os_), st), "rasterize_forward")
 
 
 def render_chunked(ctx, m, p, stream=None, sync=True):
