@@ -63,8 +63,8 @@ __device__ __forceinline__ void load16(const float* p, float (&v)[16]) {
 // (fp32x2) with operands that lie in pairs as they are stored: prediction and target side by side, and so their means, their
 // squares, and the two maps with a per-pixel factor; the product moment and the third map are paired over two rows (A) or two
 // columns (C). A thread makes four or eight outputs from one window, so that a value read from shared memory feeds eleven to
-// forty-four multiply-adds. Measured against the same pipeline with scalar multiply-adds and a CTA per channel: 187 -> 125 us on
-// a 1920x1080 view, 101 -> 95 us on a masked 1024x1024 one, 26 -> 21 us on 333x217. Other arrangements on 1920x1080: packed,
+// forty-four multiply-adds. Measured against the same pipeline with scalar multiply-adds and a CTA per channel: 187 -> 129 us on
+// a 1920x1080 view, 101 -> 96 us on a masked 1024x1024 one, 26 -> 21 us on 333x217. Other arrangements on 1920x1080: packed,
 // a CTA per channel 133 to 147; channels of one CTA with a barrier each 130; the pairs in plain order (two-way bank conflicts in
 // stages A and D) 139; two columns per thread in stage B 142.
 constexpr int STRIP_W = 54;                   // output columns of a strip
@@ -232,36 +232,50 @@ __global__ void __launch_bounds__(STRIP_THREADS, STRIP_CTAS_PER_SM) photometric_
         const bool col_in = xg >= 0 && xg < W, col_own = xg >= x0 && xg < x_end;
         MapRow* out = sh.maps + ring_slot(b);
 #pragma unroll
-        for (int o = 0; o < 4; o++) {
+        for (int o = 0; o < 4; o += 2) {   // two rows to a packed operation
           // Outside the image the weight is zero; the expressions below stay finite there (both images are zero).
           const int y = b + o;
-          const bool in = col_in && y >= 0 && y < H;
-          float M = in ? norm * lp.ssim_w : 0.f;
-          if constexpr (MASKED) {
-            if (in) {
-              const size_t q = (size_t)y * W + xg;
-              if (weights) M *= (float)weights[q] * (1.f / 255.f);
-              if (lp.mask) M *= byte_unit(gt[q], 3);
+          bool in[2], own[2];
+          float2 M;
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            in[u] = col_in && y + u >= 0 && y + u < H; own[u] = col_own && y + u >= y0 && y + u < y1;
+            float m = in[u] ? norm * lp.ssim_w : 0.f;
+            if constexpr (MASKED) {
+              if (in[u]) {
+                const size_t q = (size_t)(y + u) * W + xg;
+                if (weights) m *= (float)weights[q] * (1.f / 255.f);
+                if (lp.mask) m *= byte_unit(gt[q], 3);
+              }
             }
+            (u ? M.y : M.x) = m;
           }
-          const float mu1 = mean[o].x, mu2 = mean[o].y, mu12 = mu1 * mu2;
-          const float2 mu_sq = __fmul2_rn(mean[o], mean[o]);
-          // The variances are small differences: one rounding each, not two.
-          const float2 raw_var = __ffma2_rn(make_float2(-mu1, -mu2), mean[o], square[o]);
-          const float s1_raw = raw_var.x, s2_raw = raw_var.y, sigma12 = fmaf(-mu1, mu2, cross[o]);
-          const float A1 = 2.f * mu12 + C1, A2 = 2.f * sigma12 + C2, B1 = mu_sq.x + mu_sq.y + C1, B2 = fmaxf(0.f, s1_raw) + fmaxf(0.f, s2_raw) + C2;
-          const float inv_BB = fast_rcp(B1 * B2);   // approximate division, as in the reference's fast-math build
-          const float raw = A1 * A2 * inv_BB;
-          const float ssim = fminf(fmaxf(raw, -1.f), 1.f);
-          if (col_own && y >= y0 && y < y1) loss_local += M * ssim;
-          const float k = raw > -1.f && raw < 1.f ? M : 0.f;   // the clamp has zero slope
-          const float d_mu1 = 2.f * inv_BB * (mu2 * A2 - mu1 * ssim * B2);
-          const float d_s1 = s1_raw > 0.f ? -ssim * (inv_BB * B1) : 0.f;
-          const float Bv = k * d_s1, Cc = k * (2.f * A1 * inv_BB);
+          const float2 mu1 = make_float2(mean[o].x, mean[o + 1].x), mu2 = make_float2(mean[o].y, mean[o + 1].y), mu1_sq = __fmul2_rn(mu1, mu1), two = make_float2(2.f, 2.f);
+          const float2 neg1 = make_float2(-mu1.x, -mu1.y), neg2 = make_float2(-mu2.x, -mu2.y), dbl1 = __fadd2_rn(mu1, mu1), dbl2 = __fadd2_rn(mu2, mu2);
+          const float2 c1 = make_float2(C1, C1), c2 = make_float2(C2, C2);
+          // The expressions round as they always have (where a product is fused into a sum matters here: variances are small
+          // differences, and so is the gradient below).
+          const float2 s1_raw = __ffma2_rn(make_float2(-1.f, -1.f), mu1_sq, make_float2(square[o].x, square[o + 1].x));
+          const float2 s2_raw = __ffma2_rn(neg2, mu2, make_float2(square[o].y, square[o + 1].y));
+          const float2 sigma12 = __ffma2_rn(neg1, mu2, make_float2(cross[o], cross[o + 1]));
+          const float2 A1 = __ffma2_rn(dbl1, mu2, c1), A2 = __ffma2_rn(two, sigma12, c2), B1 = __fadd2_rn(__ffma2_rn(mu2, mu2, mu1_sq), c1);
+          const float2 B2 = __fadd2_rn(__fadd2_rn(make_float2(fmaxf(0.f, s1_raw.x), fmaxf(0.f, s1_raw.y)), make_float2(fmaxf(0.f, s2_raw.x), fmaxf(0.f, s2_raw.y))), c2);
+          const float2 BB = __fmul2_rn(B1, B2);
+          // approximate divisions, as in the reference's fast-math build
+          const float2 inv_BB = make_float2(fast_rcp(BB.x), fast_rcp(BB.y)), inv_B1 = make_float2(fast_rcp(B1.x), fast_rcp(B1.y)), inv_B2 = make_float2(fast_rcp(B2.x), fast_rcp(B2.y));
+          const float2 raw = __fmul2_rn(__fmul2_rn(A1, A2), inv_BB);
+          const float2 ssim = make_float2(fminf(fmaxf(raw.x, -1.f), 1.f), fminf(fmaxf(raw.y, -1.f), 1.f));
+          loss_local += (own[0] ? M.x * ssim.x : 0.f) + (own[1] ? M.y * ssim.y : 0.f);
+          const float2 k = make_float2(raw.x > -1.f && raw.x < 1.f ? M.x : 0.f, raw.y > -1.f && raw.y < 1.f ? M.y : 0.f);   // the clamp has zero slope
+          const float2 held = __fmul2_rn(__fmul2_rn(dbl1, ssim), inv_B1), d_mu1 = __ffma2_rn(__fmul2_rn(dbl2, A2), inv_BB, make_float2(-held.x, -held.y));
+          const float2 share = __fmul2_rn(ssim, inv_B2), d_s1 = make_float2(s1_raw.x > 0.f ? -share.x : 0.f, s1_raw.y > 0.f ? -share.y : 0.f);
+          const float2 Bv = __fmul2_rn(k, d_s1), Cc = __fmul2_rn(k, __fmul2_rn(__fadd2_rn(A1, A1), inv_BB)), pull = __fmul2_rn(Bv, mu1);
           // gradient = blur(Am) + 2 p blur(Bv) - 2 blur(Bv mu1) + target blur(Cc) - blur(Cc mu2): the three maps
           // without a per-pixel factor are blurred as one.
-          out->e12[at] = make_float2(Bv, Cc);
-          out->e0[col] = k * d_mu1 - 2.f * (Bv * mu1) - Cc * mu2;
+          const float2 e0 = __ffma2_rn(Cc, neg2, __ffma2_rn(k, d_mu1, __fmul2_rn(make_float2(-2.f, -2.f), pull)));
+          out->e12[at] = make_float2(Bv.x, Cc.x); out->e0[col] = e0.x;
+          out = ring_next(out, sh.maps);
+          out->e12[at] = make_float2(Bv.y, Cc.y); out->e0[col] = e0.y;
           out = ring_next(out, sh.maps);
         }
       }
