@@ -146,3 +146,25 @@ def test_loss_strips(W, H, masked):
     assert abs(float(h.ctx.loss_accum[0].item()) - want) <= 2e-5 * abs(want)
     v = h.ctx.v_out.cpu().numpy()
     assert rel_l2(v, v_out) <= 2e-4 and np.max(np.abs(v - v_out)) <= 2e-3 * np.max(np.abs(v_out))
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 31, 32, 33, 100])
+def test_forward_groups_and_colours_that_are_not_finite(n):
+    W = H = 64
+    scene, cam = stack_scene(n, W, H)
+    scene["pos_op"][:, 3] = -1.0
+    h = Harness(scene, cam, bg=(0.2, 0.1, 0.3), want_depth=True)
+    h.forward()
+    p0, p1, p2 = (t[:n].cpu().numpy().astype(np.float64) for t in (h.ctx.proj0, h.ctx.proj1, h.ctx.proj2))
+    vals, ranges = h.u32(h.ctx.vals_sorted, h.ctx.num_isect), h.u32(h.ctx.tile_ranges).reshape(-1, 2)
+    want = orc.raster_fwd(W, H, np.concatenate([p0, p1], 1), p2[:, :3], vals, ranges, np.array((0.2, 0.1, 0.3)), want_depth=True)
+    assert rel_l2(h.ctx.out_rgba.cpu().numpy(), want[0]) <= 1e-6
+    # An infinite colour shows in the pixels that see the splat and nowhere else.
+    images = []
+    for colour in (0.0, 1.0, float("inf")):
+        h.ctx.proj2[n // 2, 0] = colour
+        h.api.rasterize_forward(h.ctx, h.rp)
+        images.append(h.ctx.out_rgba.cpu().numpy())
+    sees = images[0][:, 0] != images[1][:, 0]
+    assert sees.any() and np.all(np.isposinf(images[2][sees, 0])) and np.array_equal(images[2][~sees], images[0][~sees])
+    assert np.array_equal(images[2][:, 1:], images[0][:, 1:])
