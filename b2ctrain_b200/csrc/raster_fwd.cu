@@ -1,23 +1,29 @@
-// Forward compositing: one warp per 8x8 tile walks the tile's depth-ordered fragment list front to back, each lane
-// carrying two horizontally adjacent pixels. Reference semantics: raster_fwd_kernel (src/gpu/raster_fwd.cu:9-71); the
-// optional expected-depth output follows the mean-depth mode of probe_kernel (src/gpu/probe.cu:30-46).
+// Forward compositing: each 8x8 tile's depth-ordered fragment list is walked front to back. Reference semantics:
+// raster_fwd_kernel (src/gpu/raster_fwd.cu:9-71); the optional expected-depth output follows the mean-depth mode of
+// probe_kernel (src/gpu/probe.cu:30-46).
 //
 // Bound by instruction issue where tiles fill the GPU and by the latency of one list where they do not; memory traffic is the
-// gather of 48 B per staged fragment, served mostly by L2. Fragments are gathered one batch of 32 ahead and staged per warp in
-// shared memory; warps never synchronise with each other. A lane's two pixels share packed operations (fp32x2), whose constant
-// operands are staged in pairs; the hit test is one comparison; a pixel that does not see a fragment takes it with weight zero
-// instead of branching around it (a vote and a branch per fragment cost more than the ten operations they saved). Measured
-// against scalar pixels with a vote: 1920x1080 view of 500k splats 143 -> 123 us, 4K with depth 847 -> 740, 1001x751 with
-// features 85 -> 69, 1237x822 117 -> 92, 64x64 (one list at a time) 50 -> 38. Images are the same bit for bit.
+// gather of 48 B per staged fragment, served mostly by L2. Fragments are gathered one batch ahead and staged in shared memory
+// as operands of packed arithmetic (fp32x2); the hit test is one comparison; a pixel that does not see a fragment takes it with
+// weight zero instead of branching around it (a vote and a branch per fragment cost more than the ten operations they saved).
+// Two kernels with the same arithmetic, bit for bit:
+//   raster_fwd_half_kernel  two warps to a tile, a lane one pixel, two consecutive fragments to a packed operation: the chain of
+//                           one list is half as long. For whole views and two chunks, where a visit to a tile is a long list.
+//   raster_fwd_kernel       one warp to a tile, a lane two pixels that share packed operations: twice as many tiles in flight.
+//                           For three and more depth chunks, whose visits are many and short.
+// Measured, us (scalar pixels with a vote / one warp / two warps): 64x64 50 / 38 / 23, 333x217 54 / 42 / 28, 1001x751 with
+// features 85 / 69 / 54, 1237x822 in two chunks 117 / 92 / 76, 1920x1080 in two 143 / 123 / 118; 1024x1024 over 1M in four
+// 231 / 187 / 206, 4K over 6M with depth in five 847 / 740 / 953, sixteen views of 3M in four on eight streams 20.6 / 21.6 ms.
 #include "common.cuh"
 
 namespace b2k {
 namespace {
 
 constexpr int FWD_WARPS = 4;
-constexpr int FWD_BATCH = 32;
-static_assert(FWD_BATCH == 1 << SEG_SHIFT_MIN, "a segment of the backward is a whole number of batches");
-constexpr int FWD_GROUP = 4;                             // fragments whose state-independent math is issued together (8: the same within 3 %, more registers)
+constexpr int FWD_TILES = FWD_WARPS / 2;                 // of a block of raster_fwd_half_kernel
+constexpr int FWD_BATCH = 64, FWD_SEG = 32;              // fragments staged at a time; between possible checkpoints
+static_assert(FWD_SEG == 1 << SEG_SHIFT_MIN, "checkpoints");
+constexpr int FWD_GROUP = 4;                             // fragments (one warp) or pairs of fragments (two) whose state-independent math is issued together
 
 // CHUNKED: the view is composited in depth chunks (chunk `chunk` of `n_chunks`, one launch each, nearest first). Between
 // launches a pixel's state lives in the output buffers: the colour sums in out_feat.xyz, the transmittance in
@@ -25,12 +31,21 @@ constexpr int FWD_GROUP = 4;                             // fragments whose stat
 // after every chunk, so a launch only touches tiles that received fragments. With DEPTH the depth sum travels in
 // out_depth and the last chunk visits every pixel to divide it out. The tile's bit in `alive` tells the binning of the next
 // chunk whether any pixel of the tile can still take a fragment.
-__device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float& at(float2& v, int p) { return p == 0 ? v.x : v.y; }
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 __device__ __forceinline__ float fast_ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+
+// Barrier of the 64 threads of a tile; whether `p` holds for any of them.
+__device__ __forceinline__ bool pair_any(int id, bool p) {
+  uint32_t r;
+  asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; barrier.cta.red.or.pred q, %2, 64, p; selp.u32 %0, 1, 0, q; }" : "=r"(r) : "r"((uint32_t)p), "r"(id) : "memory");
+  return r != 0u;
+}
 
 constexpr uint32_t DONE_BIT = 0x80000000u;
 
+__device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float& at(float2& v, int p) { return p == 0 ? v.x : v.y; }
 // Alpha of a staged fragment at the two pixels, zero where a pixel does not see it.
 __device__ __forceinline__ float2 fragment_alpha(const float4& q0, const float4& q1, const float4& q2, const float2& pcx, const float2& pcy) {
   const float2 dy = __fadd2_rn(pcy, make_float2(q0.z, q0.w)), dx = __fadd2_rn(pcx, make_float2(q0.x, q0.y));
@@ -44,11 +59,25 @@ __device__ __forceinline__ float2 fragment_alpha(const float4& q0, const float4&
   return make_float2(a0, a1);
 }
 
+// Two fragments that follow each other in a list, the nearer in the first of each pair of lanes.
+constexpr int STAGED = 5;   // (-x, -y), (c00 / 2, c01), (c11 / 2, opacity), (power, r), (g, b); then (z, feature 0), (feature 1, 2)
+// Alpha of the two at the lane's pixel, zero where it does not see one.
+__device__ __forceinline__ float2 pair_alpha(const float4& q0, const float4& q1, const float4& q2, float2 power, float2 pcx, float2 pcy) {
+  const float2 dx = __fadd2_rn(pcx, lo2(q0)), dy = __fadd2_rn(pcy, hi2(q0));
+  const float2 sigma = __ffma2_rn(dx, __ffma2_rn(dx, lo2(q1), __fmul2_rn(hi2(q1), dy)), __fmul2_rn(__fmul2_rn(lo2(q2), dy), dy));
+  const float2 e = __fmul2_rn(sigma, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+  const float2 al = __fmul2_rn(hi2(q2), make_float2(fast_ex2(e.x), fast_ex2(e.y)));
+  // alpha >= 1/255 is 0 <= sigma <= power: one comparison of bit patterns (neither is ever -0). The exponent is at most
+  // log2(255) in size there, so that flushing denormals changes nothing.
+  return make_float2(__float_as_uint(sigma.x) <= __float_as_uint(power.x) ? fminf(ALPHA_MAX, al.x) : 0.f,
+                     __float_as_uint(sigma.y) <= __float_as_uint(power.y) ? fminf(ALPHA_MAX, al.y) : 0.f);
+}
+
 // What the forward leaves for the backward (common.cuh): nothing, checkpoints of the running sums, or of each segment's sums.
 enum Checkpoints { NONE = 0, RUNNING = 1, PER_SEGMENT = 2 };
 
 template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
-__global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
+__global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
@@ -58,7 +87,186 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
   // pixel travel in feat_acc and move into out_feat.xyz when the last chunk, which then visits every pixel, is done.
   static_assert(!(FEAT && CHUNKED && BWD), "the chunked backward reads the colour sums from out_feat.xyz");
-  __shared__ float4 s_staged[FWD_WARPS][FWD_BATCH][FEAT ? 6 : 5];   // a fragment's constants, most of them twice, as operands of packed arithmetic
+  constexpr int RECORDS = FEAT ? STAGED + 2 : DEPTH ? STAGED + 1 : STAGED;
+  __shared__ float4 s_staged[FWD_TILES][2][FWD_BATCH / 2][RECORDS];   // [tile][buffer][pair]
+  __shared__ uint32_t s_last[FWD_WARPS], s_odd[FWD_WARPS][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = warp & 1;
+  const int tile = blockIdx.x * FWD_TILES + (warp >> 1);
+  if (tile >= n_tiles) return;
+  const int tx = tile % tiles_x, ty = tile / tiles_x, in_tile = half * 32 + lane;   // the lane's pixel in its tile
+  const int px = tx * RT_W + (in_tile & 7), py = ty * RT_W + (in_tile >> 3), pix = py * W + px;
+  const bool inside = px < W && py < H;
+  const float2 pcx = make_float2((float)px + 0.5f, (float)px + 0.5f), pcy = make_float2((float)py + 0.5f, (float)py + 0.5f);
+  const uint2 range = tile_ranges[tile];
+  const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
+  if (CHUNKED && !first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
+  float T = 1.f, r = 0.f, g = 0.f, b = 0.f, zs = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;   // f: composited feature lanes (raster_fwd.cu:52)
+  bool open = inside;   // the pixel can take another fragment
+  uint32_t last = range.x;
+  if (CHUNKED && !first && inside) {
+    const float4 acc = out_feat[pix];
+    r = acc.x; g = acc.y; b = acc.z; T = acc.w;
+    if constexpr (DEPTH) zs = out_depth[pix];
+    if constexpr (FEAT) { const float4 fa = feat_acc[pix]; f0 = fa.x; f1 = fa.y; f2 = fa.z; }
+    const uint32_t l = last_idx[pix];
+    open = (l & DONE_BIT) == 0u;
+    last = l & ~DONE_BIT;
+  }
+  // Checkpoints for the backward's segmented replay (see common.cuh): the state a later chunk starts a tile with, and
+  // the state before every (1 << seg_shift)-th fragment of the list.
+  const int q = CHUNKED ? chunk * n_tiles + tile : tile;
+  float sr = 0.f, sg = 0.f, sb = 0.f;   // PER_SEGMENT: colour sums of the segment at hand
+  uint32_t seg_now = 0;
+  auto checkpoint = [&](uint32_t seg) {
+    float4* dst = ckpt + (size_t)ckpt_slot(range.x, q, seg, seg_shift) * RT_PX + in_tile;
+    if constexpr (CKPT == PER_SEGMENT) { *dst = make_float4(sr, sg, sb, T); sr = sg = sb = 0.f; }   // the sums of the segment before the boundary
+    else *dst = make_float4(r, g, b, T);
+    seg_now = seg;
+  };
+  if (BWD && CHUNKED && !first && range.y > range.x) checkpoint(0u);
+  // The records of a batch are gathered one batch ahead, into registers, half by each warp: the two dependent loads (list
+  // entry, then the splat's records) are in flight while the batch before them is composited.
+  float4 n0, n1, n2;
+  float2 n3;
+  auto gather = [&](uint32_t from) {
+    n0 = n1 = n2 = make_float4(0.f, 0.f, 0.f, 0.f); n3 = make_float2(0.f, 0.f);   // beyond the list: opacity zero
+    if (from < range.y && (uint32_t)in_tile < range.y - from) {
+      const uint32_t gid = vals_sorted[from + in_tile];
+      n0 = proj0[gid]; n1 = proj1[gid]; n2 = proj2[gid];
+      if constexpr (FEAT) n3 = proj3[gid];
+    }
+  };
+  gather(range.x);
+  int buf = 0;
+  bool any_open = true;
+  for (uint32_t start = range.x;; start += FWD_BATCH, buf ^= 1) {
+    float4 (*staged)[RECORDS] = s_staged[warp >> 1][buf];
+    {
+      float* s = reinterpret_cast<float*>(staged[in_tile >> 1]) + (lane & 1);
+      const float cr = fmaxf(n2.x, 0.f), cg = fmaxf(n2.y, 0.f), cb = fmaxf(n2.z, 0.f);
+      s[0] = -n0.x; s[2] = -n0.y; s[4] = 0.5f * n0.z; s[6] = n0.w; s[8] = 0.5f * n1.x; s[10] = n1.y; s[12] = n1.w; s[14] = cr; s[16] = cg; s[18] = cb;
+      bool strange = fmaxf(cr, fmaxf(cg, cb)) == INFINITY;   // a colour or feature that is not finite may not be added with weight zero
+      if constexpr (DEPTH || FEAT) { s[20] = n1.z; s[22] = n2.w; }
+      if constexpr (FEAT) { s[24] = n3.x; s[26] = n3.y; strange = strange || !(isfinite(n2.w) && isfinite(n3.x) && isfinite(n3.y)); }
+      const uint32_t any_strange = __any_sync(0xffffffffu, strange);
+      if (lane == 0) s_odd[warp][buf] = any_strange;
+    }
+    // One barrier of the tile's two warps per batch: the batch is staged, the one before it is done with (it lies in the other
+    // buffer), and whether any pixel is still open.
+    any_open = pair_any(1 + (warp >> 1), open);
+    if (start >= range.y || !any_open) break;
+    gather(start + FWD_BATCH);
+    const bool odd = (s_odd[warp][buf] | s_odd[warp ^ 1][buf]) != 0u;
+    // Takes one fragment of weight `al` with transmittance `next_T` behind it: the one that would saturate a pixel closes it and is
+    // not taken. A pixel that does not see the fragment has its transmittance multiplied by one, and its sums take zeros.
+    auto take = [&](float al, float through, float cr, float cg, float cb, float z, float e0, float e1, float e2, uint32_t end) {
+      const float next_T = T * through;
+      open = open && next_T > T_CUTOFF;
+      const float a = open ? al : 0.f, vis = a * T;
+      r += cr * vis; g += cg * vis; b += cb * vis;
+      if constexpr (CKPT == PER_SEGMENT) { sr += cr * vis; sg += cg * vis; sb += cb * vis; }
+      if constexpr (DEPTH) zs += vis * z;
+      if constexpr (FEAT) { f0 += e0 * vis; f1 += e1 * vis; f2 += e2 * vis; }
+      T = open ? next_T : T;
+      if constexpr (BWD || CHUNKED) last = a != 0.f ? end : last;
+    };
+    // Pairs are taken FWD_GROUP at a time: first everything that does not depend on the pixel's running state (sigma, the hit test,
+    // alpha with its exponential) for the whole group, so that those chains overlap, then the short serial part (transmittance and
+    // colour sums) fragment by fragment in list order.
+    for (uint32_t t_begin = 0; t_begin < FWD_BATCH && t_begin < range.y - start; t_begin += FWD_SEG) {   // a segment of the backward is a whole number of these
+      const uint32_t at = start + t_begin - range.x, t_end = min(t_begin + FWD_SEG, range.y - start);
+      if (BWD && at != 0u && (at & ((1u << seg_shift) - 1u)) == 0u) checkpoint(at >> seg_shift);
+      if (!__any_sync(0xffffffffu, open)) continue;   // only the other half is still at it
+      if (odd) {
+#pragma unroll 1
+        for (uint32_t t = t_begin; t < t_end; t++) {
+          const float4* f = staged[t >> 1];
+          const float2 al2 = pair_alpha(f[0], f[1], f[2], lo2(f[3]), pcx, pcy);
+          const int k = t & 1;
+          const float al = k ? al2.y : al2.x;
+          const float* c = reinterpret_cast<const float*>(f) + k;
+          const float z = DEPTH ? c[RECORDS > 5 ? 20 : 0] : 0.f, e0 = FEAT ? c[RECORDS > 6 ? 22 : 0] : 0.f, e1 = FEAT ? c[RECORDS > 6 ? 24 : 0] : 0.f, e2 = FEAT ? c[RECORDS > 6 ? 26 : 0] : 0.f;
+          if (al != 0.f && open) {
+            if (T * (1.f - al) > T_CUTOFF) take(al, 1.f - al, c[14], c[16], c[18], z, e0, e1, e2, start + t + 1);
+            else open = false;
+          }
+        }
+        continue;
+      }
+      for (uint32_t t0 = t_begin; t0 < t_end; t0 += 2 * FWD_GROUP) {
+        float2 alpha[FWD_GROUP], through[FWD_GROUP], red[FWD_GROUP];
+#pragma unroll
+        for (int u = 0; u < FWD_GROUP; u++) {
+          const float4* f = staged[t0 / 2 + u];
+          const float4 q3 = f[3];
+          alpha[u] = pair_alpha(f[0], f[1], f[2], lo2(q3), pcx, pcy);
+          through[u] = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[u].x, -alpha[u].y));
+          red[u] = hi2(q3);
+        }
+#pragma unroll
+        for (int u = 0; u < FWD_GROUP; u++) {
+          const float4* f = staged[t0 / 2 + u];
+          const float4 q4 = f[4], q5 = DEPTH || FEAT ? f[RECORDS > 5 ? 5 : 0] : make_float4(0.f, 0.f, 0.f, 0.f), q6 = FEAT ? f[RECORDS > 6 ? 6 : 0] : q5;
+          const uint32_t end = start + t0 + 2 * u + 1;
+          take(alpha[u].x, through[u].x, red[u].x, q4.x, q4.z, q5.x, q5.z, q6.x, q6.z, end);
+          take(alpha[u].y, through[u].y, red[u].y, q4.y, q4.w, q5.y, q5.w, q6.y, q6.w, end + 1);
+        }
+      }
+    }
+  }
+  if (inside) {
+    out_rgba[pix] = make_float4(r + T * bg.x, g + T * bg.y, b + T * bg.z, 1.f - T);
+    if constexpr (CHUNKED) {
+      if (FEAT && final) out_feat[pix] = make_float4(f0, f1, f2, T);
+      else out_feat[pix] = make_float4(r, g, b, T);
+      if constexpr (FEAT) { if (!final) feat_acc[pix] = make_float4(f0, f1, f2, 0.f); }
+      if constexpr (DEPTH) out_depth[pix] = !final ? zs : ((1.f - T) > 0.05f ? zs / (1.f - T) : INFINITY);
+      last_idx[pix] = last | (open ? 0u : DONE_BIT);
+    } else {
+      out_feat[pix] = make_float4(f0, f1, f2, T);
+      if constexpr (DEPTH) out_depth[pix] = (1.f - T) > 0.05f ? zs / (1.f - T) : INFINITY;
+      if constexpr (BWD) last_idx[pix] = last;
+    }
+  }
+  if constexpr (!BWD && !CHUNKED) return;
+  // What the tile's two warps settle together: whether any pixel is still open, and the last fragment any pixel used.
+  const uint32_t mine = __reduce_max_sync(0xffffffffu, last);
+  if (lane == 0) s_last[warp] = mine;
+  any_open = pair_any(1 + (warp >> 1), open);
+  if (CHUNKED && !final && in_tile == 0 && !any_open)
+    atomicAnd(alive + (size_t)(ty >> 3) * ((tiles_x + 7) >> 3) + (tx >> 3), ~(1ull << ((ty & 7) * 8 + (tx & 7))));
+  if constexpr (BWD) {
+    // The backward never needs to look past the last fragment any pixel used. (A pixel whose last fragment lies in an
+    // earlier chunk contributes this chunk's start: an empty range.)
+    uint32_t m = max(s_last[warp], s_last[warp ^ 1]);
+    if constexpr (CHUNKED) m = min(max(m, range.x), range.y);
+    if (in_tile == 0) tile_ranges[tile].y = m;
+    if (m > range.x) {
+      const uint32_t segs = (m - range.x + (1u << seg_shift) - 1u) >> seg_shift;
+      if constexpr (CKPT == PER_SEGMENT) {
+        // Slot 0 has no segment before it: its colour takes the sums of the range's last segment (which is the one at hand
+        // unless nothing after its boundary was seen).
+        float* dst = reinterpret_cast<float*>(ckpt + (size_t)ckpt_slot(range.x, q, 0u, seg_shift) * RT_PX + in_tile);
+        const float4 v = segs - 1u == seg_now ? make_float4(sr, sg, sb, 0.f) : ckpt[(size_t)ckpt_slot(range.x, q, segs, seg_shift) * RT_PX + in_tile];
+        dst[0] = v.x; dst[1] = v.y; dst[2] = v.z;
+      }
+    }
+  }
+}
+
+// One warp to a tile, for views in depth chunks.
+template <int CKPT, bool DEPTH, bool FEAT>
+__global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
+    uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
+    const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
+    float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc) {
+  after_previous();
+  constexpr bool BWD = CKPT != NONE;
+  // FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
+  // pixel travel in feat_acc and move into out_feat.xyz when the last chunk, which then visits every pixel, is done.
+  static_assert(!(FEAT && BWD), "the chunked backward reads the colour sums from out_feat.xyz");
+  __shared__ float4 s_staged[FWD_WARPS][FWD_SEG][FEAT ? 6 : 5];   // a fragment's constants, most of them twice, as operands of packed arithmetic
   float2 f0 = splat2(0.f), f1 = f0, f2 = f0;   // composited feature lanes (raster_fwd.cu:52)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = blockIdx.x * FWD_WARPS + warp;
@@ -68,12 +276,12 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   const bool in0 = px0 < W && py < H, in1 = px0 + 1 < W && py < H;
   const float2 pcx = make_float2((float)px0 + 0.5f, (float)px0 + 1.5f), pcy = splat2((float)py + 0.5f);
   const uint2 range = tile_ranges[tile];
-  const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
-  if (CHUNKED && !first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
+  const bool first = chunk == 0, final = chunk == n_chunks - 1;
+  if (!first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
   float2 T = splat2(1.f), r = splat2(0.f), g = r, b = r, zs = r;   // of the two pixels
   bool open[2] = {in0, in1};   // the pixel can take another fragment
   uint32_t last[2] = {range.x, range.x};
-  if (CHUNKED && !first) {
+  if (!first) {
 #pragma unroll
     for (int p = 0; p < 2; p++) {
       if (p == 0 ? in0 : in1) {
@@ -90,7 +298,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   }
   // Checkpoints for the backward's segmented replay (see common.cuh): the state a later chunk starts a tile with, and
   // the state before every (1 << seg_shift)-th fragment of the list.
-  const int q = CHUNKED ? chunk * n_tiles + tile : tile;
+  const int q = chunk * n_tiles + tile;
   float2 sr = splat2(0.f), sg = sr, sb = sr;   // PER_SEGMENT: colour sums of the segment at hand
   uint32_t seg_now = 0;
   auto checkpoint = [&](uint32_t seg) {
@@ -103,7 +311,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
       dst[0] = make_float4(r.x, g.x, b.x, T.x); dst[1] = make_float4(r.y, g.y, b.y, T.y);
     }
   };
-  if (BWD && CHUNKED && !first && range.y > range.x) checkpoint(0u);
+  if (BWD && !first && range.y > range.x) checkpoint(0u);
   // The records of a batch are gathered one batch ahead, into registers: the two dependent loads (list entry, then the
   // splat's records) are in flight while the batch before them is composited.
   float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0, n2 = n0;
@@ -117,7 +325,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     }
   };
   gather(range.x);
-  for (uint32_t start = range.x; start < range.y; start += FWD_BATCH) {
+  for (uint32_t start = range.x; start < range.y; start += FWD_SEG) {
     if (!__any_sync(0xffffffffu, open[0] || open[1])) break;
     if (BWD && start != range.x && ((start - range.x) & ((1u << seg_shift) - 1u)) == 0u) checkpoint((start - range.x) >> seg_shift);
     __syncwarp();
@@ -138,12 +346,12 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
       odd = __ballot_sync(0xffffffffu, strange);
     }
     __syncwarp();
-    gather(start + FWD_BATCH);
+    gather(start + FWD_SEG);
     // Fragments are taken FWD_GROUP at a time: first everything that does not depend on the pixels' running state (sigma,
     // the hit test, alpha with its exponential) for the whole group, so that those chains overlap, then the short serial
     // part (transmittance and colour sums) fragment by fragment in list order.
     const float4 (*staged)[FEAT ? 6 : 5] = s_staged[warp];
-    const uint32_t remaining = min((uint32_t)FWD_BATCH, range.y - start);
+    const uint32_t remaining = min((uint32_t)FWD_SEG, range.y - start);
     if (odd) {
 #pragma unroll 1
       for (uint32_t t = 0; t < remaining; t++) {
@@ -201,20 +409,14 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     if (p == 0 ? in0 : in1) {
       const int pix = py * W + px0 + p;
       out_rgba[pix] = make_float4(at(r, p) + at(T, p) * bg.x, at(g, p) + at(T, p) * bg.y, at(b, p) + at(T, p) * bg.z, 1.f - at(T, p));
-      if constexpr (CHUNKED) {
-        if (FEAT && final) out_feat[pix] = make_float4(at(f0, p), at(f1, p), at(f2, p), at(T, p));
-        else out_feat[pix] = make_float4(at(r, p), at(g, p), at(b, p), at(T, p));
-        if constexpr (FEAT) { if (!final) feat_acc[pix] = make_float4(at(f0, p), at(f1, p), at(f2, p), 0.f); }
-        if constexpr (DEPTH) out_depth[pix] = !final ? at(zs, p) : ((1.f - at(T, p)) > 0.05f ? at(zs, p) / (1.f - at(T, p)) : INFINITY);
-        last_idx[pix] = last[p] | (open[p] ? 0u : DONE_BIT);
-      } else {
-        out_feat[pix] = make_float4(at(f0, p), at(f1, p), at(f2, p), at(T, p));
-        if constexpr (DEPTH) out_depth[pix] = (1.f - at(T, p)) > 0.05f ? at(zs, p) / (1.f - at(T, p)) : INFINITY;
-        if constexpr (BWD) last_idx[pix] = last[p];
-      }
+      if (FEAT && final) out_feat[pix] = make_float4(at(f0, p), at(f1, p), at(f2, p), at(T, p));
+      else out_feat[pix] = make_float4(at(r, p), at(g, p), at(b, p), at(T, p));
+      if constexpr (FEAT) { if (!final) feat_acc[pix] = make_float4(at(f0, p), at(f1, p), at(f2, p), 0.f); }
+      if constexpr (DEPTH) out_depth[pix] = !final ? at(zs, p) : ((1.f - at(T, p)) > 0.05f ? at(zs, p) / (1.f - at(T, p)) : INFINITY);
+      last_idx[pix] = last[p] | (open[p] ? 0u : DONE_BIT);
     }
   }
-  if (CHUNKED && !final) {
+  if (!final) {
     const bool more = __any_sync(0xffffffffu, open[0] || open[1]);
     if (lane == 0 && !more) atomicAnd(alive + (size_t)(ty >> 3) * ((tiles_x + 7) >> 3) + (tx >> 3), ~(1ull << ((ty & 7) * 8 + (tx & 7))));
   }
@@ -224,7 +426,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     uint32_t m = max(last[0], last[1]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if constexpr (CHUNKED) m = min(max(m, range.x), range.y);
+    m = min(max(m, range.x), range.y);
     if (lane == 0) tile_ranges[tile].y = m;
     if (CKPT == PER_SEGMENT && m > range.x) {
       // Slot 0 has no segment before it: its colour takes the sums of the range's last segment (which is the one at hand
@@ -251,19 +453,23 @@ namespace b2k {
 int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_chunks, unsigned long long* alive, cudaStream_t s) {
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
   uint2* ranges = (uint2*)c->tile_ranges + (n_chunks > 1 ? (size_t)chunk * c->n_tiles : 0);
-#define L(B, D, C, F) launch_next(raster_fwd_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, \
-    (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, \
-    chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(c->n_tiles), (n_chunks > 1 && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr)
-#define LB(B) do { if (n_chunks > 1) { if (c->out_depth) L(B, true, true, false); else L(B, false, true, false); } \
-    else if (o->feat_mode != 0) { if (c->out_depth) L(B, true, false, true); else L(B, false, false, true); } \
-    else { if (c->out_depth) L(B, true, false, false); else L(B, false, false, false); } } while (0)
-  if (n_chunks > 1 && o->feat_mode != 0) {   // forward only (checked by the caller): the scratch of the backward carries the feature sums
-    if (c->out_depth) L(NONE, true, true, true); else L(NONE, false, true, true);
-  } else if (!o->bwd_info) LB(NONE);
+  const bool chunked = n_chunks > 1, halves = n_chunks <= 2;   // (measured above)
+#define ARGS s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, \
+    (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, \
+    seg_shift_of(c->n_tiles), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr
+#define HALF(B, D, C, F) launch_next(raster_fwd_half_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_TILES), FWD_WARPS * 32, 0, ARGS)
+#define L(B, D, F) do { if (!chunked) HALF(B, D, false, F); else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
+    else launch_next(raster_fwd_kernel<B, D, (F) && (B) == NONE>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS); } while (0)
+#define LD(B, D) do { if (o->feat_mode != 0) L(B, D, true); else L(B, D, false); } while (0)   // a chunked view with features is forward only (checked by the caller)
+#define LB(B) do { if (c->out_depth) LD(B, true); else LD(B, false); } while (0)
+  if (!o->bwd_info) LB(NONE);
   else if (short_segments(c->n_tiles)) LB(PER_SEGMENT);
   else LB(RUNNING);
 #undef LB
+#undef LD
 #undef L
+#undef HALF
+#undef ARGS
   return check_launch();
 }
 }  // namespace b2k
