@@ -576,6 +576,16 @@ def render_forward(ctx, m, p, stream=None, sync=True):
     _check(lib().b2k_raster_fwd(C.byref(cs), C.byref(os_), st), "rasterize_forward")
 
 
+def forward_fits(ctx, stream=None):
+    """Waits for a render_forward(sync=False) and says whether its intersections fitted the context's buffers."""
+    cs, total = ctx.struct(), C.c_uint32(0)
+    st = lib().b2k_read_num_isect(C.byref(cs), _stream(stream), C.byref(total))
+    ctx.num_isect = int(total.value)
+    if st != B2K_ERR_OVERFLOW:
+        _check(st, "forward_fits")
+    return st != B2K_ERR_OVERFLOW
+
+
 def render_chunked(ctx, m, p, stream=None, sync=True):
     """b2k_render_chunked; with sync the slot count is read back and the view redone with larger buffers on overflow."""
     while True:

@@ -24,12 +24,22 @@ class Evidence:
         use_normals = normal_weight > 0.0 and view.normals is not None
         if use_normals:
             rp.feat = "Normals"
-        api.render_forward(ctx, m, rp, stream, sync=True)
-        self.view_acc.zero_()
-        cs, ms = ctx.struct(), m.struct()
-        masked_alpha = int(bool(masked and has_alpha))
-        api._check(api.lib().b2k_evidence_view(C.byref(cs), api._ptr(view.rgba), api._ptr(view.normals) if use_normals else None, api._ptr(view.weights),
-                                               masked_alpha, C.c_float(normal_weight), api._ptr(self.view_acc), api._stream(stream)), "evidence_view")
+        masked_alpha, ms = int(bool(masked and has_alpha)), m.struct()
+
+        def replay():
+            self.view_acc.zero_()
+            cs = ctx.struct()
+            api._check(api.lib().b2k_evidence_view(C.byref(cs), api._ptr(view.rgba), api._ptr(view.normals) if use_normals else None, api._ptr(view.weights),
+                                                   masked_alpha, C.c_float(normal_weight), api._ptr(self.view_acc), api._stream(stream)), "evidence_view")
+
+        # The intersection total is read back behind the replay, so that the GPU does not wait for the host in between. Lists that
+        # did not fit make it a replay of truncated lists into an accumulator of this view's own: it is redone.
+        api.render_forward(ctx, m, rp, stream, sync=False)
+        replay()
+        if not api.forward_fits(ctx, stream):
+            api.render_forward(ctx, m, rp, stream, sync=True)
+            replay()
+        cs = ctx.struct()
         if labels is not None:
             if self.votes is None:
                 self.votes = torch.zeros((m.n, self.bins), dtype=torch.float32, device=self.device)

@@ -168,3 +168,41 @@ def test_forward_groups_and_colours_that_are_not_finite(n):
     sees = images[0][:, 0] != images[1][:, 0]
     assert sees.any() and np.all(np.isposinf(images[2][sees, 0])) and np.array_equal(images[2][~sees], images[0][~sees])
     assert np.array_equal(images[2][:, 1:], images[0][:, 1:])
+
+
+@pytest.mark.parametrize("chunks", [1, 3])
+@pytest.mark.parametrize("n", [1, 3, 4, 31, 32, 33, 65])
+def test_evidence_rows_and_odd_batches(n, chunks):
+    import torch
+    from b2ctrain_b200 import api
+    from b2ctrain_b200.evidence import Evidence
+    W, H = 61, 40
+    scene, cam = stack_scene(n, W, H)
+    scene["pos_op"][:, 3] = -1.0
+    m = api.Model("cuda:0").upload(scene)
+    ctx = api.RenderCtx("cuda:0").setup(W, H, n, n_chunks=chunks)
+    rng = np.random.Generator(np.random.PCG64(n))
+    gt = rng.integers(0, 2 ** 32, W * H, dtype=np.uint64).astype(np.uint32)
+    wts = rng.integers(0, 256, W * H).astype(np.uint8)
+    ev = Evidence(m)
+    ev.add_view(ctx, cam, api.ViewGPU(torch.from_numpy(gt.view(np.int32)).cuda(), torch.from_numpy(wts).cuda(), W, H))
+    p0, p1 = (t[:n].cpu().numpy().astype(np.float64) for t in (ctx.proj0, ctx.proj1))
+    vals, ranges = ctx.vals_sorted.cpu().numpy().view(np.uint32), ctx.tile_ranges.cpu().numpy().view(np.uint32).reshape(chunks, -1, 2)
+    last, rgba = ctx.last_idx.cpu().numpy().view(np.uint32) & 0x7FFFFFFF, ctx.out_rgba.cpu().numpy().astype(np.float64)
+    want = np.zeros((n, 3))
+    for y in range(H):
+        for x in range(W):
+            i, T, a = y * W + x, 1.0, (gt[y * W + x] >> 24) / 255.0
+            w = wts[i] / 255.0
+            res = sum(abs(rgba[i, c] - ((gt[i] >> np.uint32(8 * c)) & 255) / 255.0) for c in range(3)) / 3.0
+            for ch in range(chunks):
+                b, e = ranges[ch, (y // 8) * ctx.tiles_x + x // 8]
+                for f in range(b, min(e, last[i])):
+                    s = vals[f]
+                    dx, dy = x + 0.5 - p0[s, 0], y + 0.5 - p0[s, 1]
+                    sigma = 0.5 * (p0[s, 2] * dx * dx + p1[s, 0] * dy * dy) + p0[s, 3] * dx * dy
+                    if 0.0 <= sigma <= p1[s, 3]:
+                        alpha = min(0.999, p1[s, 1] * np.exp(-sigma))
+                        want[s] += T * alpha * w * np.array([a, a * res, 1.0])
+                        T *= 1.0 - alpha
+    assert rel_l2(ev.view_acc.cpu().numpy(), want) <= 1e-4
