@@ -206,3 +206,18 @@ def test_evidence_rows_and_odd_batches(n, chunks):
                         want[s] += T * alpha * w * np.array([a, a * res, 1.0])
                         T *= 1.0 - alpha
     assert rel_l2(ev.view_acc.cpu().numpy(), want) <= 1e-4
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("W,H", [(1, 1), (31, 7), (32, 32), (33, 31), (64, 65), (130, 3)])
+def test_metrics_tiles(W, H, masked):
+    scene, cam = stack_scene(4, W, H)
+    rng = np.random.Generator(np.random.PCG64(W * 64 + H))
+    gt = rng.integers(0, 2 ** 32, W * H, dtype=np.uint64).astype(np.uint32)
+    pred = rng.uniform(-0.1, 1.1, (W * H, 4)).astype(np.float32)
+    h = Harness(scene, cam, gt)
+    h.ctx.out_rgba.copy_(h.torch.from_numpy(pred))
+    h.ctx.loss_accum.zero_()
+    h.api.eval_metrics(h.ctx, h.view, masked)
+    got, want = h.ctx.loss_accum[4:6].cpu().numpy(), orc.eval_metrics(W, H, pred, gt, masked)
+    assert np.allclose(got, np.array(want[:2], dtype=np.float64), rtol=2e-5, atol=1e-5)
