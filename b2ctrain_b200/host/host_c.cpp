@@ -80,13 +80,7 @@ extern "C" int b2ch_trainer_info(void* h, uint64_t* out8) {
 
 extern "C" int b2ch_trainer_download(void* h, float* pos_op, float* quat, float* lscale, float* sh) {
   return guarded([&] {
-    const SplatCloud c = ((StepTrainer*)h)->model.download(0);
-    for (size_t i = 0; i < c.n; i++) {
-      for (int k = 0; k < 3; k++) { pos_op[i * 4 + k] = c.pos[i * 3 + k]; lscale[i * 4 + k] = c.log_scale[i * 3 + k]; }
-      pos_op[i * 4 + 3] = c.opacity[i]; lscale[i * 4 + 3] = c.floor[i];
-      for (int k = 0; k < 4; k++) quat[i * 4 + k] = c.quat[i * 4 + k];
-    }
-    std::memcpy(sh, c.sh.data(), c.sh.size() * sizeof(float));
+    ((StepTrainer*)h)->download(pos_op, quat, lscale, sh);
   });
 }
 

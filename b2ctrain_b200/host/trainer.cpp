@@ -43,6 +43,10 @@ StepTrainer::StepTrainer(const SplatCloud& cloud, int W_, int H_, const StepConf
     staged_evt_.push_back(a); free_evt_.push_back(b);
   }
   cuda(cudaEventCreateWithFlags(&start_evt_, cudaEventDisableTiming), "event");
+  cuda(cudaEventCreateWithFlags(&binned_evt_, cudaEventDisableTiming), "event");
+  cuda(cudaEventCreateWithFlags(&counted_evt_, cudaEventDisableTiming), "event");
+  cuda(cudaEventCreateWithFlags(&done_evt_, cudaEventDisableTiming), "event");
+  for (cudaEvent_t& e : rows_evt_) cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
   cuda(cudaEventCreateWithFlags(&cleared_evt_, cudaEventDisableTiming), "event");
   for (auto& m : mark_) cuda(cudaEventCreate(&m), "event");
   h_isect_.reserve((size_t)lanes);
@@ -76,6 +80,7 @@ void StepTrainer::share_buffers() {
 }
 
 RefineStats StepTrainer::refine(const RefineParams& p, cudaStream_t stream) {
+  follow(stream);
   const bool sharded = world > 1 && cfg.shard_update;
   if (grad_clear_pending_) { cuda(cudaStreamWaitEvent(stream, cleared_evt_, 0), "wait"); grad_clear_pending_ = false; }
   if (sharded) {   // moments, the Adam-mini second moment and the lazy-update stamp: whole on every rank again
@@ -113,7 +118,7 @@ StepTrainer::~StepTrainer() {
   for (cudaEvent_t e : lane_done_) cudaEventDestroy(e);
   for (cudaEvent_t e : staged_evt_) cudaEventDestroy(e);
   for (cudaEvent_t e : free_evt_) cudaEventDestroy(e);
-  if (start_evt_) cudaEventDestroy(start_evt_);
+  for (cudaEvent_t e : {start_evt_, binned_evt_, counted_evt_, done_evt_, rows_evt_[0], rows_evt_[1]}) if (e) cudaEventDestroy(e);
   if (cleared_evt_) cudaEventDestroy(cleared_evt_);
   for (cudaEvent_t e : mark_) if (e) cudaEventDestroy(e);
 }
@@ -168,6 +173,12 @@ void StepTrainer::view_pass(int lane, int view, int slot, cudaStream_t s, bool f
   rp.sh_degree = model.degree; rp.bwd_info = true;
   { const B2kCtx cv = view_of(ctx); check(b2k_loss_zero(&cv, 0, 2, s), "loss_accum.zero"); }
   render_forward_async(ctx, model, rp, s);
+  if (fused) {   // the view's total goes to the host beside the rest of the step
+    cuda(cudaEventRecord(binned_evt_, s), "record");
+    cuda(cudaStreamWaitEvent(clear_stream_, binned_evt_, 0), "wait");
+    cuda(cudaMemcpyAsync(h_isect_.ptr, ctx.d_num_isect.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, clear_stream_), "readback");
+    cuda(cudaEventRecord(counted_evt_, clear_stream_), "record");
+  }
   ViewGPU vg; vg.rgba = target(view, slot, s, from_host); vg.W = W; vg.H = H;
   LossParams lp;
   lp.l1_w = 1.f - cfg.ssim_weight; lp.ssim_w = -cfg.ssim_weight;
@@ -205,7 +216,15 @@ void StepTrainer::run_views(const std::vector<int>& mine, cudaStream_t stream, b
   for (int lane = 1; lane < used; lane++) fold_loss(*ctxs[0], *ctxs[lane], stream);
 }
 
-bool StepTrainer::overflowed(cudaStream_t stream) {
+// Of a fused step only the total is waited for: loss, backward and update run on while the host sets up the next step. (Waiting
+// for the whole step left the GPU idle for the launch of a step's first kernels: 16 steps on 200x150 about 2,520 -> 2,410 us.)
+bool StepTrainer::overflowed(cudaStream_t stream, bool fused) {
+  if (fused) {
+    cuda(cudaEventSynchronize(counted_evt_), "sync");
+    if ((size_t)h_isect_.ptr[0] <= ctxs[0]->isect_cap) return false;
+    cuda(cudaStreamSynchronize(stream), "sync");
+    return grow_intersections(*ctxs[0], h_isect_.ptr[0]);
+  }
   for (size_t l = 0; l < ctxs.size(); l++)
     cuda(cudaMemcpyAsync(h_isect_.ptr + l, ctxs[l]->d_num_isect.ptr + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream), "readback");
   cuda(cudaStreamSynchronize(stream), "sync");
@@ -237,8 +256,37 @@ void StepTrainer::update(cudaStream_t stream) {
   grad_clear_pending_ = true;
 }
 
+// Work on another stream than the last step's follows that step.
+void StepTrainer::follow(cudaStream_t stream) {
+  if (stepped_ && stream != last_stream_) cuda(cudaStreamWaitEvent(stream, done_evt_, 0), "wait");
+}
+// The kernel writes rows straight into pinned memory, a slice at a time, while the slice before is copied out.
+void StepTrainer::download(float* pos_op, float* quat, float* lscale, float* sh) {
+  const size_t n = (size_t)model.n, lanes = 3 * (size_t)model.K(), per = 12 + lanes, most = (size_t)1 << 20;
+  if (n == 0) return;
+  const size_t slice = std::min((n + 3) & ~(size_t)3, most / per & ~(size_t)3), slices = (n + slice - 1) / slice;   // of four splats: every part stays 16-byte aligned
+  rows_.reserve(slice * per * std::min<size_t>(slices, 2));
+  const B2kModel mv = view_of(model);
+  if (stepped_) cuda(cudaStreamWaitEvent(clear_stream_, done_evt_, 0), "wait");
+  auto part = [&](size_t k, int which) { return rows_.ptr + (k & 1) * slice * per + (size_t)which * slice * 4; };
+  for (size_t k = 0; k <= slices; k++) {
+    if (k < slices) {
+      const size_t first = k * slice, count = std::min(slice, n - first);
+      check(b2k_model_rows(&mv, (int32_t)first, (int32_t)count, part(k, 0), part(k, 1), part(k, 2), part(k, 3), clear_stream_), "b2k_model_rows");
+      cuda(cudaEventRecord(rows_evt_[k & 1], clear_stream_), "record");
+    }
+    if (k == 0) continue;
+    const size_t p = k - 1, first = p * slice, count = std::min(slice, n - first);
+    cuda(cudaEventSynchronize(rows_evt_[p & 1]), "sync");
+    std::memcpy(pos_op + first * 4, part(p, 0), count * 16); std::memcpy(quat + first * 4, part(p, 1), count * 16); std::memcpy(lscale + first * 4, part(p, 2), count * 16);
+    std::memcpy(sh + first * lanes, part(p, 3), count * lanes * sizeof(float));
+  }
+}
+void StepTrainer::settle() { if (stepped_) cuda(cudaEventSynchronize(done_evt_), "sync"); }
+
 void StepTrainer::step(const std::vector<int>& all, cudaStream_t stream, bool from_host) {
   if (all.empty()) return;
+  follow(stream);
   model.adam_t++;
   step_no++;
   const std::vector<int> mine = my_share(all);
@@ -246,7 +294,7 @@ void StepTrainer::step(const std::vector<int>& all, cudaStream_t stream, bool fr
   if (profile) cuda(cudaEventRecord(mark_[0], stream), "record");
   for (;;) {
     if (!mine.empty()) run_views(mine, stream, from_host, fused); else for (auto& c : ctxs) step_begin(*c, stream);
-    if (!overflowed(stream)) break;
+    if (!overflowed(stream, fused)) break;
     overflow_redos++;
     if (!fused) {
       if (grad_clear_pending_) cuda(cudaStreamWaitEvent(stream, cleared_evt_, 0), "wait");
@@ -255,6 +303,8 @@ void StepTrainer::step(const std::vector<int>& all, cudaStream_t stream, bool fr
   }
   if (profile) cuda(cudaEventRecord(mark_[1], stream), "record");
   if (!fused) update(stream);
+  cuda(cudaEventRecord(done_evt_, stream), "record");
+  last_stream_ = stream; stepped_ = true;
   if (profile) {
     cuda(cudaEventRecord(mark_[2], stream), "record");
     cuda(cudaEventSynchronize(mark_[2]), "sync");
@@ -271,11 +321,13 @@ void StepTrainer::step(const std::vector<int>& all, cudaStream_t stream, bool fr
 }
 
 void StepTrainer::read_loss(float* out16, cudaStream_t stream) {
+  follow(stream);
   cuda(cudaMemcpyAsync(out16, ctxs[0]->loss_accum.ptr, 16 * sizeof(float), cudaMemcpyDeviceToHost, stream), "loss readback");
   cuda(cudaStreamSynchronize(stream), "sync");
 }
 
 void StepTrainer::reduce_statistics(cudaStream_t stream) {
+  follow(stream);
   if (world == 1) return;
   check(b2k_dp_allreduce_stat(dp_, model.refine_norm.ptr, (uint64_t)model.n, 1, stream), "refine_norm");
   check(b2k_dp_allreduce_stat(dp_, model.max_screen.ptr, (uint64_t)model.n, 1, stream), "max_screen");
@@ -284,6 +336,7 @@ void StepTrainer::reduce_statistics(cudaStream_t stream) {
 }
 
 uint64_t StepTrainer::replica_checksum(cudaStream_t stream) {
+  follow(stream);
   uint64_t sum = 0;
   auto add = [&](const void* p, size_t bytes) {
     std::vector<uint32_t> h(bytes / 4);

@@ -55,6 +55,11 @@ class StepTrainer {
   // and on the lanes' own streams, which are joined back into `stream` before the update; the call returns after one
   // host readback per step (the lanes' largest intersection totals), having redone the views with larger buffers if one
   // did not fit. from_host: targets are copied in from pinned memory, double-buffered on a copy stream.
+  // When a step of one view returns, its intersections have fitted and its work may still run on the stream; the methods below
+  // order themselves behind it on whatever stream they are given. settle() waits for it: before `model` is read in another way.
+  void settle();
+  // The model's splats as rows (pos_op, quat, lscale [n][4], sh [n][K][3]) into host memory of any kind.
+  void download(float* pos_op, float* quat, float* lscale, float* sh);
   void step(const std::vector<int>& views, cudaStream_t stream, bool from_host = false);
   // loss_accum of lane 0 after the last step: [0] last view's loss, [2] sum over this rank's views, [3] their count.
   void read_loss(float* out16, cudaStream_t stream);
@@ -86,7 +91,8 @@ class StepTrainer {
  private:
   void run_views(const std::vector<int>& mine, cudaStream_t stream, bool from_host, bool fused);
   void view_pass(int lane, int view, int slot, cudaStream_t s, bool from_host, bool fused, bool first_of_lane);
-  bool overflowed(cudaStream_t stream);
+  bool overflowed(cudaStream_t stream, bool fused);
+  void follow(cudaStream_t stream);
   void update(cudaStream_t stream);
   OptimParams optim_params(const CameraGPU& cam) const;
   const uint32_t* target(int view, int slot, cudaStream_t s, bool from_host);
@@ -100,8 +106,13 @@ class StepTrainer {
   cudaStream_t copy_stream_ = nullptr, clear_stream_ = nullptr;
   std::vector<DevBuf<uint32_t>> stage_;
   std::vector<cudaEvent_t> staged_evt_, free_evt_, lane_done_;
+  cudaEvent_t binned_evt_ = nullptr, counted_evt_ = nullptr, done_evt_ = nullptr;
+  cudaStream_t last_stream_ = nullptr;
+  bool stepped_ = false;
   cudaEvent_t start_evt_ = nullptr, cleared_evt_ = nullptr, mark_[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   PinnedBuf<uint32_t> h_isect_;
+  PinnedBuf<float> rows_;   // two slices of a download, at most 4 MB each
+  cudaEvent_t rows_evt_[2] = {nullptr, nullptr};
   bool grad_clear_pending_ = false;
 };
 

@@ -148,7 +148,7 @@ class HostTrainer:
 
     def download(self):
         K = (self.degree + 1) ** 2
-        a = [np.zeros((self.n, 4), np.float32) for _ in range(3)] + [np.zeros((self.n, K, 3), np.float32)]
+        a = [np.empty((self.n, 4), np.float32) for _ in range(3)] + [np.empty((self.n, K, 3), np.float32)]
         _check(lib().b2ch_trainer_download(self.h, *[x.ctypes.data_as(_P) for x in a]), "b2ch_trainer_download")
         return dict(n=self.n, degree=self.degree, pos_op=a[0], quat=a[1], lscale=a[2], sh=a[3])
 

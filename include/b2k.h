@@ -366,6 +366,9 @@ uint64_t b2k_select_tmp_words(int32_t n);
 int b2k_select_flagged(const uint32_t* keep, int32_t n, uint32_t* idx, uint32_t* count, uint32_t* tmp, b2k_stream_t s);
 int b2k_gather_lanes(const void* src, void* dst, const uint32_t* idx, int32_t count, int32_t lanes, uint64_t stride, int32_t elem_bytes,
                      b2k_stream_t s);
+/* Splats [first, first + count) as rows: pos_op, quat, lscale [count][4] and sh [count][K][3] (the model's SH is planar). The
+ * outputs may be device memory or pinned host memory; all 16-byte aligned. */
+int b2k_model_rows(const B2kModel* m, int32_t first, int32_t count, float* pos_op, float* quat, float* lscale, float* sh, b2k_stream_t s);
 /* pack_kernel, src/train/teacher.cu:11-17: float RGBA -> packed RGBA8 target. alpha_override < 0 keeps the image's. */
 int b2k_pack_rgba8(const float* rgba, uint32_t* out, int32_t n_pixels, int32_t alpha_override, b2k_stream_t s);
 /* The 8-bit image the render front end writes (src/render/renderer.cpp:353-358: lround(clamp(x, 0, 1) * 255) per channel,

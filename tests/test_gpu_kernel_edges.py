@@ -221,3 +221,21 @@ def test_metrics_tiles(W, H, masked):
     h.api.eval_metrics(h.ctx, h.view, masked)
     got, want = h.ctx.loss_accum[4:6].cpu().numpy(), orc.eval_metrics(W, H, pred, gt, masked)
     assert np.allclose(got, np.array(want[:2], dtype=np.float64), rtol=2e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("degree", range(5))
+@pytest.mark.parametrize("first,count", [(0, 1), (0, 63), (0, 64), (3, 65), (64, 130)])
+def test_model_rows(degree, first, count):
+    import ctypes as C
+    import torch
+    from b2ctrain_b200 import api
+    n, K = 200, (degree + 1) ** 2
+    scene = scenes.make_splats(n, degree, 5)
+    m = api.Model("cuda:0").upload(scene)
+    ms = m.struct()
+    want = m.download()
+    out = [torch.full((count * w + 4,), 7.0).pin_memory() for w in (4, 4, 4, 3 * K)]
+    assert api.lib().b2k_model_rows(C.byref(ms), first, count, *[api._ptr(t) for t in out], api._stream(None)) == api.B2K_OK
+    torch.cuda.synchronize()
+    for t, k in zip(out, ("pos_op", "quat", "lscale", "sh")):
+        assert np.array_equal(t[:-4].numpy(), want[k][first : first + count].reshape(-1)) and bool((t[-4:] == 7.0).all())
