@@ -103,13 +103,14 @@ __device__ __forceinline__ unsigned long long mask_bits(const uint4& hi, const B
 }
 
 // The bins a splat's box overlaps, inside the band.
-struct BinSpan { int bx0, by0, w, count; };
+struct BinSpan { int bx0, by0, w, h, count; };
 __device__ __forceinline__ BinSpan span_of(const Box& b, const Band& g) {
-  BinSpan s{0, 0, 0, 0};
+  BinSpan s{0, 0, 0, 0, 0};
   if (b.x1 <= b.x0 || b.y1 <= b.y0) return s;
   const int by0 = max(b.y0 / BIN_W, g.bin_row0), by1 = min((b.y1 - 1) / BIN_W + 1, g.bin_row0 + g.bin_rows);
   s.bx0 = b.x0 / BIN_W; s.by0 = by0; s.w = (b.x1 - 1) / BIN_W + 1 - s.bx0;
-  s.count = by1 > by0 ? s.w * (by1 - by0) : 0;
+  s.h = max(by1 - by0, 0);
+  s.count = s.w * s.h;
   return s;
 }
 
@@ -155,6 +156,35 @@ __device__ __forceinline__ bool takes_bin(const unsigned long long* s_alive, con
 // The band's alive words, in shared memory.
 __device__ __forceinline__ void load_alive(const View& v, const Band& g, unsigned long long* s_alive) {
   for (int i = threadIdx.x; i < band_bins(g); i += blockDim.x) s_alive[i] = v.alive ? v.alive[g.bin_row0 * g.bins_x + i] : ~0ull;
+}
+// Running sums over the band's bins that hold a live tile, (bins_x + 1) to a row: any rectangle of bins is counted in four reads.
+// In the later chunks most splats lie behind saturated bins only, and would otherwise ask each bin in turn (1M large splats on
+// 1024x1024 in four chunks: bin_count 98 -> 49 us a view; 6M small ones on 4K 245 -> 236).
+inline size_t live_sums_bytes(const Band& g) { return ((size_t)(g.bins_x + 1) * (g.bin_rows + 1) * sizeof(uint16_t) + 15) / 16 * 16; }
+__device__ __forceinline__ void sum_live(const Band& g, const unsigned long long* s_alive, uint16_t* s_sum) {   // synchronises
+  const int tid = threadIdx.x, lane = tid & 31, pitch = g.bins_x + 1;
+  for (int x = tid; x < pitch; x += blockDim.x) s_sum[x] = 0;
+  for (int y = tid >> 5; y < g.bin_rows; y += blockDim.x >> 5) {
+    uint16_t* row = s_sum + (y + 1) * pitch;
+    uint32_t at = 0;
+    if (lane == 0) row[0] = 0;
+    for (int x0 = 0; x0 < g.bins_x; x0 += 32) {
+      const uint32_t m = __ballot_sync(FULL, x0 + lane < g.bins_x && s_alive[y * g.bins_x + x0 + lane] != 0ull);
+      if (x0 + lane < g.bins_x) row[x0 + lane + 1] = (uint16_t)(at + __popc(m & (0xFFFFFFFFu >> (31 - lane))));
+      at += __popc(m);
+    }
+  }
+  __syncthreads();
+  for (int x = tid; x < pitch; x += blockDim.x) {
+    uint32_t at = 0;
+    for (int y = 1; y <= g.bin_rows; y++) { at += s_sum[y * pitch + x]; s_sum[y * pitch + x] = (uint16_t)at; }
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ bool any_live(const Band& g, const uint16_t* s_sum, const BinSpan& s) {
+  const int pitch = g.bins_x + 1;
+  const uint16_t *top = s_sum + (s.by0 - g.bin_row0) * pitch + s.bx0, *bottom = top + s.h * pitch;
+  return (int)bottom[s.w] - (int)bottom[0] - (int)top[s.w] + (int)top[0] != 0;
 }
 // The few bins of a lane's own splat that it goes into, as bits in the order of its span; zero for a wide splat.
 template <bool WHOLE>
@@ -223,6 +253,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
   extern __shared__ __align__(16) unsigned long long s_alive[];   // [bins], then [bins] counts
   const int bins = band_bins(g), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_alive + (WHOLE ? 0 : bins));
+  uint16_t* s_sum = reinterpret_cast<uint16_t*>(s_cnt + bins);   // of a chunk behind the first
   __shared__ uint32_t s_live[2][COUNT_THREADS / 32], s_warp[32];
   for (int i = tid; i < bins; i += COUNT_THREADS) s_cnt[i] = 0u;
   if (!WHOLE) load_alive(v, g, s_alive);
@@ -231,6 +262,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
     if (v.first_band) { t.st[S_SLOT] = v.words ? v.words[CW_BASE + v.chunk] : 0u; if (!v.words || v.chunk == 0) t.st[S_OVER] = 0u; }
   }
   __syncthreads();
+  if (!WHOLE && v.alive) sum_live(g, s_alive, s_sum);
   uint32_t r0, r1;
   view_ranks(v, r0, r1);
   const uint32_t len = run_len(r1 - r0, gridDim.x);
@@ -239,8 +271,9 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
   int parity = 0;
   RankReader<WHOLE> ranks(v, g, v.order, begin, end);
   for (uint64_t at = begin; at < end; at += COUNT_THREADS, parity ^= 1) {
-    const Rank k = ranks.next();
+    Rank k = ranks.next();
     tiles += k.tiles;
+    if (!WHOLE && v.alive && k.span.count && !any_live(g, s_sum, k.span)) k.span.count = 0;
     const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
     for (uint32_t b = take; b; b &= b - 1u) atomicAdd(&s_cnt[own_bin(g, k, __ffs(b) - 1)], 1u);
     const bool wide = wide_bins<WHOLE>(s_alive, g, k, [&](int, uint32_t, int bin) { atomicAdd(&s_cnt[bin], 1u); });
@@ -653,7 +686,7 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
     const int tiles = (std::min((row + g.bin_rows) * BIN_W, c->tiles_y) - row * BIN_W) * c->tiles_x, scan_blocks = div_up(tiles, SCAN_TILES);
 #define L(WHOLE) do { \
     const size_t alive_bytes = WHOLE ? 0 : bins * sizeof(unsigned long long); \
-    launch_next(bin_count_kernel<WHOLE>, blocks, COUNT_THREADS, alive_bytes + bins * sizeof(uint32_t), s, v, g, t, c->depth_keys); \
+    launch_next(bin_count_kernel<WHOLE>, blocks, COUNT_THREADS, alive_bytes + bins * sizeof(uint32_t) + (WHOLE ? 0 : live_sums_bytes(g)), s, v, g, t, c->depth_keys); \
     launch_next(bin_rows_kernel, div_up(bins, ROWS_BINS), ROWS_THREADS, 0, s, blocks, bins, cap, t); \
     launch_next(bin_scatter_kernel<WHOLE>, blocks, L1_THREADS, alive_bytes + bins * (L1_WARPS + 1) * sizeof(uint32_t), s, v, g, t, cap, c->depth_keys, c->keys, c->tile_off); \
     launch_next(item_count_kernel<WHOLE>, item_blocks, L2_THREADS, 0, s, v, g, t, cap, c->keys, c->vals, c->keys_sorted); } while (0)
