@@ -7,6 +7,7 @@
 // many blur taps are spent per output. The loss kernel streams down column strips and pays for a halo in one direction
 // only; every blur is register-tiled (a thread makes four consecutive outputs from a fourteen-wide sliding window).
 #include "common.cuh"
+#include <algorithm>
 
 namespace b2k {
 namespace {
@@ -31,7 +32,7 @@ struct LossArgs {
 };
 
 // ---- The loss kernel --------------------------------------------------------------------------------------------------
-// One CTA owns a strip of STRIP_W output columns and a segment of rows, all three channels, and walks the segment four rows at
+// One CTA owns a strip of STRIP_W output columns and a segment of rows, all three channels (or one, in a small image), and walks the segment four rows at
 // a time. Both blurs are separable, so only the horizontal direction pays for a halo: the row-blurred moments and the
 // derivative maps of the last RING rows live in shared-memory rings, and the four stages of the chain run side by side as a
 // pipeline, each on its own warps (six to a channel) and on its own rows, with one barrier per four rows:
@@ -48,7 +49,7 @@ struct LossArgs {
 // (fp32x2) with operands that lie in pairs as they are stored: prediction and target side by side, and so their means, their
 // squares, and the two maps with a per-pixel factor; the product moment and the third map are paired over two rows (A) or two
 // columns (C). A thread makes four or eight outputs from one window, so that a value read from shared memory feeds eleven to
-// forty-four multiply-adds. Measured against the same pipeline with scalar multiply-adds and a CTA per channel: 187 -> 129 us on
+// forty-four multiply-adds. Measured against the same pipeline with scalar multiply-adds and a CTA per channel: 187 -> 124 us on
 // a 1920x1080 view, 101 -> 96 us on a masked 1024x1024 one, 26 -> 21 us on 333x217. Other arrangements on 1920x1080: packed,
 // a CTA per channel 133 to 147; channels of one CTA with a barrier each 130; the pairs in plain order (two-way bank conflicts in
 // stages A and D) 139; two columns per thread in stage B 142.
@@ -60,8 +61,7 @@ constexpr int RING = 18;                      // rows of a ring: the 14 a column
 constexpr int BV_S = STRIP_ST + 16;           // row stride of stage C's output: the last row window overruns into zero padding
 constexpr int PX_RING = 32;                   // rows of the ring that keeps pixels for stage D: a + 7 down to a - 22 are in use
 constexpr int PX_S = 64;                      // its columns: STRIP_W, padded likewise
-constexpr int CH_WARPS = 6, STRIP_THREADS = 3 * CH_WARPS * 32;
-constexpr int STRIP_CTAS_PER_SM = 1;
+constexpr int CH_WARPS = 6, CH_THREADS = CH_WARPS * 32;
 static_assert(STRIP_ST == 64 && STRIP_IN >= STRIP_W + 4 * HALO && STRIP_IN % 4 == 0, "strip geometry");
 
 // One ring row of row-blurred moments, and one of derivative maps: everything of a row behind one address.
@@ -80,12 +80,13 @@ struct ChannelShare {
   float2 b12[2][STRIP_ROWS][BV_S];        // [buffer] the maps blurred down the column
   float b0[2][STRIP_ROWS][BV_S];
 };
+template <int CHANNELS>
 struct StripShare {
-  ChannelShare ch[3];
+  ChannelShare ch[CHANNELS];
   float out[2][STRIP_ROWS][PX_S][4];      // [buffer] gradient of the step's pixels
   float red[20];
 };
-static_assert(sizeof(StripShare) % 16 == 0 && sizeof(StripShare) <= 227 * 1024 && STRIP_THREADS / 32 <= 20, "one CTA per SM");
+static_assert(sizeof(StripShare<3>) % 16 == 0 && sizeof(StripShare<1>) % 16 == 0 && sizeof(StripShare<3>) <= 227 * 1024, "one CTA per SM");
 
 __device__ __forceinline__ int ring_slot(int row) { return (row + RING * 256) % RING; }
 template <class ROW>
@@ -98,45 +99,57 @@ __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x,
 __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 
 // MASKED: per-pixel weights or the target's alpha scale the loss, or there is an alpha lane.
-template <bool MASKED>
-__global__ void __launch_bounds__(STRIP_THREADS, STRIP_CTAS_PER_SM) photometric_strip_kernel(const float4* __restrict__ pred, const uint32_t* __restrict__ gt,
+// CHANNELS: 3, or 1 with a CTA per channel, which a small image has SMs to spare for.
+template <bool MASKED, int CHANNELS>
+__global__ void __launch_bounds__(CHANNELS * CH_THREADS, 1) photometric_strip_kernel(const float4* __restrict__ pred, const uint32_t* __restrict__ gt,
                                                                           const uint8_t* __restrict__ weights, int W, int H, int seg_rows, LossArgs lp,
                                                                           Gauss2 gauss, float4* __restrict__ v_out, float* __restrict__ loss_accum) {
   extern __shared__ __align__(16) unsigned char s_bytes[];
-  StripShare& all = *reinterpret_cast<StripShare*>(s_bytes);
-  const int tid = threadIdx.x, lane = tid & 31, c = (tid >> 5) / CH_WARPS, warp = (tid >> 5) % CH_WARPS;   // channel, role
-  ChannelShare& sh = all.ch[c];
+  constexpr int THREADS = CHANNELS * CH_THREADS;
+  StripShare<CHANNELS>& all = *reinterpret_cast<StripShare<CHANNELS>*>(s_bytes);
+  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) % CH_WARPS;   // warp: role
+  const int held = CHANNELS == 1 ? 0 : (tid >> 5) / CH_WARPS, c = CHANNELS == 1 ? (int)blockIdx.z : held;   // the CTA's channel, the image's
+  ChannelShare& sh = all.ch[held];
   const int x0 = blockIdx.x * STRIP_W, y0 = blockIdx.y * seg_rows, y1 = min(y0 + seg_rows, H);
   const int x_end = min(x0 + STRIP_W, W);
   const float norm = lp.scale / (3.f * (float)W * (float)H);
   const float alpha_norm = lp.match_alpha_weight * lp.scale / ((float)W * (float)H);
 
-  for (int i = tid; i < (int)(sizeof(StripShare) / 16); i += STRIP_THREADS) reinterpret_cast<float4*>(s_bytes)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = tid; i < (int)(sizeof(all) / 16); i += THREADS) reinterpret_cast<float4*>(s_bytes)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   after_previous();
   __syncthreads();
-  // The input pixel a thread fetches (zero outside the image and in the row pad): which one, and whether its column is inside
+  // The input pixels a thread fetches (zero outside the image and in the row pad): which, and whether their columns are inside
   // the image, does not change from step to step.
-  const int f_row = tid / STRIP_IN, f_col = tid - f_row * STRIP_IN, f_x = x0 - 2 * HALO + f_col;
-  const bool f_thread = tid < STRIP_ROWS * STRIP_IN;
-  const bool f_ok = f_thread && f_col < STRIP_W + 4 * HALO && f_x >= 0 && f_x < W;
-  static_assert(STRIP_ROWS * STRIP_IN <= STRIP_THREADS, "one pixel a thread");
-  float3 f_p = make_float3(0.f, 0.f, 0.f);
-  uint32_t f_t = 0xFF000000u;
+  constexpr int FETCH = (STRIP_ROWS * STRIP_IN + THREADS - 1) / THREADS;
+  float3 f_p[FETCH];
+  uint32_t f_t[FETCH];
   auto fetch = [&](int row0) {
-    const int y = row0 + f_row;
-    f_p = make_float3(0.f, 0.f, 0.f); f_t = 0xFF000000u;   // an opaque black target is zero with any background
-    if (f_ok && y >= 0 && y < H) { const size_t q = (size_t)y * W + f_x; f_t = gt[q]; const float4 v = pred[q]; f_p = make_float3(v.x, v.y, v.z); }
+#pragma unroll
+    for (int u = 0; u < FETCH; u++) {
+      const int e = tid + u * THREADS, row = e / STRIP_IN, col = e - row * STRIP_IN, x = x0 - 2 * HALO + col, y = row0 + row;
+      f_p[u] = make_float3(0.f, 0.f, 0.f); f_t[u] = 0xFF000000u;   // an opaque black target is zero with any background
+      if (e < STRIP_ROWS * STRIP_IN && col < STRIP_W + 4 * HALO && (unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H) {
+        const size_t q = (size_t)y * W + x;
+        f_t[u] = gt[q];
+        if constexpr (CHANNELS == 1) f_p[u].x = reinterpret_cast<const float*>(pred)[q * 4 + c];
+        else { const float4 v = pred[q]; f_p[u] = make_float3(v.x, v.y, v.z); }
+      }
+    }
   };
   auto store = [&](int buf, int row0) {
-    if (!f_thread) return;
-    const float p[3] = {f_p.x, f_p.y, f_p.z};
-    const float behind = lp.composite ? 1.f - byte_unit(f_t, 3) : 0.f;
-    const int px = f_col - 2 * HALO, slot = (row0 + f_row) & (PX_RING - 1);
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const float2 v = make_float2(p[k], byte_unit(f_t, k) + behind * lp.bg[k]);
-      all.ch[k].in[buf][f_row][pair_at(f_col)] = v;
-      if (px >= 0 && px < PX_S) all.ch[k].px[slot][pair_at(px)] = v;
+    for (int u = 0; u < FETCH; u++) {
+      const int e = tid + u * THREADS, row = e / STRIP_IN, col = e - row * STRIP_IN, px = col - 2 * HALO, slot = (row0 + row) & (PX_RING - 1);
+      if (e >= STRIP_ROWS * STRIP_IN) break;
+      const float p[3] = {f_p[u].x, f_p[u].y, f_p[u].z};
+      const float behind = lp.composite ? 1.f - byte_unit(f_t[u], 3) : 0.f;
+#pragma unroll
+      for (int k = 0; k < CHANNELS; k++) {
+        const int channel = CHANNELS == 1 ? c : k;
+        const float2 v = make_float2(p[k], byte_unit(f_t[u], channel) + behind * lp.bg[channel]);
+        all.ch[k].in[buf][row][pair_at(col)] = v;
+        if (px >= 0 && px < PX_S) all.ch[k].px[slot][pair_at(px)] = v;
+      }
     }
   };
   fetch(y0 - 2 * HALO);
@@ -343,8 +356,18 @@ __global__ void __launch_bounds__(STRIP_THREADS, STRIP_CTAS_PER_SM) photometric_
     }
     {
       // The gradient rows that stage D left in the step before.
-      const int row = tid / PX_S, col = tid - row * PX_S, y = d - STRIP_ROWS + row, x = x0 + col;
-      if (row < STRIP_ROWS && col < STRIP_W && x < x_end && y >= y0 && y < y1) v_out[(size_t)y * W + x] = *reinterpret_cast<const float4*>(all.out[buf ^ 1][row][col]);
+      constexpr int DRAIN = (STRIP_ROWS * PX_S + THREADS - 1) / THREADS;
+#pragma unroll
+      for (int u = 0; u < DRAIN; u++) {
+        const int e = tid + u * THREADS, row = e / PX_S, col = e - row * PX_S, y = d - STRIP_ROWS + row, x = x0 + col;
+        if (row >= STRIP_ROWS || col >= STRIP_W || x >= x_end || y < y0 || y >= y1) continue;
+        const float4 v = *reinterpret_cast<const float4*>(all.out[buf ^ 1][row][col]);
+        if constexpr (CHANNELS == 1) {
+          float* out = reinterpret_cast<float*>(v_out + (size_t)y * W + x);
+          out[c] = c == 0 ? v.x : (c == 1 ? v.y : v.z);
+          if (c == 0) out[3] = v.w;
+        } else v_out[(size_t)y * W + x] = v;
+      }
     }
     if (more) store(buf ^ 1, a + STRIP_ROWS);   // consumed by stage A in the next step
     __syncthreads();
@@ -354,7 +377,7 @@ __global__ void __launch_bounds__(STRIP_THREADS, STRIP_CTAS_PER_SM) photometric_
   __syncthreads();
   if (tid == 0) {
     float t = 0.f;
-    for (int i = 0; i < STRIP_THREADS / 32; i++) t += all.red[i];
+    for (int i = 0; i < THREADS / 32; i++) t += all.red[i];
     if (t != 0.f) atomicAdd(loss_accum, t);
   }
 }
@@ -495,21 +518,32 @@ extern "C" int b2k_loss_photometric(const B2kCtx* c, const B2kLoss* lp, b2k_stre
   static bool attr_set[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !attr_set[dev]) {
-    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare)));
-    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare)));
+    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare<3>)));
+    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare<3>)));
+    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare<1>)));
+    B2K_CUDA(cudaFuncSetAttribute(photometric_strip_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StripShare<1>)));
     attr_set[dev] = true;
   }
-  // Rows per segment: as many segments as fill the resident CTA slots once (a second, partial wave costs more than the
-  // eight pipeline-fill steps a longer segment amortises), in whole steps of four rows.
-  const int strips = div_up(c->W, STRIP_W), slots = sm_count() * STRIP_CTAS_PER_SM;
-  int segs = slots / strips;
-  segs = segs < 1 ? 1 : segs;
-  int seg_rows = div_up(div_up(c->H, segs), STRIP_ROWS) * STRIP_ROWS;
-  if (seg_rows < 8) seg_rows = 8;
-  const dim3 grid(strips, div_up(c->H, seg_rows));
-#define L(MASKED) launch_next(photometric_strip_kernel<MASKED>, grid, STRIP_THREADS, sizeof(StripShare), (cudaStream_t)stream, (const float4*)c->out_rgba, lp->rgba, lp->weights, c->W, c->H, \
-    seg_rows, a, g2, (float4*)c->v_out, c->loss_accum)
-  if (lp->weights || lp->mask || lp->alpha_lane) L(true); else L(false);
+  // Rows per segment: as many segments as there are SMs (a second, partial wave costs more than the eight pipeline-fill
+  // steps a longer segment amortises), in whole steps of four rows.
+  const int strips = div_up(c->W, STRIP_W);
+  auto rows_for = [&](int columns) {   // CTAs side by side
+    const int segs = std::max(1, sm_count() / columns);
+    return std::max(8, div_up(div_up(c->H, segs), STRIP_ROWS) * STRIP_ROWS);
+  };
+  auto steps_of = [](int rows) { return 8 + rows / STRIP_ROWS; };
+  // A CTA per channel steps faster than one of three channels (64x64 0.96 against 1.46 us a step, 333x217 with mask 1.7 against
+  // 2.0) but leaves a third of the SMs to cut the rows for: taken where its segments are at most a fifth longer in steps (64x64
+  // 14.6 -> 9.6 us, 200x150 14.9 -> 11.8; 333x217 would go from 22.4 to 27.2).
+  const int rows3 = rows_for(strips), rows1 = rows_for(strips * 3);
+  const bool apart = steps_of(rows1) * 5 <= steps_of(rows3) * 6 && strips * 3 <= sm_count();
+  const int seg_rows = apart ? rows1 : rows3;
+  const dim3 grid(strips, div_up(c->H, seg_rows), apart ? 3 : 1);
+#define L(MASKED, CHANNELS) launch_next(photometric_strip_kernel<MASKED, CHANNELS>, grid, CHANNELS * CH_THREADS, sizeof(StripShare<CHANNELS>), (cudaStream_t)stream, \
+    (const float4*)c->out_rgba, lp->rgba, lp->weights, c->W, c->H, seg_rows, a, g2, (float4*)c->v_out, c->loss_accum)
+  const bool masked = lp->weights || lp->mask || lp->alpha_lane;
+  if (apart) { if (masked) L(true, 1); else L(false, 1); }
+  else { if (masked) L(true, 3); else L(false, 3); }
 #undef L
   return check_launch();
 }
