@@ -381,7 +381,6 @@ def bench_train(args, cfg, scene, cams, device, rank, world, barrier, max_over_r
         phases["views_fastest_rank"] = -max_over_ranks(-mine_ms["views"])
         phases["update_form"] = ("Adam from the accumulator (one rank)" if world == 1 else "all-reduce + replicated Adam" if args.allreduce
                                  else "sharded: peer-memory reduce + Adam + parameter broadcast in one kernel")
-    tile_bits = info["tile_bits"]
     cap = info["isect_cap"]
     tr.close()
     del tr
@@ -399,11 +398,8 @@ def bench_train(args, cfg, scene, cams, device, rank, world, barrier, max_over_r
     views_per_step = n_views
     value = views_per_step * args.steps / (ms / 1e3)
     e2e_value = views_per_step * args.steps / (ms_e2e / 1e3)
-    from b2ctrain_b200 import api as _api
-    passes = int(_api.lib().b2k_sort_passes(int(tile_bits)))
-    launches_view = 1 + (1 + 12 + 2 + 3 * passes + 1) + 1 + 1 + 1 + 1 + 1
-    if args.chunks > 1:   # projection 2, depth sort 13, chunk words 1, per chunk 6 (+1 after the first) + the tile-sort passes, then loss .. projection backward
-        launches_view = 2 + 13 + 1 + sum(6 + (2 if ch else 0) + 3 * passes for ch in range(args.chunks)) + 5
+    # the view's loss cleared, render, loss, accumulate, backward (clear, list, replay), touched list (clear, list), projection backward or update
+    launches_view = 1 + render_launches(n, W, H, args.chunks) + 2 + 3 + (2 if n > 8192 else 1) + 1
     launches = args.steps * (n_views * launches_view + (0 if (world == 1 and n_views == 1) else world))   # all ranks
     res = {"metric": "train views/s", "value": value, "unit": "views/s", "ms_per_step": ms / args.steps, "scaling": "strong",
            "config": {"views_per_step": views_per_step, "render": ("front to back in %d depth chunks, saturated tiles stop emitting" % args.chunks) if args.chunks > 1 else "whole view binned before compositing", "splats": n, "sh_degree": deg, "resolution": f"{W}x{H}", "parallelism": f"dp{world} by view",
@@ -496,13 +492,12 @@ def stage_roofline(args, tr, cams, targets, mine, stats, clocks=None):
     nv = len(views)
     st = stats[0]
     V, I, Is, Ib, n, P, tiles = st["V"], st["I"], st["I_sorted"], st["I_b"], m.n, ctx.W * ctx.H, ctx.n_tiles
-    passes = int(api.lib().b2k_sort_passes(int(ctx.tile_bits)))
     alg = {"project": 48 * n + 12 * K * V + 48 * V + 28 * n,
-           "bin_sort": 16 * n * 4 + 24 * n + 8 * I + 16 * I * passes + 4 * I + 8 * tiles,
+           "bin_sort": 16 * n * 3 + 56 * n + 8 * I + 8 * tiles,   # three sort passes; boxes and records; lists and tile ids
            "raster_fwd": 52 * Ib + 36 * P,
-           # chunked renderer: records + colours of every splat, the depth sort, per chunk the rank / box words, then emit, tile
-           # sort and ranges on the pairs that survive, and the compositing of what the ranges hold
-           "render_chunked": (48 * n + 12 * K * V + 64 * n) + 16 * n * 4 + 20 * n + (8 + 16 * passes + 4) * Is + 8 * tiles * max(chunks, 1) + 52 * Ib + 36 * P,
+           # chunked renderer: records + colours of every splat, three passes of the depth sort, the box of every splat once, the
+           # lists of the hits that survive, ranges, and the compositing of what the ranges hold
+           "render_chunked": (48 * n + 12 * K * V + 72 * n) + 16 * n * 3 + 20 * n + 4 * Is + 8 * tiles * max(chunks, 1) + 52 * Ib + 36 * P,
            "loss": 20 * P + 16 * P, "raster_bwd": 28 * P + 52 * Ib + 52 * touched,
            "proj_bwd": (52 + 48 + 12 * K) * touched + 2 * 4 * (11 + 3 * K) * touched + 8 * n}   # flags of all splats, records of the touched ones
     # Loss: per pixel and channel 64/54 x (5 + 5 + 3) + 3 eleven-tap blurs (the strip's horizontal halo) = 203 FMA, plus the
@@ -515,8 +510,7 @@ def stage_roofline(args, tr, cams, targets, mine, stats, clocks=None):
             api.project_splats(ctx, m, api.RenderParams(cams[v], sh_degree=m.degree, bwd_info=True))
             ph += np.array(api.bin_and_sort_profile(ctx, m))
         ph /= nv
-        stages["bin_sort"]["phases_ms"] = {"depth_sort": ph[0], "scan_emit": ph[1], "tile_count": [ph[2 + 2 * p] for p in range(min(passes, 3))],
-                                           "tile_scatter": [ph[3 + 2 * p] for p in range(min(passes, 3))], "tile_ranges": ph[8], "total": ph[9]}
+        stages["bin_sort"]["phases_ms"] = {"depth_sort": ph[0], "lists": ph[1], "tile_ids": ph[8], "total": ph[9]}
     props = torch.cuda.get_device_properties(ctx.last_idx.device)
     sm_mhz = float((clocks or {}).get("sm_mhz") or 1965.0)   # median SM clock sampled during the timed region
     fp32_peak = 2 * 128 * props.multi_processor_count * sm_mhz * 1e6
@@ -530,22 +524,16 @@ def stage_roofline(args, tr, cams, targets, mine, stats, clocks=None):
                                "note": "stages of the timed form (" + ("chunked" if chunks > 1 else "whole-view") + " rendering) back to back on one stream; the "
                                        "optimizer update (once per step) is not included"}
     # The roofline object: the single-kernel stage with the largest time per view (the chunked renderer is ~70 launches, not one kernel).
-    kernel_of = {"project": "project_kernel", "raster_fwd": "raster_fwd_kernel", "loss": "photometric_strip_kernel", "raster_bwd": "raster_bwd_kernel", "proj_bwd": "proj_bwd_kernel"}
+    kernel_of = {"project": "project_kernel", "raster_fwd": "raster_fwd_half_kernel", "loss": "photometric_strip_kernel", "raster_bwd": "raster_bwd_kernel", "proj_bwd": "proj_bwd_kernel"}
     kernel_ms = {kernel_of[nm]: stages[nm]["ms"] for nm in names if nm in kernel_of}
-    if chunks <= 1:
-        kernel_ms["radix_scatter_kernel"] = float(np.mean(stages["bin_sort"]["phases_ms"]["tile_scatter"]))
     top = max(kernel_ms, key=kernel_ms.get)
     per_launch_ms = kernel_ms[top]
-    if top == "radix_scatter_kernel":
-        stage, bytes_launch, traffic = "bin_sort", 16 * I, int(16.7 * I)   # dram read + write per launch: ncu capture at half the splat count, scaled by pairs
-        note = f"{passes} launches per view on I = {I} pairs; 16 B per pair per launch"
-    else:
-        stage = [k for k, v in kernel_of.items() if v == top][0]
-        bytes_launch, traffic, note = alg[stage], None, "one launch per view"
-        if top == "raster_bwd_kernel":
-            traffic = int(80.7 * Ib)   # dram read + write per launch from an ncu capture at half the splat count (100.3 MB at I_b = 1,243,915), scaled by fragments
-        elif top == "photometric_strip_kernel":
-            traffic = int(22.7 * P)    # ncu capture of one 1920x1080 view: 43.1 MB read + 4.0 MB written (the gradient image stays in L2)
+    stage = [k for k, v in kernel_of.items() if v == top][0]
+    bytes_launch, traffic, note = alg[stage], None, "one launch per view"
+    if top == "raster_bwd_kernel":
+        traffic = int(80.7 * Ib)   # dram read + write per launch, from an ncu capture of a view of 500k splats at 1920x1080, scaled by fragments
+    elif top == "photometric_strip_kernel":
+        traffic = int(22.7 * P)   # the same capture: images in, gradient image out as far as it left the L2
     a = bytes_launch / (per_launch_ms * 1e-3) / 1e9
     hbm_view = {"achieved": a, "peak": hbm, "unit": "GB/s", "frac": a / hbm, "traffic": traffic, "peak_source": peak_src, "algorithmic_bytes_per_launch": int(bytes_launch)}
     if stage in flop:   # the compositing kernels are bound by FP32 issue: that roof is the headline, the HBM figure rides beside it
@@ -561,6 +549,16 @@ def stage_roofline(args, tr, cams, targets, mine, stats, clocks=None):
     return roof, stages
 
 
+def render_launches(n, W, H, chunks):
+    """Kernels of one render: the whole view (clear, projection, big boxes, depth sort, binning, tile ids, compositing) or depth
+    chunks (projection, depth sort, chunk words, per chunk binning and compositing). The binning takes seven kernels per band
+    of at most 2,048 bins of 8x8 tiles; the depth sort one up to 8,192 splats, ten above."""
+    bins_x, bin_rows = -(-W // 64), -(-H // 64)
+    bands = -(-bin_rows // (2048 // bins_x))
+    sort = 1 if n <= 8192 else 10
+    return 1 + sort + 1 + chunks * (7 * bands + 1) if chunks > 1 else 3 + sort + 7 * bands + 2
+
+
 def bench_render(args, scene, cams, device, rank, world, barrier, max_over_ranks, sampler):
     import torch
     from b2ctrain_b200.trainer import Renderer
@@ -569,7 +567,7 @@ def bench_render(args, scene, cams, device, rank, world, barrier, max_over_ranks
     from b2ctrain_b200 import host_trainer as ht
     r = Renderer(scene, W, H, device, rank, world, want_depth=True, render_chunks=args.chunks)
     stats = presize(r, cams, mine, None, False)   # counts of the first camera through the Python mirror, outside any timed region
-    tile_bits, r_cap = r.ctx.tile_bits, r.ctx.isect_cap
+    r_cap = r.ctx.isect_cap
     del r
     torch.cuda.empty_cache()
     # The timed loops run in the C++ host (b2c::StreamRenderer). e2e: every camera's RGBA8 image and depth map land in pinned
@@ -604,11 +602,7 @@ def bench_render(args, scene, cams, device, rank, world, barrier, max_over_ranks
     ms_e2e = timed(args.steps, True)
     hr.close()
     mpix = len(cams) * W * H * args.steps / 1e6
-    from b2ctrain_b200 import api as _api
-    passes = int(_api.lib().b2k_sort_passes(int(tile_bits)))
-    launches_view = 1 + (1 + 12 + 2 + 3 * passes + 1) + 1
-    if args.chunks > 1:
-        launches_view = 2 + 13 + 1 + sum(6 + (2 if ch else 0) + 3 * passes for ch in range(args.chunks))
+    launches_view = render_launches(scene["n"], W, H, args.chunks)
     return {"metric": "render Mpix/s", "value": mpix / (ms / 1e3), "unit": "Mpix/s", "ms_per_step": ms / args.steps, "scaling": "strong",
             "config": {"cameras": len(cams), "render": ("front to back in %d depth chunks, saturated tiles stop emitting" % args.chunks) if args.chunks > 1 else "whole view binned before compositing", "splats": scene["n"], "sh_degree": scene["degree"], "resolution": f"{W}x{H}", "parallelism": f"cameras over {world} GPUs", "cameras_in_flight": lanes,
                        "l2_policy": "inputs larger than L2", "scene_counts_view0": stats[0] if stats else None},
