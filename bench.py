@@ -531,9 +531,9 @@ def stage_roofline(args, tr, cams, targets, mine, stats, clocks=None):
     stage = [k for k, v in kernel_of.items() if v == top][0]
     bytes_launch, traffic, note = alg[stage], None, "one launch per view"
     if top == "raster_bwd_kernel":
-        traffic = int(80.7 * Ib)   # dram read + write per launch, from an ncu capture of a view of 500k splats at 1920x1080, scaled by fragments
+        traffic = int(63.8 * Ib)   # dram read + write per launch, from an ncu capture of a view of 500k splats at 1920x1080, scaled by fragments
     elif top == "photometric_strip_kernel":
-        traffic = int(22.7 * P)   # the same capture: images in, gradient image out as far as it left the L2
+        traffic = int(21.3 * P)   # the same capture: images in, gradient image out as far as it left the L2
     a = bytes_launch / (per_launch_ms * 1e-3) / 1e9
     hbm_view = {"achieved": a, "peak": hbm, "unit": "GB/s", "frac": a / hbm, "traffic": traffic, "peak_source": peak_src, "algorithmic_bytes_per_launch": int(bytes_launch)}
     if stage in flop:   # the compositing kernels are bound by FP32 issue: that roof is the headline, the HBM figure rides beside it
