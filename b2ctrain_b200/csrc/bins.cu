@@ -566,30 +566,29 @@ __global__ void __launch_bounds__(COL_GROUPS * BIN_TILES) item_columns_kernel(Ba
 }
 
 // Ranges of the band's tiles, row-major: block b starts behind the hits of the blocks before it. Empty tiles get (0, 0);
-// ranges end with the buffers. The last block to finish moves the view's slot on.
+// ranges end with the buffers. The last block to finish moves the view's slot on. All loads are issued before the one
+// scan of the block (two scans one after the other and a fence took 5.4 to 7.8 us, this 2.8 to 5.8).
 __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, Tables t, uint32_t cap, uint2* __restrict__ ranges, uint32_t* __restrict__ num_isect) {
   after_previous();
-  __shared__ uint32_t s_warp[32];
-  const int tid = threadIdx.x;
+  __shared__ uint32_t s_warp[32], s_slot;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int tile0 = g.bin_row0 * BIN_W * g.tiles_x, tiles = (min((g.bin_row0 + g.bin_rows) * BIN_W, g.tiles_y) - g.bin_row0 * BIN_W) * g.tiles_x;
   const int mine = blockIdx.x * SCAN_TILES + tid;
-  uint32_t all, before;
-  {
-    const uint32_t seg = tid < (int)gridDim.x ? t.segments[tid] : 0u;
-    const uint32_t incl = block_scan(seg, s_warp, all);
-    __shared__ uint32_t s_before;
-    if (tid == (int)blockIdx.x) s_before = incl - seg;
-    __syncthreads();
-    before = s_before;
-  }
-  const uint32_t slot = t.st[S_SLOT];
   const uint32_t c = mine < tiles ? ranges[tile0 + mine].x : 0u;
+  if (tid == 0) s_slot = t.st[S_SLOT];
+  uint32_t all = 0, before = 0;   // hits of the band, and of the blocks before this one: every warp adds them up for itself
+  {
+    uint32_t seg[BINS_SEGMENTS / 32];
+#pragma unroll
+    for (int u = 0; u < BINS_SEGMENTS / 32; u++) seg[u] = u * 32 + lane < (int)gridDim.x ? t.segments[u * 32 + lane] : 0u;
+#pragma unroll
+    for (int u = 0; u < BINS_SEGMENTS / 32; u++) { all += seg[u]; before += u * 32 + lane < (int)blockIdx.x ? seg[u] : 0u; }
+    all = __reduce_add_sync(FULL, all); before = __reduce_add_sync(FULL, before);
+  }
   uint32_t total;
-  const uint32_t start = slot + before + block_scan(c, s_warp, total) - c;
+  const uint32_t in_block = block_scan(c, s_warp, total) - c, slot = s_slot, start = slot + before + in_block;
   if (mine < tiles) ranges[tile0 + mine] = c ? make_uint2(min(start, cap), min(start + c, cap)) : make_uint2(0u, 0u);
-  __threadfence();
-  __syncthreads();
-  if (tid == 0 && atomicAdd(t.st + S_DONE_TILES, 1u) == gridDim.x - 1u) {   // every block has read the slot
+  if (tid == 0 && atomicAdd(t.st + S_DONE_TILES, 1u) == gridDim.x - 1u) {   // every block has read the slot (its first thread did)
     uint32_t end = slot + all;
     if (v.last_band) {
       if (v.words) { v.words[CW_COUNT + v.chunk] = end - v.words[CW_BASE + v.chunk]; v.words[CW_BASE + v.chunk + 1] = (end + 31u) & ~31u; }
