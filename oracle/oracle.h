@@ -95,11 +95,14 @@ double orc_loss(int W, int H, const double* pred, const uint32_t* gt, const uint
                 double* v_out);
 
 /* Per-pixel reverse replay (raster_bwd.cu:11-143). v_splat: [n][13] (zeroed here, lanes: xy 2, conic 3, rgb 3,
- * opacity 1, refine 1, feat 3 (always 0)); vis_flag: [n]; vis_weight: [n] (zeroed here). */
+ * opacity 1, refine 1, feat 3 (always 0)); vis_flag: [n]; vis_weight: [n] (zeroed here). bound (optional): [n][13], for each
+ * of the first ten lanes what single-precision rounding may move it by, however much the lane itself cancels (a running
+ * error analysis; from_totals: of a replay that finds the colour behind a fragment by subtracting from the pixel's total);
+ * lane 10 counts the splat's fragment-pixels on the edge of the opacity cut, which may fall either way. */
 void orc_raster_bwd(int n, int W, int H, const double* geo, const double* col, const uint32_t* vals_sorted,
                     const uint32_t* tile_ranges, const double* bg, const double* out_rgba, const double* out_T,
                     const uint32_t* last_idx, const double* v_out, double* v_splat, uint32_t* vis_flag,
-                    double* vis_weight);
+                    double* vis_weight, double* bound, int from_totals);
 
 /* Projection backward (optim.cu:100-297): screen-space lanes -> parameter gradients [n][11+3K]
  * (pos 3, opacity 1, quat 4, log-scale 3, SH K*3), the layout of OptimParams::grad_out (optim.cu:292-297). */

@@ -202,7 +202,7 @@ extern "C" double orc_step(int n, int degree, int active_degree, const float* po
   }
   if (backward && gt && grad) {
     std::vector<double> v_splat((size_t)n * 13), visw(n); std::vector<uint32_t> vis(n);
-    orc_raster_bwd(n, W, H, geo.data(), col.data(), vals.data(), ranges.data(), bg, rgba, outT.data(), last.data(), v_out.data(), v_splat.data(), vis.data(), visw.data());
+    orc_raster_bwd(n, W, H, geo.data(), col.data(), vals.data(), ranges.data(), bg, rgba, outT.data(), last.data(), v_out.data(), v_splat.data(), vis.data(), visw.data(), nullptr, 0);
     orc_proj_bwd(n, degree, active_degree, pos_op, quat, lscale, sh, cam, v_splat.data(), vis.data(), tile_count.data(), grad);
   }
   return loss;

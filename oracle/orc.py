@@ -263,11 +263,12 @@ def eval_metrics(W, H, pred, gt, mask_weighted=False):
     return se, ssim_sum
 
 
-def raster_bwd(n, W, H, geo, col, vals, ranges, bg, rgba, T, last, v_out):
+def raster_bwd(n, W, H, geo, col, vals, ranges, bg, rgba, T, last, v_out, bound=None, from_totals=False):
+    """bound: optional float64 [n][13] that receives the error bounds of a single-precision replay (oracle.h)."""
     v_splat = np.zeros((n, 13)); vis = np.zeros(n, np.uint32); visw = np.zeros(n)
     vals = _u32(vals) if len(vals) else np.zeros(1, np.uint32)
     lib().orc_raster_bwd(n, W, H, _p(_f64(geo)), _p(_f64(col)), _p(vals), _p(_u32(ranges)), _p(_f64(bg)), _p(_f64(rgba)),
-                         _p(_f64(T)), _p(_u32(last)), _p(_f64(v_out)), _p(v_splat), _p(vis), _p(visw))
+                         _p(_f64(T)), _p(_u32(last)), _p(_f64(v_out)), _p(v_splat), _p(vis), _p(visw), _p(bound), int(from_totals))
     return v_splat, vis, visw
 
 
