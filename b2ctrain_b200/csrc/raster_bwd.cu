@@ -98,12 +98,14 @@ __global__ void __launch_bounds__(256) bwd_items_kernel(const uint2* __restrict_
 
 // Short segments: the same list, and the segments' colour sums that the forward left turned into the colour behind each
 // boundary. One warp per tile walks its checkpoints from the far end: slot j of a range holds the sums of segment j - 1,
-// slot 0 those of the last one; afterwards slot j holds the colour from boundary j on.
+// slot 0 those of the last one; afterwards slot j holds the colour from boundary j on. A second backward on the same forward
+// finds them so (BWD_SUMMED, which the forward clears and the replay sets) and lists the items only.
 __global__ void __launch_bounds__(128) bwd_suffix_kernel(const uint2* __restrict__ tile_ranges, int n_tiles, int n_chunks, int seg_shift, uint2* __restrict__ items,
                                                          uint32_t* __restrict__ work, float4* __restrict__ ckpt) {
   after_previous();
   const int lane = threadIdx.x & 31, tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (tile >= n_tiles) return;
+  const bool summed = work[BWD_SUMMED] != 0u;
   float3 acc[2] = {make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
   for (int c = n_chunks - 1; c >= 0; c--) {
     const int q = c * n_tiles + tile;
@@ -114,6 +116,7 @@ __global__ void __launch_bounds__(128) bwd_suffix_kernel(const uint2* __restrict
     if (lane == 0) base = atomicAdd(work, segs);
     base = __shfl_sync(FULL, base, 0);
     for (uint32_t s = lane; s < segs; s += 32) items[base + s] = make_uint2((uint32_t)q, s);
+    if (summed) continue;
     float4* at = ckpt + (size_t)ckpt_slot(range.x, q, 0u, seg_shift) * RT_PX + lane * 2;
     float4 own[2] = {at[0], at[1]};   // the sums of the segment behind the boundary that comes next
     for (uint32_t hi = segs; hi > 0u;) {   // boundaries hi - 1 .. hi - count, four in flight
@@ -157,6 +160,7 @@ __global__ void __launch_bounds__(BWD_WARPS * 32, BWD_CTAS_PER_SM) raster_bwd_ke
   const int red_p = lane % RED_P, red_row = lane / RED_P;   // in a reduction: this lane's pair and tile row
   const float2 aspect2 = f2(aspect);
   const uint32_t n_items = work[0];
+  if (FORM == SHORT && blockIdx.x == 0 && threadIdx.x == 0) work[BWD_SUMMED] = 1u;
 
   for (;;) {
     uint32_t it = 0;

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
-    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc) {
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
   const float2 pcx = make_float2((float)px + 0.5f, (float)px + 0.5f), pcy = make_float2((float)py + 0.5f, (float)py + 0.5f);
   const uint2 range = tile_ranges[tile];
   const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
+  if (CKPT == PER_SEGMENT && first && tile == 0 && in_tile == 0) bwd_work[BWD_SUMMED] = 0u;
   if (CHUNKED && !first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
   float T = 1.f, r = 0.f, g = 0.f, b = 0.f, zs = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;   // f: composited feature lanes (raster_fwd.cu:52)
   bool open = inside;   // the pixel can take another fragment
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
-    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc) {
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   // FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
@@ -261,6 +262,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   const float2 pcx = make_float2((float)px0 + 0.5f, (float)px0 + 1.5f), pcy = splat2((float)py + 0.5f);
   const uint2 range = tile_ranges[tile];
   const bool first = chunk == 0, final = chunk == n_chunks - 1;
+  if (CKPT == PER_SEGMENT && first && tile == 0 && lane == 0) bwd_work[BWD_SUMMED] = 0u;
   if (!first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
   float2 T = splat2(1.f), r = splat2(0.f), g = r, b = r, zs = r;   // of the two pixels
   bool open[2] = {in0, in1};   // the pixel can take another fragment
@@ -440,7 +442,7 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
   const bool chunked = n_chunks > 1, halves = n_chunks <= 2;   // (measured above)
 #define ARGS s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, \
     (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, \
-    seg_shift_of(c->n_tiles), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr
+    seg_shift_of(c->n_tiles), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr, bwd_work_ptr(c)
 #define HALF(B, D, C, F) launch_next(raster_fwd_half_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_TILES), FWD_WARPS * 32, 0, ARGS)
 #define L(B, D, F) do { if (!chunked) HALF(B, D, false, F); else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
     else launch_next(raster_fwd_kernel<B, D, (F) && (B) == NONE>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS); } while (0)

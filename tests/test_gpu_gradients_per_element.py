@@ -102,3 +102,27 @@ def test_opacity_gradients_of_a_step_of_several_views_per_element(W, H):
     got = tr.grad[:, 3].cpu().numpy().astype(np.float64)
     sure = edge == 0
     assert sure.mean() > 0.5 and np.all(np.abs(got - total)[sure] <= limit[sure])
+
+
+@pytest.mark.parametrize("chunks", [1, 3])
+@pytest.mark.parametrize("W,H", [(512, 512), (520, 512)])       # segments of 32 and of 128 fragments
+def test_backward_repeats_on_one_forward(W, H, chunks):
+    """Two backwards with different pixel gradients after one forward, the second through the scaled entry: each gives the
+    lanes of its own pixel gradients."""
+    import ctypes as C
+    scene, cam = stack_scene(300, W, H)
+    n, bg, rng = scene["n"], (0.2, 0.1, 0.3), np.random.Generator(np.random.PCG64(21))
+    h = Harness(scene, cam, bg=bg)
+    h.forward()
+    ctx = h.api.RenderCtx("cuda:0")
+    ctx.setup(W, H, h.model.cap, n_chunks=chunks)
+    h.api.render_forward(ctx, h.model, h.rp)
+    for scale in (1.0, 8.0, 1.0):
+        v_out = (rng.standard_normal((W * H, 4)) * 1e-3).astype(np.float32)
+        want, bound, _ = wanted(n, W, H, h, v_out, bg, W > 512)
+        ctx.v_out.copy_(h.torch.from_numpy(v_out * np.float32(scale)))
+        ctx.v_splat.zero_()
+        ctx.vis_flag.zero_()
+        cs, ms, opts = ctx.struct(), h.model.struct(), h.rp.struct()
+        h.api._check(h.api.lib().b2k_raster_bwd_scaled(C.byref(cs), C.byref(ms), C.byref(opts), C.c_float(scale), h.api._stream(None)), "b2k_raster_bwd_scaled")
+        check(ctx.v_splat[:n].cpu().numpy().astype(np.float64), want, bound, scale)
