@@ -256,9 +256,10 @@ void StepTrainer::update(cudaStream_t stream) {
   grad_clear_pending_ = true;
 }
 
-// Work on another stream than the last step's follows that step.
+// Work on any stream follows the last step, also where the handle is the same: cudaStreamPerThread names a stream of each host
+// thread's own, and a destroyed stream's handle may come back while its work still runs.
 void StepTrainer::follow(cudaStream_t stream) {
-  if (stepped_ && stream != last_stream_) cuda(cudaStreamWaitEvent(stream, done_evt_, 0), "wait");
+  if (stepped_) cuda(cudaStreamWaitEvent(stream, done_evt_, 0), "wait");
 }
 // The kernel writes rows straight into pinned memory, a slice at a time, while the slice before is copied out.
 void StepTrainer::download(float* pos_op, float* quat, float* lscale, float* sh) {
@@ -304,7 +305,7 @@ void StepTrainer::step(const std::vector<int>& all, cudaStream_t stream, bool fr
   if (profile) cuda(cudaEventRecord(mark_[1], stream), "record");
   if (!fused) update(stream);
   cuda(cudaEventRecord(done_evt_, stream), "record");
-  last_stream_ = stream; stepped_ = true;
+  stepped_ = true;
   if (profile) {
     cuda(cudaEventRecord(mark_[2], stream), "record");
     cuda(cudaEventSynchronize(mark_[2]), "sync");

@@ -107,7 +107,6 @@ class StepTrainer {
   std::vector<DevBuf<uint32_t>> stage_;
   std::vector<cudaEvent_t> staged_evt_, free_evt_, lane_done_;
   cudaEvent_t binned_evt_ = nullptr, counted_evt_ = nullptr, done_evt_ = nullptr;
-  cudaStream_t last_stream_ = nullptr;
   bool stepped_ = false;
   cudaEvent_t start_evt_ = nullptr, cleared_evt_ = nullptr, mark_[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   PinnedBuf<uint32_t> h_isect_;

@@ -85,6 +85,35 @@ def test_cpp_step_matches_python_step(views, lanes, cap):
 
 
 @pytest.mark.gpu
+def test_steps_from_several_host_threads_on_their_own_default_streams():
+    """cudaStreamPerThread is one handle for as many streams as there are host threads: steps that take turns between threads
+    on it, and a read of the loss on it, follow one another all the same."""
+    import threading
+    import torch
+    from b2ctrain_b200 import host_trainer as ht
+    PER_THREAD = 2                       # cudaStreamPerThread
+    scene, cams, targets = case(n=20000)
+    runs = []
+    for stream, threads in ((torch.cuda.current_stream().cuda_stream, False), (PER_THREAD, True)):
+        t = ht.HostTrainer(scene, 160, 120, views_in_flight=1, lr_mean=1e-4, sparse=True)
+        for cam, target in zip(cams, targets):
+            t.add_view(cam, target)
+        for k in range(8):
+            if threads:
+                worker = threading.Thread(target=t.step, args=([k % 6], stream))
+                worker.start()
+                worker.join()
+            else:
+                t.step([k % 6], stream)
+        runs.append((t.read_loss(stream), t.download()))
+        t.close()
+    (la, a), (lb, b) = runs
+    assert abs(la[2] - lb[2]) <= 1e-4 * abs(la[2]) and la[3] == lb[3]
+    for k in ("pos_op", "quat", "lscale", "sh"):   # eight steps whose small gradients follow the order of the atomics: a norm, not the largest
+        assert np.linalg.norm(a[k] - b[k]) <= 1e-4 * np.linalg.norm(a[k]), k
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("shard", [1, 0])
 def test_two_rank_data_parallel_step_matches_one_rank(shard):
     """Two ranks on two GPUs (child processes, NCCL without NVLS): three steps of six views sharded by view, with the
