@@ -61,7 +61,7 @@ extern "C" int b2ch_trainer_add_view(void* h, const B2kCamera* cam, const uint32
 }
 
 extern "C" int b2ch_trainer_step(void* h, const int32_t* views, int32_t n_views, void* stream, int32_t from_host) {
-  return guarded([&] { ((StepTrainer*)h)->step(std::vector<int>(views, views + n_views), (cudaStream_t)stream, from_host != 0); });
+  return guarded([&] { ((StepTrainer*)h)->step_ahead(std::vector<int>(views, views + n_views), (cudaStream_t)stream, from_host != 0); });
 }
 
 extern "C" int b2ch_trainer_read_loss(void* h, float* out16, void* stream) { return guarded([&] { ((StepTrainer*)h)->read_loss(out16, (cudaStream_t)stream); }); }

@@ -32,7 +32,8 @@ void* b2ch_trainer_create(int32_t n, int32_t degree, const float* pos_op, const 
 void b2ch_trainer_destroy(void* trainer);
 /* Registers a view (camera record with intrinsics for W x H, packed RGBA8 target on the host); returns its index or -1. */
 int b2ch_trainer_add_view(void* trainer, const B2kCamera* cam, const uint32_t* rgba);
-/* One optimisation step over the listed views (the whole step's list on every rank). */
+/* One optimisation step over the listed views (the whole step's list on every rank). With one view it returns once the view is
+ * known to have fitted; every other call on the handle follows the step on whatever stream it is given. */
 int b2ch_trainer_step(void* trainer, const int32_t* views, int32_t n_views, void* stream, int32_t from_host);
 int b2ch_trainer_read_loss(void* trainer, float* out16, void* stream);
 int b2ch_trainer_set_profile(void* trainer, int32_t on);

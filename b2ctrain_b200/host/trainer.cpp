@@ -286,6 +286,11 @@ void StepTrainer::download(float* pos_op, float* quat, float* lscale, float* sh)
 void StepTrainer::settle() { if (stepped_) cuda(cudaEventSynchronize(done_evt_), "sync"); }
 
 void StepTrainer::step(const std::vector<int>& all, cudaStream_t stream, bool from_host) {
+  step_ahead(all, stream, from_host);
+  if (world == 1 && all.size() == 1) settle();
+}
+
+void StepTrainer::step_ahead(const std::vector<int>& all, cudaStream_t stream, bool from_host) {
   if (all.empty()) return;
   follow(stream);
   model.adam_t++;

@@ -55,12 +55,15 @@ class StepTrainer {
   // and on the lanes' own streams, which are joined back into `stream` before the update; the call returns after one
   // host readback per step (the lanes' largest intersection totals), having redone the views with larger buffers if one
   // did not fit. from_host: targets are copied in from pinned memory, double-buffered on a copy stream.
-  // When a step of one view returns, its intersections have fitted and its work may still run on the stream; the methods below
-  // order themselves behind it on whatever stream they are given. settle() waits for it: before `model` is read in another way.
+  // A one-view step is complete when the call returns; the update of a step of several views may still run on `stream`.
+  void step(const std::vector<int>& views, cudaStream_t stream, bool from_host = false);
+  // step() that returns as soon as the views are known to have fitted, the rest of the work still on the stream: for callers
+  // that reach the model through this object's methods only (they order themselves behind it, on any stream), or call
+  // settle(), which waits for it, before they read `model` themselves.
+  void step_ahead(const std::vector<int>& views, cudaStream_t stream, bool from_host = false);
   void settle();
   // The model's splats as rows (pos_op, quat, lscale [n][4], sh [n][K][3]) into host memory of any kind.
   void download(float* pos_op, float* quat, float* lscale, float* sh);
-  void step(const std::vector<int>& views, cudaStream_t stream, bool from_host = false);
   // loss_accum of lane 0 after the last step: [0] last view's loss, [2] sum over this rank's views, [3] their count.
   void read_loss(float* out16, cudaStream_t stream);
   // The refinement statistics made global over the ranks (max: refine_norm, max_screen; sum: vis_count, vis_weight).

@@ -88,3 +88,47 @@ def test_reference_test_harness_compiles_against_the_mirror_headers(tmp_path):
     r = subprocess.run(["g++", "-std=c++17", "-O1", f"-I{HOST}", f"-I{cuda}/include", str(src), "-o", str(tmp_path / "ref_harness"), f"-L{pkg}", "-lb2chost", "-lb2k",
                         f"-L{cuda}/lib64", "-lcudart", f"-Wl,-rpath,{pkg}", f"-Wl,-rpath,{cuda}/lib64"], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-3000:]
+
+
+STEP_PROGRAM = r"""
+#include "trainer.h"
+#include <cstdio>
+#include <random>
+using namespace b2c;
+int main() {
+  std::mt19937 rng(7);
+  std::uniform_real_distribution<float> u(-1.f, 1.f);
+  SplatCloud c; c.resize(100000, 1);
+  for (float& p : c.pos) p = u(rng);
+  for (float& s : c.log_scale) s = -4.f;
+  for (float& s : c.sh) s = 0.5f * u(rng);
+  Camera cam; cam.width = 1280; cam.height = 720; cam.fx = cam.fy = 720.f; cam.cx = 640.f; cam.cy = 360.f; cam.t[2] = 4.f; cam.update_pos();
+  std::vector<uint32_t> target(1280 * 720, 0xFF808080u);
+  StepConfig cfg; cfg.views_in_flight = 1; cfg.isect_cap = 1 << 24; cfg.lr_mean = 1e-4f;
+  StepTrainer tr(c, 1280, 720, cfg);
+  tr.add_view(cam, target.data());
+  cudaStream_t s = nullptr;
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return 2;
+  int running = 0;
+  for (int k = 0; k < 4; k++) { tr.step({0}, s); running += cudaStreamQuery(s) != cudaSuccess; }
+  printf("running after step: %d\n", running);
+  tr.step_ahead({0}, s);
+  tr.settle();
+  printf("running after settle: %d\n", (int)(cudaStreamQuery(s) != cudaSuccess));
+  return 0;
+}
+"""
+
+
+@pytest.mark.gpu
+def test_one_view_step_is_complete_when_it_returns(tmp_path):
+    """StepTrainer::step of one view leaves nothing on the stream, so that a caller may read the public model at once, in any way."""
+    build_harness()
+    src, exe = tmp_path / "step.cpp", tmp_path / "step"
+    src.write_text(STEP_PROGRAM)
+    cuda, pkg = os.environ.get("CUDA_HOME", "/usr/local/cuda"), os.path.join(ROOT, "b2ctrain_b200")
+    r = subprocess.run(["g++", "-std=c++17", "-O1", f"-I{HOST}", f"-I{cuda}/include", str(src), "-o", str(exe), f"-L{pkg}", "-lb2chost", "-lb2k", f"-L{cuda}/lib64", "-lcudart",
+                        f"-Wl,-rpath,{pkg}", f"-Wl,-rpath,{cuda}/lib64"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.split("\n")[:2] == ["running after step: 0", "running after settle: 0"], r.stdout + r.stderr
