@@ -227,16 +227,17 @@ __device__ __forceinline__ bool wide_bins(const unsigned long long* s_alive, con
   return took;
 }
 
-// Inclusive scan over the block of one value per thread (at most 1024 threads); s_warp holds 32 words. Synchronises.
-__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t& total) {
+// Inclusive scan over the block of one value per thread (at most 1024 threads); s_warp holds 32 values. Synchronises.
+template <class T>
+__device__ __forceinline__ T block_scan(T v, T* s_warp, T& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(FULL, v, o); if (lane >= o) v += u; }
+  for (int o = 1; o < 32; o <<= 1) { const T u = __shfl_up_sync(FULL, v, o); if (lane >= o) v += u; }
   __syncthreads();
   if (lane == 31) s_warp[warp] = v;
   __syncthreads();
-  uint32_t pre = 0, all = 0;
-  for (int w = 0; w < warps; w++) { const uint32_t t = s_warp[w]; if (w < warp) pre += t; all += t; }
+  T pre = 0, all = 0;
+  for (int w = 0; w < warps; w++) { const T t = s_warp[w]; if (w < warp) pre += t; all += t; }
   total = all;
   return v + pre;
 }
@@ -300,11 +301,14 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
 }
 
 // A warp per bin turns the bin's counts into offsets. The last block to finish lays out the band: first pair of every bin,
-// and the items (runs of pairs of one bin) that level 2 works on. An item is 256 pairs unless that made too many.
+// and the items (runs of pairs of one bin) that level 2 works on. An item is 256 pairs unless that made too many. The band's pairs
+// are added up in 64 bits: two million splats over a whole 4K image make more than 2^32, and a sum that wrapped around would
+// give items that are too short, and more of them than there is room for.
 constexpr int ROWS_THREADS = 512, ROWS_BINS = ROWS_THREADS / 32, ROWS_PER = 16;   // at most 32 * ROWS_PER blocks of level 1
 __global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int bins, uint32_t cap, Tables t) {
   after_previous();
   __shared__ uint32_t s_warp[32];
+  __shared__ unsigned long long s_sums[32];
   __shared__ bool s_last;
   const int tid = threadIdx.x, lane = tid & 31, bin = blockIdx.x * ROWS_BINS + (tid >> 5);
   if (bin < bins) {
@@ -330,26 +334,28 @@ __global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int 
   if (!s_last) return;
   __threadfence();
   constexpr int PER = MAX_BINS / ROWS_THREADS;
-  uint32_t tot[PER], sum = 0;
+  uint32_t tot[PER];
+  unsigned long long sum = 0, pairs;
 #pragma unroll
   for (int u = 0; u < PER; u++) { const int b = tid * PER + u; tot[u] = b < bins ? __ldcg(t.totals + b) : 0u; sum += tot[u]; }
-  uint32_t pairs;
-  uint32_t at = block_scan(sum, s_warp, pairs) - sum;
-  const uint32_t room = MAX_ITEMS - (uint32_t)bins, len = 256u * (pairs / (256u * room) + 1u);   // items <= pairs / len + bins <= MAX_ITEMS
+  unsigned long long at = block_scan(sum, s_sums, pairs) - sum;
+  const uint32_t room = MAX_ITEMS - (uint32_t)bins, len = 256u * (uint32_t)(pairs / (256u * room) + 1u);   // items <= pairs / len + bins <= MAX_ITEMS
   uint32_t items = 0, n_items;
 #pragma unroll
   for (int u = 0; u < PER; u++) items += (tot[u] + len - 1u) / len;
   uint32_t it = block_scan(items, s_warp, n_items) - items;
+  auto in_cap = [&](unsigned long long p) { return (uint32_t)(p < cap ? p : cap); };   // pairs beyond the buffers are not written
 #pragma unroll
   for (int u = 0; u < PER; u++) {
     const int b = tid * PER + u;
-    if (b < bins) { t.base[b] = at; t.first_item[b] = it; }
+    if (b < bins) { t.base[b] = in_cap(at); t.first_item[b] = it; }
     at += tot[u]; it += (tot[u] + len - 1u) / len;
   }
   if (tid == 0) {
-    t.base[bins] = pairs; t.first_item[bins] = n_items;
-    t.st[S_PAIRS] = pairs; t.st[S_ITEMS] = n_items; t.st[S_ITEM_LEN] = len;
-    if (pairs > cap && pairs > t.st[S_OVER]) t.st[S_OVER] = pairs;   // level 1's own pairs did not fit: the caller grows the buffers
+    const uint32_t total = (uint32_t)(pairs < 0xFFFFFFFFull ? pairs : 0xFFFFFFFFull);
+    t.base[bins] = in_cap(pairs); t.first_item[bins] = n_items;
+    t.st[S_PAIRS] = total; t.st[S_ITEMS] = n_items; t.st[S_ITEM_LEN] = len;
+    if (total > cap && total > t.st[S_OVER]) t.st[S_OVER] = total;   // level 1's own pairs did not fit: the caller grows the buffers
   }
   if (tid < BINS_SEGMENTS) t.segments[tid] = 0u;
 }
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
   }
   if (begin >= end && !(offsets && blockIdx.x == gridDim.x - 1)) return;
   for (int i = tid; i < bins * L1_WARPS; i += L1_THREADS) s_bits[i] = 0u;
-  for (int i = tid; i < bins; i += L1_THREADS) s_next[i] = t.base[i] + t.cells[(size_t)i * gridDim.x + blockIdx.x];
+  for (int i = tid; i < bins; i += L1_THREADS) s_next[i] = (uint32_t)min((unsigned long long)t.base[i] + t.cells[(size_t)i * gridDim.x + blockIdx.x], (unsigned long long)cap);
   if (!WHOLE) load_alive(v, g, s_alive);
   uint32_t tiles_before = 0;
   if (offsets) {
@@ -450,8 +456,9 @@ struct Item { uint32_t first, end; int bx, by; };
 __device__ __forceinline__ Item item_of(const Tables& t, const Band& g, uint32_t it, uint32_t cap) {
   const uint32_t bin = t.item_bin[it], len = t.st[S_ITEM_LEN];
   Item m;
-  m.first = t.base[bin] + (it - t.first_item[bin]) * len;
-  m.end = min(min(m.first + len, t.base[bin + 1]), cap);
+  const unsigned long long first = t.base[bin] + (unsigned long long)(it - t.first_item[bin]) * len;
+  m.first = (uint32_t)min(first, (unsigned long long)cap);
+  m.end = (uint32_t)min(first + len, (unsigned long long)min(t.base[bin + 1], cap));
   m.bx = (int)bin % g.bins_x; m.by = g.bin_row0 + (int)bin / g.bins_x;
   return m;
 }

@@ -239,3 +239,36 @@ def test_model_rows(degree, first, count):
     torch.cuda.synchronize()
     for t, k in zip(out, ("pos_op", "quat", "lscale", "sh")):
         assert np.array_equal(t[:-4].numpy(), want[k][first : first + count].reshape(-1)) and bool((t[-4:] == 7.0).all())
+
+
+def test_more_bin_pairs_than_a_word_counts():
+    """Three million splats over a whole 4K image: 4.6 billion pairs of (splat, 8x8-tile bin) in the second chunk. The view
+    reports that it does not fit, writes nothing outside its buffers, and the context renders an ordinary view afterwards."""
+    import ctypes as C
+    import torch
+    from b2ctrain_b200 import api
+    n, W, H = 3_000_000, 3840, 2160
+    cam = scenes.look_at_camera((0.0, 0.0, 4.0), W, H, float(H))
+    m = api.Model("cuda:0")
+    rng = np.random.Generator(np.random.PCG64(2))
+    scene = scenes.make_splats(20000, 0, 3)
+    big = {k: np.tile(v, (n // 20000,) + (1,) * (v.ndim - 1)) for k, v in scene.items() if hasattr(v, "ndim")}
+    big["pos_op"][:, :3] = rng.uniform(-0.1, 0.1, (n, 3))
+    big["pos_op"][:, 3] = -4.0
+    big["lscale"][:, :3] = 2.0
+    m.upload(dict(scene, n=n, **big))
+    ctx = api.RenderCtx("cuda:0")
+    ctx.setup(W, H, m.cap, isect_cap=1 << 20, n_chunks=2)
+    rp = api.RenderParams(cam, sh_degree=0, bwd_info=False)
+    api.render_chunked(ctx, m, rp, sync=False)
+    total = C.c_uint32(0)
+    cs = ctx.struct()
+    assert api.lib().b2k_read_num_isect(C.byref(cs), api._stream(None), C.byref(total)) == api.B2K_ERR_OVERFLOW
+    assert total.value > 1 << 20
+    small = api.Model("cuda:0").upload(scenes.floor_for_cameras(scene, [cam]))
+    fresh = api.RenderCtx("cuda:0")
+    fresh.setup(W, H, small.cap, isect_cap=1 << 22, n_chunks=2)
+    ctx._alloc_isect(1 << 22)
+    for c in (ctx, fresh):
+        api.render_chunked(c, small, rp, sync=True)
+    assert torch.equal(ctx.out_rgba, fresh.out_rgba) and ctx.num_isect == fresh.num_isect
