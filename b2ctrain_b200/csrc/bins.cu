@@ -60,7 +60,7 @@ struct Tables {
   uint32_t* segments;    // [BINS_SEGMENTS] hits per tile_scan block
   uint32_t* st;          // [16] see S_*
 };
-enum { S_PAIRS = 0, S_ITEMS, S_ITEM_LEN, S_DONE_ROWS, S_DONE_TILES, S_SLOT, S_OVER, S_TOTAL };
+enum { S_PAIRS = 0, S_ITEMS, S_ITEM_LEN, S_DONE_ROWS, S_DONE_TILES, S_SLOT, S_OVER, S_TOTAL, S_KEPT };
 
 __device__ __forceinline__ void view_ranks(const View& v, uint32_t& r0, uint32_t& r1) {
   if (!v.words) { r0 = 0u; r1 = (uint32_t)v.n; return; }
@@ -113,6 +113,17 @@ __device__ __forceinline__ BinSpan span_of(const Box& b, const Band& g) {
   s.count = s.w * s.h;
   return s;
 }
+
+// Where level 1's pairs lie. A view has fewer pairs than hits as a rule, but a long needle's box overlaps many bins without a hit,
+// and a chunk does not test them: pairs may be more than the lists have room for although the hits are not. Up to `cap` they lie
+// in the first buffer, and the second and third keep their hit words. More of them, up to ROOM times the lists' room, go on into
+// those; then no hit words are kept (S_KEPT) and the emission makes the tests again. Still more do not fit, and their number is reported.
+constexpr uint32_t ROOM = 3;
+struct Pairs {
+  uint32_t *first, *lo, *hi; uint32_t cap;   // cap: entries of each buffer
+  __host__ __device__ __forceinline__ uint32_t room() const { return (uint32_t)((unsigned long long)cap * ROOM < 0xFFFF0000ull ? (unsigned long long)cap * ROOM : cap > 0xFFFF0000u ? cap : 0xFFFF0000u); }
+  __device__ __forceinline__ uint32_t* at(uint32_t p) const { return p < cap ? first + p : p - cap < cap ? lo + (p - cap) : hi + (p - cap - cap); }   // p < room()
+};
 
 // One rank's splat as level 1 sees it.
 struct Rank { uint32_t splat, tiles; uint4 hi; Box box; BinSpan span; };
@@ -305,7 +316,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
 // are added up in 64 bits: two million splats over a whole 4K image make more than 2^32, and a sum that wrapped around would
 // give items that are too short, and more of them than there is room for.
 constexpr int ROWS_THREADS = 512, ROWS_BINS = ROWS_THREADS / 32, ROWS_PER = 16;   // at most 32 * ROWS_PER blocks of level 1
-__global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int bins, uint32_t cap, Tables t) {
+__global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int bins, uint32_t cap, uint32_t room_pairs, Tables t) {
   after_previous();
   __shared__ uint32_t s_warp[32];
   __shared__ unsigned long long s_sums[32];
@@ -344,18 +355,19 @@ __global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int 
 #pragma unroll
   for (int u = 0; u < PER; u++) items += (tot[u] + len - 1u) / len;
   uint32_t it = block_scan(items, s_warp, n_items) - items;
-  auto in_cap = [&](unsigned long long p) { return (uint32_t)(p < cap ? p : cap); };   // pairs beyond the buffers are not written
+  const bool kept = pairs <= cap || pairs > room_pairs;   // the last: a view that does not fit, cut short
+  auto in_room = [&](unsigned long long p) { return (uint32_t)(p < room_pairs ? p : room_pairs); };   // pairs beyond the buffers are not written
 #pragma unroll
   for (int u = 0; u < PER; u++) {
     const int b = tid * PER + u;
-    if (b < bins) { t.base[b] = in_cap(at); t.first_item[b] = it; }
+    if (b < bins) { t.base[b] = in_room(at); t.first_item[b] = it; }
     at += tot[u]; it += (tot[u] + len - 1u) / len;
   }
   if (tid == 0) {
     const uint32_t total = (uint32_t)(pairs < 0xFFFFFFFFull ? pairs : 0xFFFFFFFFull);
-    t.base[bins] = in_cap(pairs); t.first_item[bins] = n_items;
-    t.st[S_PAIRS] = total; t.st[S_ITEMS] = n_items; t.st[S_ITEM_LEN] = len;
-    if (total > cap && total > t.st[S_OVER]) t.st[S_OVER] = total;   // level 1's own pairs did not fit: the caller grows the buffers
+    t.base[bins] = in_room(pairs); t.first_item[bins] = n_items;
+    t.st[S_PAIRS] = total; t.st[S_ITEMS] = n_items; t.st[S_ITEM_LEN] = len; t.st[S_KEPT] = kept ? 1u : 0u;
+    if (total > room_pairs && total > t.st[S_OVER]) t.st[S_OVER] = total;   // level 1's own pairs did not fit: the caller grows the buffers
   }
   if (tid < BINS_SEGMENTS) t.segments[tid] = 0u;
 }
@@ -363,7 +375,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) bin_rows_kernel(int blocks, int 
 // The pairs to their places, stable: bit l of s_bits[bin][w] says that lane l of warp w adds a pair to the bin in this round.
 // The splat that adds a bin's first pair of the round afterwards moves the bin's place on and clears its bits.
 template <bool WHOLE>
-__global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ live, uint32_t* __restrict__ pairs,
+__global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g, Tables t, Pairs pr, const uint32_t* __restrict__ live,
                                                                  uint32_t* __restrict__ tile_off) {
   after_previous();
   extern __shared__ __align__(16) uint32_t s_bits[];   // [bins][8], then [bins] alive words, then [bins] next free place
@@ -377,13 +389,14 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
   const uint64_t begin = (uint64_t)r0 + (uint64_t)blockIdx.x * len;
   const uint64_t end = WHOLE ? (begin + len < (uint64_t)r1 ? begin + len : (uint64_t)r1) : begin + t.block_sums[blockIdx.x];
   const bool offsets = WHOLE && v.first_band;
+  const uint32_t room = pr.room();
   for (int b = blockIdx.x * L1_WARPS + warp; b < bins; b += gridDim.x * L1_WARPS) {   // the items' bins, a warp per bin
     const uint32_t e = t.first_item[b + 1];
     for (uint32_t k = t.first_item[b] + (uint32_t)lane; k < e; k += 32) t.item_bin[k] = (uint32_t)b;
   }
   if (begin >= end && !(offsets && blockIdx.x == gridDim.x - 1)) return;
   for (int i = tid; i < bins * L1_WARPS; i += L1_THREADS) s_bits[i] = 0u;
-  for (int i = tid; i < bins; i += L1_THREADS) s_next[i] = (uint32_t)min((unsigned long long)t.base[i] + t.cells[(size_t)i * gridDim.x + blockIdx.x], (unsigned long long)cap);
+  for (int i = tid; i < bins; i += L1_THREADS) s_next[i] = (uint32_t)min((unsigned long long)t.base[i] + t.cells[(size_t)i * gridDim.x + blockIdx.x], (unsigned long long)room);
   if (!WHOLE) load_alive(v, g, s_alive);
   uint32_t tiles_before = 0;
   if (offsets) {
@@ -408,32 +421,37 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
     const uint32_t added = __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w) + __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
     if (added) { s_next[bin] += added; b4[0] = make_uint4(0u, 0u, 0u, 0u); b4[1] = make_uint4(0u, 0u, 0u, 0u); }
   };
-  RankReader<WHOLE> ranks(v, g, WHOLE ? v.order : live, begin, end);
-  for (uint64_t at = begin; at < end; at += L1_THREADS) {
-    const Rank k = ranks.next();
-    const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
-    for (uint32_t b = take; b; b &= b - 1u) atomicOr(&s_bits[own_bin(g, k, __ffs(b) - 1) * L1_WARPS + warp], 1u << lane);
-    wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t, int bin) { atomicOr(&s_bits[bin * L1_WARPS + warp], 1u << l); });
-    if (offsets) {
-      uint32_t total;
-      const uint32_t incl = block_scan(k.tiles, s_warp, total);
-      if (at + tid < end) tile_off[at + tid] = tiles_before + incl;
-      tiles_before += total;
+  auto spread = [&](auto put) {
+    RankReader<WHOLE> ranks(v, g, WHOLE ? v.order : live, begin, end);
+    for (uint64_t at = begin; at < end; at += L1_THREADS) {
+      const Rank k = ranks.next();
+      const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
+      for (uint32_t b = take; b; b &= b - 1u) atomicOr(&s_bits[own_bin(g, k, __ffs(b) - 1) * L1_WARPS + warp], 1u << lane);
+      wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t, int bin) { atomicOr(&s_bits[bin * L1_WARPS + warp], 1u << l); });
+      if (offsets) {
+        uint32_t total;
+        const uint32_t incl = block_scan(k.tiles, s_warp, total);
+        if (at + tid < end) tile_off[at + tid] = tiles_before + incl;
+        tiles_before += total;
+      }
+      const bool any_wide = __syncthreads_or(k.span.count > SERIAL_BINS);
+      uint32_t first = 0u;
+      for (uint32_t b = take; b; b &= b - 1u) {
+        const int bin = own_bin(g, k, __ffs(b) - 1);
+        const uint32_t n = earlier(bin, lane), pos = s_next[bin] + n;
+        put(pos, k.splat);
+        if (n == 0u) first |= b & (0u - b);
+      }
+      wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t splat, int bin) { const uint32_t pos = s_next[bin] + earlier(bin, l); put(pos, splat); });
+      __syncthreads();
+      if (any_wide) { for (int i = tid; i < bins; i += L1_THREADS) move_on(i); }
+      else { for (uint32_t b = first; b; b &= b - 1u) move_on(own_bin(g, k, __ffs(b) - 1)); }
+      __syncthreads();
     }
-    const bool any_wide = __syncthreads_or(k.span.count > SERIAL_BINS);
-    uint32_t first = 0u;
-    for (uint32_t b = take; b; b &= b - 1u) {
-      const int bin = own_bin(g, k, __ffs(b) - 1);
-      const uint32_t n = earlier(bin, lane), pos = s_next[bin] + n;
-      if (pos < cap) pairs[pos] = k.splat;
-      if (n == 0u) first |= b & (0u - b);
-    }
-    wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t splat, int bin) { const uint32_t pos = s_next[bin] + earlier(bin, l); if (pos < cap) pairs[pos] = splat; });
-    __syncthreads();
-    if (any_wide) { for (int i = tid; i < bins; i += L1_THREADS) move_on(i); }
-    else { for (uint32_t b = first; b; b &= b - 1u) move_on(own_bin(g, k, __ffs(b) - 1)); }
-    __syncthreads();
-  }
+  };
+  // (one of two loops: a test of the place against both limits inside it, and the kernel takes 42 us for 39)
+  if (t.st[S_KEPT]) spread([&](uint32_t pos, uint32_t splat) { if (pos < pr.cap) pr.first[pos] = splat; });
+  else spread([&](uint32_t pos, uint32_t splat) { if (pos < room) *pr.at(pos) = splat; });
   if (offsets && blockIdx.x == gridDim.x - 1 && tid == 0) t.st[S_TOTAL] = tiles_before;   // the view's hits, also when the pairs did not fit
 }
 
@@ -453,20 +471,19 @@ __device__ __forceinline__ uint32_t transpose_bits(uint32_t x) {
 
 // The pairs of one item and the bin's corner.
 struct Item { uint32_t first, end; int bx, by; };
-__device__ __forceinline__ Item item_of(const Tables& t, const Band& g, uint32_t it, uint32_t cap) {
+__device__ __forceinline__ Item item_of(const Tables& t, const Band& g, uint32_t it, uint32_t limit) {
   const uint32_t bin = t.item_bin[it], len = t.st[S_ITEM_LEN];
   Item m;
   const unsigned long long first = t.base[bin] + (unsigned long long)(it - t.first_item[bin]) * len;
-  m.first = (uint32_t)min(first, (unsigned long long)cap);
-  m.end = (uint32_t)min(first + len, (unsigned long long)min(t.base[bin + 1], cap));
+  m.first = (uint32_t)min(first, (unsigned long long)limit);
+  m.end = (uint32_t)min(first + len, (unsigned long long)min(t.base[bin + 1], limit));
   m.bx = (int)bin % g.bins_x; m.by = g.bin_row0 + (int)bin / g.bins_x;
   return m;
 }
 
 // Hit word of every pair of an item (bit = row * 8 + column of the tile in its bin), and the item's hits per tile.
 template <bool WHOLE>
-__global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ pairs, uint32_t* __restrict__ hit_lo,
-                                                                uint32_t* __restrict__ hit_hi) {
+__global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, Tables t, Pairs pr) {
   after_previous();
   struct WarpShare { float4 rec[64]; unsigned long long hits[32]; uint32_t unit[32 * BIN_W]; };   // unit: pair | row << 5 | columns << 8
   __shared__ WarpShare s_share[L2_WARPS];
@@ -474,15 +491,16 @@ __global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   WarpShare& ws = s_share[warp];
   const uint32_t n_items = t.st[S_ITEMS];
+  const bool kept = t.st[S_KEPT] != 0u;
   for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const Item m = item_of(t, g, it, cap);
+    const Item m = item_of(t, g, it, kept ? pr.cap : pr.room());
     const unsigned long long alive = !WHOLE && v.alive ? v.alive[m.by * g.bins_x + m.bx] : ~0ull;
     uint32_t c_lo = 0, c_hi = 0;   // this warp's hits on tiles `lane` and `lane + 32`
     for (uint32_t p0 = m.first; p0 < m.end; p0 += L2_THREADS) {
       const uint32_t p = p0 + tid;
       unsigned long long hits = 0ull, todo = 0ull;   // todo: tiles to test
       if (p < m.end) {
-        const uint32_t i = pairs[p];
+        const uint32_t i = kept ? pr.first[p] : *pr.at(p);
         const uint4 hi = v.hit_info[i];
         const Box b = box_of(hi);
         if (WHOLE && hi.z != 0xFFFFFFFFu) {
@@ -528,7 +546,7 @@ __global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, 
         hits |= ws.hits[lane];
         __syncwarp();
       }
-      if (p < m.end) { hit_lo[p] = (uint32_t)hits; hit_hi[p] = (uint32_t)(hits >> 32); }
+      if (kept && p < m.end) { pr.lo[p] = (uint32_t)hits; pr.hi[p] = (uint32_t)(hits >> 32); }
       c_lo += __popc(transpose_bits((uint32_t)hits)); c_hi += __popc(transpose_bits((uint32_t)(hits >> 32)));
     }
     s_cnt[warp][lane] = c_lo; s_cnt[warp][lane + 32] = c_hi;
@@ -605,17 +623,33 @@ __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, T
   }
 }
 
+// A pair's hit word by itself, where none was kept.
+template <bool WHOLE>
+__device__ __forceinline__ unsigned long long hits_again(const View& v, int bx, int by, unsigned long long alive, uint32_t i) {
+  const uint4 hi = v.hit_info[i];
+  const Box b = box_of(hi);
+  if (WHOLE && hi.z != 0xFFFFFFFFu) return mask_bits(hi, b, bx, by);
+  const float4 q0 = v.proj0[i], q1 = v.proj1[i];
+  const TileRec rec = make_tile_rec(q0.x, q0.y, q0.z, q0.w, q1.x, q1.w);
+  unsigned long long out = 0ull;
+  for (unsigned long long todo = rect_bits(b, bx, by) & alive; todo; todo &= todo - 1ull) {
+    const int tile = __ffsll((long long)todo) - 1;
+    if (tile_hit(bx * BIN_W + (tile & 7), by * BIN_W + (tile >> 3), rec)) out |= 1ull << tile;
+  }
+  return out;
+}
+
 // The hits of an item to their tiles' lists, in the order of the pairs: for each tile the warp takes the 32 pairs of one hit
 // word at a time, and the lanes with a hit write side by side.
-__global__ void __launch_bounds__(L2_THREADS) item_emit_kernel(Band g, Tables t, uint32_t cap, const uint32_t* __restrict__ pairs, const uint32_t* __restrict__ hit_lo,
-                                                               const uint32_t* __restrict__ hit_hi, const uint2* __restrict__ ranges, uint32_t* __restrict__ vals) {
-  after_previous();
-  __shared__ uint32_t s_splat[L2_THREADS], s_word[L2_WARPS][BIN_TILES];
+template <bool WHOLE, bool KEPT>
+__device__ __forceinline__ void emit_items(const View& v, const Band& g, const Tables& t, const Pairs& pr, const uint2* __restrict__ ranges, uint32_t* __restrict__ vals,
+                                           uint32_t (&s_splat)[L2_THREADS], uint32_t (&s_word)[L2_WARPS][BIN_TILES]) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lane_lt = (1u << lane) - 1u, n_items = t.st[S_ITEMS];
+  const uint32_t cap = pr.cap;
   constexpr int TPW = BIN_TILES / L2_WARPS;   // tiles a warp writes
   for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const Item m = item_of(t, g, it, cap);
+    const Item m = item_of(t, g, it, KEPT ? cap : pr.room());
     uint32_t next = 0;   // lane k < TPW: next place of the warp's k-th tile
     if (lane < TPW) {
       const int tile = warp * TPW + lane, x = m.bx * BIN_W + (tile & 7), y = m.by * BIN_W + (tile >> 3);
@@ -624,9 +658,18 @@ __global__ void __launch_bounds__(L2_THREADS) item_emit_kernel(Band g, Tables t,
     for (uint32_t p0 = m.first; p0 < m.end; p0 += L2_THREADS) {
       const uint32_t p = p0 + tid;
       const bool valid = p < m.end;
-      s_splat[tid] = valid ? pairs[p] : 0u;
-      s_word[warp][lane] = transpose_bits(valid ? hit_lo[p] : 0u);
-      s_word[warp][lane + 32] = transpose_bits(valid ? hit_hi[p] : 0u);
+      uint32_t splat = 0u, lo = 0u, hi = 0u;
+      if (valid) {
+        if constexpr (KEPT) { splat = pr.first[p]; lo = pr.lo[p]; hi = pr.hi[p]; }
+        else {
+          splat = *pr.at(p);
+          const unsigned long long hits = hits_again<WHOLE>(v, m.bx, m.by, !WHOLE && v.alive ? v.alive[m.by * g.bins_x + m.bx] : ~0ull, splat);
+          lo = (uint32_t)hits; hi = (uint32_t)(hits >> 32);
+        }
+      }
+      s_splat[tid] = splat;
+      s_word[warp][lane] = transpose_bits(lo);
+      s_word[warp][lane + 32] = transpose_bits(hi);
       __syncthreads();
 #pragma unroll
       for (int k = 0; k < TPW; k++) {
@@ -645,6 +688,13 @@ __global__ void __launch_bounds__(L2_THREADS) item_emit_kernel(Band g, Tables t,
     }
   }
 }
+template <bool WHOLE>
+__global__ void __launch_bounds__(L2_THREADS, 4) item_emit_kernel(View v, Band g, Tables t, Pairs pr, const uint2* __restrict__ ranges, uint32_t* __restrict__ vals) {
+  after_previous();
+  __shared__ uint32_t s_splat[L2_THREADS], s_word[L2_WARPS][BIN_TILES];
+  if (t.st[S_KEPT]) emit_items<WHOLE, true>(v, g, t, pr, ranges, vals, s_splat, s_word);
+  else emit_items<WHOLE, false>(v, g, t, pr, ranges, vals, s_splat, s_word);
+}
 
 // Tile ids of the sorted list, for callers of the whole-view binning: a warp per tile.
 __global__ void __launch_bounds__(256) fill_keys_kernel(int n_tiles, const uint2* __restrict__ ranges, uint32_t* __restrict__ keys) {
@@ -659,7 +709,7 @@ __global__ void __launch_bounds__(256) fill_keys_kernel(int n_tiles, const uint2
 }  // namespace
 
 // Bins the ranks of one depth chunk (words != nullptr) or of the whole view into vals_sorted and `ranges`. Level 1's pairs
-// take ctx->keys, the hit words ctx->vals and ctx->keys_sorted, a chunk's live splats the scratch of the depth sort.
+// take ctx->keys, the hit words (or more pairs) ctx->vals and ctx->keys_sorted, a chunk's live splats the scratch of the depth sort.
 int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, int hi_num, const unsigned long long* alive, uint32_t* tables, cudaStream_t s) {
   Tables t;
   t.cells = tables;
@@ -675,6 +725,7 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
     attr_set[dev] = true;
   }
   const uint32_t cap = (uint32_t)c->isect_cap;
+  const Pairs pr{c->keys, c->vals, c->keys_sorted, cap};
   uint2* ranges = (uint2*)c->tile_ranges + (words ? (size_t)chunk * c->n_tiles : 0);
   const int bins_x = div_up(c->tiles_x, BIN_W), bin_rows = div_up(c->tiles_y, BIN_W);
   if (bins_x > MAX_BINS) return B2K_ERR_UNSUPPORTED;   // tile boxes hold twelve bits of a tile's column: the caller's own limit is lower
@@ -693,15 +744,16 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
 #define L(WHOLE) do { \
     const size_t alive_bytes = WHOLE ? 0 : bins * sizeof(unsigned long long); \
     launch_next(bin_count_kernel<WHOLE>, blocks, COUNT_THREADS, alive_bytes + bins * sizeof(uint32_t) + (WHOLE ? 0 : live_sums_bytes(g)), s, v, g, t, c->depth_keys); \
-    launch_next(bin_rows_kernel, div_up(bins, ROWS_BINS), ROWS_THREADS, 0, s, blocks, bins, cap, t); \
-    launch_next(bin_scatter_kernel<WHOLE>, blocks, L1_THREADS, alive_bytes + bins * (L1_WARPS + 1) * sizeof(uint32_t), s, v, g, t, cap, c->depth_keys, c->keys, c->tile_off); \
-    launch_next(item_count_kernel<WHOLE>, item_blocks, L2_THREADS, 0, s, v, g, t, cap, c->keys, c->vals, c->keys_sorted); } while (0)
+    launch_next(bin_rows_kernel, div_up(bins, ROWS_BINS), ROWS_THREADS, 0, s, blocks, bins, cap, pr.room(), t); \
+    launch_next(bin_scatter_kernel<WHOLE>, blocks, L1_THREADS, alive_bytes + bins * (L1_WARPS + 1) * sizeof(uint32_t), s, v, g, t, pr, c->depth_keys, c->tile_off); \
+    launch_next(item_count_kernel<WHOLE>, item_blocks, L2_THREADS, 0, s, v, g, t, pr); } while (0)
     if (words) L(false); else L(true);
 #undef L
     if (bins >= 2 * sm_count()) launch_next(item_columns_kernel<4>, bins, 4 * BIN_TILES, 0, s, g, t, ranges);
     else launch_next(item_columns_kernel<16>, bins, 16 * BIN_TILES, 0, s, g, t, ranges);
     launch_next(tile_scan_kernel, scan_blocks, SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect);
-    launch_next(item_emit_kernel, item_blocks, L2_THREADS, 0, s, g, t, cap, c->keys, c->vals, c->keys_sorted, ranges, c->vals_sorted);
+    if (words) launch_next(item_emit_kernel<false>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
+    else launch_next(item_emit_kernel<true>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
   }
   return check_launch();
 }

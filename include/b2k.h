@@ -71,9 +71,11 @@ typedef struct {
   uint32_t* order_in;      /* [n] scratch of the depth sort */
   uint32_t* order;         /* [n] after b2k_project: identity; after b2k_bin_sort: splat index by depth rank (culled last) */
   uint32_t* tile_off;      /* [n] inclusive scan of tile counts in depth order */
-  uint32_t *keys, *vals, *keys_sorted, *vals_sorted; /* [isect_cap] scratch, scratch; tile id / splat index by tile, then depth */
+  uint32_t *keys, *vals, *keys_sorted, *vals_sorted; /* [isect_cap] scratch, scratch; tile id / splat index by tile, then depth
+                              (the first three are scratch of the binning together) */
   uint64_t isect_cap;
-  uint32_t* num_isect;     /* [4] device words: [0] intersections of this view (may exceed isect_cap: overflow);
+  uint32_t* num_isect;     /* [4] device words: [0] intersections of this view (may exceed isect_cap: overflow; also where the
+                              binning would need more than 3 * isect_cap words of scratch, which it then reports instead);
                               [1] entries of vis_list; [2] largest [0] since the caller cleared it (b2k_loss_accumulate) */
   void* sort_tmp;          /* scratch of b2k_sort_tmp_bytes() bytes */
   uint64_t sort_tmp_bytes;

@@ -272,3 +272,42 @@ def test_more_bin_pairs_than_a_word_counts():
     for c in (ctx, fresh):
         api.render_chunked(c, small, rp, sync=True)
     assert torch.equal(ctx.out_rgba, fresh.out_rgba) and ctx.num_isect == fresh.num_isect
+
+
+@pytest.mark.parametrize("chunks", [1, 2, 3])
+@pytest.mark.parametrize("W,H", [(2000, 2000), (3001, 2999)])    # one band of bins, and two
+def test_lists_fit_into_buffers_of_exactly_their_size(W, H, chunks):
+    """Diagonal needles across the image: their boxes overlap more bins than they hit tiles, so that level 1's pairs do not fit
+    where the lists do. Buffers of the lists' size hold the view all the same, and the lists are those of larger buffers."""
+    import torch
+    from b2ctrain_b200 import api
+    n = 40
+    scene = scenes.make_splats(n, 0, 3)
+    rng = np.random.Generator(np.random.PCG64(8))
+    scene["pos_op"][:, :3] = rng.uniform(-0.05, 0.05, (n, 3))
+    scene["pos_op"][:, 3] = -1.0
+    turn = np.deg2rad(45.0 + rng.uniform(-2, 2, n)) / 2 * np.where(np.arange(n) % 2, 1, -1)
+    scene["quat"][:] = np.stack([np.cos(turn), 0 * turn, 0 * turn, np.sin(turn)], 1)
+    scene["lscale"][:, :3] = [0.0, -9.0, -9.0]
+    scene["pos_op"][-1, :] = [0.0, 0.0, 0.3, 1.0]              # and one splat with a mask, in front of them
+    scene["lscale"][-1, :3] = -5.0
+    cam = scenes.look_at_camera((0.0, 0.0, 4.0), W, H, float(H))
+    scene = scenes.floor_for_cameras(scene, [cam])
+    m = api.Model("cuda:0").upload(scene)
+    rp = api.RenderParams(cam, sh_degree=0, bwd_info=False)
+    wide = api.RenderCtx("cuda:0")
+    wide.setup(W, H, m.cap, n_chunks=chunks)
+    api.render_forward(wide, m, rp)
+    hits = wide.num_isect
+    exact = api.RenderCtx("cuda:0")
+    exact.setup(W, H, m.cap, isect_cap=hits, n_chunks=chunks)
+    api.render_forward(exact, m, rp)
+    assert exact.isect_cap == hits and exact.num_isect == hits
+    assert torch.equal(exact.out_rgba, wide.out_rgba) and torch.equal(exact.tile_ranges, wide.tile_ranges)
+    ranges = wide.tile_ranges.cpu().numpy().reshape(-1, 2)
+    a, b = exact.vals_sorted.cpu().numpy(), wide.vals_sorted.cpu().numpy()
+    assert all(np.array_equal(a[x:y], b[x:y]) for x, y in ranges if y > x)
+    less = api.RenderCtx("cuda:0")                              # one too few is still too few
+    less.setup(W, H, m.cap, isect_cap=hits - 1, n_chunks=chunks)
+    api.render_forward(less, m, rp)
+    assert less.isect_cap > hits - 1 and torch.equal(less.out_rgba, wide.out_rgba)
