@@ -126,15 +126,18 @@ struct Range { uint32_t lo[MAX_BLOCKS], hi[MAX_BLOCKS]; Digits digits; };   // p
 // Elements a block owns: whole tiles of `tile` pairs.
 __device__ __forceinline__ uint32_t run_of(uint32_t n, uint32_t blocks, uint32_t tile) { return ((n + blocks - 1) / blocks + tile - 1) / tile * tile; }
 
+// Keys are read four at a time where the caller's array allows it.
+__device__ __forceinline__ bool by_quads(const uint32_t* keys) { return ((uintptr_t)keys & 15u) == 0u; }
+
 __global__ void __launch_bounds__(CNT_THREADS) key_range_kernel(const uint32_t* __restrict__ keys, uint32_t n, Range* __restrict__ range) {
   after_previous();
   __shared__ uint32_t s_lo[CNT_THREADS / 32], s_hi[CNT_THREADS / 32];
   uint32_t lo = CULLED, hi = 0u;
   auto see = [&](uint32_t k) { if (k != CULLED) { lo = min(lo, k); hi = max(hi, k); } };
-  const uint32_t quads = n / 4, stride = gridDim.x * CNT_THREADS;
+  const uint32_t quads = by_quads(keys) ? n / 4 : 0u, stride = gridDim.x * CNT_THREADS;
 #pragma unroll 8
   for (uint32_t q = blockIdx.x * CNT_THREADS + threadIdx.x; q < quads; q += stride) { const uint4 k = reinterpret_cast<const uint4*>(keys)[q]; see(k.x); see(k.y); see(k.z); see(k.w); }
-  if (blockIdx.x == 0 && threadIdx.x < (n & 3u)) see(keys[quads * 4 + threadIdx.x]);
+  for (uint32_t i = quads * 4 + blockIdx.x * CNT_THREADS + threadIdx.x; i < n; i += stride) see(keys[i]);
   lo = __reduce_min_sync(FULL, lo); hi = __reduce_max_sync(FULL, hi);
   if ((threadIdx.x & 31) == 0) { s_lo[threadIdx.x >> 5] = lo; s_hi[threadIdx.x >> 5] = hi; }
   __syncthreads();
@@ -184,14 +187,14 @@ __global__ void __launch_bounds__(CNT_THREADS) digit_count_kernel(const uint32_t
   const uint32_t len = run_of(n, gridDim.x, tile);
   const uint64_t begin64 = (uint64_t)blockIdx.x * len;
   const uint32_t begin = begin64 < n ? (uint32_t)begin64 : n, end = begin64 + len < n ? (uint32_t)(begin64 + len) : n;   // a multiple of four
-  const uint32_t whole = begin + ((end - begin) & ~3u);
+  const uint32_t whole = by_quads(keys) ? begin + ((end - begin) & ~3u) : begin;
 #pragma unroll 4
   for (uint32_t i = begin + threadIdx.x * 4; i < whole; i += CNT_THREADS * 4) {
     const uint4 k = *reinterpret_cast<const uint4*>(keys + i);
     atomicAdd(&hist[digit_at<COMPRESS>(k.x, d, pass)], 1u); atomicAdd(&hist[digit_at<COMPRESS>(k.y, d, pass)], 1u);
     atomicAdd(&hist[digit_at<COMPRESS>(k.z, d, pass)], 1u); atomicAdd(&hist[digit_at<COMPRESS>(k.w, d, pass)], 1u);
   }
-  if (threadIdx.x < end - whole) atomicAdd(&hist[digit_at<COMPRESS>(keys[whole + threadIdx.x], d, pass)], 1u);
+  for (uint64_t i = (uint64_t)whole + threadIdx.x; i < end; i += CNT_THREADS) atomicAdd(&hist[digit_at<COMPRESS>(keys[i], d, pass)], 1u);
   __syncthreads();
   for (uint32_t g = threadIdx.x; g < radix; g += CNT_THREADS) {
     uint32_t t = 0;

@@ -311,3 +311,39 @@ def test_lists_fit_into_buffers_of_exactly_their_size(W, H, chunks):
     less.setup(W, H, m.cap, isect_cap=hits - 1, n_chunks=chunks)
     api.render_forward(less, m, rp)
     assert less.isect_cap > hits - 1 and torch.equal(less.out_rgba, wide.out_rgba)
+
+
+@pytest.mark.parametrize("n", [1, 5, 511, 512, 5000, 70001])
+def test_pairs_sort_at_any_word(n):
+    """Keys and values that start one word behind a 16-byte boundary."""
+    import torch
+    from b2ctrain_b200 import api
+    rng = np.random.Generator(np.random.PCG64(n))
+    keys = rng.integers(0, 2 ** 32, n, dtype=np.uint64).astype(np.uint32) & np.uint32(0xFFFF00FF)
+    order = np.argsort(keys, kind="stable")
+    for at in (1, 2, 3):
+        arrays = [torch.zeros(n + 4, dtype=torch.int32, device="cuda:0")[at:at + n] for _ in range(4)]
+        arrays[0].copy_(torch.from_numpy(keys.view(np.int32)))
+        arrays[1].copy_(torch.arange(n, dtype=torch.int32))
+        size = api.lib().b2k_sort_pairs_tmp_bytes()
+        tmp = torch.zeros(size, dtype=torch.uint8, device="cuda:0")
+        assert api.lib().b2k_sort_pairs_u32(*[api._ptr(t) for t in arrays], n, api._ptr(tmp), size, api._stream(None)) == api.B2K_OK
+        assert np.array_equal(arrays[0].cpu().numpy().view(np.uint32), keys[order]) and np.array_equal(arrays[1].cpu().numpy(), order)
+
+
+@pytest.mark.parametrize("chunks", [1, 3])
+def test_depth_sort_scratch_at_any_word(chunks):
+    """The offsets' array, which the depth sort of many splats borrows, one word behind a 16-byte boundary."""
+    import torch
+    from b2ctrain_b200 import api
+    scene = scenes.make_splats(9001, 0, 4)
+    cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 30.0, 10.0), 320, 200, 200.0)
+    m = api.Model("cuda:0").upload(scenes.floor_for_cameras(scene, [cam]))
+    images = []
+    for at in (0, 1):
+        ctx = api.RenderCtx("cuda:0")
+        ctx.setup(320, 200, m.cap, n_chunks=chunks)
+        ctx.tile_off = torch.zeros(m.cap + 4, dtype=torch.int32, device="cuda:0")[at:at + m.cap]
+        api.render_forward(ctx, m, api.RenderParams(cam, sh_degree=0))
+        images.append((ctx.out_rgba.clone(), ctx.order[:m.n].clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*images))
