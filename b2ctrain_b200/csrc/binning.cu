@@ -115,7 +115,7 @@ extern "C" int b2k_render_chunked(const B2kModel* m, const B2kCamera* cam, const
     if (st) return st;
   }
   uint32_t* words = c->chunk_words;
-  unsigned long long* alive = (unsigned long long*)(words + CW_WORDS);
+  unsigned long long* alive = (unsigned long long*)(((uintptr_t)(words + CW_WORDS) + 7) & ~(uintptr_t)7);   // the caller's array may start at any word
   if (n == 0) {
     B2K_CUDA(cudaMemsetAsync(c->tile_ranges, 0, sizeof(uint32_t) * 2 * (size_t)c->n_tiles * C, s));
     B2K_CUDA(cudaMemsetAsync(c->num_isect, 0, sizeof(uint32_t), s));

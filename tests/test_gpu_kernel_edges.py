@@ -347,3 +347,22 @@ def test_depth_sort_scratch_at_any_word(chunks):
         api.render_forward(ctx, m, api.RenderParams(cam, sh_degree=0))
         images.append((ctx.out_rgba.clone(), ctx.order[:m.n].clone()))
     assert all(torch.equal(a, b) for a, b in zip(*images))
+
+
+def test_chunk_words_at_any_word():
+    """The alive words of a chunked view, 64 bits each, in an array of 32-bit words that starts at an odd one."""
+    import torch
+    from b2ctrain_b200 import api
+    W, H = 520, 264
+    scene = scenes.make_splats(20000, 0, 4, log_scale=(-2.5, 0.5))
+    cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 30.0, 10.0), W, H, 264.0)
+    m = api.Model("cuda:0").upload(scenes.floor_for_cameras(scene, [cam]))
+    images = []
+    for at in (0, 1):
+        ctx = api.RenderCtx("cuda:0")
+        ctx.setup(W, H, m.cap, n_chunks=3)
+        words = 32 + ctx.n_tiles + (ctx.tiles_x + 1) * (ctx.tiles_y + 1)
+        ctx.chunk_words = torch.zeros(words + 2, dtype=torch.int32, device="cuda:0")[at:at + words]
+        api.render_forward(ctx, m, api.RenderParams(cam, sh_degree=0))
+        images.append((ctx.out_rgba.clone(), ctx.tile_ranges.clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*images))
