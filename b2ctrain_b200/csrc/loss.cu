@@ -536,7 +536,9 @@ extern "C" int b2k_loss_photometric(const B2kCtx* c, const B2kLoss* lp, b2k_stre
   // 2.0) but leaves a third of the SMs to cut the rows for: taken where its segments are at most a fifth longer in steps (64x64
   // 14.6 -> 9.6 us, 200x150 14.9 -> 11.8; 333x217 would go from 22.4 to 27.2).
   const int rows3 = rows_for(strips), rows1 = rows_for(strips * 3);
-  const bool apart = steps_of(rows1) * 5 <= steps_of(rows3) * 6 && strips * 3 <= sm_count();
+  // It is also the one that writes the gradient by single floats: taken where the caller's array is not aligned for whole pixels.
+  const bool whole_pixels = (((uintptr_t)c->out_rgba | (uintptr_t)c->v_out) & 15) == 0;
+  const bool apart = !whole_pixels || (steps_of(rows1) * 5 <= steps_of(rows3) * 6 && strips * 3 <= sm_count());
   const int seg_rows = apart ? rows1 : rows3;
   const dim3 grid(strips, div_up(c->H, seg_rows), apart ? 3 : 1);
 #define L(MASKED, CHANNELS) launch_next(photometric_strip_kernel<MASKED, CHANNELS>, grid, CHANNELS * CH_THREADS, sizeof(StripShare<CHANNELS>), (cudaStream_t)stream, \

@@ -366,3 +366,26 @@ def test_chunk_words_at_any_word():
         api.render_forward(ctx, m, api.RenderParams(cam, sh_degree=0))
         images.append((ctx.out_rgba.clone(), ctx.tile_ranges.clone()))
     assert all(torch.equal(a, b) for a, b in zip(*images))
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("W,H", [(54, 9), (1001, 300), (3100, 40)])
+def test_loss_gradient_at_any_word(W, H, masked):
+    """The pixel gradients' array one float behind a 16-byte boundary."""
+    rng = np.random.Generator(np.random.PCG64(W))
+    scene, cam = stack_scene(4, W, H)
+    gt = rng.integers(0, 2 ** 32, W * H, dtype=np.uint64).astype(np.uint32)
+    wts = rng.integers(64, 256, W * H).astype(np.uint8) if masked else None
+    lp = dict(l1_w=0.8, ssim_w=-0.2, bg=(0.2, 0.1, 0.3), composite=not masked, mask=masked, alpha_lane=masked, match_alpha_weight=0.3, scale=1.7, grad_scale=1.0)
+    h = Harness(scene, cam, gt, wts, lp)
+    h.ctx.out_rgba.copy_(h.torch.from_numpy(rng.random((W * H, 4)).astype(np.float32)))
+    got = []
+    for at in (0, 1):
+        buffer = h.torch.full((W * H * 4 + 8,), 7.0, device="cuda:0")
+        h.ctx.v_out = buffer[at:at + W * H * 4].view(W * H, 4)
+        h.ctx.loss_accum.zero_()
+        h.api.photometric_loss(h.ctx, h.view, h.lp)
+        assert bool((buffer[:at] == 7.0).all()) and bool((buffer[at + W * H * 4:] == 7.0).all())
+        got.append((h.ctx.v_out.cpu().numpy(), float(h.ctx.loss_accum[0].item())))
+    (a, la), (b, lb) = got
+    assert rel_l2(b, a) <= 1e-6 and abs(la - lb) <= 1e-5 * abs(la)
