@@ -227,30 +227,7 @@ def _fields(obj, names, get):
 _MODEL_GET = attrgetter(*_MODEL_PTRS)
 
 
-class _Recorded:
-    """An object whose C record is kept until one of its attributes is set or deleted: a step passes the same context to six
-    calls and the same model to four, and reading forty-seven tensors' addresses each time cost more than the launches of a
-    small step. Tensors are swapped by setting the attribute; one whose storage is exchanged in place (Tensor.set_,
-    Tensor.resize_) has to be set again."""
-    _kept = None
-
-    def __setattr__(self, name, value):
-        self.__dict__["_kept"] = None
-        self.__dict__[name] = value
-
-    def __delattr__(self, name):
-        self.__dict__["_kept"] = None
-        object.__delattr__(self, name)
-
-    def struct(self):
-        """A record of its own for the caller, who may change it."""
-        s = self._kept
-        if s is None:
-            s = self.__dict__["_kept"] = self._record()
-        return type(s).from_buffer_copy(s)
-
-
-class Model(_Recorded):
+class Model:
     """Device splat model: parameters, Adam moments and refine statistics (src/model.h:14-40). Capacity doubles from
     1024 (src/model.cu:10-11); SH is planar with stride `cap`."""
 
@@ -343,7 +320,7 @@ class Model(_Recorded):
         n, K = self.n, self.K()
         return torch.cat([dc, hi], 0)[:, :n].t().reshape(n, K, 3).contiguous().cpu().numpy()
 
-    def _record(self):
+    def struct(self):
         return B2kModel.from_buffer_copy(_MODEL_PACK.pack(self.n, self.cap, self.degree, *map(_addr, _fields(self, _MODEL_PTRS, _MODEL_GET))))
 
 
@@ -354,7 +331,7 @@ _CTX_PTRS = ("proj0", "proj1", "proj2", "tile_count", "hit_info", "depth_keys", 
 _CTX_GET = attrgetter(*_CTX_PTRS)
 
 
-class RenderCtx(_Recorded):
+class RenderCtx:
     """Per-view scratch (src/gpu/render.h:66-95); member names follow the reference. `setup` sizes everything; the
     intersection buffers start at 2^22 entries (src/gpu/render.cu:20) and double on overflow."""
 
@@ -414,7 +391,8 @@ class RenderCtx(_Recorded):
         self.bwd_scratch = torch.zeros(int(lib().b2k_bwd_scratch_bytes(self.W, self.H, self.n_chunks, self.isect_cap)), dtype=torch.uint8,
                                        device=self.device)
 
-    def _record(self):
+    def struct(self):
+        """The context's record, from the tensors as they are now: one may have been given other storage in place."""
         p = [0 if t is None else t.data_ptr() for t in _fields(self, _CTX_PTRS, _CTX_GET)]
         return B2kCtx.from_buffer_copy(_CTX_PACK.pack(
             self.W, self.H, self.tiles_x, self.tiles_y, self.n_tiles, self.tile_bits, self.n_cap, *p[:14], self.isect_cap, self.d_num_isect.data_ptr(), p[14],

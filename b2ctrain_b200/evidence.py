@@ -24,28 +24,28 @@ class Evidence:
         use_normals = normal_weight > 0.0 and view.normals is not None
         if use_normals:
             rp.feat = "Normals"
-        masked_alpha, ms = int(bool(masked and has_alpha)), m.struct()
+        masked_alpha = int(bool(masked and has_alpha))
 
         def replay():
-            self.view_acc.zero_()
             cs = ctx.struct()
+            self.view_acc.zero_()
             api._check(api.lib().b2k_evidence_view(C.byref(cs), api._ptr(view.rgba), api._ptr(view.normals) if use_normals else None, api._ptr(view.weights),
                                                    masked_alpha, C.c_float(normal_weight), api._ptr(self.view_acc), api._stream(stream)), "evidence_view")
+            return cs
 
         # The intersection total is read back behind the replay, so that the GPU does not wait for the host in between. Lists that
         # did not fit make it a replay of truncated lists into an accumulator of this view's own: it is redone.
         api.render_forward(ctx, m, rp, stream, sync=False)
-        replay()
+        cs = replay()
+        ms, pos = m.struct(), (C.c_float * 3)(*[float(x) for x in cam["pos"]])
         if not api.forward_fits(ctx, stream):
             api.render_forward(ctx, m, rp, stream, sync=True)
-            replay()
-        cs = ctx.struct()
+            cs = replay()
         if labels is not None:
             if self.votes is None:
                 self.votes = torch.zeros((m.n, self.bins), dtype=torch.float32, device=self.device)
             api._check(api.lib().b2k_label_vote(C.byref(cs), api._ptr(view.rgba), api._ptr(labels), api._ptr(view.weights), masked_alpha, api._ptr(self.votes),
                                                 api._stream(stream)), "label_vote")
-        pos = (C.c_float * 3)(*[float(x) for x in cam["pos"]])
         api._check(api.lib().b2k_evidence_fold(C.byref(ms), api._ptr(self.view_acc), pos, api._ptr(self.acc), api._stream(stream)), "evidence_fold")
 
     def reduce(self, world):

@@ -6,7 +6,7 @@ import re
 
 import pytest
 
-from b2ctrain_b200 import api, build
+from b2ctrain_b200 import api, build, scenes
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -64,3 +64,24 @@ def test_unsupported_lanes_raise():
         api.OptimParams(dict(), frozen=True).struct()
     with pytest.raises(RuntimeError, match="unsupported lane"):
         api.LossParams(normal_scale=0.5).struct(api.ViewGPU(None))
+
+
+def test_records_follow_tensors_whose_storage_changes_in_place():
+    """A tensor of a model or context may get other memory without being set anew (Tensor.data, set_, resize_, the instance's
+    dictionary): the record of the next call has its present address."""
+    import torch
+    m, ctx = api.Model("cpu"), api.RenderCtx("cpu")
+    m.upload(scenes.make_splats(100, 1, 1))
+    ctx.setup(64, 48, m.cap)
+    for owner, name, field in ((m, "pos_op", "pos_op"), (m, "sh_hi", "sh_hi"), (ctx, "v_out", "v_out"), (ctx, "d_num_isect", "num_isect"), (ctx, "sort_tmp", "sort_tmp")):
+        t = getattr(owner, name)
+        assert getattr(owner.struct(), field) == t.data_ptr()
+        t.data = torch.zeros_like(t)
+        assert getattr(owner.struct(), field) == t.data_ptr()
+        t.set_(torch.zeros_like(t))
+        assert getattr(owner.struct(), field) == t.data_ptr()
+        t.resize_(t.numel() * 64)
+        assert getattr(owner.struct(), field) == t.data_ptr()
+        vars(owner)[name] = torch.zeros_like(t)
+        assert getattr(owner.struct(), field) == vars(owner)[name].data_ptr()
+    assert ctx.struct().sort_tmp_bytes == ctx.sort_tmp.numel()
