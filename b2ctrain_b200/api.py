@@ -82,10 +82,24 @@ for _record, _pack in ((B2kCamera, _CAMERA_PACK), (B2kRenderOpts, _OPTS_PACK), (
     assert C.sizeof(_record) == _pack.size, _record
 
 
-def _floats(a, n):
-    """The first n entries of a list or an array, as what a pack accepts."""
+def _packed(record, pack, *values):
+    """A record from its fields' values in order, arrays entry by entry."""
+    try:
+        return record.from_buffer_copy(pack.pack(*values))
+    except (OverflowError, _st.error):   # what a pack refuses and an assignment takes: a float beyond the range is infinite, an integer wraps around
+        s, values = record(), iter(values)
+        for name, kind in record._fields_:
+            if issubclass(kind, C.Array):
+                getattr(s, name)[:] = [next(values) for _ in range(kind._length_)]
+            else:
+                setattr(s, name, next(values))
+        return s
+
+
+def _floats(a, n=None):
+    """The (first n) entries of a list or an array as floats."""
     a = a.tolist() if hasattr(a, "tolist") else a
-    return a if len(a) == n else [a[i] for i in range(n)]
+    return [float(x) for x in a] if n is None or len(a) == n else [float(a[i]) for i in range(n)]
 
 
 def _addr(t):
@@ -205,8 +219,8 @@ _CAMERA_LIMITS = itemgetter("lim_pos_x", "lim_pos_y", "lim_neg_x", "lim_neg_y")
 
 def camera_from(cam):
     """CameraGPU record from a camera dict of b2ctrain_b200.scenes (CameraGPU::from, src/gpu/render.h:15-24)."""
-    return B2kCamera.from_buffer_copy(_CAMERA_PACK.pack(*_floats(cam["R"], 9), *_floats(cam["t"], 3), *_floats(cam["pos"], 3), *_CAMERA_HEAD(cam),
-                                                        *map(int, _CAMERA_SIZE(cam)), *_CAMERA_LIMITS(cam)))
+    return _packed(B2kCamera, _CAMERA_PACK, *_floats(cam["R"], 9), *_floats(cam["t"], 3), *_floats(cam["pos"], 3), *_floats(_CAMERA_HEAD(cam)),
+                   *map(int, _CAMERA_SIZE(cam)), *_floats(_CAMERA_LIMITS(cam)))
 
 
 def _capacity_for(n):
@@ -321,7 +335,7 @@ class Model:
         return torch.cat([dc, hi], 0)[:, :n].t().reshape(n, K, 3).contiguous().cpu().numpy()
 
     def struct(self):
-        return B2kModel.from_buffer_copy(_MODEL_PACK.pack(self.n, self.cap, self.degree, *map(_addr, _fields(self, _MODEL_PTRS, _MODEL_GET))))
+        return _packed(B2kModel, _MODEL_PACK, self.n, self.cap, self.degree, *map(_addr, _fields(self, _MODEL_PTRS, _MODEL_GET)))
 
 
 # The pointers of a context in the order of its record (num_isect, which is d_num_isect here, goes between vals_sorted and sort_tmp).
@@ -394,9 +408,8 @@ class RenderCtx:
     def struct(self):
         """The context's record, from the tensors as they are now: one may have been given other storage in place."""
         p = [0 if t is None else t.data_ptr() for t in _fields(self, _CTX_PTRS, _CTX_GET)]
-        return B2kCtx.from_buffer_copy(_CTX_PACK.pack(
-            self.W, self.H, self.tiles_x, self.tiles_y, self.n_tiles, self.tile_bits, self.n_cap, *p[:14], self.isect_cap, self.d_num_isect.data_ptr(), p[14],
-            self.sort_tmp.numel(), *p[15:25], self.n_chunks, *p[25:], self.bwd_scratch.numel()))
+        return _packed(B2kCtx, _CTX_PACK, self.W, self.H, self.tiles_x, self.tiles_y, self.n_tiles, self.tile_bits, self.n_cap, *p[:14], self.isect_cap,
+                       self.d_num_isect.data_ptr(), p[14], self.sort_tmp.numel(), *p[15:25], self.n_chunks, *p[25:], self.bwd_scratch.numel())
 
 
 class RenderParams:
@@ -419,9 +432,8 @@ class RenderParams:
             raise RuntimeError("RenderParams: mip / warp / sh_frame / app / hollow lanes are not implemented (unsupported lane)")
         if self.feat not in self._FEAT or (self.feat == "Buffer") != (self.feat_buffer is not None):
             raise RuntimeError("RenderParams: feat is None, Normals or Buffer, and feat_buffer goes with Buffer")
-        return B2kRenderOpts.from_buffer_copy(_OPTS_PACK.pack(
-            *_floats(self.bg, 3), int(self.sh_degree), bool(self.bwd_info), _addr(self.pos_override), _addr(self.quat_override), _addr(self.lscale_override),
-            self._FEAT[self.feat], _addr(self.feat_buffer)))
+        return _packed(B2kRenderOpts, _OPTS_PACK, *_floats(self.bg, 3), int(self.sh_degree), int(bool(self.bwd_info)), _addr(self.pos_override),
+                       _addr(self.quat_override), _addr(self.lscale_override), self._FEAT[self.feat], _addr(self.feat_buffer))
 
     def camera(self):
         return self.cam if isinstance(self.cam, B2kCamera) else camera_from(self.cam)
@@ -451,9 +463,8 @@ class LossParams:
     def struct(self, view):
         if self.normal_scale != 0.0:
             raise RuntimeError("LossParams: the normal-supervision lane is not implemented (unsupported lane)")
-        return B2kLoss.from_buffer_copy(_LOSS_PACK.pack(
-            _addr(view.rgba), _addr(view.weights), self.l1_w, self.ssim_w, *_floats(self.bg, 3), int(self.composite), int(self.mask), int(self.alpha_lane),
-            self.match_alpha_weight, self.scale, self.grad_scale))
+        return _packed(B2kLoss, _LOSS_PACK, _addr(view.rgba), _addr(view.weights), self.l1_w, self.ssim_w, *_floats(self.bg, 3), int(self.composite), int(self.mask),
+                       int(self.alpha_lane), self.match_alpha_weight, self.scale, self.grad_scale)
 
 
 class OptimParams:
@@ -485,10 +496,9 @@ class OptimParams:
     def struct(self):
         if self.mip or self.frozen or any(getattr(self, k) is not None for k in self._UNSUPPORTED):
             raise RuntimeError("OptimParams: cage / deformation / sparsification lanes are not implemented (unsupported lane)")
-        return B2kOptim.from_buffer_copy(_OPTIM_PACK.pack(
-            self.active_sh_degree, self.t, self.beta1, self.beta2, self.eps, self.lr_mean, self.lr_rot, self.lr_scale, self.lr_opac, self.lr_dc, self.lr_sh_rest,
-            self.noise_weight, self.noise_clamp, self.seed & 0xFFFFFFFF, self.step & 0xFFFFFFFF, bool(self.sparse), _addr(self.pos_override),
-            _addr(self.quat_override), _addr(self.lscale_override), _addr(self.grad_out), _addr(self.touched_out)))
+        return _packed(B2kOptim, _OPTIM_PACK, self.active_sh_degree, self.t, self.beta1, self.beta2, self.eps, self.lr_mean, self.lr_rot, self.lr_scale, self.lr_opac,
+                       self.lr_dc, self.lr_sh_rest, self.noise_weight, self.noise_clamp, self.seed, self.step, int(bool(self.sparse)), _addr(self.pos_override),
+                       _addr(self.quat_override), _addr(self.lscale_override), _addr(self.grad_out), _addr(self.touched_out))
 
     def camera(self):
         return self.cam if isinstance(self.cam, B2kCamera) else camera_from(self.cam)

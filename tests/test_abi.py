@@ -85,3 +85,26 @@ def test_records_follow_tensors_whose_storage_changes_in_place():
         vars(owner)[name] = torch.zeros_like(t)
         assert getattr(owner.struct(), field) == vars(owner)[name].data_ptr()
     assert ctx.struct().sort_tmp_bytes == ctx.sort_tmp.numel()
+
+
+def test_records_take_what_an_assignment_takes():
+    """Values that a native-layout pack refuses: floats beyond single precision, integers beyond 32 bits, numbers as text."""
+    import math
+    import numpy as np
+    cam = scenes.look_at_camera((0.0, 0.0, 4.0), 64, 48, 60.0)
+    plain = api.camera_from(cam)
+    odd = api.camera_from(dict(cam, fx="60.0", lim_pos_x=1e39, lim_neg_y=-1e300, W="64", R=[np.float64(x) for x in np.asarray(cam["R"]).reshape(-1)]))
+    assert odd.fx == plain.fx and odd.lim_pos_x == math.inf and odd.lim_neg_y == -math.inf and odd.W == 64 and list(odd.R) == list(plain.R) and list(odd.pos) == list(plain.pos)
+    op = api.OptimParams(cam, t=2 ** 31 + 5, seed=-3, step=2 ** 32 + 7, lr_mean=1e40, active_sh_degree=2).struct()
+    assert op.t == 5 - 2 ** 31 and op.seed == 2 ** 32 - 3 and op.step == 7 and op.lr_mean == math.inf and op.active_sh_degree == 2 and op.sparse in (0, 1)
+    rp = api.RenderParams(cam, bg=(1e39, "0.5", np.float32(0.25)), sh_degree=3).struct()
+    assert list(rp.bg) == [math.inf, 0.5, 0.25] and rp.sh_degree == 3 and not rp.pos_override
+    lp = api.LossParams(scale=1e39, bg=(0.25, 0.5, 1.0), mask=True)
+
+    class View:
+        rgba = weights = None
+
+    ls = lp.struct(View)
+    assert ls.scale == math.inf and list(ls.bg) == [0.25, 0.5, 1.0] and ls.mask == 1 and not ls.rgba
+    with pytest.raises(TypeError):
+        api.LossParams(scale="1").struct(View)
