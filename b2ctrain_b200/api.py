@@ -169,6 +169,7 @@ SIGNATURES = {
     "b2k_quantize_rgba8": (C.c_int, [_P, _P, C.c_int32, _S]),
     "b2k_error_string": (C.c_char_p, [C.c_int]),
     "b2k_last_cuda_error": (C.c_int, []),
+    "b2k_launches_repeated": (C.c_uint64, []),
     "b2k_version": (C.c_char_p, []),
 }
 

@@ -11,6 +11,7 @@
 namespace b2k {
 
 int g_last_cuda_error = 0;
+std::atomic<uint64_t> g_launches_repeated{0};
 int check_launch() {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return B2K_ERR_CUDA; }
@@ -344,4 +345,5 @@ static const char* kErrors[] = {"ok", "bad argument", "buffer capacity exceeded"
                                 "intersection buffers overflowed"};
 extern "C" const char* b2k_error_string(int status) { return status >= 0 && status <= 5 ? kErrors[status] : "unknown status"; }
 extern "C" int b2k_last_cuda_error(void) { return g_last_cuda_error; }
+extern "C" uint64_t b2k_launches_repeated(void) { return g_launches_repeated.load(std::memory_order_relaxed); }
 extern "C" const char* b2k_version(void) { return "b2k 0.1 (sm_100a)"; }

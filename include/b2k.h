@@ -379,6 +379,9 @@ int b2k_quantize_rgba8(const float* rgba, uint32_t* out, int32_t n_pixels, b2k_s
 
 const char* b2k_error_string(int status);
 int b2k_last_cuda_error(void);
+/* Launches of this process that the runtime refused with programmatic stream serialisation and that went out without it: zero
+ * unless something is wrong. The results are the same. */
+uint64_t b2k_launches_repeated(void);
 const char* b2k_version(void);
 
 #ifdef __cplusplus
