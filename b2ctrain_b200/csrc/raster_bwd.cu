@@ -406,7 +406,7 @@ using namespace b2k;
 extern "C" uint64_t b2k_bwd_scratch_bytes(int32_t W, int32_t H, int32_t n_chunks, uint64_t isect_cap) {
   if (W <= 0 || H <= 0) return 0;
   const uint64_t tiles = (uint64_t)div_up(W, RT_W) * div_up(H, RT_W), chunks = n_chunks > 1 ? (uint64_t)n_chunks : 1u;
-  const uint64_t slots = bwd_slots(isect_cap, tiles * chunks, seg_shift_of(tiles));
+  const uint64_t slots = bwd_slots(isect_cap, tiles * chunks, seg_shift_of(short_segments(tiles, isect_cap)));
   return sizeof(uint32_t) * BWD_HEADER_WORDS + sizeof(uint2) * slots + sizeof(float4) * RT_PX * slots;
 }
 
@@ -427,8 +427,8 @@ extern "C" int b2k_raster_bwd_scaled(const B2kCtx* c, const B2kModel* m, const B
   uint2* items = bwd_items_ptr(c);
   launch_clear(work, 2, nullptr, 0, s);
   const int n_ranges = chunks * c->n_tiles;
-  const int seg_shift = seg_shift_of(c->n_tiles);
-  const bool brief = short_segments(c->n_tiles);
+  const bool brief = short_segments(c);
+  const int seg_shift = seg_shift_of(brief);
   if (brief) launch_next(bwd_suffix_kernel, div_up(c->n_tiles, 4), 128, 0, s, (const uint2*)c->tile_ranges, c->n_tiles, chunks, seg_shift, items, work, bwd_ckpt_ptr(c));
   else launch_next(bwd_items_kernel, min(div_up(n_ranges, 256), sm_count() * 4), 256, 0, s, (const uint2*)c->tile_ranges, n_ranges, seg_shift, items, work);
   // Persistent grid: as many CTAs as an SM holds.

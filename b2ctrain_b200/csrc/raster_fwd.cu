@@ -442,14 +442,14 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
   const bool chunked = n_chunks > 1, halves = n_chunks <= 2;   // (measured above)
 #define ARGS s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, \
     (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, \
-    seg_shift_of(c->n_tiles), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr, bwd_work_ptr(c)
+    seg_shift_of(short_segments(c)), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr, bwd_work_ptr(c)
 #define HALF(B, D, C, F) launch_next(raster_fwd_half_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_TILES), FWD_WARPS * 32, 0, ARGS)
 #define L(B, D, F) do { if (!chunked) HALF(B, D, false, F); else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
     else launch_next(raster_fwd_kernel<B, D, (F) && (B) == NONE>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS); } while (0)
 #define LD(B, D) do { if (o->feat_mode != 0) L(B, D, true); else L(B, D, false); } while (0)   // a chunked view with features is forward only (checked by the caller)
 #define LB(B) do { if (c->out_depth) LD(B, true); else LD(B, false); } while (0)
   if (!o->bwd_info) LB(NONE);
-  else if (short_segments(c->n_tiles)) LB(PER_SEGMENT);
+  else if (short_segments(c)) LB(PER_SEGMENT);
   else LB(RUNNING);
 #undef LB
 #undef LD

@@ -219,12 +219,14 @@ int b2k_loss_fold(const B2kCtx* dst, const B2kCtx* src, b2k_stream_t s);
 /* eval_metrics, src/gpu/loss.h:41 (eval_kernel, src/gpu/loss.cu:241-293). */
 int b2k_eval_metrics(const B2kCtx* ctx, const uint32_t* rgba, int32_t mask_weighted, b2k_stream_t s);
 
-/* Bytes of ctx->bwd_scratch for a context of this image size, chunk count (0 or 1: whole view) and intersection capacity. */
+/* Bytes of ctx->bwd_scratch for a context of this image size, chunk count (0 or 1: whole view) and intersection capacity: about
+ * 1 KB per 32 intersections in images of up to 4,096 tiles with a capacity of up to 2^24, per 128 otherwise. */
 uint64_t b2k_bwd_scratch_bytes(int32_t W, int32_t H, int32_t n_chunks, uint64_t isect_cap);
 
 /* ---- backward ---- */
 /* rasterize_backward, src/gpu/render.h:106 (raster_bwd_kernel, src/gpu/raster_bwd.cu:11-143). Same gradients; the
- * tile lists are replayed in segments of 32 or 64 fragments from the forward's checkpoints in ctx->bwd_scratch. */
+ * tile lists are replayed in segments of 32 or 128 fragments from the forward's checkpoints in ctx->bwd_scratch, as
+ * often as asked for one forward. */
 int b2k_raster_bwd(const B2kCtx* ctx, const B2kModel* m, const B2kRenderOpts* opts, b2k_stream_t s);
 /* rasterize_backward_tc, src/gpu/render.h:107-109 (raster_bwd_tc_kernel, src/gpu/raster_bwd_tc.cu:30-225), as far as its
  * contract goes: the pixel gradients in v_out were produced with LossParams::grad_scale applied and the per-splat

@@ -126,3 +126,21 @@ def test_backward_repeats_on_one_forward(W, H, chunks):
         cs, ms, opts = ctx.struct(), h.model.struct(), h.rp.struct()
         h.api._check(h.api.lib().b2k_raster_bwd_scaled(C.byref(cs), C.byref(ms), C.byref(opts), C.c_float(scale), h.api._stream(None)), "b2k_raster_bwd_scaled")
         check(ctx.v_splat[:n].cpu().numpy().astype(np.float64), want, bound, scale)
+
+
+def test_segments_are_long_again_where_short_ones_would_take_too_much_memory():
+    """Buffers for more than 2^24 intersections in a small image: checkpoints every 128 fragments, and the same gradients."""
+    from b2ctrain_b200 import api
+    W = H = 256
+    size = lambda cap: api.lib().b2k_bwd_scratch_bytes(W, H, 1, cap)
+    assert size(1 << 24) < 600e6 and size((1 << 24) + 1) < 150e6 and size(1 << 25) < 300e6
+    scene, cam = stack_scene(300, W, H)
+    n, bg = scene["n"], (0.2, 0.1, 0.3)
+    v_out = (np.random.Generator(np.random.PCG64(3)).standard_normal((W * H, 4)) * 1e-3).astype(np.float32)
+    for cap in (1 << 24, 1 << 25):
+        h = Harness(scene, cam, bg=bg, isect_cap=cap)
+        h.forward()
+        h.ctx.v_out.copy_(h.torch.from_numpy(v_out))
+        h.api.rasterize_backward(h.ctx, h.model, h.rp)
+        want, bound, _ = wanted(n, W, H, h, v_out, bg, cap > 1 << 24)
+        check(h.ctx.v_splat[:n].cpu().numpy().astype(np.float64), want, bound, cap)
