@@ -108,3 +108,16 @@ def test_records_take_what_an_assignment_takes():
     assert ls.scale == math.inf and list(ls.bg) == [0.25, 0.5, 1.0] and ls.mask == 1 and not ls.rgba
     with pytest.raises(TypeError):
         api.LossParams(scale="1").struct(View)
+
+
+def test_rows_of_the_model_need_aligned_outputs(lib):
+    """b2k_model_rows writes 16 bytes at a time: an output at another address is an argument error, not a fault."""
+    import torch
+    m = api.Model("cpu").upload(scenes.make_splats(8, 1, 1))
+    ms = m.struct()
+    out = [torch.zeros(8 * w + 4) for w in (4, 4, 4, 12)]
+    assert all(t.data_ptr() % 16 == 0 for t in out)
+    for k in range(4):
+        ptrs = [C.c_void_p(t.data_ptr() + (4 if j == k else 0)) for j, t in enumerate(out)]
+        assert lib.b2k_model_rows(C.byref(ms), 0, 0, *ptrs, None) == api.B2K_ERR_ARG
+    assert lib.b2k_model_rows(C.byref(ms), 0, 0, *[C.c_void_p(t.data_ptr()) for t in out], None) == api.B2K_OK
