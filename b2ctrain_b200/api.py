@@ -96,10 +96,14 @@ def _packed(record, pack, *values):
         return s
 
 
-def _floats(a, n=None):
-    """The (first n) entries of a list or an array as floats."""
+def _first(a, n):
+    """The first n entries of a list or an array."""
     a = a.tolist() if hasattr(a, "tolist") else a
-    return [float(x) for x in a] if n is None or len(a) == n else [float(a[i]) for i in range(n)]
+    return a if len(a) == n else [a[i] for i in range(n)]
+
+
+def _floats(a, n=None):
+    return [float(x) for x in (a if n is None else _first(a, n))]
 
 
 def _addr(t):
@@ -220,8 +224,12 @@ _CAMERA_LIMITS = itemgetter("lim_pos_x", "lim_pos_y", "lim_neg_x", "lim_neg_y")
 
 def camera_from(cam):
     """CameraGPU record from a camera dict of b2ctrain_b200.scenes (CameraGPU::from, src/gpu/render.h:15-24)."""
-    return _packed(B2kCamera, _CAMERA_PACK, *_floats(cam["R"], 9), *_floats(cam["t"], 3), *_floats(cam["pos"], 3), *_floats(_CAMERA_HEAD(cam)),
-                   *map(int, _CAMERA_SIZE(cam)), *_floats(_CAMERA_LIMITS(cam)))
+    size = map(int, _CAMERA_SIZE(cam))
+    try:
+        return B2kCamera.from_buffer_copy(_CAMERA_PACK.pack(*_first(cam["R"], 9), *_first(cam["t"], 3), *_first(cam["pos"], 3), *_CAMERA_HEAD(cam), *size, *_CAMERA_LIMITS(cam)))
+    except (OverflowError, _st.error):
+        return _packed(B2kCamera, _CAMERA_PACK, *_floats(cam["R"], 9), *_floats(cam["t"], 3), *_floats(cam["pos"], 3), *_floats(_CAMERA_HEAD(cam)), *map(int, _CAMERA_SIZE(cam)),
+                       *_floats(_CAMERA_LIMITS(cam)))
 
 
 def _capacity_for(n):
@@ -599,59 +607,86 @@ def render_chunked(ctx, m, p, stream=None, sync=True):
         return ctx.num_isect
 
 
+# Records of the calls that read a few fields only, with those fields: a whole one takes about 4 us of the host's time, and
+# the launches of a small step leave it little more than a step's GPU time (64x64 step: host 106 us with whole records, 91 so).
+def _loss_record(ctx):
+    s = B2kCtx()
+    s.loss_accum, s.num_isect = _addr(ctx.loss_accum), _addr(ctx.d_num_isect)
+    return s
+
+
+def _image_record(ctx):
+    s = B2kCtx()
+    s.W, s.H, s.out_rgba, s.v_out, s.loss_accum = ctx.W, ctx.H, _addr(ctx.out_rgba), _addr(ctx.v_out), _addr(ctx.loss_accum)
+    return s
+
+
 def photometric_loss(ctx, view, lp, stream=None):
-    cs, ls = ctx.struct(), lp.struct(view)
+    cs, ls = _image_record(ctx), lp.struct(view)
     _check(lib().b2k_loss_photometric(C.byref(cs), C.byref(ls), _stream(stream)), "photometric_loss")
 
 
 def accumulate_loss(ctx, stream=None):
-    cs = ctx.struct()
+    cs = _loss_record(ctx)
     _check(lib().b2k_loss_accumulate(C.byref(cs), _stream(stream)), "accumulate_loss")
 
 
 def zero_loss(ctx, first=0, count=16, stream=None):
     """loss_accum[first : first + count] = 0 on the stream."""
-    cs = ctx.struct()
+    cs = _loss_record(ctx)
     _check(lib().b2k_loss_zero(C.byref(cs), int(first), int(count), _stream(stream)), "zero_loss")
 
 
 def step_begin(ctx, stream=None):
     """Clears the context's loss accumulator and its running intersection maximum (start of a training step)."""
-    cs = ctx.struct()
+    cs = _loss_record(ctx)
     _check(lib().b2k_step_begin(C.byref(cs), _stream(stream)), "step_begin")
 
 
 def fold_loss(dst_ctx, src_ctx, stream=None):
     """Adds the running loss sum and view count of src_ctx into dst_ctx's."""
-    a, b = dst_ctx.struct(), src_ctx.struct()
+    a, b = _loss_record(dst_ctx), _loss_record(src_ctx)
     _check(lib().b2k_loss_fold(C.byref(a), C.byref(b), _stream(stream)), "fold_loss")
 
 
 def eval_metrics(ctx, view, mask_weighted=False, stream=None):
-    cs = ctx.struct()
+    cs = _image_record(ctx)
     _check(lib().b2k_eval_metrics(C.byref(cs), _ptr(view.rgba), int(mask_weighted), _stream(stream)), "eval_metrics")
 
 
+def _weight_record(m):
+    s = B2kModel()
+    s.n, s.cap, s.degree, s.vis_weight = m.n, m.cap, m.degree, _addr(getattr(m, "vis_weight", None))
+    return s
+
+
 def rasterize_backward(ctx, m, p, stream=None):
-    cs, ms, os_ = ctx.struct(), m.struct(), p.struct()
+    cs, ms, os_ = ctx.struct(), _weight_record(m), p.struct()
     _check(lib().b2k_raster_bwd(C.byref(cs), C.byref(ms), C.byref(os_), _stream(stream)), "rasterize_backward")
 
 
 def rasterize_backward_tc(ctx, m, p, grad_scale, stream=None):
     """rasterize_backward_tc (src/gpu/render.h:107-109): v_out carries grad_scale, the per-splat lanes leave divided by it."""
-    cs, ms, os_ = ctx.struct(), m.struct(), p.struct()
+    cs, ms, os_ = ctx.struct(), _weight_record(m), p.struct()
     _check(lib().b2k_raster_bwd_scaled(C.byref(cs), C.byref(ms), C.byref(os_), C.c_float(grad_scale), _stream(stream)), "rasterize_backward_tc")
 
 
+def _lanes_record(ctx):
+    s = B2kCtx()
+    s.n_cap, s.isect_cap, s.num_isect = ctx.n_cap, ctx.isect_cap, _addr(ctx.d_num_isect)
+    s.v_splat, s.vis_flag, s.tile_count, s.vis_list = _addr(ctx.v_splat), _addr(ctx.vis_flag), _addr(ctx.tile_count), _addr(getattr(ctx, "vis_list", None))
+    return s
+
+
 def optimizer_step(ctx, m, op, stream=None):
-    cs, ms, os_, cam = ctx.struct(), m.struct(), op.struct(), op.camera()
+    cs, ms, os_, cam = _lanes_record(ctx), m.struct(), op.struct(), op.camera()
     _check(lib().b2k_optim_fused(C.byref(cs), C.byref(ms), C.byref(cam), C.byref(os_), _stream(stream)), "optimizer_step")
 
 
 # ---- data-parallel split of optimizer_step ----
 
 def projection_backward(ctx, m, op, grad, stream=None):
-    cs, ms, os_, cam = ctx.struct(), m.struct(), op.struct(), op.camera()
+    cs, ms, os_, cam = _lanes_record(ctx), m.struct(), op.struct(), op.camera()
     _check(lib().b2k_proj_bwd(C.byref(cs), C.byref(ms), C.byref(cam), C.byref(os_), _ptr(grad), _stream(stream)), "projection_backward")
 
 
