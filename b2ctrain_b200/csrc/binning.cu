@@ -8,9 +8,10 @@ namespace b2k {
 namespace {
 
 // Optional timing marks for b2k_bin_sort_profile: when armed, an event is recorded on the stream at each mark.
-struct Marks { cudaEvent_t ev[32]; int n = 0; bool armed = false; };
+constexpr int MARKS = 4;   // start, depth sort done, lists done, keys done
+struct Marks { cudaEvent_t ev[MARKS]; int n = 0; bool armed = false; };
 thread_local Marks g_marks;
-void mark(cudaStream_t s) { if (g_marks.armed && g_marks.n < 32) cudaEventRecord(g_marks.ev[g_marks.n++], s); }
+void mark(cudaStream_t s) { if (g_marks.armed && g_marks.n < MARKS) cudaEventRecord(g_marks.ev[g_marks.n++], s); }
 
 // ---- front-to-back rendering in depth chunks ------------------------------------------------------------------------
 // The view's splats are taken in a few chunks of increasing depth rank. A chunk is binned (its hits distributed to the
@@ -141,18 +142,17 @@ extern "C" int b2k_render_chunked(const B2kModel* m, const B2kCamera* cam, const
 extern "C" int b2k_bin_sort_profile(const B2kCtx* c, int32_t n, b2k_stream_t stream, float* ms) {
   B2K_REQUIRE(c && ms);
   Marks& mk = g_marks;
-  for (int i = 0; i < 32; i++) B2K_CUDA(cudaEventCreate(&mk.ev[i]));
+  for (int i = 0; i < MARKS; i++) B2K_CUDA(cudaEventCreate(&mk.ev[i]));
   mk.n = 0; mk.armed = true;
   const int st = b2k_bin_sort(c, n, stream);
   mk.armed = false;
   cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
-  const int expect = 4;   // start, depth sort done, lists done, keys done
   for (int i = 0; i < 10; i++) ms[i] = 0.f;
-  if (st == B2K_OK && e == cudaSuccess && mk.n == expect && n > 0) {
+  if (st == B2K_OK && e == cudaSuccess && mk.n == MARKS && n > 0) {
     auto dt = [&](int a, int b) { float t = 0.f; cudaEventElapsedTime(&t, mk.ev[a], mk.ev[b]); return t; };
-    ms[0] = dt(0, expect - 3); ms[1] = dt(expect - 3, expect - 2); ms[8] = dt(expect - 2, expect - 1); ms[9] = dt(0, expect - 1);
+    ms[0] = dt(0, 1); ms[1] = dt(1, 2); ms[8] = dt(2, 3); ms[9] = dt(0, 3);
   }
-  for (int i = 0; i < 32; i++) cudaEventDestroy(mk.ev[i]);
+  for (int i = 0; i < MARKS; i++) cudaEventDestroy(mk.ev[i]);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return B2K_ERR_CUDA; }
   return st;
 }
