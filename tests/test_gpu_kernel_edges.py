@@ -24,7 +24,7 @@ def stack_scene(n, W, H, seed=3):
     return scenes.floor_for_cameras(scene, [cam]), cam
 
 
-@pytest.mark.parametrize("W,H", [(512, 512), (520, 512)])       # 4,096 and 4,160 tiles: segments of 32 and of 64 fragments
+@pytest.mark.parametrize("W,H", [(512, 512), (520, 512)])       # 4,096 and 4,160 tiles: segments of 32 and of 128 fragments
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 65, 129])
 def test_backward_segments_and_odd_batches(n, W, H):
     scene, cam = stack_scene(n, W, H)

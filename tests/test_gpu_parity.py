@@ -69,9 +69,9 @@ def test_binning_bit_exact():
     assert np.array_equal(order, want_order.astype(np.uint32))
 
 
-def test_binning_bit_exact_at_4k_where_the_tile_sort_uses_nine_bit_digits():
-    """A 3840x2160 image has 129,600 tiles, 17 bits of tile id: the tile sort runs two passes of nine-bit digits instead of
-    three of eight. Same contract as above, plus the chunked renderer on the same view."""
+def test_binning_bit_exact_at_4k_over_many_bins():
+    """A 3840x2160 image has 129,600 tiles (17 bits of tile id) in 2,040 bins of 8x8 tiles, nearly all that one band of the
+    binning holds. Same contract as above, plus the chunked renderer on the same view."""
     import torch
     scene, cam = small_scene(n=1200, W=3840, H=2160)
     h = Harness(scene, cam)
