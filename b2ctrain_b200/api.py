@@ -608,7 +608,7 @@ def render_chunked(ctx, m, p, stream=None, sync=True):
 
 
 # Records of the calls that read a few fields only, with those fields: a whole one takes about 4 us of the host's time, and
-# the launches of a small step leave it little more than a step's GPU time (64x64 step: host 106 us with whole records, 91 so).
+# the launches of a small step leave it little more than a step's GPU time (64x64 step: host 106 us with whole records, 93 so).
 def _loss_record(ctx):
     s = B2kCtx()
     s.loss_accum, s.num_isect = _addr(ctx.loss_accum), _addr(ctx.d_num_isect)
