@@ -35,7 +35,7 @@ namespace b2k {
 namespace {
 
 constexpr int BWD_WARPS = 4;                 // warps per CTA (independent: the CTA shape only sets the residency granularity)
-constexpr int BWD_CTAS_PER_SM = 5;            // 94 registers: 131 us on the view below; 138 with 4 CTAs, 140 with 5.5, 139 with 6
+constexpr int BWD_CTAS_PER_SM = 5;            // 96 registers: 131 us on the view below; 138 with 4 CTAs, 140 with 5.5, 139 with 6
 constexpr int BWD_BATCH = 32;                 // fragments staged per warp and batch
 constexpr int RED_P = 4;                      // fragment pairs pending before a reduction (8 save shuffles, but cost the memory of a third of the warps: 136 us)
 constexpr int RED_STRIDE = 33;                // 16-byte words per pending pair, one of skew: conflict-free reads
