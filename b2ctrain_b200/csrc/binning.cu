@@ -78,14 +78,14 @@ extern "C" int b2k_bin_sort(const B2kCtx* c, int32_t n, b2k_stream_t stream) {
   uint32_t* tables = sort_tables_ptr(c);
   // 1. Splats by depth: key = bits of view z (culled splats carry 0xFFFFFFFF and land last), value = index.
   mark(s);
-  int st = depth_sort(c, n, false, tables, s);   // a view is binned again after its buffers have grown
+  int st = depth_sort(c, n, false, walks(c, n), tables, s);   // a view is binned again after its buffers have grown
   if (st) return st;
   mark(s);
   // 2. Hits to the tiles' lists, depth order surviving inside each tile; 3. the tile ids of the list.
   st = launch_bins(c, n, nullptr, 0, 0, 256, nullptr, tables, s);
   if (st) return st;
   mark(s);
-  st = launch_fill_keys(c, s);
+  if (!walks(c, n)) st = launch_fill_keys(c, s);
   mark(s);
   return st;
 }
@@ -125,7 +125,7 @@ extern "C" int b2k_render_chunked(const B2kModel* m, const B2kCamera* cam, const
   }
   if (c->sort_tmp_bytes < b2k_sort_tmp_bytes(c->n_cap, c->isect_cap) || c->isect_cap == 0 || c->isect_cap > 0x7FFFFFF0ull) return B2K_ERR_CAPACITY;
   uint32_t* tables = sort_tables_ptr(c);
-  st = depth_sort(c, n, true, tables, s);
+  st = depth_sort(c, n, true, false, tables, s);
   if (st) return st;
   const int bins = div_up(c->tiles_x, 8) * div_up(c->tiles_y, 8);
   launch_next(chunk_prepare_kernel, div_up(bins, 256), 256, 0, s, c->depth_keys_sorted, n, words, alive, bins);

@@ -22,84 +22,20 @@
 // pairs and two radix passes over them, sum of the stage's kernels per view: 4K, 6M splats, 37.5M hits 2,660 -> 960 us;
 // 1080p, 500k splats, 4.4M hits 330 -> 150; 1024x1024, 1M splats of which a tenth cover hundreds of tiles 1,350 -> 390.
 // Inside that, the tests of a warp's 32 pairs shared out by tile row (not a pair per lane): 455 -> 286 us at 4K.
-#include "common.cuh"
+#include "bins.cuh"
 #include <algorithm>
 
 namespace b2k {
 namespace {
 
-constexpr int BIN_W = 8;                      // tiles along a bin's edge
-constexpr int BIN_TILES = BIN_W * BIN_W;
-constexpr int MAX_BINS = 2048;                // bins of one band: what a block's tables in shared memory hold; larger images take several bands of bin rows
-constexpr int MAX_ITEMS = 8192;               // items of one band: BINS_TABLE_WORDS / 64
 constexpr int L1_THREADS = 256, L1_WARPS = L1_THREADS / 32;
-constexpr int L2_THREADS = 256, L2_WARPS = L2_THREADS / 32;
 constexpr int SERIAL_BINS = 12;               // a splat over more bins is spread by its whole warp (4K view: 8 -> 12 takes 360 + 338 to 264 + 204 us)
-constexpr int SCAN_TILES = 1024;              // tiles per block of tile_scan
-constexpr unsigned FULL = 0xffffffffu;
 static_assert((size_t)MAX_ITEMS * BIN_TILES <= BINS_TABLE_WORDS, "the counts of the items take the place of level 1's table");
 static_assert(MAX_BINS * BIN_TILES / SCAN_TILES <= BINS_SEGMENTS, "one sum per tile_scan block");
 
-// The bins and tiles of one band.
-struct Band { int tiles_x, tiles_y, bins_x, bin_row0, bin_rows; };
-__device__ __forceinline__ int band_bins(const Band& g) { return g.bins_x * g.bin_rows; }
-
-// What a call works on. words == nullptr: the whole view, from exact hit masks; else depth chunk `chunk` of a chunked view.
-struct View {
-  const uint32_t* order; const uint4* hit_info; const uint32_t* tile_count; const float4* proj0; const float4* proj1;
-  int n; uint32_t* words; int chunk, lo_num, hi_num; const unsigned long long* alive; int first_band, last_band;
-};
-
-struct Tables {
-  uint32_t* cells;       // [bin][block] of level 1, then [item][64] of level 2
-  uint32_t* totals;      // [MAX_BINS] pairs per bin
-  uint32_t* base;        // [MAX_BINS + 1] first pair of each bin
-  uint32_t* first_item;  // [MAX_BINS + 1]
-  uint32_t* item_bin;    // [MAX_ITEMS]
-  uint32_t* block_sums;  // [1024] tile counts of level 1's blocks (whole view)
-  uint32_t* segments;    // [BINS_SEGMENTS] hits per tile_scan block
-  uint32_t* st;          // [16] see S_*
-};
-enum { S_PAIRS = 0, S_ITEMS, S_ITEM_LEN, S_DONE_ROWS, S_DONE_TILES, S_SLOT, S_OVER, S_TOTAL, S_KEPT };
-
-__device__ __forceinline__ void view_ranks(const View& v, uint32_t& r0, uint32_t& r1) {
-  if (!v.words) { r0 = 0u; r1 = (uint32_t)v.n; return; }
-  const uint64_t V = v.words[CW_V];
-  r0 = (uint32_t)((V * (uint64_t)v.lo_num) >> 8);
-  r1 = (uint32_t)((V * (uint64_t)v.hi_num) >> 8);
-}
 __device__ __forceinline__ uint32_t run_len(uint32_t n, uint32_t blocks) {
   const uint32_t per = (n + blocks - 1) / blocks;
   return (per + L1_THREADS - 1) / L1_THREADS * L1_THREADS;
-}
-
-// A splat's tile box, half open; empty when x1 == x0.
-struct Box { int x0, y0, x1, y1; };
-__device__ __forceinline__ Box box_of(const uint4& hi) {
-  Box b;
-  if (hi.z == 0xFFFFFFFFu) {
-    b.x0 = (int)(hi.x & 0xFFFFu); b.y0 = (int)(hi.x >> 16);
-    b.x1 = b.x0 + (int)(hi.y & 0xFFFFu); b.y1 = b.y0 + (int)(hi.y >> 16);
-  } else {
-    b.x0 = (int)(hi.z & 0xFFFu); b.y0 = (int)((hi.z >> 12) & 0xFFFu);
-    b.x1 = b.x0 + (int)(hi.z >> 24); b.y1 = b.y0 + (int)hi.w;
-  }
-  return b;
-}
-// The box's tiles inside bin (bx, by), bit = row * 8 + column.
-__device__ __forceinline__ unsigned long long rect_bits(const Box& b, int bx, int by) {
-  const int lx0 = max(b.x0 - bx * BIN_W, 0), lx1 = min(b.x1 - bx * BIN_W, BIN_W), ly0 = max(b.y0 - by * BIN_W, 0), ly1 = min(b.y1 - by * BIN_W, BIN_W);
-  const unsigned long long row = ((1u << (lx1 - lx0)) - 1u) << lx0;
-  return (row * 0x0101010101010101ull) & ((~0ull >> (64 - BIN_W * (ly1 - ly0))) << (BIN_W * ly0));
-}
-// The same from the exact hit mask of a box of at most 64 tiles (row-major inside the box).
-__device__ __forceinline__ unsigned long long mask_bits(const uint4& hi, const Box& b, int bx, int by) {
-  const unsigned long long mask = ((unsigned long long)hi.y << 32) | hi.x;
-  const int xs = max(b.x0, bx * BIN_W), xe = min(b.x1, bx * BIN_W + BIN_W), ys = max(b.y0, by * BIN_W), ye = min(b.y1, by * BIN_W + BIN_W), bw = b.x1 - b.x0;
-  unsigned long long out = 0ull;
-  for (int y = ys; y < ye; y++)
-    out |= ((mask >> ((y - b.y0) * bw + (xs - b.x0))) & ((1ull << (xe - xs)) - 1ull)) << ((y - by * BIN_W) * BIN_W + (xs - bx * BIN_W));
-  return out;
 }
 
 // The bins a splat's box overlaps, inside the band.
@@ -236,21 +172,6 @@ __device__ __forceinline__ bool wide_bins(const unsigned long long* s_alive, con
     if (lane == src) took = any;
   }
   return took;
-}
-
-// Inclusive scan over the block of one value per thread (at most 1024 threads); s_warp holds 32 values. Synchronises.
-template <class T>
-__device__ __forceinline__ T block_scan(T v, T* s_warp, T& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) { const T u = __shfl_up_sync(FULL, v, o); if (lane >= o) v += u; }
-  __syncthreads();
-  if (lane == 31) s_warp[warp] = v;
-  __syncthreads();
-  T pre = 0, all = 0;
-  for (int w = 0; w < warps; w++) { const T t = s_warp[w]; if (w < warp) pre += t; all += t; }
-  total = all;
-  return v + pre;
 }
 
 // ---- level 1 -----------------------------------------------------------------------------------------------------------
@@ -457,18 +378,6 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
 
 // ---- level 2 -----------------------------------------------------------------------------------------------------------
 
-// Transposes the 32x32 bit matrix whose row i is lane i's word.
-__device__ __forceinline__ uint32_t transpose_bits(uint32_t x) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const uint32_t m = o == 16 ? 0x0000FFFFu : o == 8 ? 0x00FF00FFu : o == 4 ? 0x0F0F0F0Fu : o == 2 ? 0x33333333u : 0x55555555u;   // columns without bit o
-    const uint32_t y = __shfl_xor_sync(FULL, x, o);
-    x = (lane & o) ? (x & ~m) | ((y >> o) & m) : (x & m) | ((y & m) << o);
-  }
-  return x;
-}
-
 // The pairs of one item and the bin's corner.
 struct Item { uint32_t first, end; int bx, by; };
 __device__ __forceinline__ Item item_of(const Tables& t, const Band& g, uint32_t it, uint32_t limit) {
@@ -485,7 +394,6 @@ __device__ __forceinline__ Item item_of(const Tables& t, const Band& g, uint32_t
 template <bool WHOLE>
 __global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, Tables t, Pairs pr) {
   after_previous();
-  struct WarpShare { float4 rec[64]; unsigned long long hits[32]; uint32_t unit[32 * BIN_W]; };   // unit: pair | row << 5 | columns << 8
   __shared__ WarpShare s_share[L2_WARPS];
   __shared__ uint32_t s_cnt[L2_WARPS][BIN_TILES];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -508,44 +416,10 @@ __global__ void __launch_bounds__(L2_THREADS) item_count_kernel(View v, Band g, 
         } else {
           todo = rect_bits(b, m.bx, m.by) & alive;
           const float4 q0 = v.proj0[i], q1 = v.proj1[i];
-          const TileRec rec = make_tile_rec(q0.x, q0.y, q0.z, q0.w, q1.x, q1.w);
-          ws.rec[lane * 2] = make_float4(rec.mx, rec.my, rec.c00, rec.c01);
-          ws.rec[lane * 2 + 1] = make_float4(rec.c11, rec.power, rec.ia, rec.ib);
+          share_record(ws, q0, q1);
         }
       }
-      // The tests of the warp's pairs are shared out by tile row: boxes hold one to 64 tiles of the bin, and with a pair per
-      // lane most lanes wait for the largest.
-      uint32_t rows = 0u;
-#pragma unroll
-      for (int r = 0; r < BIN_W; r++) rows |= ((uint32_t)(todo >> (8 * r)) & 0xFFu) ? 1u << r : 0u;
-      uint32_t at = __popc(rows);
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(FULL, at, o); if (lane >= o) at += u; }
-      const uint32_t units = __shfl_sync(FULL, at, 31);
-      if (units) {
-        at -= __popc(rows);
-        for (uint32_t b = rows; b; b &= b - 1u, at++) {
-          const int r = __ffs(b) - 1;
-          ws.unit[at] = (uint32_t)lane | ((uint32_t)r << 5) | (((uint32_t)(todo >> (8 * r)) & 0xFFu) << 8);
-        }
-        ws.hits[lane] = 0ull;
-        __syncwarp();
-        for (uint32_t u = lane; u < units; u += 32) {
-          const uint32_t e = ws.unit[u], owner = e & 31u, r = (e >> 5) & 7u;
-          const float4 a = ws.rec[owner * 2], b = ws.rec[owner * 2 + 1];
-          const TileRec rec{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-          const TileRow row = tile_row(m.by * BIN_W + (int)r, rec);
-          uint32_t out = 0u;
-          for (uint32_t cols = e >> 8; cols; cols &= cols - 1u) {
-            const int c = __ffs(cols) - 1;
-            if (tile_hit(m.bx * BIN_W + c, row, rec)) out |= 1u << c;
-          }
-          reinterpret_cast<unsigned char*>(ws.hits + owner)[r] = (unsigned char)out;
-        }
-        __syncwarp();
-        hits |= ws.hits[lane];
-        __syncwarp();
-      }
+      hits |= shared_tests(ws, todo, m.bx, m.by);
       if (kept && p < m.end) { pr.lo[p] = (uint32_t)hits; pr.hi[p] = (uint32_t)(hits >> 32); }
       c_lo += __popc(transpose_bits((uint32_t)hits)); c_hi += __popc(transpose_bits((uint32_t)(hits >> 32)));
     }
@@ -623,22 +497,6 @@ __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, T
   }
 }
 
-// A pair's hit word by itself, where none was kept.
-template <bool WHOLE>
-__device__ __forceinline__ unsigned long long hits_again(const View& v, int bx, int by, unsigned long long alive, uint32_t i) {
-  const uint4 hi = v.hit_info[i];
-  const Box b = box_of(hi);
-  if (WHOLE && hi.z != 0xFFFFFFFFu) return mask_bits(hi, b, bx, by);
-  const float4 q0 = v.proj0[i], q1 = v.proj1[i];
-  const TileRec rec = make_tile_rec(q0.x, q0.y, q0.z, q0.w, q1.x, q1.w);
-  unsigned long long out = 0ull;
-  for (unsigned long long todo = rect_bits(b, bx, by) & alive; todo; todo &= todo - 1ull) {
-    const int tile = __ffsll((long long)todo) - 1;
-    if (tile_hit(bx * BIN_W + (tile & 7), by * BIN_W + (tile >> 3), rec)) out |= 1ull << tile;
-  }
-  return out;
-}
-
 // The hits of an item to their tiles' lists, in the order of the pairs: for each tile the warp takes the 32 pairs of one hit
 // word at a time, and the lanes with a hit write side by side.
 template <bool WHOLE, bool KEPT>
@@ -711,11 +569,7 @@ __global__ void __launch_bounds__(256) fill_keys_kernel(int n_tiles, const uint2
 // Bins the ranks of one depth chunk (words != nullptr) or of the whole view into vals_sorted and `ranges`. Level 1's pairs
 // take ctx->keys, the hit words (or more pairs) ctx->vals and ctx->keys_sorted, a chunk's live splats the scratch of the depth sort.
 int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, int hi_num, const unsigned long long* alive, uint32_t* tables, cudaStream_t s) {
-  Tables t;
-  t.cells = tables;
-  t.totals = t.cells + BINS_TABLE_WORDS; t.base = t.totals + MAX_BINS; t.first_item = t.base + MAX_BINS + 1; t.item_bin = t.first_item + MAX_BINS + 1;
-  t.block_sums = t.item_bin + MAX_ITEMS; t.segments = t.block_sums + 1024; t.st = t.segments + BINS_SEGMENTS;
-  static_assert(MAX_BINS + 2 * (MAX_BINS + 1) + MAX_ITEMS + 1024 + BINS_SEGMENTS + 16 <= BINS_EXTRA_WORDS, "scratch");
+  const Tables t = bins_tables(tables);
   static bool attr_set[64] = {false};
   int dev = 0;
   constexpr int smem_max = MAX_BINS * ((L1_WARPS + 1) * (int)sizeof(uint32_t) + 8);
@@ -731,16 +585,17 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
   if (bins_x > MAX_BINS) return B2K_ERR_UNSUPPORTED;   // tile boxes hold twelve bits of a tile's column: the caller's own limit is lower
   const int rows_per_band = MAX_BINS / bins_x;
   View v{c->order, (const uint4*)c->hit_info, c->tile_count, (const float4*)c->proj0, (const float4*)c->proj1, n, words, chunk, lo_num, hi_num, alive, 0, 0};
+  const long long most = words ? (long long)n * (hi_num - lo_num) / 256 + 1 : n;   // ranks
+  if (!words && walks(c, n)) return launch_walk(c, v, tables, s);
   for (int row = 0; row < bin_rows; row += rows_per_band) {
     Band g{c->tiles_x, c->tiles_y, bins_x, row, std::min(rows_per_band, bin_rows - row)};
     v.first_band = row == 0; v.last_band = row + g.bin_rows == bin_rows;
     const int bins = g.bins_x * g.bin_rows;
     // Blocks of level 1: two per SM, no more than the table holds rows for, none without a rank.
-    const long long ranks = words ? (long long)n * (hi_num - lo_num) / 256 + 1 : n;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>({2LL * sm_count(), 32LL * ROWS_PER, (long long)(BINS_TABLE_WORDS / bins), (ranks + L1_THREADS - 1) / L1_THREADS}));
+    const int blocks = (int)std::max<long long>(1, std::min<long long>({2LL * sm_count(), 32LL * ROWS_PER, (long long)(BINS_TABLE_WORDS / bins), (most + L1_THREADS - 1) / L1_THREADS}));
     // Items are read on the device: a grid that fills the GPU, or what few splats can make at most.
-    const int item_blocks = (int)std::min<long long>(sm_count() * 8LL, bins + ranks * std::min(bins, 64) / L2_THREADS);
-    const int tiles = (std::min((row + g.bin_rows) * BIN_W, c->tiles_y) - row * BIN_W) * c->tiles_x, scan_blocks = div_up(tiles, SCAN_TILES);
+    const int item_blocks = (int)std::min<long long>(sm_count() * 8LL, bins + most * std::min(bins, 64) / L2_THREADS);
+    const int tiles = (std::min((row + g.bin_rows) * BIN_W, c->tiles_y) - row * BIN_W) * c->tiles_x;
 #define L(WHOLE) do { \
     const size_t alive_bytes = WHOLE ? 0 : bins * sizeof(unsigned long long); \
     launch_next(bin_count_kernel<WHOLE>, blocks, COUNT_THREADS, alive_bytes + bins * sizeof(uint32_t) + (WHOLE ? 0 : live_sums_bytes(g)), s, v, g, t, c->depth_keys); \
@@ -751,7 +606,7 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
 #undef L
     if (bins >= 2 * sm_count()) launch_next(item_columns_kernel<4>, bins, 4 * BIN_TILES, 0, s, g, t, ranges);
     else launch_next(item_columns_kernel<16>, bins, 16 * BIN_TILES, 0, s, g, t, ranges);
-    launch_next(tile_scan_kernel, scan_blocks, SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect);
+    launch_next(tile_scan_kernel, div_up(tiles, SCAN_TILES), SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect);
     if (words) launch_next(item_emit_kernel<false>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
     else launch_next(item_emit_kernel<true>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
   }

@@ -11,13 +11,12 @@
 // Bound by latency (launches, barriers) up to a few hundred thousand splats, by the scatter's issue and writes above. Against
 // four passes of eight bits with tiles of 4,096 at every size, first launch to last: 2,000 splats 89 -> 12 us, 100,000 94 ->
 // 52, 500,000 103 -> 64, three million 176 -> 132, six million 254 -> 204.
-#include "common.cuh"
+#include "bins.cuh"
 #include <algorithm>
 
 namespace b2k {
 namespace {
 
-constexpr unsigned FULL = 0xffffffffu;
 constexpr uint32_t CULLED = 0xFFFFFFFFu;
 constexpr int MAX_RADIX = 2048;             // eleven bits: any keys; depths that this library projected fit ten (see DEPTH_RADIX)
 constexpr int DEPTH_RADIX = 1024;           // the projection keeps depths of 0.01 .. 1e10: 29 bits of range, three digits of ten
@@ -27,6 +26,11 @@ __device__ __forceinline__ uint32_t warp_incl(uint32_t v) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(FULL, v, o); if (lane >= o) v += u; }
   return v;
+}
+
+// walk.cu's tile totals are zero when its kernels begin: a kernel of the sort clears them on the way (nullptr: no walk follows).
+__device__ __forceinline__ void clear_totals(uint32_t* totals) {
+  if (totals) for (int i = threadIdx.x; i < WALK_TILES; i += blockDim.x) totals[i] = 0u;
 }
 
 // How keys are cut into digits: `compress` from the range of the keys, else plain bytes.
@@ -48,7 +52,7 @@ constexpr size_t small_smem(int items) { return (size_t)SMALL_THREADS * items * 
 // A warp owns a contiguous run of 32 * ITEMS pairs, held in registers from one pass to the write of the next; pair j * 32 + l
 // of the run is lane l's j-th.
 template <int ITEMS>
-__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* keys_out, uint32_t* vals_out) { after_previous();   // may work in place
+__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* keys_out, uint32_t* vals_out, uint32_t* totals) { after_previous();   // may work in place
   extern __shared__ __align__(16) uint32_t s_mem[];
   uint32_t* s_key = s_mem;
   uint32_t* s_val = s_key + SMALL_THREADS * ITEMS;
@@ -57,6 +61,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_
   __shared__ uint32_t s_red[2][SMALL_WARPS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int first = warp * (32 * ITEMS) + lane;
+  clear_totals(totals);
   uint32_t key[ITEMS], val[ITEMS], lo = CULLED, hi = 0u;
 #pragma unroll
   for (int j = 0; j < ITEMS; j++) {
@@ -129,8 +134,9 @@ __device__ __forceinline__ uint32_t run_of(uint32_t n, uint32_t blocks, uint32_t
 // Keys are read four at a time where the caller's array allows it.
 __device__ __forceinline__ bool by_quads(const uint32_t* keys) { return ((uintptr_t)keys & 15u) == 0u; }
 
-__global__ void __launch_bounds__(CNT_THREADS) key_range_kernel(const uint32_t* __restrict__ keys, uint32_t n, Range* __restrict__ range) {
+__global__ void __launch_bounds__(CNT_THREADS) key_range_kernel(const uint32_t* __restrict__ keys, uint32_t n, Range* __restrict__ range, uint32_t* __restrict__ totals) {
   after_previous();
+  if (blockIdx.x == gridDim.x - 1) clear_totals(totals);
   __shared__ uint32_t s_lo[CNT_THREADS / 32], s_hi[CNT_THREADS / 32];
   uint32_t lo = CULLED, hi = 0u;
   auto see = [&](uint32_t k) { if (k != CULLED) { lo = min(lo, k); hi = max(hi, k); } };
@@ -383,31 +389,32 @@ int one_pass(const Shape& sh, const uint32_t* ki, const uint32_t* vi, uint32_t* 
 }
 
 template <int ITEMS>
-int small_sort(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* ko, uint32_t* vo, cudaStream_t s) {
+int small_sort(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* ko, uint32_t* vo, uint32_t* totals, cudaStream_t s) {
   static bool attr_set[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !attr_set[dev]) {
     B2K_CUDA(cudaFuncSetAttribute(small_sort_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(ITEMS)));
     attr_set[dev] = true;
   }
-  launch_next(small_sort_kernel<ITEMS>, 1, SMALL_THREADS, small_smem(ITEMS), s, keys, vals, n, ko, vo);
+  launch_next(small_sort_kernel<ITEMS>, 1, SMALL_THREADS, small_smem(ITEMS), s, keys, vals, n, ko, vo, totals);
   return check_launch();
 }
 
-int depth_sort(const B2kCtx* c, int n, bool identity, uint32_t* tables, cudaStream_t s) {
+int depth_sort(const B2kCtx* c, int n, bool identity, bool for_walk, uint32_t* tables, cudaStream_t s) {
   const uint32_t* in = c->depth_keys_sorted;
   const uint32_t* index = identity ? nullptr : c->order;
+  uint32_t* cleared = for_walk ? bins_tables(tables).tile_totals : nullptr;
   if (n <= SMALL_N) {   // one block reads everything before it writes: in place
     const int items = div_up(n, SMALL_THREADS);
-    return items <= 2 ? small_sort<2>(in, index, n, c->depth_keys_sorted, c->order, s) : items <= 4 ? small_sort<4>(in, index, n, c->depth_keys_sorted, c->order, s)
-                                                                                               : small_sort<SMALL_ITEMS>(in, index, n, c->depth_keys_sorted, c->order, s);
+    uint32_t *k = c->depth_keys_sorted, *v = c->order;
+    return items <= 2 ? small_sort<2>(in, index, n, k, v, cleared, s) : items <= 4 ? small_sort<4>(in, index, n, k, v, cleared, s) : small_sort<SMALL_ITEMS>(in, index, n, k, v, cleared, s);
   }
   uint32_t *table = tables, *totals = table + BINS_TABLE_WORDS;
   Range* range = (Range*)(totals + MAX_RADIX);
-  static_assert(MAX_RADIX + sizeof(Range) / sizeof(uint32_t) <= BINS_EXTRA_WORDS, "scratch");
+  static_assert(MAX_RADIX + sizeof(Range) / sizeof(uint32_t) <= BINS_EXTRA_WORDS - WALK_TILES, "scratch");
   const Shape sh = shape_of((uint32_t)n);
   const int range_blocks = std::min<int>(std::min(2 * sm_count(), MAX_BLOCKS), div_up(n, CNT_THREADS * 16));
-  launch_next(key_range_kernel, range_blocks, CNT_THREADS, 0, s, in, (uint32_t)n, range);
+  launch_next(key_range_kernel, range_blocks, CNT_THREADS, 0, s, in, (uint32_t)n, range, cleared);
   // Three passes by way of two scratch pairs (the second: tile_off and the projection's list, both free here).
   uint32_t* list = big_list_ptr(c);
   const uint32_t* ki[3] = {in, c->depth_keys, c->tile_off};

@@ -389,3 +389,24 @@ def test_loss_gradient_at_any_word(W, H, masked):
         got.append((h.ctx.v_out.cpu().numpy(), float(h.ctx.loss_accum[0].item())))
     (a, la), (b, lb) = got
     assert rel_l2(b, a) <= 1e-6 and abs(la - lb) <= 1e-5 * abs(la)
+
+
+@pytest.mark.parametrize("W,H,n,wide", [(8, 8, 1, 0), (8, 8, 257, 3), (64, 64, 255, 3), (64, 64, 256, 0), (65, 63, 513, 9), (200, 150, 8193, 40),
+                                        (512, 512, 5000, 30), (520, 512, 5000, 30), (1000, 24, 4000, 90)])
+@pytest.mark.parametrize("room", [True, False])
+def test_small_views_walked(W, H, n, wide, room):
+    """Whole views of up to 4,096 tiles are binned by walking the ranks for every bin, given room for the hit words; in buffers of just
+    the lists' size some take the general distribution. Runs of 256 ranks, one tile, one bin, ragged bins, large boxes."""
+    scene, cam = bin_scene(n, W, H, wide, seed=n)
+    h = Harness(scene, cam, isect_cap=1 << 22)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    tc_o, vals_o, keys_o, ranges_o = orc.bin_sort(h.ctx.proj0[:n].cpu().numpy(), h.ctx.proj1[:n].cpu().numpy(), W, H)
+    if not room:
+        h.ctx._alloc_isect(len(vals_o))
+    for again in range(2):                                     # the second time from keys and an order that are sorted already
+        h.api.bin_and_sort(h.ctx, h.model)
+        tc = h.u32(h.ctx.tile_count, n)
+        assert h.ctx.num_isect == len(vals_o) > 0 and np.array_equal(tc, tc_o)
+        assert np.array_equal(h.u32(h.ctx.vals_sorted, len(vals_o)), vals_o) and np.array_equal(h.u32(h.ctx.keys_sorted, len(vals_o)), keys_o)
+        assert np.array_equal(h.u32(h.ctx.tile_ranges).reshape(-1, 2), ranges_o)
+        assert np.array_equal(h.u32(h.ctx.tile_off, n), np.cumsum(tc[h.u32(h.ctx.order, n)], dtype=np.uint32))
