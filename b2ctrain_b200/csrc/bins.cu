@@ -150,6 +150,18 @@ __device__ __forceinline__ int own_bin(const Band& g, const Rank& k, int c) {
   const int dy = c / k.span.w;
   return (k.span.by0 + dy - g.bin_row0) * g.bins_x + k.span.bx0 + c - dy * k.span.w;
 }
+// The bins of a splat over many of them, shared out over the lanes of a warp: f(local bin). Returns whether the lane called f.
+template <bool WHOLE, class F>
+__device__ __forceinline__ bool spread_bins(const unsigned long long* s_alive, const Band& g, const uint4& hi, F f) {
+  const Box b = box_of(hi);
+  const BinSpan s = span_of(b, g);
+  bool any = false;
+  for (int c = threadIdx.x & 31; c < s.count; c += 32) {
+    const int dy = c / s.w, bx = s.bx0 + c - dy * s.w, by = s.by0 + dy, bin = (by - g.bin_row0) * g.bins_x + bx;
+    if (takes_bin<WHOLE>(s_alive, hi, b, bx, by, bin, s.count)) { any = true; f(bin); }
+  }
+  return any;
+}
 // Splats over many bins are spread by the whole warp, one after the other: f(lane of the splat, splat, local bin) for every
 // bin. All lanes call this together; returns whether this lane's own splat is wide and went into any bin.
 template <bool WHOLE, class F>
@@ -161,14 +173,7 @@ __device__ __forceinline__ bool wide_bins(const unsigned long long* s_alive, con
     uint4 hi;
     hi.x = __shfl_sync(FULL, k.hi.x, src); hi.y = __shfl_sync(FULL, k.hi.y, src); hi.z = __shfl_sync(FULL, k.hi.z, src); hi.w = __shfl_sync(FULL, k.hi.w, src);
     const uint32_t splat = __shfl_sync(FULL, k.splat, src);
-    const Box b = box_of(hi);
-    const BinSpan s = span_of(b, g);
-    bool any = false;
-    for (int c = lane; c < s.count; c += 32) {
-      const int dy = c / s.w, bx = s.bx0 + c - dy * s.w, by = s.by0 + dy, bin = (by - g.bin_row0) * g.bins_x + bx;
-      if (takes_bin<WHOLE>(s_alive, hi, b, bx, by, bin, s.count)) { any = true; f(src, splat, bin); }
-    }
-    any = __any_sync(FULL, any);
+    const bool any = __any_sync(FULL, spread_bins<WHOLE>(s_alive, g, hi, [&](int bin) { f(src, splat, bin); }));
     if (lane == src) took = any;
   }
   return took;
@@ -303,7 +308,9 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
   const int bins = band_bins(g), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long* s_alive = reinterpret_cast<unsigned long long*>(s_bits + (size_t)bins * L1_WARPS);
   uint32_t* s_next = reinterpret_cast<uint32_t*>(s_alive + (WHOLE ? 0 : bins));
-  __shared__ uint32_t s_warp[32];
+  __shared__ uint32_t s_warp[32], s_wides;
+  __shared__ uint4 s_wide[L1_THREADS];
+  __shared__ uint2 s_wide_of[L1_THREADS];     // splat, thread
   uint32_t r0, r1;
   view_ranks(v, r0, r1);
   const uint32_t len = run_len(r1 - r0, gridDim.x);
@@ -317,6 +324,7 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
   }
   if (begin >= end && !(offsets && blockIdx.x == gridDim.x - 1)) return;
   for (int i = tid; i < bins * L1_WARPS; i += L1_THREADS) s_bits[i] = 0u;
+  if (tid == 0) s_wides = 0u;
   for (int i = tid; i < bins; i += L1_THREADS) s_next[i] = (uint32_t)min((unsigned long long)t.base[i] + t.cells[(size_t)i * gridDim.x + blockIdx.x], (unsigned long long)room);
   if (!WHOLE) load_alive(v, g, s_alive);
   uint32_t tiles_before = 0;
@@ -327,13 +335,13 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
     tiles_before = total;
   }
   __syncthreads();
-  auto earlier = [&](int bin, int l) {   // pairs of this round before lane l of this warp
+  auto earlier = [&](int bin, int of_warp, int l) {   // pairs of this round before lane l of a warp
     const uint4* b4 = reinterpret_cast<const uint4*>(s_bits + bin * L1_WARPS);
     const uint4 a = b4[0], b = b4[1];
     const uint32_t w[L1_WARPS] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     uint32_t n = 0;
 #pragma unroll
-    for (int k = 0; k < L1_WARPS; k++) n += (uint32_t)__popc(k < warp ? w[k] : k == warp ? w[k] & ((1u << l) - 1u) : 0u);
+    for (int k = 0; k < L1_WARPS; k++) n += (uint32_t)__popc(k < of_warp ? w[k] : k == of_warp ? w[k] & ((1u << l) - 1u) : 0u);
     return n;
   };
   auto move_on = [&](int bin) {
@@ -348,22 +356,37 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
       const Rank k = ranks.next();
       const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
       for (uint32_t b = take; b; b &= b - 1u) atomicOr(&s_bits[own_bin(g, k, __ffs(b) - 1) * L1_WARPS + warp], 1u << lane);
-      wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t, int bin) { atomicOr(&s_bits[bin * L1_WARPS + warp], 1u << l); });
+      // Splats over many bins are listed, and the block's warps share them: behind the first chunks they are most of what is left, and with
+      // each to its own warp a few warps spread thirty while the others wait.
+      const bool wide = k.span.count > SERIAL_BINS;
+      if (wide) { const uint32_t at = atomicAdd(&s_wides, 1u); s_wide[at] = k.hi; s_wide_of[at] = make_uint2(k.splat, (uint32_t)tid); }
       if (offsets) {
         uint32_t total;
         const uint32_t incl = block_scan(k.tiles, s_warp, total);
         if (at + tid < end) tile_off[at + tid] = tiles_before + incl;
         tiles_before += total;
       }
-      const bool any_wide = __syncthreads_or(k.span.count > SERIAL_BINS);
+      const bool any_wide = __syncthreads_or(wide);
+      const uint32_t wides = any_wide ? s_wides : 0u;
+      if (any_wide) {
+        for (uint32_t e = warp; e < wides; e += L1_WARPS) {
+          const uint32_t of = s_wide_of[e].y;
+          spread_bins<WHOLE>(s_alive, g, s_wide[e], [&](int bin) { atomicOr(&s_bits[bin * L1_WARPS + (of >> 5)], 1u << (of & 31u)); });
+        }
+        __syncthreads();
+        if (tid == 0) s_wides = 0u;
+      }
       uint32_t first = 0u;
       for (uint32_t b = take; b; b &= b - 1u) {
         const int bin = own_bin(g, k, __ffs(b) - 1);
-        const uint32_t n = earlier(bin, lane), pos = s_next[bin] + n;
+        const uint32_t n = earlier(bin, warp, lane), pos = s_next[bin] + n;
         put(pos, k.splat);
         if (n == 0u) first |= b & (0u - b);
       }
-      wide_bins<WHOLE>(s_alive, g, k, [&](int l, uint32_t splat, int bin) { const uint32_t pos = s_next[bin] + earlier(bin, l); put(pos, splat); });
+      for (uint32_t e = warp; e < wides; e += L1_WARPS) {
+        const uint2 of = s_wide_of[e];
+        spread_bins<WHOLE>(s_alive, g, s_wide[e], [&](int bin) { put(s_next[bin] + earlier(bin, (int)(of.y >> 5), (int)(of.y & 31u)), of.x); });
+      }
       __syncthreads();
       if (any_wide) { for (int i = tid; i < bins; i += L1_THREADS) move_on(i); }
       else { for (uint32_t b = first; b; b &= b - 1u) move_on(own_bin(g, k, __ffs(b) - 1)); }

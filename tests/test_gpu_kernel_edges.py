@@ -410,3 +410,18 @@ def test_small_views_walked(W, H, n, wide, room):
         assert np.array_equal(h.u32(h.ctx.vals_sorted, len(vals_o)), vals_o) and np.array_equal(h.u32(h.ctx.keys_sorted, len(vals_o)), keys_o)
         assert np.array_equal(h.u32(h.ctx.tile_ranges).reshape(-1, 2), ranges_o)
         assert np.array_equal(h.u32(h.ctx.tile_off, n), np.cumsum(tc[h.u32(h.ctx.order, n)], dtype=np.uint32))
+
+
+def test_chunks_of_wide_splats():
+    """Hundreds of splats over most bins in one round of the distribution: shared out over the block's warps."""
+    import torch
+    W, H, n = 1040, 264, 6000
+    scene, cam = bin_scene(n, W, H, 2000)
+    scene["pos_op"][:, 3] = -3.0
+    h = Harness(scene, cam, isect_cap=1 << 23)
+    h.forward()
+    for chunks in (2, 3):
+        ctx = h.api.RenderCtx("cuda:0")
+        ctx.setup(W, H, h.model.cap, n_chunks=chunks, isect_cap=1 << 23)
+        h.api.render_forward(ctx, h.model, h.rp)
+        assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
