@@ -33,10 +33,68 @@ namespace {
 
 constexpr int PROJ_BLOCK = 256;
 
-// Tile boxes of at most this many tiles are tested by the projecting thread and remembered as a bit mask; larger
-// ones go to a list that a warp-per-splat kernel counts (and later emits) cooperatively.
-constexpr int MASK_TILES = 64;
+// Tile boxes of at most MASK_TILES tiles are remembered as a bit mask of the tiles hit. The tests of boxes of at most WARP_TILES tiles
+// are shared out over the splats' warp; larger ones go to a list that a warp-per-splat kernel counts, so that no warp waits for a few of them.
+constexpr int MASK_TILES = 64, WARP_TILES = 1024;
 
+// The tile tests of a warp's 32 splats, shared out in units of up to eight tiles of one row: boxes hold one to a thousand tiles, and with
+// a splat per lane most lanes wait for the largest.
+struct TileShare { float4 rec[64]; uint32_t corner[32], width[32], end[32], mask[64], count[32]; };
+// box: the lane's tile box (empty: none); returns the tiles hit, and for boxes of at most MASK_TILES tiles their mask. All lanes call this.
+__device__ __forceinline__ uint32_t shared_hits(TileShare& ts, const TileRec& rec, const TileBox& b, int area, uint32_t& mask_lo, uint32_t& mask_hi) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, bw = b.max_x - b.min_x;
+  const int units = area > 0 ? (b.max_y - b.min_y) * ((bw + 7) >> 3) : 0;
+  int end = units;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(ALL, end, o); if (lane >= o) end += u; }
+  const int total = __shfl_sync(ALL, end, 31);
+  mask_lo = mask_hi = 0u;
+  if (total == 0) return 0u;
+  ts.rec[lane * 2] = make_float4(rec.mx, rec.my, rec.c00, rec.c01);
+  ts.rec[lane * 2 + 1] = make_float4(rec.c11, rec.power, rec.ia, rec.ib);
+  ts.corner[lane] = (uint32_t)b.min_x | (uint32_t)b.min_y << 16; ts.width[lane] = (uint32_t)bw | (area <= MASK_TILES ? 0x80000000u : 0u); ts.end[lane] = (uint32_t)end;
+  ts.mask[lane * 2] = ts.mask[lane * 2 + 1] = 0u; ts.count[lane] = 0u;
+  __syncwarp();
+  for (int u = lane; u < total; u += 32) {
+    int owner = 0;   // the first lane whose units end behind u
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) owner += (int)ts.end[owner + step - 1] <= u ? step : 0;
+    const uint32_t corner = ts.corner[owner], wide = ts.width[owner], w = wide & 0xFFFFu, per_row = (w + 7u) >> 3;
+    const uint32_t at = (uint32_t)u - (owner ? ts.end[owner - 1] : 0u), row_in_box = per_row == 1u ? at : at / per_row, x0 = (at - row_in_box * per_row) * 8u;
+    const float4 a = ts.rec[owner * 2], c = ts.rec[owner * 2 + 1];
+    const TileRec r{a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+    const TileRow row = tile_row((int)((corner >> 16) + row_in_box), r);
+    const uint32_t tiles = min(w - x0, 8u);
+    uint32_t out = 0u;
+    for (uint32_t k = 0; k < tiles; k++) out |= tile_hit((int)((corner & 0xFFFFu) + x0 + k), row, r) ? 1u << k : 0u;
+    if (out == 0u) continue;
+    atomicAdd(&ts.count[owner], (uint32_t)__popc(out));
+    if (wide >> 31) {
+      const uint32_t bit = row_in_box * w + x0;
+      const unsigned long long word = (unsigned long long)out << (bit & 31u);
+      atomicOr(&ts.mask[owner * 2 + (bit >> 5)], (uint32_t)word);
+      if (word >> 32) atomicOr(&ts.mask[owner * 2 + 1], (uint32_t)(word >> 32));
+    }
+  }
+  __syncwarp();
+  mask_lo = ts.mask[lane * 2]; mask_hi = ts.mask[lane * 2 + 1];
+  return ts.count[lane];
+}
+
+// What a splat's record says about its tiles: tiles hit, the words of hit_info, whether it goes to the list of large boxes. All lanes of
+// the warp call this; `drawn`: the splat has a record and its box is on the image.
+struct TileHits { uint32_t hits, w0, w1, box, height; bool big; };
+__device__ __forceinline__ TileHits decide_tiles(TileShare& ts, const TileRec& rec, const TileBox& b, bool drawn) {
+  const int bw = drawn ? b.max_x - b.min_x : 0, bh = drawn ? b.max_y - b.min_y : 0, area = bw > 0 && bh > 0 ? bw * bh : 0;
+  TileHits t{0u, 0u, 0u, 0u, drawn ? (uint32_t)bh : 0u, area > WARP_TILES};
+  t.hits = shared_hits(ts, rec, b, t.big ? 0 : area, t.w0, t.w1);
+  if (area > MASK_TILES) {   // no mask: the box itself
+    t.box = 0xFFFFFFFFu;
+    t.w0 = (uint32_t)b.min_x | ((uint32_t)b.min_y << 16); t.w1 = (uint32_t)bw | ((uint32_t)bh << 16);
+  } else if (area > 0) t.box = (uint32_t)b.min_x | ((uint32_t)b.min_y << 12) | ((uint32_t)bw << 24);
+  return t;
+}
 
 // Feature lanes of a splat (src/gpu/project.cu:62-77). Mode 1: pseudo-normal = the local axis of the shortest scale,
 // turned to face the camera, in camera space. Mode 2: the caller's per-splat buffer, clamped to +-100, non-finite -> 0.
@@ -84,57 +142,50 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
     uint4* __restrict__ hit_info, uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in, float* __restrict__ max_screen,
     uint32_t* __restrict__ big_list, uint32_t* __restrict__ big_count, int feat_mode, const float* __restrict__ feat_in, float2* __restrict__ proj3) {
   after_previous();
+  __shared__ TileShare s_share[PROJ_BLOCK / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 po = pos_op[i], q = quat[i], ls = lscale[i];
+  const bool valid = i < n;
+  float4 po = make_float4(0.f, 0.f, 0.f, 0.f), q = po, ls = po;
+  if (valid) { po = pos_op[i]; q = quat[i]; ls = lscale[i]; }
   Proj pr;
-  uint32_t hits = 0, mask_lo = 0, mask_hi = 0, box = 0, height = 0;
-  bool shade = false, big = false;
-  if (project_one(po, q, ls, cam, pr)) {
-    const TileRec rec = make_tile_rec(pr.mx, pr.my, pr.c00, pr.c01, pr.c11, pr.power);
-    TileBox bb;
-    if (tile_box(rec, cam.W, cam.H, tiles_x, tiles_y, bb)) {
-      const int bw = bb.max_x - bb.min_x, bh = bb.max_y - bb.min_y;
-      height = (uint32_t)bh;
-      if (bw * bh > MASK_TILES) {
-        big = true; shade = true;
-        box = 0xFFFFFFFFu;
-        mask_lo = (uint32_t)bb.min_x | ((uint32_t)bb.min_y << 16); mask_hi = (uint32_t)bw | ((uint32_t)bh << 16);   // no mask: the box itself
-        big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
-      } else if (bw > 0 && bh > 0) {
-        int bit = 0;
-        for (int ty = bb.min_y; ty < bb.max_y; ty++)
-          for (int tx = bb.min_x; tx < bb.max_x; tx++, bit++)
-            if (tile_hit(tx, ty, rec)) { hits++; if (bit < 32) mask_lo |= 1u << bit; else mask_hi |= 1u << (bit - 32); }
-        box = (uint32_t)bb.min_x | ((uint32_t)bb.min_y << 12) | ((uint32_t)bw << 24);
-        shade = hits != 0;
-      }
-      const float detc = pr.c00 * pr.c11 - pr.c01 * pr.c01;
-      const float ex = sqrtf(2.f * pr.power * pr.c11 / detc), ey = sqrtf(2.f * pr.power * pr.c00 / detc);
-      if (max_screen) { const float ms = fmaxf(ex / (float)cam.W, ey / (float)cam.H); if (ms > max_screen[i]) atomic_max_nonneg(max_screen + i, ms); }
+  TileRec rec{};
+  TileBox bb{0, 0, 0, 0};
+  bool drawn = false;
+  if (valid) {
+    if (project_one(po, q, ls, cam, pr)) {
+      rec = make_tile_rec(pr.mx, pr.my, pr.c00, pr.c01, pr.c11, pr.power);
+      drawn = tile_box(rec, cam.W, cam.H, tiles_x, tiles_y, bb);
+      proj0[i] = make_float4(pr.mx, pr.my, pr.c00, pr.c01);
+      proj1[i] = make_float4(pr.c11, pr.opac, pr.mean_c.z, pr.power);
+    } else {
+      proj1[i] = make_float4(0.f, 0.f, 0.f, -1.f);   // no record
     }
-    proj0[i] = make_float4(pr.mx, pr.my, pr.c00, pr.c01);
-    proj1[i] = make_float4(pr.c11, pr.opac, pr.mean_c.z, pr.power);
-    if (shade) {
-      float4 col = splat_colour<DEG>(i, cap, make_float3(po.x, po.y, po.z), cam.pos, active, sh_dc, sh_hi);
-      if (feat_mode != 0) {
-        const float3 f = splat_feature(feat_mode, i, po, ls, pr.Rq, cam, feat_in);
-        col.w = f.x;
-        proj3[i] = make_float2(f.y, f.z);
-      }
-      proj2[i] = col;
-    }
-  } else {
-    proj1[i] = make_float4(0.f, 0.f, 0.f, -1.f);   // no record
   }
-  hit_info[i] = make_uint4(mask_lo, mask_hi, box, height);
+  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn);
+  if (!valid) return;
+  if (t.big) big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
+  if (drawn && max_screen) {
+    const float detc = pr.c00 * pr.c11 - pr.c01 * pr.c01;
+    const float ex = sqrtf(2.f * pr.power * pr.c11 / detc), ey = sqrtf(2.f * pr.power * pr.c00 / detc);
+    const float ms = fmaxf(ex / (float)cam.W, ey / (float)cam.H);
+    if (ms > max_screen[i]) atomic_max_nonneg(max_screen + i, ms);
+  }
+  if (t.hits || t.big) {
+    float4 col = splat_colour<DEG>(i, cap, make_float3(po.x, po.y, po.z), cam.pos, active, sh_dc, sh_hi);
+    if (feat_mode != 0) {
+      const float3 f = splat_feature(feat_mode, i, po, ls, pr.Rq, cam, feat_in);
+      col.w = f.x;
+      proj3[i] = make_float2(f.y, f.z);
+    }
+    proj2[i] = col;
+  }
+  hit_info[i] = make_uint4(t.w0, t.w1, t.box, t.height);
   order_in[i] = (uint32_t)i;
-  if (!big) {   // big splats get their count and key from count_big_kernel
-    tile_count[i] = hits;
-    depth_keys[i] = hits ? __float_as_uint(pr.mean_c.z) : 0xFFFFFFFFu;
+  if (!t.big) {   // the others get their count and key from count_big_kernel
+    tile_count[i] = t.hits;
+    depth_keys[i] = t.hits ? __float_as_uint(pr.mean_c.z) : 0xFFFFFFFFu;
   }
 }
-
 
 // The projection of the chunked renderer, which decides tiles later and only for the splats whose tile box still holds
 // a live tile: records, colours, the tile box, the depth key, the screen-size statistic.
@@ -228,33 +279,24 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
                                                                  uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in,
                                                                  uint32_t* __restrict__ big_list, uint32_t* __restrict__ big_count) {
   after_previous();
+  __shared__ TileShare s_share[PROJ_BLOCK / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 a = proj0[i], b = proj1[i];
-  uint32_t hits = 0, mask_lo = 0, mask_hi = 0, box = 0, height = 0;
-  bool big = false;
+  const bool valid = i < n;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = make_float4(0.f, 0.f, 0.f, -1.f);
+  if (valid) { a = proj0[i]; b = proj1[i]; }
+  TileRec rec{};
+  TileBox bb{0, 0, 0, 0};
+  bool drawn = false;
   if (b.w > -0.5f) {
-    const TileRec rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
-    TileBox bb;
-    if (tile_box(rec, W, H, tiles_x, tiles_y, bb)) {
-      const int bw = bb.max_x - bb.min_x, bh = bb.max_y - bb.min_y;
-      height = (uint32_t)bh;
-      if (bw * bh > MASK_TILES) {
-        big = true; box = 0xFFFFFFFFu;
-        mask_lo = (uint32_t)bb.min_x | ((uint32_t)bb.min_y << 16); mask_hi = (uint32_t)bw | ((uint32_t)bh << 16);
-        big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
-      } else if (bw > 0 && bh > 0) {
-        int bit = 0;
-        for (int ty = bb.min_y; ty < bb.max_y; ty++)
-          for (int tx = bb.min_x; tx < bb.max_x; tx++, bit++)
-            if (tile_hit(tx, ty, rec)) { hits++; if (bit < 32) mask_lo |= 1u << bit; else mask_hi |= 1u << (bit - 32); }
-        box = (uint32_t)bb.min_x | ((uint32_t)bb.min_y << 12) | ((uint32_t)bw << 24);
-      }
-    }
+    rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
+    drawn = tile_box(rec, W, H, tiles_x, tiles_y, bb);
   }
-  hit_info[i] = make_uint4(mask_lo, mask_hi, box, height);
+  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn);
+  if (!valid) return;
+  if (t.big) big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
+  hit_info[i] = make_uint4(t.w0, t.w1, t.box, t.height);
   order_in[i] = (uint32_t)i;
-  if (!big) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
+  if (!t.big) { tile_count[i] = t.hits; depth_keys[i] = t.hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
 }
 
 // A few words to zero. (A memset node would break the chain of overlapped launches on both sides.)

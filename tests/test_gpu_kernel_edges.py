@@ -425,3 +425,26 @@ def test_chunks_of_wide_splats():
         ctx.setup(W, H, h.model.cap, n_chunks=chunks, isect_cap=1 << 23)
         h.api.render_forward(ctx, h.model, h.rp)
         assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
+
+
+def test_tile_boxes_of_every_size():
+    """The tile tests are shared out over a warp in units of eight tiles of a row: masks up to 64 tiles, counts up to 1,024, a list above."""
+    W, H, n = 1040, 720, 3001
+    scene = scenes.make_splats(n, 0, 11, log_scale=(-4.5, 1.6))
+    cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 25.0, 10.0), W, H, float(max(W, H)))
+    scene = scenes.floor_for_cameras(scene, [cam])
+    h = Harness(scene, cam, isect_cap=1 << 23)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    tc_o = orc.bin_sort(h.ctx.proj0[:n].cpu().numpy(), h.ctx.proj1[:n].cpu().numpy(), W, H)[0]
+    info = h.u32(h.ctx.hit_info[:n]).reshape(-1, 4)
+    large = info[:, 2] == 0xFFFFFFFF
+    area = np.where(large, (info[:, 1] & 0xFFFF) * (info[:, 1] >> 16), (info[:, 2] >> 24) * info[:, 3])
+    assert (area[~large] == 64).any() and (area == 1).any() and ((area > 64) & (area <= 1024)).any() and (area > 1024).any()
+    masks = np.array([bin(int(a)).count("1") + bin(int(b)).count("1") for a, b in info[:, :2]])
+    for project in (False, True):
+        assert np.array_equal(h.u32(h.ctx.tile_count, n), tc_o)
+        assert np.array_equal(masks[~large], tc_o[~large])
+        if not project:
+            h.ctx.tile_count.zero_(); h.ctx.hit_info.zero_()
+            h.api.count_tiles(h.ctx, h.model)
+            assert np.array_equal(h.u32(h.ctx.hit_info[:n]).reshape(-1, 4)[tc_o > 0], info[tc_o > 0])
