@@ -6,6 +6,8 @@
 // gather of 48 B per staged fragment, served mostly by L2. Fragments are gathered one batch ahead and staged in shared memory
 // as operands of packed arithmetic (fp32x2); the hit test is one comparison; a pixel that does not see a fragment takes it with
 // weight zero instead of branching around it (a vote and a branch per fragment cost more than the ten operations they saved).
+// Transmittances are multiplied up for a group of fragments first, and fragments are compared and selected one by one only where a
+// pixel of the warp closes inside the group (none_closes): 1024x1024 over 1M in four chunks 184 -> 172 us, 4K over 6M in five 734 -> 705.
 // Two kernels with the same arithmetic, bit for bit:
 //   raster_fwd_half_kernel  two warps to a tile, a lane one pixel, two consecutive fragments to a packed operation: the chain of
 //                           one list is half as long. For whole views and two chunks, where a visit to a tile is a long list.
@@ -41,7 +43,15 @@ __device__ __forceinline__ bool pair_any(int id, bool p) {
   return r != 0u;
 }
 
+// Expected depth from the depth sum of a pixel and its transmittance.
+__device__ __forceinline__ float finished_depth(float zs, float T) { return (1.f - T) > 0.05f ? zs / (1.f - T) : INFINITY; }
+
 constexpr uint32_t DONE_BIT = 0x80000000u;
+
+// A pixel carries its transmittance while it is open and zero once it has closed (the last value then waits in a variable of its own).
+// So a group of fragments multiplies up the transmittances first, one operation a fragment, and only if some pixel of the warp closes
+// inside the group (the product passes the cut-off: it never rises again) are fragments compared and selected one by one. Whether none does:
+__device__ __forceinline__ bool none_closes(float behind_group) { return __float_as_uint(behind_group) - 1u >= __float_as_uint(T_CUTOFF); }   // zero, or above the cut-off
 
 // Two fragments that follow each other in a list, the nearer in the first of each pair of lanes.
 constexpr int STAGED = 5;   // (-x, -y), (c00 / 2, c01), (c11 / 2, opacity), (power, r), (g, b); then (z, feature 0), (feature 1, 2)
@@ -59,6 +69,85 @@ __device__ __forceinline__ float2 pair_alpha(const float4& q0, const float4& q1,
 
 // What the forward leaves for the backward (common.cuh): nothing, checkpoints of the running sums, or of each segment's sums.
 enum Checkpoints { NONE = 0, RUNNING = 1, PER_SEGMENT = 2 };
+
+// What the kernels that give a lane one pixel keep of it.
+template <int CKPT, bool DEPTH, bool FEAT, bool TRACKED>
+struct Pixel {
+  float r = 0.f, g = 0.f, b = 0.f, zs = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;   // f: composited feature lanes (raster_fwd.cu:52)
+  float sr = 0.f, sg = 0.f, sb = 0.f;   // PER_SEGMENT: colour sums of the segment at hand
+  float T = 0.f, T_closed = 1.f;        // transmittance of a pixel that can take another fragment; else zero, and the transmittance it closed with
+  uint32_t last = 0u;                   // TRACKED: behind the last fragment the pixel took
+  // Adds a fragment that the pixel sees with blend weight `vis` (zero where it does not see it).
+  __device__ __forceinline__ void add(float vis, float cr, float cg, float cb, float z, float e0, float e1, float e2, uint32_t end) {
+    r += cr * vis; g += cg * vis; b += cb * vis;
+    if constexpr (CKPT == PER_SEGMENT) { sr += cr * vis; sg += cg * vis; sb += cb * vis; }
+    if constexpr (DEPTH) zs += vis * z;
+    if constexpr (FEAT) { f0 += e0 * vis; f1 += e1 * vis; f2 += e2 * vis; }
+    if constexpr (TRACKED) last = vis != 0.f ? end : last;
+  }
+  // The blend weight of a fragment of weight `al` and transmittance `through`, and the pixel's transmittance moved on: the fragment that
+  // would saturate a pixel closes it and is not taken.
+  __device__ __forceinline__ float weigh(float al, float through) {
+    const float next_T = T * through;
+    const bool stays = next_T > T_CUTOFF;
+    const float vis = stays ? al * T : 0.f;
+    T_closed = !stays && T != 0.f ? T : T_closed;
+    T = stays ? next_T : 0.f;
+    return vis;
+  }
+  __device__ __forceinline__ float now() const { return T != 0.f ? T : T_closed; }
+  // The state before a boundary, for the backward.
+  __device__ __forceinline__ void checkpoint(float4* dst) {
+    if constexpr (CKPT == PER_SEGMENT) { *dst = make_float4(sr, sg, sb, now()); sr = sg = sb = 0.f; }   // the sums of the segment before the boundary
+    else *dst = make_float4(r, g, b, now());
+  }
+  // 2 * PAIRS fragments in list order; `end`: behind the first. A pixel that does not see a fragment has its transmittance multiplied by
+  // one, and its sums take zeros.
+  template <int PAIRS, int RECORDS>
+  __device__ __forceinline__ void take_pairs(const float2 (&alpha)[PAIRS], const float4 (*staged)[RECORDS], uint32_t end) {
+    float2 vis[PAIRS], through[PAIRS];
+    float ahead = T;
+#pragma unroll
+    for (int u = 0; u < PAIRS; u++) {
+      through[u] = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[u].x, -alpha[u].y));
+      vis[u].x = alpha[u].x * ahead; ahead *= through[u].x; vis[u].y = alpha[u].y * ahead; ahead *= through[u].y;
+    }
+    if (__all_sync(0xffffffffu, none_closes(ahead))) T = ahead;
+    else {
+#pragma unroll
+      for (int u = 0; u < PAIRS; u++) { vis[u].x = weigh(alpha[u].x, through[u].x); vis[u].y = weigh(alpha[u].y, through[u].y); }
+    }
+#pragma unroll
+    for (int u = 0; u < PAIRS; u++) {
+      const float4* f = staged[u];
+      const float2 red = hi2(f[3]);
+      const float4 q4 = f[4], q5 = DEPTH || FEAT ? f[RECORDS > 5 ? 5 : 0] : make_float4(0.f, 0.f, 0.f, 0.f), q6 = FEAT ? f[RECORDS > 6 ? 6 : 0] : q5;
+      add(vis[u].x, red.x, q4.x, q4.z, q5.x, q5.z, q6.x, q6.z, end + 2 * u);
+      add(vis[u].y, red.y, q4.y, q4.w, q5.y, q5.w, q6.y, q6.w, end + 2 * u + 1);
+    }
+  }
+  // The same one by one, for colours or features that are not finite, which may not be added with weight zero. al: the fragment's alpha.
+  template <int RECORDS>
+  __device__ __forceinline__ void take_odd(float al, const float4* f, int k, uint32_t end) {
+    if (al == 0.f || T == 0.f) return;
+    const float* c = reinterpret_cast<const float*>(f) + k;
+    const float z = DEPTH ? c[RECORDS > 5 ? 20 : 0] : 0.f, e0 = FEAT ? c[RECORDS > 6 ? 22 : 0] : 0.f, e1 = FEAT ? c[RECORDS > 6 ? 24 : 0] : 0.f, e2 = FEAT ? c[RECORDS > 6 ? 26 : 0] : 0.f;
+    const float vis = weigh(al, 1.f - al);
+    if (vis != 0.f) add(vis, c[14], c[16], c[18], z, e0, e1, e2, end);
+  }
+};
+
+// A record's place in its staged pair (k: the pair's first or second); whether its colour or a feature is not finite.
+template <bool DEPTH, bool FEAT>
+__device__ __forceinline__ bool stage_record(float4* pair, int k, const float4& n0, const float4& n1, const float4& n2, const float2& n3) {
+  float* s = reinterpret_cast<float*>(pair) + k;
+  const float cr = fmaxf(n2.x, 0.f), cg = fmaxf(n2.y, 0.f), cb = fmaxf(n2.z, 0.f);
+  s[0] = -n0.x; s[2] = -n0.y; s[4] = 0.5f * n0.z; s[6] = n0.w; s[8] = 0.5f * n1.x; s[10] = n1.y; s[12] = n1.w; s[14] = cr; s[16] = cg; s[18] = cb;
+  bool strange = fmaxf(cr, fmaxf(cg, cb)) == INFINITY;
+  if constexpr (DEPTH || FEAT) { s[20] = n1.z; s[22] = n2.w; }
+  if constexpr (FEAT) { s[24] = n3.x; s[26] = n3.y; strange = strange || !(isfinite(n2.w) && isfinite(n3.x) && isfinite(n3.y)); }
+  return strange;
+}
 
 template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
 __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
@@ -85,29 +174,23 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
   const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
   if (CKPT == PER_SEGMENT && first && tile == 0 && in_tile == 0) bwd_work[BWD_SUMMED] = 0u;
   if (CHUNKED && !first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
-  float T = 1.f, r = 0.f, g = 0.f, b = 0.f, zs = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;   // f: composited feature lanes (raster_fwd.cu:52)
-  bool open = inside;   // the pixel can take another fragment
-  uint32_t last = range.x;
+  Pixel<CKPT, DEPTH, FEAT, BWD || CHUNKED> P;
+  P.T = inside ? 1.f : 0.f;
+  P.last = range.x;
   if (CHUNKED && !first && inside) {
     const float4 acc = out_feat[pix];
-    r = acc.x; g = acc.y; b = acc.z; T = acc.w;
-    if constexpr (DEPTH) zs = out_depth[pix];
-    if constexpr (FEAT) { const float4 fa = feat_acc[pix]; f0 = fa.x; f1 = fa.y; f2 = fa.z; }
+    P.r = acc.x; P.g = acc.y; P.b = acc.z;
+    if constexpr (DEPTH) P.zs = out_depth[pix];
+    if constexpr (FEAT) { const float4 fa = feat_acc[pix]; P.f0 = fa.x; P.f1 = fa.y; P.f2 = fa.z; }
     const uint32_t l = last_idx[pix];
-    open = (l & DONE_BIT) == 0u;
-    last = l & ~DONE_BIT;
+    P.T = (l & DONE_BIT) == 0u ? acc.w : 0.f; P.T_closed = acc.w;
+    P.last = l & ~DONE_BIT;
   }
   // Checkpoints for the backward's segmented replay (see common.cuh): the state a later chunk starts a tile with, and
   // the state before every (1 << seg_shift)-th fragment of the list.
   const int q = CHUNKED ? chunk * n_tiles + tile : tile;
-  float sr = 0.f, sg = 0.f, sb = 0.f;   // PER_SEGMENT: colour sums of the segment at hand
   uint32_t seg_now = 0;
-  auto checkpoint = [&](uint32_t seg) {
-    float4* dst = ckpt + (size_t)ckpt_slot(range.x, q, seg, seg_shift) * RT_PX + in_tile;
-    if constexpr (CKPT == PER_SEGMENT) { *dst = make_float4(sr, sg, sb, T); sr = sg = sb = 0.f; }   // the sums of the segment before the boundary
-    else *dst = make_float4(r, g, b, T);
-    seg_now = seg;
-  };
+  auto checkpoint = [&](uint32_t seg) { P.checkpoint(ckpt + (size_t)ckpt_slot(range.x, q, seg, seg_shift) * RT_PX + in_tile); seg_now = seg; };
   if (BWD && CHUNKED && !first && range.y > range.x) checkpoint(0u);
   // The records of a batch are gathered one batch ahead, into registers, half by each warp: the two dependent loads (list
   // entry, then the splat's records) are in flight while the batch before them is composited.
@@ -127,95 +210,62 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
   for (uint32_t start = range.x;; start += FWD_BATCH, buf ^= 1) {
     float4 (*staged)[RECORDS] = s_staged[warp >> 1][buf];
     {
-      float* s = reinterpret_cast<float*>(staged[in_tile >> 1]) + (lane & 1);
-      const float cr = fmaxf(n2.x, 0.f), cg = fmaxf(n2.y, 0.f), cb = fmaxf(n2.z, 0.f);
-      s[0] = -n0.x; s[2] = -n0.y; s[4] = 0.5f * n0.z; s[6] = n0.w; s[8] = 0.5f * n1.x; s[10] = n1.y; s[12] = n1.w; s[14] = cr; s[16] = cg; s[18] = cb;
-      bool strange = fmaxf(cr, fmaxf(cg, cb)) == INFINITY;   // a colour or feature that is not finite may not be added with weight zero
-      if constexpr (DEPTH || FEAT) { s[20] = n1.z; s[22] = n2.w; }
-      if constexpr (FEAT) { s[24] = n3.x; s[26] = n3.y; strange = strange || !(isfinite(n2.w) && isfinite(n3.x) && isfinite(n3.y)); }
+      const bool strange = stage_record<DEPTH, FEAT>(staged[in_tile >> 1], lane & 1, n0, n1, n2, n3);
       const uint32_t any_strange = __any_sync(0xffffffffu, strange);
       if (lane == 0) s_odd[warp][buf] = any_strange;
     }
     // One barrier of the tile's two warps per batch: the batch is staged, the one before it is done with (it lies in the other
     // buffer), and whether any pixel is still open.
-    any_open = pair_any(1 + (warp >> 1), open);
+    any_open = pair_any(1 + (warp >> 1), P.T != 0.f);
     if (start >= range.y || !any_open) break;
     gather(start + FWD_BATCH);
     const bool odd = (s_odd[warp][buf] | s_odd[warp ^ 1][buf]) != 0u;
-    // Takes one fragment of weight `al` with transmittance `next_T` behind it: the one that would saturate a pixel closes it and is
-    // not taken. A pixel that does not see the fragment has its transmittance multiplied by one, and its sums take zeros.
-    auto take = [&](float al, float through, float cr, float cg, float cb, float z, float e0, float e1, float e2, uint32_t end) {
-      const float next_T = T * through;
-      open = open && next_T > T_CUTOFF;
-      const float a = open ? al : 0.f, vis = a * T;
-      r += cr * vis; g += cg * vis; b += cb * vis;
-      if constexpr (CKPT == PER_SEGMENT) { sr += cr * vis; sg += cg * vis; sb += cb * vis; }
-      if constexpr (DEPTH) zs += vis * z;
-      if constexpr (FEAT) { f0 += e0 * vis; f1 += e1 * vis; f2 += e2 * vis; }
-      T = open ? next_T : T;
-      if constexpr (BWD || CHUNKED) last = a != 0.f ? end : last;
-    };
     // Pairs are taken FWD_GROUP at a time: first everything that does not depend on the pixel's running state (sigma, the hit test,
-    // alpha with its exponential) for the whole group, so that those chains overlap, then the short serial part (transmittance and
-    // colour sums) fragment by fragment in list order.
+    // alpha with its exponential) for the whole group, so that those chains overlap, then the transmittances, then the sums, fragment by
+    // fragment in list order.
     for (uint32_t t_begin = 0; t_begin < FWD_BATCH && t_begin < range.y - start; t_begin += FWD_SEG) {   // a segment of the backward is a whole number of these
       const uint32_t at = start + t_begin - range.x, t_end = min(t_begin + FWD_SEG, range.y - start);
       if (BWD && at != 0u && (at & ((1u << seg_shift) - 1u)) == 0u) checkpoint(at >> seg_shift);
-      if (!__any_sync(0xffffffffu, open)) continue;   // only the other half is still at it
+      if (!__any_sync(0xffffffffu, P.T != 0.f)) continue;   // only the other half is still at it
       if (odd) {
 #pragma unroll 1
         for (uint32_t t = t_begin; t < t_end; t++) {
           const float4* f = staged[t >> 1];
-          const float2 al2 = pair_alpha(f[0], f[1], f[2], lo2(f[3]), pcx, pcy);
-          const int k = t & 1;
-          const float al = k ? al2.y : al2.x;
-          const float* c = reinterpret_cast<const float*>(f) + k;
-          const float z = DEPTH ? c[RECORDS > 5 ? 20 : 0] : 0.f, e0 = FEAT ? c[RECORDS > 6 ? 22 : 0] : 0.f, e1 = FEAT ? c[RECORDS > 6 ? 24 : 0] : 0.f, e2 = FEAT ? c[RECORDS > 6 ? 26 : 0] : 0.f;
-          if (al != 0.f && open) {
-            if (T * (1.f - al) > T_CUTOFF) take(al, 1.f - al, c[14], c[16], c[18], z, e0, e1, e2, start + t + 1);
-            else open = false;
-          }
+          const float2 al = pair_alpha(f[0], f[1], f[2], lo2(f[3]), pcx, pcy);
+          P.template take_odd<RECORDS>(t & 1 ? al.y : al.x, f, t & 1, start + t + 1);
         }
         continue;
       }
       for (uint32_t t0 = t_begin; t0 < t_end; t0 += 2 * FWD_GROUP) {
-        float2 alpha[FWD_GROUP], through[FWD_GROUP], red[FWD_GROUP];
+        float2 alpha[FWD_GROUP];
 #pragma unroll
         for (int u = 0; u < FWD_GROUP; u++) {
           const float4* f = staged[t0 / 2 + u];
-          const float4 q3 = f[3];
-          alpha[u] = pair_alpha(f[0], f[1], f[2], lo2(q3), pcx, pcy);
-          through[u] = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[u].x, -alpha[u].y));
-          red[u] = hi2(q3);
+          alpha[u] = pair_alpha(f[0], f[1], f[2], lo2(f[3]), pcx, pcy);
         }
-#pragma unroll
-        for (int u = 0; u < FWD_GROUP; u++) {
-          const float4* f = staged[t0 / 2 + u];
-          const float4 q4 = f[4], q5 = DEPTH || FEAT ? f[RECORDS > 5 ? 5 : 0] : make_float4(0.f, 0.f, 0.f, 0.f), q6 = FEAT ? f[RECORDS > 6 ? 6 : 0] : q5;
-          const uint32_t end = start + t0 + 2 * u + 1;
-          take(alpha[u].x, through[u].x, red[u].x, q4.x, q4.z, q5.x, q5.z, q6.x, q6.z, end);
-          take(alpha[u].y, through[u].y, red[u].y, q4.y, q4.w, q5.y, q5.w, q6.y, q6.w, end + 1);
-        }
+        P.take_pairs(alpha, staged + t0 / 2, start + t0 + 1);
       }
     }
   }
+  const bool open = P.T != 0.f;
+  const float T = P.now();
   if (inside) {
-    out_rgba[pix] = make_float4(r + T * bg.x, g + T * bg.y, b + T * bg.z, 1.f - T);
+    out_rgba[pix] = make_float4(P.r + T * bg.x, P.g + T * bg.y, P.b + T * bg.z, 1.f - T);
     if constexpr (CHUNKED) {
-      if (FEAT && final) out_feat[pix] = make_float4(f0, f1, f2, T);
-      else out_feat[pix] = make_float4(r, g, b, T);
-      if constexpr (FEAT) { if (!final) feat_acc[pix] = make_float4(f0, f1, f2, 0.f); }
-      if constexpr (DEPTH) out_depth[pix] = !final ? zs : ((1.f - T) > 0.05f ? zs / (1.f - T) : INFINITY);
-      last_idx[pix] = last | (open ? 0u : DONE_BIT);
+      if (FEAT && final) out_feat[pix] = make_float4(P.f0, P.f1, P.f2, T);
+      else out_feat[pix] = make_float4(P.r, P.g, P.b, T);
+      if constexpr (FEAT) { if (!final) feat_acc[pix] = make_float4(P.f0, P.f1, P.f2, 0.f); }
+      if constexpr (DEPTH) out_depth[pix] = !final ? P.zs : finished_depth(P.zs, T);
+      last_idx[pix] = P.last | (open ? 0u : DONE_BIT);
     } else {
-      out_feat[pix] = make_float4(f0, f1, f2, T);
-      if constexpr (DEPTH) out_depth[pix] = (1.f - T) > 0.05f ? zs / (1.f - T) : INFINITY;
-      if constexpr (BWD) last_idx[pix] = last;
+      out_feat[pix] = make_float4(P.f0, P.f1, P.f2, T);
+      if constexpr (DEPTH) out_depth[pix] = finished_depth(P.zs, T);
+      if constexpr (BWD) last_idx[pix] = P.last;
     }
   }
   if constexpr (!BWD && !CHUNKED) return;
   // What the tile's two warps settle together: whether any pixel is still open, and the last fragment any pixel used.
-  const uint32_t mine = __reduce_max_sync(0xffffffffu, last);
+  const uint32_t mine = __reduce_max_sync(0xffffffffu, P.last);
   if (lane == 0) s_last[warp] = mine;
   any_open = pair_any(1 + (warp >> 1), open);
   if (CHUNKED && !final && in_tile == 0 && !any_open)
@@ -232,7 +282,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
         // Slot 0 has no segment before it: its colour takes the sums of the range's last segment (which is the one at hand
         // unless nothing after its boundary was seen).
         float* dst = reinterpret_cast<float*>(ckpt + (size_t)ckpt_slot(range.x, q, 0u, seg_shift) * RT_PX + in_tile);
-        const float4 v = segs - 1u == seg_now ? make_float4(sr, sg, sb, 0.f) : ckpt[(size_t)ckpt_slot(range.x, q, segs, seg_shift) * RT_PX + in_tile];
+        const float4 v = segs - 1u == seg_now ? make_float4(P.sr, P.sg, P.sb, 0.f) : ckpt[(size_t)ckpt_slot(range.x, q, segs, seg_shift) * RT_PX + in_tile];
         dst[0] = v.x; dst[1] = v.y; dst[2] = v.z;
       }
     }
@@ -264,8 +314,8 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   const bool first = chunk == 0, final = chunk == n_chunks - 1;
   if (CKPT == PER_SEGMENT && first && tile == 0 && lane == 0) bwd_work[BWD_SUMMED] = 0u;
   if (!first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
-  float2 T = splat2(1.f), r = splat2(0.f), g = r, b = r, zs = r;   // of the two pixels
-  bool open[2] = {in0, in1};   // the pixel can take another fragment
+  float2 r = splat2(0.f), g = r, b = r, zs = r;   // of the two pixels
+  float2 T = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f), T_closed = splat2(1.f);   // transmittance of a pixel that can take another fragment, else zero and the one it closed with
   uint32_t last[2] = {range.x, range.x};
   if (!first) {
 #pragma unroll
@@ -273,11 +323,11 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
       if (p == 0 ? in0 : in1) {
         const int pix = py * W + px0 + p;
         const float4 acc = out_feat[pix];
-        at(r, p) = acc.x; at(g, p) = acc.y; at(b, p) = acc.z; at(T, p) = acc.w;
+        at(r, p) = acc.x; at(g, p) = acc.y; at(b, p) = acc.z; at(T_closed, p) = acc.w;
         if constexpr (DEPTH) at(zs, p) = out_depth[pix];
         if constexpr (FEAT) { const float4 fa = feat_acc[pix]; at(f0, p) = fa.x; at(f1, p) = fa.y; at(f2, p) = fa.z; }
         const uint32_t l = last_idx[pix];
-        open[p] = (l & DONE_BIT) == 0u;
+        at(T, p) = (l & DONE_BIT) == 0u ? acc.w : 0.f;
         last[p] = l & ~DONE_BIT;
       }
     }
@@ -289,12 +339,13 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   uint32_t seg_now = 0;
   auto checkpoint = [&](uint32_t seg) {
     float4* dst = ckpt + (size_t)ckpt_slot(range.x, q, seg, seg_shift) * RT_PX + lane * 2;
+    const float2 now = make_float2(T.x != 0.f ? T.x : T_closed.x, T.y != 0.f ? T.y : T_closed.y);
     if constexpr (CKPT == PER_SEGMENT) {   // the sums of the segment before the boundary
-      dst[0] = make_float4(sr.x, sg.x, sb.x, T.x); dst[1] = make_float4(sr.y, sg.y, sb.y, T.y);
+      dst[0] = make_float4(sr.x, sg.x, sb.x, now.x); dst[1] = make_float4(sr.y, sg.y, sb.y, now.y);
       sr = sg = sb = splat2(0.f);
       seg_now = seg;
     } else {
-      dst[0] = make_float4(r.x, g.x, b.x, T.x); dst[1] = make_float4(r.y, g.y, b.y, T.y);
+      dst[0] = make_float4(r.x, g.x, b.x, now.x); dst[1] = make_float4(r.y, g.y, b.y, now.y);
     }
   };
   if (BWD && !first && range.y > range.x) checkpoint(0u);
@@ -312,7 +363,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   };
   gather(range.x);
   for (uint32_t start = range.x; start < range.y; start += FWD_SEG) {
-    if (!__any_sync(0xffffffffu, open[0] || open[1])) break;
+    if (!__any_sync(0xffffffffu, T.x != 0.f || T.y != 0.f)) break;
     if (BWD && start != range.x && ((start - range.x) & ((1u << seg_shift) - 1u)) == 0u) checkpoint((start - range.x) >> seg_shift);
     __syncwarp();
     uint32_t odd;   // fragments whose colour or feature is not finite: they may not be added with weight zero
@@ -334,8 +385,18 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     __syncwarp();
     gather(start + FWD_SEG);
     // Fragments are taken FWD_GROUP at a time: first everything that does not depend on the pixels' running state (sigma,
-    // the hit test, alpha with its exponential) for the whole group, so that those chains overlap, then the short serial
-    // part (transmittance and colour sums) fragment by fragment in list order.
+    // the hit test, alpha with its exponential) for the whole group, so that those chains overlap, then the transmittances, then the
+    // sums, fragment by fragment in list order. A pixel that does not see a fragment has its transmittance multiplied by one, and its
+    // sums take zeros.
+    // The blend weight of a fragment, and the pixel's transmittance moved on: the fragment that would saturate a pixel closes it and is
+    // not taken.
+    auto weigh = [&](int p, float al, float through) {
+      const float now = at(T, p), next_T = now * through;
+      const bool stays = next_T > T_CUTOFF;
+      at(T_closed, p) = !stays && now != 0.f ? now : at(T_closed, p);
+      at(T, p) = stays ? next_T : 0.f;
+      return stays ? al * now : 0.f;
+    };
     const float4 (*staged)[FEAT ? 6 : 5] = s_staged[warp];
     const uint32_t remaining = min((uint32_t)FWD_SEG, range.y - start);
     if (odd) {
@@ -345,15 +406,14 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
         const float4 q3 = staged[t][3], q4 = staged[t][4];
 #pragma unroll
         for (int p = 0; p < 2; p++) {
-          const float al = p == 0 ? alpha.x : alpha.y, next_T = at(T, p) * (1.f - al);
-          open[p] = open[p] && next_T > T_CUTOFF;
-          if (!open[p] || al == 0.f) continue;
-          const float vis = al * at(T, p);
+          const float al = p == 0 ? alpha.x : alpha.y;
+          if (al == 0.f || at(T, p) == 0.f) continue;
+          const float vis = weigh(p, al, 1.f - al);
+          if (vis == 0.f) continue;
           at(r, p) += q3.x * vis; at(g, p) += q3.z * vis; at(b, p) += q4.x * vis;
           if constexpr (CKPT == PER_SEGMENT) { at(sr, p) += q3.x * vis; at(sg, p) += q3.z * vis; at(sb, p) += q4.x * vis; }
           if constexpr (DEPTH) at(zs, p) += vis * q4.z;
           if constexpr (FEAT) { const float4 q5 = staged[t][5]; at(f0, p) += q5.x * vis; at(f1, p) += q5.y * vis; at(f2, p) += q5.z * vis; }
-          at(T, p) = next_T;
           last[p] = start + t + 1;
         }
       }
@@ -368,28 +428,35 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
         alpha[u] = fragment_alpha(q0, q1, q2, pcx, pcy);
         through[u] = __fadd2_rn(splat2(1.f), make_float2(-alpha[u].x, -alpha[u].y));
       }
+      float2 vis[FWD_GROUP];
+      {
+        float2 ahead = T;
+#pragma unroll
+        for (int u = 0; u < FWD_GROUP; u++) { vis[u] = __fmul2_rn(alpha[u], ahead); ahead = __fmul2_rn(ahead, through[u]); }
+        if (__all_sync(0xffffffffu, none_closes(ahead.x) && none_closes(ahead.y))) T = ahead;
+        else {
+#pragma unroll
+          for (int u = 0; u < FWD_GROUP; u++) vis[u] = make_float2(weigh(0, alpha[u].x, through[u].x), weigh(1, alpha[u].y, through[u].y));
+        }
+      }
 #pragma unroll
       for (int u = 0; u < FWD_GROUP; u++) {
         const uint32_t t = t0 + (uint32_t)u;
-        // The fragment that would saturate a pixel closes it, and is not taken. A pixel that does not see the fragment has its
-        // transmittance multiplied by one, and its sums take zeros.
-        const float2 next_T = __fmul2_rn(T, through[u]);
-        open[0] = open[0] && next_T.x > T_CUTOFF; open[1] = open[1] && next_T.y > T_CUTOFF;
-        const float2 a = make_float2(open[0] ? alpha[u].x : 0.f, open[1] ? alpha[u].y : 0.f);
         const float4 q3 = staged[t][3], q4 = staged[t][4];
-        const float2 vis = __fmul2_rn(a, T), cr = make_float2(q3.x, q3.y), cg = make_float2(q3.z, q3.w), cb = make_float2(q4.x, q4.y);
-        r = __ffma2_rn(cr, vis, r); g = __ffma2_rn(cg, vis, g); b = __ffma2_rn(cb, vis, b);
-        if constexpr (CKPT == PER_SEGMENT) { sr = __ffma2_rn(cr, vis, sr); sg = __ffma2_rn(cg, vis, sg); sb = __ffma2_rn(cb, vis, sb); }
-        if constexpr (DEPTH) zs = __ffma2_rn(vis, make_float2(q4.z, q4.w), zs);
+        const float2 cr = make_float2(q3.x, q3.y), cg = make_float2(q3.z, q3.w), cb = make_float2(q4.x, q4.y);
+        r = __ffma2_rn(cr, vis[u], r); g = __ffma2_rn(cg, vis[u], g); b = __ffma2_rn(cb, vis[u], b);
+        if constexpr (CKPT == PER_SEGMENT) { sr = __ffma2_rn(cr, vis[u], sr); sg = __ffma2_rn(cg, vis[u], sg); sb = __ffma2_rn(cb, vis[u], sb); }
+        if constexpr (DEPTH) zs = __ffma2_rn(vis[u], make_float2(q4.z, q4.w), zs);
         if constexpr (FEAT) {
           const float4 q5 = staged[t][5];
-          f0 = __ffma2_rn(splat2(q5.x), vis, f0); f1 = __ffma2_rn(splat2(q5.y), vis, f1); f2 = __ffma2_rn(splat2(q5.z), vis, f2);
+          f0 = __ffma2_rn(splat2(q5.x), vis[u], f0); f1 = __ffma2_rn(splat2(q5.y), vis[u], f1); f2 = __ffma2_rn(splat2(q5.z), vis[u], f2);
         }
-        T.x = open[0] ? next_T.x : T.x; T.y = open[1] ? next_T.y : T.y;
-        last[0] = a.x != 0.f ? start + t + 1 : last[0]; last[1] = a.y != 0.f ? start + t + 1 : last[1];
+        last[0] = vis[u].x != 0.f ? start + t + 1 : last[0]; last[1] = vis[u].y != 0.f ? start + t + 1 : last[1];
       }
     }
   }
+  const bool open[2] = {T.x != 0.f, T.y != 0.f};
+  T = make_float2(open[0] ? T.x : T_closed.x, open[1] ? T.y : T_closed.y);
 #pragma unroll
   for (int p = 0; p < 2; p++) {
     if (p == 0 ? in0 : in1) {
@@ -398,7 +465,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
       if (FEAT && final) out_feat[pix] = make_float4(at(f0, p), at(f1, p), at(f2, p), at(T, p));
       else out_feat[pix] = make_float4(at(r, p), at(g, p), at(b, p), at(T, p));
       if constexpr (FEAT) { if (!final) feat_acc[pix] = make_float4(at(f0, p), at(f1, p), at(f2, p), 0.f); }
-      if constexpr (DEPTH) out_depth[pix] = !final ? at(zs, p) : ((1.f - at(T, p)) > 0.05f ? at(zs, p) / (1.f - at(T, p)) : INFINITY);
+      if constexpr (DEPTH) out_depth[pix] = !final ? at(zs, p) : finished_depth(at(zs, p), at(T, p));
       last_idx[pix] = last[p] | (open[p] ? 0u : DONE_BIT);
     }
   }
