@@ -7,7 +7,7 @@
 // as operands of packed arithmetic (fp32x2); the hit test is one comparison; a pixel that does not see a fragment takes it with
 // weight zero instead of branching around it (a vote and a branch per fragment cost more than the ten operations they saved).
 // Transmittances are multiplied up for a group of fragments first, and fragments are compared and selected one by one only where a
-// pixel of the warp closes inside the group (none_closes): 1024x1024 over 1M in four chunks 184 -> 172 us, 4K over 6M in five 734 -> 705.
+// pixel of the warp closes inside the group (none_closes): 1024x1024 over 1M in four chunks 184 -> 172 us, 4K over 6M in five 681 -> 652.
 // Two kernels with the same arithmetic, bit for bit:
 //   raster_fwd_half_kernel  two warps to a tile, a lane one pixel, two consecutive fragments to a packed operation: the chain of
 //                           one list is half as long. For whole views and two chunks, where a visit to a tile is a long list.
@@ -31,7 +31,8 @@ constexpr int FWD_GROUP = 4;                             // fragments (one warp)
 // launches a pixel's state lives in the output buffers: the colour sums in out_feat.xyz, the transmittance in
 // out_feat.w, and last_idx with bit 31 set once the pixel has reached the cutoff; out_rgba holds the finished pixel
 // after every chunk, so a launch only touches tiles that received fragments. With DEPTH the depth sum travels in
-// out_depth and the last chunk visits every pixel to divide it out. The tile's bit in `alive` tells the binning of the next
+// out_depth, and the last chunk divides it out in every pixel, which is all it does in a tile that it leaves nothing in (the last of five
+// visits to a 4K view 183 -> 130 us). The tile's bit in `alive` tells the binning of the next
 // chunk whether any pixel of the tile can still take a fragment.
 __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
@@ -173,7 +174,10 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
   const uint2 range = tile_ranges[tile];
   const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
   if (CKPT == PER_SEGMENT && first && tile == 0 && in_tile == 0) bwd_work[BWD_SUMMED] = 0u;
-  if (CHUNKED && !first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
+  if (CHUNKED && !first && range.y <= range.x && !(final && FEAT)) {   // nothing of this chunk lands here: pixels, state and flag stay
+    if (DEPTH && final && inside) out_depth[pix] = finished_depth(out_depth[pix], out_feat[pix].w);
+    return;
+  }
   Pixel<CKPT, DEPTH, FEAT, BWD || CHUNKED> P;
   P.T = inside ? 1.f : 0.f;
   P.last = range.x;
@@ -313,7 +317,14 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   const uint2 range = tile_ranges[tile];
   const bool first = chunk == 0, final = chunk == n_chunks - 1;
   if (CKPT == PER_SEGMENT && first && tile == 0 && lane == 0) bwd_work[BWD_SUMMED] = 0u;
-  if (!first && range.y <= range.x && !(final && (DEPTH || FEAT))) return;   // nothing of this chunk lands here: pixels, state and flag stay
+  if (!first && range.y <= range.x && !(final && FEAT)) {   // nothing of this chunk lands here: pixels, state and flag stay
+    if (DEPTH && final) {
+#pragma unroll
+      for (int p = 0; p < 2; p++)
+        if (p == 0 ? in0 : in1) { const int pix = py * W + px0 + p; out_depth[pix] = finished_depth(out_depth[pix], out_feat[pix].w); }
+    }
+    return;
+  }
   float2 r = splat2(0.f), g = r, b = r, zs = r;   // of the two pixels
   float2 T = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f), T_closed = splat2(1.f);   // transmittance of a pixel that can take another fragment, else zero and the one it closed with
   uint32_t last[2] = {range.x, range.x};
