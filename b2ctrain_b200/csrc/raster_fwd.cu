@@ -8,7 +8,9 @@
 // weight zero instead of branching around it (a vote and a branch per fragment cost more than the ten operations they saved).
 // Transmittances are multiplied up for a group of fragments first, and fragments are compared and selected one by one only where a
 // pixel of the warp closes inside the group (none_closes): 1024x1024 over 1M in four chunks 184 -> 172 us, 4K over 6M in five 681 -> 652.
-// Two kernels with the same arithmetic, bit for bit:
+// Three kernels with the same arithmetic, bit for bit:
+//   raster_fwd_team_kernel  eight warps to a tile: some find alphas, two composite, two gather. For whole views of so few tiles that all
+//                           are in flight at once, whose time is that of the longest list.
 //   raster_fwd_half_kernel  two warps to a tile, a lane one pixel, two consecutive fragments to a packed operation: the chain of
 //                           one list is half as long. For whole views and two chunks, where a visit to a tile is a long list.
 //   raster_fwd_kernel       one warp to a tile, a lane two pixels that share packed operations: twice as many tiles in flight.
@@ -16,6 +18,9 @@
 // Measured, us (scalar pixels with a vote / one warp / two warps): 64x64 50 / 38 / 23, 333x217 54 / 42 / 28, 1001x751 with
 // features 85 / 69 / 54, 1237x822 in two chunks 117 / 92 / 76, 1920x1080 in two 143 / 123 / 118; 1024x1024 over 1M in four
 // 231 / 187 / 206, 4K over 6M with depth in five 847 / 740 / 953, sixteen views of 3M in four on eight streams 20.6 / 21.6 ms.
+// Two warps / the team, us: 64x64 over 2k splats 21.3 / 15.1, 200x150 over 1k 11.7 / 9.9, 333x217 over 1k 11.8 / 10.0, over 20k 24.7 /
+// 18.7, over 150k 78 / 50 (1,176 tiles, a block each); 400x300 over 4k 12.9 / 16.1, over 40k 25.3 / 26.3 (1,900 tiles, the second
+// thousand waits), 512x512 over 10k 17.8 / 31.7, 1280x720 over 100k 40.7 / 70.7.
 #include "common.cuh"
 
 namespace b2k {
@@ -293,6 +298,126 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
   }
 }
 
+// Eight warps to a tile, for whole views of so few tiles that all are in flight together (TEAM_PER_SM blocks fit an SM), where the GPU is
+// idle but for the lists' own length: four warps find the alphas of
+// a batch, two warps (a pixel per lane) carry the transmittances and the sums, two warps take turns to gather and stage the records of
+// the batches ahead. A batch passes from one to the next with one barrier of the block.
+constexpr int TEAM_BATCH = FWD_SEG, TEAM_PAIRS = TEAM_BATCH / 2, TEAM_PRODUCERS = 4, TEAM_GROUP = 8, TEAM_THREADS = (2 + TEAM_PRODUCERS + 2) * 32, TEAM_PER_SM = 8;
+
+template <int CKPT, bool DEPTH, bool FEAT>
+__global__ void __launch_bounds__(TEAM_THREADS) raster_fwd_team_kernel(
+    uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
+    const float4* __restrict__ proj2, int W, int H, int tiles_x, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
+    float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, uint32_t* __restrict__ bwd_work) {
+  after_previous();
+  constexpr bool BWD = CKPT != NONE;
+  constexpr int RECORDS = FEAT ? STAGED + 2 : DEPTH ? STAGED + 1 : STAGED;
+  __shared__ float4 s_staged[3][TEAM_PAIRS][RECORDS];   // of the batches that are staged, weighed and composited
+  __shared__ float2 s_alpha[2][TEAM_PAIRS][RT_PX];
+  __shared__ uint32_t s_odd[3], s_last[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile = blockIdx.x, tx = tile % tiles_x, ty = tile / tiles_x;
+  const uint2 range = tile_ranges[tile];
+  const uint32_t batches = range.y > range.x ? (range.y - range.x + TEAM_BATCH - 1) / TEAM_BATCH : 0u;
+  if (CKPT == PER_SEGMENT && tile == 0 && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
+  const bool composites = warp < 2, weighs = !composites && warp < 2 + TEAM_PRODUCERS;
+  // The lane's pixel, of a producer its first of two.
+  const int in_tile = (composites ? warp * 32 : 0) + lane, px = tx * RT_W + (in_tile & 7), py = ty * RT_W + (in_tile >> 3), pix = py * W + px;
+  const bool inside = composites && px < W && py < H;
+  const float2 pcx = make_float2((float)px + 0.5f, (float)px + 0.5f), pcy = make_float2((float)py + 0.5f, (float)py + 0.5f);
+  Pixel<CKPT, DEPTH, FEAT, BWD> P;
+  P.T = inside ? 1.f : 0.f;
+  P.last = range.x;
+  uint32_t seg_now = 0;
+  // A gathering warp's next batch is in its registers, and the list entries of the one after that.
+  const uint32_t turn = (uint32_t)warp & 1u;
+  float4 n0, n1, n2;
+  float2 n3;
+  uint32_t gid = 0u;
+  auto entries = [&](uint32_t b) { const uint32_t at = range.x + b * TEAM_BATCH + lane; gid = b < batches && at < range.y ? vals_sorted[at] : 0xFFFFFFFFu; };
+  auto gather = [&]() {
+    n0 = n1 = n2 = make_float4(0.f, 0.f, 0.f, 0.f); n3 = make_float2(0.f, 0.f);   // beyond the list: opacity zero
+    if (gid != 0xFFFFFFFFu) {
+      n0 = proj0[gid]; n1 = proj1[gid]; n2 = proj2[gid];
+      if constexpr (FEAT) n3 = proj3[gid];
+    }
+  };
+  if (!composites && !weighs) { entries(turn); gather(); entries(turn + 2u); }
+  for (uint32_t t = 0; batches && t < batches + 2u; t++) {
+    if (!__syncthreads_or(P.T != 0.f)) break;   // (only the pixels' own warps hold a transmittance)
+    if (composites) {
+      if (t < 2u) continue;
+      const uint32_t at = (t - 2u) * TEAM_BATCH, start = range.x + at, count = min((uint32_t)TEAM_BATCH, range.y - start);
+      const float4 (*staged)[RECORDS] = s_staged[(t - 2u) % 3u];
+      const float2 (*alphas)[RT_PX] = s_alpha[t & 1u];
+      if (BWD && at != 0u && (at & ((1u << seg_shift) - 1u)) == 0u) {
+        seg_now = at >> seg_shift;
+        P.checkpoint(ckpt + (size_t)ckpt_slot(range.x, tile, seg_now, seg_shift) * RT_PX + in_tile);
+      }
+      if (!__any_sync(0xffffffffu, P.T != 0.f)) continue;   // only the other half is still at it
+      if (s_odd[(t - 2u) % 3u]) {
+#pragma unroll 1
+        for (uint32_t k = 0; k < count; k++) {
+          const float2 al = alphas[k >> 1][in_tile];
+          P.template take_odd<RECORDS>(k & 1u ? al.y : al.x, staged[k >> 1], (int)(k & 1u), start + k + 1u);
+        }
+        continue;
+      }
+      for (uint32_t k = 0; k < count; k += 2 * TEAM_GROUP) {
+        float2 alpha[TEAM_GROUP];
+#pragma unroll
+        for (int u = 0; u < TEAM_GROUP; u++) alpha[u] = alphas[k / 2 + u][in_tile];
+        P.take_pairs(alpha, staged + k / 2, start + k + 1u);
+      }
+    } else if (weighs) {
+      if (t == 0u || t > batches) continue;
+      const uint32_t start = range.x + (t - 1u) * TEAM_BATCH, count = min((uint32_t)TEAM_BATCH, range.y - start);
+      const uint32_t pairs = (count + 2 * TEAM_GROUP - 1) / (2 * TEAM_GROUP) * TEAM_GROUP;   // the sums take whole groups
+      const float4 (*staged)[RECORDS] = s_staged[(t - 1u) % 3u];
+      float2 (*alphas)[RT_PX] = s_alpha[(t - 1u) & 1u];
+      const float2 pcy1 = make_float2(pcy.x + 4.f, pcy.y + 4.f);   // exact
+#pragma unroll
+      for (uint32_t k = 0; k < TEAM_PAIRS / TEAM_PRODUCERS; k++) {
+        const uint32_t pair = k * TEAM_PRODUCERS + (uint32_t)warp - 2u;
+        if (pair >= pairs) break;
+        const float4* f = staged[pair];
+        const float4 q0 = f[0], q1 = f[1], q2 = f[2];
+        const float2 power = lo2(f[3]);
+        alphas[pair][lane] = pair_alpha(q0, q1, q2, power, pcx, pcy);
+        alphas[pair][lane + 32] = pair_alpha(q0, q1, q2, power, pcx, pcy1);
+      }
+    } else if (t < batches && (t & 1u) == turn) {
+      const bool strange = stage_record<DEPTH, FEAT>(s_staged[t % 3u][lane >> 1], lane & 1, n0, n1, n2, n3);
+      const uint32_t any_strange = __any_sync(0xffffffffu, strange);
+      if (lane == 0) s_odd[t % 3u] = any_strange;
+      gather();
+      entries(t + 4u);
+    }
+  }
+  if (!composites) return;
+  const float T = P.now();
+  if (inside) {
+    out_rgba[pix] = make_float4(P.r + T * bg.x, P.g + T * bg.y, P.b + T * bg.z, 1.f - T);
+    out_feat[pix] = make_float4(P.f0, P.f1, P.f2, T);
+    if constexpr (DEPTH) out_depth[pix] = finished_depth(P.zs, T);
+    if constexpr (BWD) last_idx[pix] = P.last;
+  }
+  if constexpr (BWD) {
+    // The backward never needs to look past the last fragment any pixel used.
+    const uint32_t mine = __reduce_max_sync(0xffffffffu, P.last);
+    if (lane == 0) s_last[warp] = mine;
+    pair_any(1, false);
+    const uint32_t m = max(s_last[0], s_last[1]);
+    if (in_tile == 0) tile_ranges[tile].y = m;
+    if (CKPT == PER_SEGMENT && m > range.x) {
+      // Slot 0 has no segment before it (see raster_fwd_half_kernel).
+      const uint32_t segs = (m - range.x + (1u << seg_shift) - 1u) >> seg_shift;
+      float* dst = reinterpret_cast<float*>(ckpt + (size_t)ckpt_slot(range.x, tile, 0u, seg_shift) * RT_PX + in_tile);
+      const float4 v = segs - 1u == seg_now ? make_float4(P.sr, P.sg, P.sb, 0.f) : ckpt[(size_t)ckpt_slot(range.x, tile, segs, seg_shift) * RT_PX + in_tile];
+      dst[0] = v.x; dst[1] = v.y; dst[2] = v.z;
+    }
+  }
+}
+
 // One warp to a tile, for views in depth chunks.
 template <int CKPT, bool DEPTH, bool FEAT>
 __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
@@ -522,7 +647,10 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
     (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, \
     seg_shift_of(short_segments(c)), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr, bwd_work_ptr(c)
 #define HALF(B, D, C, F) launch_next(raster_fwd_half_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_TILES), FWD_WARPS * 32, 0, ARGS)
-#define L(B, D, F) do { if (!chunked) HALF(B, D, false, F); else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
+#define TEAM(B, D, F) launch_next(raster_fwd_team_kernel<B, D, F>, c->n_tiles, TEAM_THREADS, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, \
+    (const float4*)c->proj2, c->W, c->H, c->tiles_x, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, (const float2*)c->proj3, \
+    o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c))
+#define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_PER_SM * sm_count()) TEAM(B, D, F); else HALF(B, D, false, F); } else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
     else launch_next(raster_fwd_kernel<B, D, (F) && (B) == NONE>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS); } while (0)
 #define LD(B, D) do { if (o->feat_mode != 0) L(B, D, true); else L(B, D, false); } while (0)   // a chunked view with features is forward only (checked by the caller)
 #define LB(B) do { if (c->out_depth) LD(B, true); else LD(B, false); } while (0)
@@ -533,6 +661,7 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
 #undef LD
 #undef L
 #undef HALF
+#undef TEAM
 #undef ARGS
   return check_launch();
 }

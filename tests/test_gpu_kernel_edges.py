@@ -448,3 +448,30 @@ def test_tile_boxes_of_every_size():
             h.ctx.tile_count.zero_(); h.ctx.hit_info.zero_()
             h.api.count_tiles(h.ctx, h.model)
             assert np.array_equal(h.u32(h.ctx.hit_info[:n]).reshape(-1, 4)[tc_o > 0], info[tc_o > 0])
+
+
+@pytest.mark.parametrize("W,H", [(64, 64), (61, 43)])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 97, 300])
+def test_forward_of_few_tiles_is_that_of_chunks(n, W, H):
+    """A team of warps to a tile, two warps, and one warp composite the same image bit for bit, whether pixels close inside a group of
+    fragments, at its ends or not at all."""
+    import torch
+    from b2ctrain_b200 import api
+    scene, cam = stack_scene(n, W, H, seed=n)
+    scene["pos_op"][:, 3] = np.linspace(-4.0, 3.0, n)
+    scene["lscale"][:, :3] = np.random.Generator(np.random.PCG64(n)).normal(-2.5, 0.7, (n, 3))
+    m = api.Model("cuda:0").upload(scenes.floor_for_cameras(scene, [cam]))
+    got = []
+    for chunks in (1, 2, 3):
+        ctx = api.RenderCtx("cuda:0")
+        ctx.want_depth = True
+        ctx.setup(W, H, m.cap, n_chunks=chunks)
+        rp = api.RenderParams(cam, bg=(0.2, 0.1, 0.3), sh_degree=1, bwd_info=False)
+        api.render_forward(ctx, m, rp)
+        plain = [ctx.out_rgba.clone(), ctx.out_feat[:, 3].clone(), ctx.out_depth.clone()]
+        rp.feat = "Normals"
+        api.render_forward(ctx, m, rp)
+        got.append(plain + [ctx.out_rgba.clone(), ctx.out_feat.clone(), ctx.out_depth.clone()])
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert torch.equal(a, b)
