@@ -475,3 +475,32 @@ def test_forward_of_few_tiles_is_that_of_chunks(n, W, H):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 500])
+@pytest.mark.parametrize("degree,active", [(0, 0), (1, 1), (2, 1), (3, 3), (4, 2), (4, 4)])
+def test_accumulator_rows_are_the_gradients(degree, active, n):
+    """A view's rows in an accumulator of zeros are the gradients of the debug lane, float for float."""
+    import torch
+    from b2ctrain_b200 import api
+    W, H = 96, 64
+    scene = scenes.floor_for_cameras(scenes.make_splats(n, degree, n + degree), [cam := scenes.look_at_camera(scenes.orbit_eye(3.0, 30.0, 10.0), W, H, 64.0)])
+    rng = np.random.Generator(np.random.PCG64(n))
+    h = Harness(scene, cam)
+    h.rp.sh_degree = active
+    got = []
+    for split in (False, True):
+        h.forward()
+        h.ctx.v_out.copy_(torch.from_numpy(np.random.Generator(np.random.PCG64(4)).standard_normal((W * H, 4)).astype(np.float32)))
+        h.ctx.v_splat.zero_(); h.ctx.vis_flag.zero_()
+        h.api.rasterize_backward(h.ctx, h.model, h.rp)
+        if not split:
+            lanes, flags = h.ctx.v_splat.clone(), h.ctx.vis_flag.clone()
+        else:
+            h.ctx.v_splat.copy_(lanes); h.ctx.vis_flag.copy_(flags)      # the order of the replay's reductions is not at issue
+        grad = torch.zeros((h.model.n, 11 + 3 * h.model.K()), device="cuda:0")
+        op = api.OptimParams(cam, active_sh_degree=active, sparse=True, grad_out=None if split else grad)
+        (api.projection_backward(h.ctx, h.model, op, grad) if split else api.optimizer_step(h.ctx, h.model, op))
+        assert not bool(h.ctx.vis_flag.any()) and not bool(h.ctx.v_splat[:n].any())
+        got.append(grad)
+    assert bool(got[0].any()) and torch.equal(got[0], got[1])
