@@ -5,6 +5,9 @@
 //    culled ones as largest + 1: the depths of a scene span 23 to 28 bits, so three digits of eight to ten bits do what four
 //    passes over 32 bits did, whatever the range (three digits of eleven hold all 32 bits). The range is found on the device.
 //  * Up to SMALL_N splats: one block sorts in its shared memory, one launch.
+//  * Up to CLUSTER_N: one cluster of eight blocks, one launch. Whole sort, us, one block or ten launches / the cluster: 3,000 splats 17.7 /
+//    15.9, 8,000 26.3 / 17.7, 16,000 30.3 / 20.1, 24,000 30.4 / 23.3, 32,000 31.0 / 27.5; 40,000 31.6 / 43.5 (and 2,000 13.0 / 15.1).
+//    Sixteen blocks take 4 us more to launch and gain nothing.
 //  * Above: three passes of the wait-free form (digit counts per block, scan over the blocks, ranked scatter); no block waits
 //    for another. A block owns one contiguous run. Scatter is staged through shared memory so that global writes go out in
 //    digit runs. Values that are the positions are not read.
@@ -12,6 +15,7 @@
 // four passes of eight bits with tiles of 4,096 at every size, first launch to last: 2,000 splats 89 -> 12 us, 100,000 94 ->
 // 52, 500,000 103 -> 64, three million 176 -> 132, six million 254 -> 204.
 #include "bins.cuh"
+#include <cooperative_groups.h>
 #include <algorithm>
 
 namespace b2k {
@@ -46,18 +50,15 @@ __device__ __forceinline__ Digits digits_of(uint32_t lo, uint32_t hi, int passes
 }
 
 // ---- one block -----------------------------------------------------------------------------------------------------------
-constexpr int SMALL_THREADS = 1024, SMALL_WARPS = 32, SMALL_ITEMS = 8, SMALL_N = SMALL_THREADS * SMALL_ITEMS;
-constexpr size_t small_smem(int items) { return (size_t)SMALL_THREADS * items * 8 + SMALL_WARPS * 256 * 2 + 256 * 4; }
+constexpr int SMALL_THREADS = 1024, SMALL_WARPS = 32, SMALL_ITEMS = 2, SMALL_N = SMALL_THREADS * SMALL_ITEMS;
 
 // A warp owns a contiguous run of 32 * ITEMS pairs, held in registers from one pass to the write of the next; pair j * 32 + l
 // of the run is lane l's j-th.
-template <int ITEMS>
-__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* keys_out, uint32_t* vals_out, uint32_t* totals) { after_previous();   // may work in place
-  extern __shared__ __align__(16) uint32_t s_mem[];
-  uint32_t* s_key = s_mem;
-  uint32_t* s_val = s_key + SMALL_THREADS * ITEMS;
-  uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_val + SMALL_THREADS * ITEMS);   // [warp][256]: digit counts, then offsets inside the digit
-  uint32_t* s_base = reinterpret_cast<uint32_t*>(s_cnt + SMALL_WARPS * 256);      // [256] first place of each digit
+__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* keys_out, uint32_t* vals_out, uint32_t* totals) {   // may work in place
+  after_previous();
+  constexpr int ITEMS = SMALL_ITEMS;
+  __shared__ uint32_t s_key[SMALL_N], s_val[SMALL_N], s_base[256];                 // s_base: first place of each digit
+  __shared__ __align__(4) uint16_t s_cnt[SMALL_WARPS * 256];                       // [warp][256]: digit counts, then offsets inside the digit
   __shared__ uint32_t s_red[2][SMALL_WARPS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int first = warp * (32 * ITEMS) + lane;
@@ -120,6 +121,101 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const uint32_
   }
 #pragma unroll
   for (int j = 0; j < ITEMS; j++) { const int i = first + j * 32; if (i < n) { keys_out[i] = key[j]; vals_out[i] = val[j]; } }
+}
+
+// ---- one cluster ---------------------------------------------------------------------------------------------------------
+// Eight blocks of a cluster hold the pairs in their registers and shared memory from the first pass to the last: digit totals and the
+// pairs themselves cross between them in distributed shared memory, two barriers of the cluster a pass. Block b owns the places
+// b * THREADS * ITEMS .. of the sorted order.
+constexpr int CLUSTER = 8, CLUSTER_N = CLUSTER * SMALL_THREADS * 4;
+constexpr size_t cluster_smem(int items) { return (size_t)SMALL_THREADS * items * 8 + SMALL_WARPS * 256 * 2; }
+
+template <int ITEMS>
+__global__ void __launch_bounds__(SMALL_THREADS) cluster_sort_kernel(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* keys_out, uint32_t* vals_out, uint32_t* totals) {   // may work in place
+  after_previous();
+  namespace cg = cooperative_groups;
+  constexpr uint32_t SHARE = SMALL_THREADS * ITEMS;
+  extern __shared__ __align__(16) uint32_t s_mem[];
+  uint2* s_pair = reinterpret_cast<uint2*>(s_mem);
+  uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_pair + SHARE);   // [warp][256]: digit counts, then offsets inside the block's digit
+  __shared__ uint32_t s_tot[256], s_base[256], s_red[2][SMALL_WARPS], s_range[2];
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t me = cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t first = warp * (32 * ITEMS) + lane, lane_lt = (1u << lane) - 1u;
+  if (me == CLUSTER - 1u) clear_totals(totals);
+  uint32_t key[ITEMS], val[ITEMS], lo = CULLED, hi = 0u;
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) {
+    const uint32_t i = me * SHARE + first + j * 32;
+    key[j] = i < (uint32_t)n ? keys[i] : CULLED;      // the fill sorts behind everything: culled, and later in the input
+    val[j] = vals && i < (uint32_t)n ? vals[i] : i;
+    if (key[j] != CULLED) { lo = min(lo, key[j]); hi = max(hi, key[j]); }
+  }
+  lo = __reduce_min_sync(FULL, lo); hi = __reduce_max_sync(FULL, hi);
+  if (lane == 0) { s_red[0][warp] = lo; s_red[1][warp] = hi; }
+  __syncthreads();
+  if (warp == 0) {
+    lo = __reduce_min_sync(FULL, s_red[0][lane]); hi = __reduce_max_sync(FULL, s_red[1][lane]);
+    if (lane == 0) { s_range[0] = lo; s_range[1] = hi; }
+  }
+  cluster.sync();
+  {
+    const uint32_t* of = cluster.map_shared_rank(s_range, lane & (CLUSTER - 1));
+    lo = __reduce_min_sync(FULL, of[0]); hi = __reduce_max_sync(FULL, of[1]);
+  }
+  const Digits d = digits_of(lo, hi, 4);
+  const int bits = max(1, 32 - __clz((int)d.span));
+  uint16_t* my_cnt = s_cnt + warp * 256;
+  for (int shift = 0; shift < bits; shift += 8) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) reinterpret_cast<uint32_t*>(my_cnt)[lane + k * 32] = 0u;
+    __syncwarp();
+    uint32_t rank[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) {
+      const uint32_t g = (compressed(key[j], d) >> shift) & 255u;
+      uint32_t peers = FULL;   // lanes with the same digit: one vote per digit bit
+#pragma unroll
+      for (int b = 0; b < 8; b++) { const bool bit = (g >> b) & 1u; const uint32_t vote = __ballot_sync(FULL, bit); peers &= bit ? vote : ~vote; }
+      const uint32_t before = my_cnt[g];
+      rank[j] = before + __popc(peers & lane_lt);
+      __syncwarp();
+      if (lane == __ffs(peers) - 1) my_cnt[g] = (uint16_t)(before + __popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    // The warps' counts of a digit become offsets inside the block's; the block's totals are there for the others to read.
+    if (tid < 256) {
+      uint32_t sum = 0;
+#pragma unroll 8
+      for (int w = 0; w < SMALL_WARPS; w++) { const uint32_t c = s_cnt[w * 256 + tid]; s_cnt[w * 256 + tid] = (uint16_t)sum; sum += c; }
+      s_tot[tid] = sum;
+    }
+    cluster.sync();            // (and the pairs of the pass before have been read)
+    uint32_t base = 0;
+    if (tid < 256) {
+      uint32_t all = 0, before = 0;
+#pragma unroll
+      for (int c = 0; c < CLUSTER; c++) { const uint32_t t = cluster.map_shared_rank(s_tot, c)[tid]; before += (uint32_t)c < me ? t : 0u; all += t; }
+      const uint32_t incl = warp_incl(all);
+      if (lane == 31) s_red[0][warp] = incl;
+      base = incl - all + before;
+    }
+    __syncthreads();
+    if (tid < 256) { for (int w = 0; w < warp; w++) base += s_red[0][w]; s_base[tid] = base; }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) {
+      const uint32_t g = (compressed(key[j], d) >> shift) & 255u, at = s_base[g] + my_cnt[g] + rank[j];
+      cluster.map_shared_rank(s_pair, at / SHARE)[at % SHARE] = make_uint2(key[j], val[j]);
+    }
+    cluster.sync();
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) { const uint2 p = s_pair[first + j * 32]; key[j] = p.x; val[j] = p.y; }
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) { const uint32_t i = me * SHARE + first + j * 32; if (i < (uint32_t)n) { keys_out[i] = key[j]; vals_out[i] = val[j]; } }
 }
 
 // ---- many blocks ---------------------------------------------------------------------------------------------------------
@@ -388,15 +484,20 @@ int one_pass(const Shape& sh, const uint32_t* ki, const uint32_t* vi, uint32_t* 
   }
 }
 
-template <int ITEMS>
 int small_sort(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* ko, uint32_t* vo, uint32_t* totals, cudaStream_t s) {
+  launch_next(small_sort_kernel, 1, SMALL_THREADS, 0, s, keys, vals, n, ko, vo, totals);
+  return check_launch();
+}
+
+template <int ITEMS>
+int cluster_sort(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* ko, uint32_t* vo, uint32_t* totals, cudaStream_t s) {
   static bool attr_set[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !attr_set[dev]) {
-    B2K_CUDA(cudaFuncSetAttribute(small_sort_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(ITEMS)));
+    B2K_CUDA(cudaFuncSetAttribute(cluster_sort_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem(ITEMS)));
     attr_set[dev] = true;
   }
-  launch_next(small_sort_kernel<ITEMS>, 1, SMALL_THREADS, small_smem(ITEMS), s, keys, vals, n, ko, vo, totals);
+  launch_clustered(CLUSTER, cluster_sort_kernel<ITEMS>, CLUSTER, SMALL_THREADS, cluster_smem(ITEMS), s, keys, vals, n, ko, vo, totals);
   return check_launch();
 }
 
@@ -404,10 +505,12 @@ int depth_sort(const B2kCtx* c, int n, bool identity, bool for_walk, uint32_t* t
   const uint32_t* in = c->depth_keys_sorted;
   const uint32_t* index = identity ? nullptr : c->order;
   uint32_t* cleared = for_walk ? bins_tables(tables).tile_totals : nullptr;
-  if (n <= SMALL_N) {   // one block reads everything before it writes: in place
-    const int items = div_up(n, SMALL_THREADS);
-    uint32_t *k = c->depth_keys_sorted, *v = c->order;
-    return items <= 2 ? small_sort<2>(in, index, n, k, v, cleared, s) : items <= 4 ? small_sort<4>(in, index, n, k, v, cleared, s) : small_sort<SMALL_ITEMS>(in, index, n, k, v, cleared, s);
+  uint32_t *k = c->depth_keys_sorted, *v = c->order;   // one block, or one cluster, reads everything before it writes: in place
+  if (n <= SMALL_N) return small_sort(in, index, n, k, v, cleared, s);
+  if (n <= CLUSTER_N) {
+    const int items = div_up(n, CLUSTER * SMALL_THREADS);
+    return items <= 1 ? cluster_sort<1>(in, index, n, k, v, cleared, s) : items <= 2 ? cluster_sort<2>(in, index, n, k, v, cleared, s)
+           : items <= 3 ? cluster_sort<3>(in, index, n, k, v, cleared, s) : cluster_sort<4>(in, index, n, k, v, cleared, s);
   }
   uint32_t *table = tables, *totals = table + BINS_TABLE_WORDS;
   Range* range = (Range*)(totals + MAX_RADIX);

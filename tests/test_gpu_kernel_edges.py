@@ -504,3 +504,11 @@ def test_accumulator_rows_are_the_gradients(degree, active, n):
         assert not bool(h.ctx.vis_flag.any()) and not bool(h.ctx.v_splat[:n].any())
         got.append(grad)
     assert bool(got[0].any()) and torch.equal(got[0], got[1])
+
+
+
+@pytest.mark.parametrize("kind", ["uniform", "wide", "same", "culled", "any_bits"])
+@pytest.mark.parametrize("n", [8191, 16384, 16385, 24577, 32768, 32769])
+def test_depth_sort_in_one_cluster(n, kind):
+    """Every number of pairs a thread, full and with one left over, and the first size above."""
+    test_depth_sort_is_stable_at_every_size(n, kind)
