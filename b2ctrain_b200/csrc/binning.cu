@@ -53,7 +53,7 @@ using namespace b2k;
 
 namespace b2k {
 namespace {
-constexpr uint64_t sort_tmp_words(uint64_t n_cap) { return BIG_HEADER_WORDS + n_cap + BINS_TABLE_WORDS + BINS_EXTRA_WORDS; }
+constexpr uint64_t sort_tmp_words(uint64_t n_cap) { return TMP_HEADER_WORDS + n_cap + BINS_TABLE_WORDS + BINS_EXTRA_WORDS; }
 }  // namespace
 }  // namespace b2k
 

@@ -34,7 +34,8 @@ namespace {
 constexpr int PROJ_BLOCK = 256;
 
 // Tile boxes of at most MASK_TILES tiles are remembered as a bit mask of the tiles hit. The tests of boxes of at most WARP_TILES tiles
-// are shared out over the splats' warp; larger ones go to a list that a warp-per-splat kernel counts, so that no warp waits for a few of them.
+// are shared out over the splats' warp; larger ones are counted by a kernel of their own, a warp to each, so that no warp waits for a few of
+// them.
 constexpr int MASK_TILES = 64, WARP_TILES = 1024;
 
 // The tile tests of a warp's 32 splats, shared out in units of up to eight tiles of one row: boxes hold one to a thousand tiles, and with
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
     const float* __restrict__ sh_dc, const float* __restrict__ sh_hi, CamDev cam, int active, int tiles_x, int tiles_y,
     float4* __restrict__ proj0, float4* __restrict__ proj1, float4* __restrict__ proj2, uint32_t* __restrict__ tile_count,
     uint4* __restrict__ hit_info, uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in, float* __restrict__ max_screen,
-    uint32_t* __restrict__ big_list, uint32_t* __restrict__ big_count, int feat_mode, const float* __restrict__ feat_in, float2* __restrict__ proj3) {
+    int feat_mode, const float* __restrict__ feat_in, float2* __restrict__ proj3) {
   after_previous();
   __shared__ TileShare s_share[PROJ_BLOCK / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -163,7 +164,6 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
   }
   const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn);
   if (!valid) return;
-  if (t.big) big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
   if (drawn && max_screen) {
     const float detc = pr.c00 * pr.c11 - pr.c01 * pr.c01;
     const float ex = sqrtf(2.f * pr.power * pr.c11 / detc), ey = sqrtf(2.f * pr.power * pr.c00 / detc);
@@ -247,28 +247,34 @@ __global__ void __launch_bounds__(PROJ_BLOCK, 4) project_lite_kernel(
   depth_keys[i] = area ? __float_as_uint(pr.mean_c.z) : 0xFFFFFFFFu;
 }
 
-// One warp per listed splat: lanes sweep the tile box 32 tiles at a time.
-__global__ void __launch_bounds__(256) count_big_kernel(const uint32_t* __restrict__ big_list, const uint32_t* __restrict__ big_count,
-                                                        const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H, int tiles_x,
-                                                        int tiles_y, uint32_t* __restrict__ tile_count, uint32_t* __restrict__ depth_keys) {
+// Boxes above WARP_TILES: a warp to each, its lanes sweep the box 32 tiles at a time. Warp w looks at every (number of warps)-th pair of
+// splats from the w-th on (a pair is a sector of hit_info), so that large splats that follow each other go to different warps. (They used to
+// go to a list, whose counter took a launch of its own to clear: 64x64 over 2k splats 80.2 -> 78.9 us a step.)
+__global__ void __launch_bounds__(256) count_big_kernel(int n, const uint4* __restrict__ hit_info, const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H,
+                                                        int tiles_x, int tiles_y, uint32_t* __restrict__ tile_count, uint32_t* __restrict__ depth_keys) {
   after_previous();
-  const int lane = threadIdx.x & 31;
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5), count = *big_count;
-  for (uint32_t e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); e < count; e += warps) {
-    const uint32_t i = big_list[e];
-    const float4 a = proj0[i], b = proj1[i];
-    const TileRec rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
-    TileBox bb;
-    uint32_t hits = 0;
-    if (tile_box(rec, W, H, tiles_x, tiles_y, bb)) {
-      const int bw = bb.max_x - bb.min_x, area = bw * (bb.max_y - bb.min_y);
-      for (int t0 = 0; t0 < area; t0 += 32) {
-        const int t = t0 + lane;
-        const bool hit = t < area && tile_hit(bb.min_x + t % bw, bb.min_y + t / bw, rec);
-        hits += __popc(__ballot_sync(0xffffffffu, hit));
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5), first = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  for (long long p0 = first; 2 * p0 < n; p0 += 16ll * warps) {
+    auto splat_of = [&](int l) { return 2 * (p0 + (long long)(l >> 1) * warps) + (l & 1); };
+    const long long mine = splat_of(lane);
+    const uint4 hi = mine < n ? hit_info[mine] : make_uint4(0u, 0u, 0u, 0u);
+    const bool big = hi.z == 0xFFFFFFFFu && (hi.y & 0xFFFFu) * (hi.y >> 16) > (uint32_t)WARP_TILES;
+    for (uint32_t todo = __ballot_sync(0xffffffffu, big); todo; todo &= todo - 1u) {
+      const long long i = splat_of(__ffs(todo) - 1);
+      const float4 a = proj0[i], b = proj1[i];
+      const TileRec rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
+      TileBox bb;
+      uint32_t hits = 0;
+      if (tile_box(rec, W, H, tiles_x, tiles_y, bb)) {
+        const int bw = bb.max_x - bb.min_x, area = bw * (bb.max_y - bb.min_y);
+        for (int t0 = 0; t0 < area; t0 += 32) {
+          const int t = t0 + lane;
+          const bool hit = t < area && tile_hit(bb.min_x + t % bw, bb.min_y + t / bw, rec);
+          hits += __popc(__ballot_sync(0xffffffffu, hit));
+        }
       }
+      if (lane == 0) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
     }
-    if (lane == 0) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
   }
 }
 
@@ -276,8 +282,7 @@ __global__ void __launch_bounds__(256) count_big_kernel(const uint32_t* __restri
 // already in proj0 / proj1 (power < -0.5 marks "no record").
 __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H,
                                                                  int tiles_x, int tiles_y, uint32_t* __restrict__ tile_count, uint4* __restrict__ hit_info,
-                                                                 uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in,
-                                                                 uint32_t* __restrict__ big_list, uint32_t* __restrict__ big_count) {
+                                                                 uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in) {
   after_previous();
   __shared__ TileShare s_share[PROJ_BLOCK / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -293,7 +298,6 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
   }
   const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn);
   if (!valid) return;
-  if (t.big) big_list[atomicAdd(big_count, 1u)] = (uint32_t)i;
   hit_info[i] = make_uint4(t.w0, t.w1, t.box, t.height);
   order_in[i] = (uint32_t)i;
   if (!t.big) { tile_count[i] = t.hits; depth_keys[i] = t.hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
@@ -312,14 +316,11 @@ int launch(const B2kModel* m, const CamDev& cam, const B2kRenderOpts* o, const B
   const float4* quat = (const float4*)(o->quat_override ? o->quat_override : m->quat);
   const float4* lscale = (const float4*)(o->lscale_override ? o->lscale_override : m->lscale);
   const int active = o->sh_degree < m->degree ? o->sh_degree : m->degree;
-  uint32_t* big_count = big_count_ptr(c);
-  uint32_t* big_list = big_list_ptr(c);
-  launch_clear(big_count, 1, nullptr, 0, s);
   launch_next(project_kernel<DEG>, div_up(m->n, PROJ_BLOCK), PROJ_BLOCK, 0, s, 
       m->n, (size_t)m->cap, pos, quat, lscale, m->sh_dc, m->sh_hi, cam, active < 0 ? 0 : active, c->tiles_x, c->tiles_y,
       (float4*)c->proj0, (float4*)c->proj1, (float4*)c->proj2, c->tile_count, (uint4*)c->hit_info, c->depth_keys_sorted, c->order, m->max_screen,
-      big_list, big_count, o->feat_mode, o->feat_buffer, (float2*)c->proj3);
-  launch_next(count_big_kernel, sm_count() * 8, 256, 0, s, big_list, big_count, (const float4*)c->proj0, (const float4*)c->proj1, cam.W, cam.H, c->tiles_x,
+      o->feat_mode, o->feat_buffer, (float2*)c->proj3);
+  launch_next(count_big_kernel, min(div_up(m->n, 16), sm_count() * 8), 256, 0, s, m->n, (const uint4*)c->hit_info, (const float4*)c->proj0, (const float4*)c->proj1, cam.W, cam.H, c->tiles_x,
                                                   c->tiles_y, c->tile_count, c->depth_keys_sorted);
   return check_launch();
 }
@@ -373,12 +374,9 @@ extern "C" int b2k_count_tiles(const B2kCtx* c, int32_t n, b2k_stream_t stream) 
   B2K_REQUIRE(c->W > 0 && c->H > 0 && c->tiles_x == div_up(c->W, RT_W) && c->tiles_y == div_up(c->H, RT_W));
   if (c->n_cap < n || c->sort_tmp_bytes < b2k_sort_tmp_bytes(c->n_cap, c->isect_cap)) return B2K_ERR_CAPACITY;
   cudaStream_t s = (cudaStream_t)stream;
-  uint32_t* big_count = big_count_ptr(c);
-  uint32_t* big_list = big_list_ptr(c);
-  launch_clear(big_count, 1, nullptr, 0, s);
   launch_next(count_tiles_kernel, div_up(n, 256), 256, 0, s, n, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y, c->tile_count,
-                                                   (uint4*)c->hit_info, c->depth_keys_sorted, c->order, big_list, big_count);
-  launch_next(count_big_kernel, sm_count() * 8, 256, 0, s, big_list, big_count, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y,
+                                                   (uint4*)c->hit_info, c->depth_keys_sorted, c->order);
+  launch_next(count_big_kernel, min(div_up(n, 16), sm_count() * 8), 256, 0, s, n, (const uint4*)c->hit_info, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y,
                                                   c->tile_count, c->depth_keys_sorted);
   return check_launch();
 }
