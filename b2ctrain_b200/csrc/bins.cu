@@ -63,18 +63,18 @@ struct Pairs {
 
 // One rank's splat as level 1 sees it.
 struct Rank { uint32_t splat, tiles; uint4 hi; Box box; BinSpan span; };
-// Walks a list of splats in rounds of blockDim.x, the dependent loads (list entry, then the splat's record) one and two rounds
-// ahead of their use.
-template <bool WHOLE>
+// Walks a list of splats (list(p) for p in [begin, end)) in rounds of blockDim.x, the dependent loads (list entry, then the splat's
+// record) one and two rounds ahead of their use.
+template <bool WHOLE, class List>
 struct RankReader {
-  const View& v; const Band& g; const uint32_t* list; uint64_t at, end;
+  const View& v; const Band& g; const List& list; uint64_t at, end;
   uint32_t i1 = 0u, i2 = 0u, t1 = 0u;
   uint4 h1 = make_uint4(0u, 0u, 0u, 0u);
-  __device__ __forceinline__ RankReader(const View& v_, const Band& g_, const uint32_t* list_, uint64_t begin, uint64_t end_) : v(v_), g(g_), list(list_), at(begin + threadIdx.x), end(end_) {
+  __device__ __forceinline__ RankReader(const View& v_, const Band& g_, const List& list_, uint64_t begin, uint64_t end_) : v(v_), g(g_), list(list_), at(begin + threadIdx.x), end(end_) {
     i1 = entry(at); i2 = entry(at + blockDim.x);
     record(at);
   }
-  __device__ __forceinline__ uint32_t entry(uint64_t p) const { return p < end ? list[p] : 0u; }
+  __device__ __forceinline__ uint32_t entry(uint64_t p) const { return p < end ? list(p) : 0u; }
   __device__ __forceinline__ void record(uint64_t p) {
     const bool valid = p < end;
     h1 = valid ? v.hit_info[i1] : make_uint4(0u, 0u, 0u, 0u);
@@ -181,10 +181,13 @@ __device__ __forceinline__ bool wide_bins(const unsigned long long* s_alive, con
 
 // ---- level 1 -----------------------------------------------------------------------------------------------------------
 
-// Pairs per bin of each block's run of ranks. A chunk also leaves the run's splats that go anywhere, in order, at the run's
-// place in `live`: in the later chunks most splats lie behind saturated tiles, and the write pass never looks at them. The
-// whole view leaves the run's tile count instead (tile_off is its running sum).
-constexpr int COUNT_THREADS = 512;
+// Pairs per bin of each block's run of ranks. Each warp takes a part of the run by itself. A chunk also leaves the part's splats that go
+// anywhere, in order, at the part's place in `live`, and their number in live_counts: in the later chunks most splats lie behind
+// saturated tiles, and the write pass never looks at them. (With one list a block, the block met after every 512 ranks and every warp
+// added up the warps before it: 478 instructions for 32 ranks, nearly all dead, in the last chunk of a 4K view of 6M splats: 130 us, now 64.)
+// The whole view leaves the run's tile count instead (tile_off is its running sum).
+constexpr int COUNT_THREADS = 512, PARTS = COUNT_THREADS / 32;
+__device__ __forceinline__ uint32_t part_len(uint32_t run) { return (run + COUNT_THREADS - 1) / COUNT_THREADS * 32; }
 template <bool WHOLE>
 __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g, Tables t, uint32_t* __restrict__ live) {
   after_previous();
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
   const int bins = band_bins(g), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_alive + (WHOLE ? 0 : bins));
   uint16_t* s_sum = reinterpret_cast<uint16_t*>(s_cnt + bins);   // of a chunk behind the first
-  __shared__ uint32_t s_live[2][COUNT_THREADS / 32], s_warp[32];
+  __shared__ uint32_t s_warp[32];
   for (int i = tid; i < bins; i += COUNT_THREADS) s_cnt[i] = 0u;
   if (!WHOLE) load_alive(v, g, s_alive);
   if (blockIdx.x == 0 && tid == 0) {    // this band's counters; the view's with its first band
@@ -200,36 +203,80 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
     if (v.first_band) { t.st[S_SLOT] = v.words ? v.words[CW_BASE + v.chunk] : 0u; if (!v.words || v.chunk == 0) t.st[S_OVER] = 0u; }
   }
   __syncthreads();
-  if (!WHOLE && v.alive) sum_live(g, s_alive, s_sum);
+  const bool some_dead = !WHOLE && v.alive;
+  if (some_dead) sum_live(g, s_alive, s_sum);
   uint32_t r0, r1;
   view_ranks(v, r0, r1);
-  const uint32_t len = run_len(r1 - r0, gridDim.x);
-  const uint64_t begin = (uint64_t)r0 + (uint64_t)blockIdx.x * len, end = begin + len < (uint64_t)r1 ? begin + len : (uint64_t)r1;
-  uint32_t tiles = 0, n_live = 0;
-  int parity = 0;
-  RankReader<WHOLE> ranks(v, g, v.order, begin, end);
-  for (uint64_t at = begin; at < end; at += COUNT_THREADS, parity ^= 1) {
-    Rank k = ranks.next();
-    tiles += k.tiles;
-    if (!WHOLE && v.alive && k.span.count && !any_live(g, s_sum, k.span)) k.span.count = 0;
+  const uint32_t len = run_len(r1 - r0, gridDim.x), part = part_len(len);
+  const uint32_t run_end = (uint32_t)min((uint64_t)r0 + (uint64_t)(blockIdx.x + 1) * len, (uint64_t)r1);
+  const uint32_t begin = (uint32_t)min((uint64_t)r0 + (uint64_t)blockIdx.x * len + warp * part, (uint64_t)run_end), end = min(begin + part, run_end);
+  uint32_t tiles = 0, n_live = 0, waiting = 0;
+  auto count = [&](const Rank& k) {     // the bins of a warp's splats, and in a chunk the list of those that go into any
     const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
     for (uint32_t b = take; b; b &= b - 1u) atomicAdd(&s_cnt[own_bin(g, k, __ffs(b) - 1)], 1u);
     const bool wide = wide_bins<WHOLE>(s_alive, g, k, [&](int, uint32_t, int bin) { atomicAdd(&s_cnt[bin], 1u); });
     if constexpr (!WHOLE) {
       const uint32_t on = __ballot_sync(FULL, take != 0u || wide);
-      if (lane == 0) s_live[parity][warp] = (uint32_t)__popc(on);
-      __syncthreads();
-      uint32_t pre = 0, all = 0;
+      if ((on >> lane) & 1u) live[begin + n_live + __popc(on & ((1u << lane) - 1u))] = k.splat;
+      n_live += __popc(on);
+    }
+  };
+  __shared__ uint4 s_hit[WHOLE ? 1 : PARTS][64];
+  __shared__ uint32_t s_splat[WHOLE ? 1 : PARTS][64];
+  auto queued = [&](uint32_t n) {       // counts the first n of the warp's queue
+    __syncwarp();
+    Rank k{0u, 0u, make_uint4(0u, 0u, 0u, 0u), Box{0, 0, 0, 0}, BinSpan{0, 0, 0, 0, 0}};
+    const int w = WHOLE ? 0 : warp;
+    if ((uint32_t)lane < n) { k.splat = s_splat[w][lane]; k.hi = s_hit[w][lane]; }
+    k.box = box_of(k.hi); k.span = span_of(k.box, g);
+    count(k);
+  };
+  constexpr int PER = 2;                // ranks of a lane on their way together
+  uint32_t next[PER];
 #pragma unroll
-      for (int w = 0; w < COUNT_THREADS / 32; w++) { const uint32_t c = s_live[parity][w]; pre += w < warp ? c : 0u; all += c; }
-      if ((on >> lane) & 1u) live[begin + n_live + pre + __popc(on & ((1u << lane) - 1u))] = k.splat;
-      n_live += all;
+  for (int u = 0; u < PER; u++) next[u] = begin + u * 32 + lane < end ? v.order[begin + u * 32 + lane] : 0u;
+  for (uint32_t at = begin; at < end; at += 32 * PER) {
+    Rank k[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      const bool valid = at + u * 32 + lane < end;
+      k[u].splat = next[u];
+      k[u].hi = valid ? v.hit_info[next[u]] : make_uint4(0u, 0u, 0u, 0u);
+      k[u].tiles = WHOLE && valid ? v.tile_count[next[u]] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < PER; u++) { const uint32_t p = at + (PER + u) * 32 + lane; next[u] = p < end ? v.order[p] : 0u; }
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      if (WHOLE && k[u].tiles == 0u) k[u].hi = make_uint4(0u, 0u, 0u, 0u);
+      tiles += k[u].tiles;
+      k[u].box = box_of(k[u].hi);
+      k[u].span = span_of(k[u].box, g);
+      if (!some_dead) { count(k[u]); continue; }
+      // Behind the first chunks few splats overlap a bin that holds a live tile. They wait in shared memory until there are a warp's
+      // worth of them: with one here and there, nearly every warp went through the bins for a lane or two.
+      const bool in = k[u].span.count != 0 && any_live(g, s_sum, k[u].span);
+      const uint32_t m = __ballot_sync(FULL, in);
+      if (m == 0u) continue;
+      const int w = WHOLE ? 0 : warp;
+      if (in) { const uint32_t q = waiting + __popc(m & ((1u << lane) - 1u)); s_splat[w][q] = k[u].splat; s_hit[w][q] = k[u].hi; }
+      waiting += __popc(m);
+      if (waiting >= 32u) {
+        queued(32u);
+        waiting -= 32u;
+        __syncwarp();
+        const bool rest = (uint32_t)lane < waiting;
+        const uint32_t i = rest ? s_splat[w][32 + lane] : 0u;
+        const uint4 h = rest ? s_hit[w][32 + lane] : make_uint4(0u, 0u, 0u, 0u);
+        if (rest) { s_splat[w][lane] = i; s_hit[w][lane] = h; }
+      }
     }
   }
+  if (waiting) queued(waiting);
   __syncthreads();
   for (int i = tid; i < bins; i += COUNT_THREADS) t.cells[(size_t)i * gridDim.x + blockIdx.x] = s_cnt[i];
   if (!WHOLE) {
-    if (tid == 0) t.block_sums[blockIdx.x] = n_live;
+    if (lane == 0) t.live_counts[blockIdx.x * PARTS + warp] = n_live;
   } else if (v.first_band) {
     uint32_t total;
     block_scan(tiles, s_warp, total);
@@ -314,8 +361,28 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
   uint32_t r0, r1;
   view_ranks(v, r0, r1);
   const uint32_t len = run_len(r1 - r0, gridDim.x);
-  const uint64_t begin = (uint64_t)r0 + (uint64_t)blockIdx.x * len;
-  const uint64_t end = WHOLE ? (begin + len < (uint64_t)r1 ? begin + len : (uint64_t)r1) : begin + t.block_sums[blockIdx.x];
+  // The run's ranks, or of a chunk the live splats that the warps of bin_count have listed part by part.
+  const uint64_t run = (uint64_t)r0 + (uint64_t)blockIdx.x * len;
+  __shared__ uint32_t s_part[PARTS + 1];      // entries of the parts before
+  if (!WHOLE) {
+    if (warp == 0) {
+      const uint32_t c = lane < PARTS ? t.live_counts[blockIdx.x * PARTS + lane] : 0u;
+      uint32_t incl = c;
+#pragma unroll
+      for (int o = 1; o < PARTS; o <<= 1) { const uint32_t u = __shfl_up_sync(FULL, incl, o); if (lane >= o) incl += u; }
+      if (lane < PARTS) s_part[lane + 1] = incl;
+      if (lane == 0) s_part[0] = 0u;
+    }
+    __syncthreads();
+  }
+  const uint64_t begin = WHOLE ? run : 0u, end = WHOLE ? (run + len < (uint64_t)r1 ? run + len : (uint64_t)r1) : s_part[PARTS];
+  auto list = [&](uint64_t p) -> uint32_t {
+    if constexpr (WHOLE) return v.order[p];
+    uint32_t k = 0;                           // the part that holds entry p
+#pragma unroll
+    for (uint32_t step = PARTS / 2; step > 0; step >>= 1) k += s_part[k + step] <= p ? step : 0u;
+    return live[run + k * part_len(len) + (p - s_part[k])];
+  };
   const bool offsets = WHOLE && v.first_band;
   const uint32_t room = pr.room();
   for (int b = blockIdx.x * L1_WARPS + warp; b < bins; b += gridDim.x * L1_WARPS) {   // the items' bins, a warp per bin
@@ -351,7 +418,7 @@ __global__ void __launch_bounds__(L1_THREADS) bin_scatter_kernel(View v, Band g,
     if (added) { s_next[bin] += added; b4[0] = make_uint4(0u, 0u, 0u, 0u); b4[1] = make_uint4(0u, 0u, 0u, 0u); }
   };
   auto spread = [&](auto put) {
-    RankReader<WHOLE> ranks(v, g, WHOLE ? v.order : live, begin, end);
+    RankReader<WHOLE, decltype(list)> ranks(v, g, list, begin, end);
     for (uint64_t at = begin; at < end; at += L1_THREADS) {
       const Rank k = ranks.next();
       const uint32_t take = own_bins<WHOLE>(s_alive, g, k);
@@ -597,6 +664,7 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
   int dev = 0;
   constexpr int smem_max = MAX_BINS * ((L1_WARPS + 1) * (int)sizeof(uint32_t) + 8);
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !attr_set[dev]) {
+    B2K_CUDA(cudaFuncSetAttribute(bin_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_BINS * 12 + (MAX_BINS + 1) * 4 + 16));
     B2K_CUDA(cudaFuncSetAttribute(bin_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     B2K_CUDA(cudaFuncSetAttribute(bin_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     attr_set[dev] = true;

@@ -34,14 +34,15 @@ struct Tables {
   uint32_t* segments;    // [BINS_SEGMENTS] hits per tile_scan block
   uint32_t* st;          // [16] see S_*
   uint32_t* tile_totals; // [WALK_TILES] hits per tile, of walk.cu
+  uint32_t* live_counts; // [512][16] live splats of the parts of level 1's runs (a chunk)
 };
 constexpr int WALK_TILES = 4096;               // tiles of a view that walk.cu takes
 inline Tables bins_tables(uint32_t* tables) {
   Tables t;
   t.cells = tables;
   t.totals = t.cells + BINS_TABLE_WORDS; t.base = t.totals + MAX_BINS; t.first_item = t.base + MAX_BINS + 1; t.item_bin = t.first_item + MAX_BINS + 1;
-  t.block_sums = t.item_bin + MAX_ITEMS; t.segments = t.block_sums + 1024; t.st = t.segments + BINS_SEGMENTS; t.tile_totals = t.st + 16;
-  static_assert(MAX_BINS + 2 * (MAX_BINS + 1) + MAX_ITEMS + 1024 + BINS_SEGMENTS + 16 + WALK_TILES <= BINS_EXTRA_WORDS, "scratch");
+  t.block_sums = t.item_bin + MAX_ITEMS; t.segments = t.block_sums + 1024; t.st = t.segments + BINS_SEGMENTS; t.tile_totals = t.st + 16; t.live_counts = t.tile_totals + WALK_TILES;
+  static_assert(MAX_BINS + 2 * (MAX_BINS + 1) + MAX_ITEMS + 1024 + BINS_SEGMENTS + 16 + WALK_TILES + 512 * 16 <= BINS_EXTRA_WORDS, "scratch");
   return t;
 }
 enum { S_PAIRS = 0, S_ITEMS, S_ITEM_LEN, S_DONE_ROWS, S_DONE_TILES, S_SLOT, S_OVER, S_TOTAL, S_KEPT };

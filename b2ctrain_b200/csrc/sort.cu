@@ -514,7 +514,7 @@ int depth_sort(const B2kCtx* c, int n, bool identity, bool for_walk, uint32_t* t
   }
   uint32_t *table = tables, *totals = table + BINS_TABLE_WORDS;
   Range* range = (Range*)(totals + MAX_RADIX);
-  static_assert(MAX_RADIX + sizeof(Range) / sizeof(uint32_t) <= BINS_EXTRA_WORDS - WALK_TILES, "scratch");
+  static_assert(MAX_RADIX + sizeof(Range) / sizeof(uint32_t) <= MAX_BINS + 2 * (MAX_BINS + 1), "scratch: in front of the counters that outlive the sort");
   const Shape sh = shape_of((uint32_t)n);
   const int range_blocks = std::min<int>(std::min(2 * sm_count(), MAX_BLOCKS), div_up(n, CNT_THREADS * 16));
   launch_next(key_range_kernel, range_blocks, CNT_THREADS, 0, s, in, (uint32_t)n, range, cleared);
