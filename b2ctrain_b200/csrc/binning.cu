@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(256) chunk_prepare_kernel(const uint32_t* __re
   if (i != 0) return;
   words[CW_V] = (uint32_t)lo;
   words[CW_BASE] = 0u;
+  for (int k = CW_LONG; k < CW_WORDS; k++) words[k] = 0u;
 }
 
 }  // namespace
@@ -120,6 +121,7 @@ extern "C" int b2k_render_chunked(const B2kModel* m, const B2kCamera* cam, const
   if (n == 0) {
     B2K_CUDA(cudaMemsetAsync(c->tile_ranges, 0, sizeof(uint32_t) * 2 * (size_t)c->n_tiles * C, s));
     B2K_CUDA(cudaMemsetAsync(c->num_isect, 0, sizeof(uint32_t), s));
+    B2K_CUDA(cudaMemsetAsync(words, 0, sizeof(uint32_t) * CW_WORDS, s));   // no tile of any chunk has a list
     for (int ch = 0; ch < C; ch++) { st = launch_raster_fwd(c, o, ch, C, alive, s); if (st) return st; }
     return B2K_OK;
   }

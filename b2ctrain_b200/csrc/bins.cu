@@ -557,7 +557,8 @@ __global__ void __launch_bounds__(COL_GROUPS * BIN_TILES) item_columns_kernel(Ba
 // Ranges of the band's tiles, row-major: block b starts behind the hits of the blocks before it. Empty tiles get (0, 0);
 // ranges end with the buffers. The last block to finish moves the view's slot on. All loads are issued before the one
 // scan of the block (two scans one after the other and a fence took 5.4 to 7.8 us, this 2.8 to 5.8).
-__global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, Tables t, uint32_t cap, uint2* __restrict__ ranges, uint32_t* __restrict__ num_isect) {
+__global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, Tables t, uint32_t cap, uint2* __restrict__ ranges, uint32_t* __restrict__ num_isect,
+                                                               uint32_t* __restrict__ list) {
   after_previous();
   __shared__ uint32_t s_warp[32], s_slot;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -577,6 +578,15 @@ __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, T
   uint32_t total;
   const uint32_t in_block = block_scan(c, s_warp, total) - c, slot = s_slot, start = slot + before + in_block;
   if (mine < tiles) ranges[tile0 + mine] = c ? make_uint2(min(start, cap), min(start + c, cap)) : make_uint2(0u, 0u);
+  if (list) {   // the chunk's tiles with a list, for the compositing: long lists from the start, short ones from the end
+    const uint32_t longs = __ballot_sync(FULL, c >= LONG_LIST), shorts = __ballot_sync(FULL, c > 0u && c < LONG_LIST), lane_lt = (1u << lane) - 1u;
+    uint32_t at_long = 0u, at_short = 0u;
+    if (lane == 0 && longs) at_long = atomicAdd(v.words + CW_LONG + v.chunk, (uint32_t)__popc(longs));
+    if (lane == 1 && shorts) at_short = atomicAdd(v.words + CW_SHORT + v.chunk, (uint32_t)__popc(shorts));
+    at_long = __shfl_sync(FULL, at_long, 0); at_short = __shfl_sync(FULL, at_short, 1);
+    if ((longs >> lane) & 1u) list[at_long + __popc(longs & lane_lt)] = (uint32_t)(tile0 + mine);
+    if ((shorts >> lane) & 1u) list[g.tiles_x * g.tiles_y - 1 - (int)(at_short + __popc(shorts & lane_lt))] = (uint32_t)(tile0 + mine);
+  }
   if (tid == 0 && atomicAdd(t.st + S_DONE_TILES, 1u) == gridDim.x - 1u) {   // every block has read the slot (its first thread did)
     uint32_t end = slot + all;
     if (v.last_band) {
@@ -697,7 +707,7 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
 #undef L
     if (bins >= 2 * sm_count()) launch_next(item_columns_kernel<4>, bins, 4 * BIN_TILES, 0, s, g, t, ranges);
     else launch_next(item_columns_kernel<16>, bins, 16 * BIN_TILES, 0, s, g, t, ranges);
-    launch_next(tile_scan_kernel, div_up(tiles, SCAN_TILES), SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect);
+    launch_next(tile_scan_kernel, div_up(tiles, SCAN_TILES), SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect, alive ? (uint32_t*)(alive + (size_t)bins_x * bin_rows) : nullptr);
     if (words) launch_next(item_emit_kernel<false>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
     else launch_next(item_emit_kernel<true>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
   }

@@ -73,6 +73,16 @@ __device__ __forceinline__ float2 pair_alpha(const float4& q0, const float4& q1,
                      __float_as_uint(sigma.y) <= __float_as_uint(power.y) ? fminf(ALPHA_MAX, al.y) : 0.f);
 }
 
+// The tiles of a chunk behind the first that have a list (tile_scan has written them down): those with long lists first.
+struct TileList {
+  const uint32_t* list; uint32_t longs, count; int n_tiles;
+  __device__ __forceinline__ int at(uint32_t w) const { return list ? (int)list[w < longs ? w : (uint32_t)n_tiles - 1u - (w - longs)] : (int)w; }
+};
+__device__ __forceinline__ TileList tile_list(const uint32_t* words, const uint32_t* list, int chunk, int n_tiles) {
+  const uint32_t longs = words[CW_LONG + chunk];
+  return {list, longs, longs + words[CW_SHORT + chunk], n_tiles};
+}
+
 // What the forward leaves for the backward (common.cuh): nothing, checkpoints of the running sums, or of each segment's sums.
 enum Checkpoints { NONE = 0, RUNNING = 1, PER_SEGMENT = 2 };
 
@@ -302,32 +312,49 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
 // idle but for the lists' own length: four warps find the alphas of
 // a batch, two warps (a pixel per lane) carry the transmittances and the sums, two warps take turns to gather and stage the records of
 // the batches ahead. A batch passes from one to the next with one barrier of the block.
-constexpr int TEAM_BATCH = FWD_SEG, TEAM_PAIRS = TEAM_BATCH / 2, TEAM_PRODUCERS = 4, TEAM_GROUP = 8, TEAM_THREADS = (2 + TEAM_PRODUCERS + 2) * 32, TEAM_PER_SM = 8;
+constexpr int TEAM_BATCH = FWD_SEG, TEAM_PAIRS = TEAM_BATCH / 2, TEAM_PRODUCERS = 4, TEAM_THREADS = (2 + TEAM_PRODUCERS + 2) * 32, TEAM_PER_SM = 8;
 
-template <int CKPT, bool DEPTH, bool FEAT>
-__global__ void __launch_bounds__(TEAM_THREADS) raster_fwd_team_kernel(
+template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
+__global__ void __launch_bounds__(TEAM_THREADS, CHUNKED ? 4 : 2) raster_fwd_team_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
-    const float4* __restrict__ proj2, int W, int H, int tiles_x, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
-    float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, uint32_t* __restrict__ bwd_work) {
+    const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
+    float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, uint32_t* __restrict__ bwd_work, const uint32_t* __restrict__ words, const uint32_t* __restrict__ list) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   constexpr int RECORDS = FEAT ? STAGED + 2 : DEPTH ? STAGED + 1 : STAGED;
   __shared__ float4 s_staged[3][TEAM_PAIRS][RECORDS];   // of the batches that are staged, weighed and composited
   __shared__ float2 s_alpha[2][TEAM_PAIRS][RT_PX];
   __shared__ uint32_t s_odd[3], s_last[2];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile = blockIdx.x, tx = tile % tiles_x, ty = tile / tiles_x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int TEAM_GROUP = CHUNKED ? 4 : 8;   // pairs whose sums are taken together: eight want registers for two blocks an SM, which is enough where tiles are few
+  static_assert(!(CHUNKED && (DEPTH || FEAT)), "the last chunk finishes depths and features in every tile");
+  const bool composites = warp < 2, weighs = !composites && warp < 2 + TEAM_PRODUCERS, final = !CHUNKED || chunk == n_chunks - 1;
+  if (CKPT == PER_SEGMENT && !CHUNKED && blockIdx.x == 0 && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
+  const TileList tiles = CHUNKED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
+  for (uint32_t w = blockIdx.x; w < tiles.count; w += gridDim.x) {
+  if (w != blockIdx.x) __syncthreads();   // the last tile's batches have been read
+  const int tile = tiles.at(w), tx = tile % tiles_x, ty = tile / tiles_x;
   const uint2 range = tile_ranges[tile];
   const uint32_t batches = range.y > range.x ? (range.y - range.x + TEAM_BATCH - 1) / TEAM_BATCH : 0u;
-  if (CKPT == PER_SEGMENT && tile == 0 && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
-  const bool composites = warp < 2, weighs = !composites && warp < 2 + TEAM_PRODUCERS;
   // The lane's pixel, of a producer its first of two.
   const int in_tile = (composites ? warp * 32 : 0) + lane, px = tx * RT_W + (in_tile & 7), py = ty * RT_W + (in_tile >> 3), pix = py * W + px;
   const bool inside = composites && px < W && py < H;
   const float2 pcx = make_float2((float)px + 0.5f, (float)px + 0.5f), pcy = make_float2((float)py + 0.5f, (float)py + 0.5f);
-  Pixel<CKPT, DEPTH, FEAT, BWD> P;
+  Pixel<CKPT, DEPTH, FEAT, BWD || CHUNKED> P;
   P.T = inside ? 1.f : 0.f;
   P.last = range.x;
+  if (CHUNKED && inside) {
+    const float4 acc = out_feat[pix];
+    P.r = acc.x; P.g = acc.y; P.b = acc.z;
+    const uint32_t l = last_idx[pix];
+    P.T = (l & DONE_BIT) == 0u ? acc.w : 0.f; P.T_closed = acc.w;
+    P.last = l & ~DONE_BIT;
+  }
+  const int q = CHUNKED ? chunk * n_tiles + tile : tile;
   uint32_t seg_now = 0;
+  auto checkpoint = [&](uint32_t seg) { P.checkpoint(ckpt + (size_t)ckpt_slot(range.x, q, seg, seg_shift) * RT_PX + in_tile); seg_now = seg; };
+  if (BWD && CHUNKED && composites) checkpoint(0u);   // the state this chunk starts the tile with
   // A gathering warp's next batch is in its registers, and the list entries of the one after that.
   const uint32_t turn = (uint32_t)warp & 1u;
   float4 n0, n1, n2;
@@ -349,10 +376,7 @@ __global__ void __launch_bounds__(TEAM_THREADS) raster_fwd_team_kernel(
       const uint32_t at = (t - 2u) * TEAM_BATCH, start = range.x + at, count = min((uint32_t)TEAM_BATCH, range.y - start);
       const float4 (*staged)[RECORDS] = s_staged[(t - 2u) % 3u];
       const float2 (*alphas)[RT_PX] = s_alpha[t & 1u];
-      if (BWD && at != 0u && (at & ((1u << seg_shift) - 1u)) == 0u) {
-        seg_now = at >> seg_shift;
-        P.checkpoint(ckpt + (size_t)ckpt_slot(range.x, tile, seg_now, seg_shift) * RT_PX + in_tile);
-      }
+      if (BWD && at != 0u && (at & ((1u << seg_shift) - 1u)) == 0u) checkpoint(at >> seg_shift);
       if (!__any_sync(0xffffffffu, P.T != 0.f)) continue;   // only the other half is still at it
       if (s_odd[(t - 2u) % 3u]) {
 #pragma unroll 1
@@ -393,48 +417,61 @@ __global__ void __launch_bounds__(TEAM_THREADS) raster_fwd_team_kernel(
       entries(t + 4u);
     }
   }
-  if (!composites) return;
+  if (!composites) continue;
+  const bool open = P.T != 0.f;
   const float T = P.now();
   if (inside) {
     out_rgba[pix] = make_float4(P.r + T * bg.x, P.g + T * bg.y, P.b + T * bg.z, 1.f - T);
-    out_feat[pix] = make_float4(P.f0, P.f1, P.f2, T);
-    if constexpr (DEPTH) out_depth[pix] = finished_depth(P.zs, T);
-    if constexpr (BWD) last_idx[pix] = P.last;
+    if constexpr (CHUNKED) {
+      out_feat[pix] = make_float4(P.r, P.g, P.b, T);
+      last_idx[pix] = P.last | (open ? 0u : DONE_BIT);
+    } else {
+      out_feat[pix] = make_float4(P.f0, P.f1, P.f2, T);
+      if constexpr (DEPTH) out_depth[pix] = finished_depth(P.zs, T);
+      if constexpr (BWD) last_idx[pix] = P.last;
+    }
   }
-  if constexpr (BWD) {
-    // The backward never needs to look past the last fragment any pixel used.
+  if constexpr (BWD || CHUNKED) {
+    // What the two warps settle together: whether any pixel is still open, and the last fragment any pixel used, which the backward never
+    // needs to look past.
     const uint32_t mine = __reduce_max_sync(0xffffffffu, P.last);
     if (lane == 0) s_last[warp] = mine;
-    pair_any(1, false);
-    const uint32_t m = max(s_last[0], s_last[1]);
-    if (in_tile == 0) tile_ranges[tile].y = m;
+    const bool any_open = pair_any(1, open);
+    if (CHUNKED && !final && in_tile == 0 && !any_open)
+      atomicAnd(alive + (size_t)(ty >> 3) * ((tiles_x + 7) >> 3) + (tx >> 3), ~(1ull << ((ty & 7) * 8 + (tx & 7))));
+    uint32_t m = max(s_last[0], s_last[1]);
+    if constexpr (CHUNKED) m = min(max(m, range.x), range.y);
+    if (BWD && in_tile == 0) tile_ranges[tile].y = m;
     if (CKPT == PER_SEGMENT && m > range.x) {
       // Slot 0 has no segment before it (see raster_fwd_half_kernel).
       const uint32_t segs = (m - range.x + (1u << seg_shift) - 1u) >> seg_shift;
-      float* dst = reinterpret_cast<float*>(ckpt + (size_t)ckpt_slot(range.x, tile, 0u, seg_shift) * RT_PX + in_tile);
-      const float4 v = segs - 1u == seg_now ? make_float4(P.sr, P.sg, P.sb, 0.f) : ckpt[(size_t)ckpt_slot(range.x, tile, segs, seg_shift) * RT_PX + in_tile];
+      float* dst = reinterpret_cast<float*>(ckpt + (size_t)ckpt_slot(range.x, q, 0u, seg_shift) * RT_PX + in_tile);
+      const float4 v = segs - 1u == seg_now ? make_float4(P.sr, P.sg, P.sb, 0.f) : ckpt[(size_t)ckpt_slot(range.x, q, segs, seg_shift) * RT_PX + in_tile];
       dst[0] = v.x; dst[1] = v.y; dst[2] = v.z;
     }
+  }
   }
 }
 
 // One warp to a tile, for views in depth chunks.
-template <int CKPT, bool DEPTH, bool FEAT>
+template <int CKPT, bool DEPTH, bool FEAT, bool LISTED>
 __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
-    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work) {
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work,
+    const uint32_t* __restrict__ words, const uint32_t* __restrict__ list) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   // FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
   // pixel travel in feat_acc and move into out_feat.xyz when the last chunk, which then visits every pixel, is done.
   static_assert(!(FEAT && BWD), "the chunked backward reads the colour sums from out_feat.xyz");
   __shared__ float4 s_staged[FWD_WARPS][FWD_SEG][FEAT ? 6 : 5];   // a fragment's constants, most of them twice, as operands of packed arithmetic
-  float2 f0 = splat2(0.f), f1 = f0, f2 = f0;   // composited feature lanes (raster_fwd.cu:52)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x * FWD_WARPS + warp;
-  if (tile >= n_tiles) return;
+  const TileList tiles = LISTED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
+  for (uint32_t w = blockIdx.x * FWD_WARPS + warp; w < tiles.count; w += gridDim.x * FWD_WARPS) {   // (once, unless LISTED)
+  const int tile = tiles.at(w);
+  float2 f0 = splat2(0.f), f1 = f0, f2 = f0;   // composited feature lanes (raster_fwd.cu:52)
   const int tx = tile % tiles_x, ty = tile / tiles_x;
   const int px0 = tx * RT_W + (lane & 3) * 2, py = ty * RT_W + (lane >> 2);
   const bool in0 = px0 < W && py < H, in1 = px0 + 1 < W && py < H;
@@ -442,7 +479,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   const uint2 range = tile_ranges[tile];
   const bool first = chunk == 0, final = chunk == n_chunks - 1;
   if (CKPT == PER_SEGMENT && first && tile == 0 && lane == 0) bwd_work[BWD_SUMMED] = 0u;
-  if (!first && range.y <= range.x && !(final && FEAT)) {   // nothing of this chunk lands here: pixels, state and flag stay
+  if (!LISTED && !first && range.y <= range.x && !(final && FEAT)) {   // nothing of this chunk lands here: pixels, state and flag stay
     if (DEPTH && final) {
 #pragma unroll
       for (int p = 0; p < 2; p++)
@@ -630,6 +667,8 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
       }
     }
   }
+  if (!LISTED) return;
+  }
 }
 
 }  // namespace
@@ -643,15 +682,20 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
   uint2* ranges = (uint2*)c->tile_ranges + (n_chunks > 1 ? (size_t)chunk * c->n_tiles : 0);
   const bool chunked = n_chunks > 1, halves = n_chunks <= 2;   // (measured above)
+  // Behind the first chunk only the tiles with a list are visited, but for the last one where it finishes depths or features.
+  const int bins = div_up(c->tiles_x, 8) * div_up(c->tiles_y, 8);
+  const uint32_t* list = chunked && chunk > 0 && !(chunk == n_chunks - 1 && (c->out_depth || o->feat_mode != 0)) ? (const uint32_t*)(alive + bins) : nullptr;
 #define ARGS s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, \
     (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, \
     seg_shift_of(short_segments(c)), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr, bwd_work_ptr(c)
 #define HALF(B, D, C, F) launch_next(raster_fwd_half_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_TILES), FWD_WARPS * 32, 0, ARGS)
-#define TEAM(B, D, F) launch_next(raster_fwd_team_kernel<B, D, F>, c->n_tiles, TEAM_THREADS, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, \
-    (const float4*)c->proj2, c->W, c->H, c->tiles_x, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, (const float2*)c->proj3, \
-    o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c))
-#define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_PER_SM * sm_count()) TEAM(B, D, F); else HALF(B, D, false, F); } else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
-    else launch_next(raster_fwd_kernel<B, D, (F) && (B) == NONE>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS); } while (0)
+#define TEAM(B, D, C, F) launch_next(raster_fwd_team_kernel<B, D, C, F>, C ? min(c->n_tiles, TEAM_PER_SM * sm_count()) : c->n_tiles, TEAM_THREADS, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, \
+    (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, \
+    (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c), c->chunk_words, list)
+#define WARP(B, D, F) do { if (list) launch_next(raster_fwd_kernel<B, D, F, true>, min(div_up(c->n_tiles, FWD_WARPS), 24 * sm_count()), FWD_WARPS * 32, 0, ARGS, c->chunk_words, list); \
+    else launch_next(raster_fwd_kernel<B, D, F, false>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS, c->chunk_words, list); } while (0)
+#define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_PER_SM * sm_count()) TEAM(B, D, false, F); else HALF(B, D, false, F); } else if (halves && list) TEAM(B, false, true, false); else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
+    else WARP(B, D, (F) && (B) == NONE); } while (0)
 #define LD(B, D) do { if (o->feat_mode != 0) L(B, D, true); else L(B, D, false); } while (0)   // a chunked view with features is forward only (checked by the caller)
 #define LB(B) do { if (c->out_depth) LD(B, true); else LD(B, false); } while (0)
   if (!o->bwd_info) LB(NONE);
@@ -662,6 +706,7 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
 #undef L
 #undef HALF
 #undef TEAM
+#undef WARP
 #undef ARGS
   return check_launch();
 }

@@ -98,7 +98,8 @@ typedef struct {
                               range per chunk and tile, indices into vals_sorted) and b2k_raster_bwd walks them all */
   float* proj3;            /* [n][2] feature lanes y, z (x rides in proj2.w), render.h:70; NULL unless a feature mode is used */
   uint32_t* chunk_words;   /* [32 + n_tiles + (tiles_x + 1)(tiles_y + 1)] device scratch of b2k_render_chunked (chunk windows
-                              and counts, one "some pixel can still take a fragment" flag per tile), or NULL when
+                              and counts, one "some pixel can still take a fragment" flag per tile, the list of a chunk's tiles
+                              that have fragments), or NULL when
                               n_chunks <= 1 */
   void* bwd_scratch;       /* b2k_bwd_scratch_bytes() bytes, needed when the forward runs with bwd_info: per-pixel (colour
                               sums, transmittance) checkpoints the forward leaves at every segment boundary of a tile's list, and

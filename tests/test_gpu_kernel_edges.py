@@ -512,3 +512,28 @@ def test_accumulator_rows_are_the_gradients(degree, active, n):
 def test_depth_sort_in_one_cluster(n, kind):
     """Every number of pairs a thread, full and with one left over, and the first size above."""
     test_depth_sort_is_stable_at_every_size(n, kind)
+
+
+
+@pytest.mark.parametrize("W,H", [(64, 64), (528, 520)])   # segments of 32 and of 128 fragments
+@pytest.mark.parametrize("chunks", [2, 3, 5])
+@pytest.mark.parametrize("n", [1, 3, 40])
+def test_chunks_without_fragments(n, chunks, W, H):
+    """Few splats leave the first chunks without any: nothing but background there, and the backward of every pass starts anew."""
+    import torch
+    scene, cam = stack_scene(n, W, H)
+    scene["pos_op"][:, 3] = 1.0
+    h = Harness(scene, cam, bg=(0.2, 0.1, 0.3))
+    ctx = h.api.RenderCtx("cuda:0")
+    ctx.setup(W, H, h.model.cap, n_chunks=chunks)
+    v_out = torch.from_numpy(np.random.Generator(np.random.PCG64(4)).standard_normal((W * H, 4)).astype(np.float32))
+    for c in (ctx, h.ctx):
+        c.out_rgba.fill_(7.0)
+    for _ in range(2):
+        for c in (ctx, h.ctx):
+            h.api.render_forward(c, h.model, h.rp)
+            c.v_out.copy_(v_out)
+            c.v_splat.zero_(); c.vis_flag.zero_()
+            h.api.rasterize_backward(c, h.model, h.rp)
+        assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
+        assert torch.equal(ctx.vis_flag[:n], h.ctx.vis_flag[:n]) and rel_l2(ctx.v_splat[:n].cpu().numpy(), h.ctx.v_splat[:n].cpu().numpy()) <= 2e-5
