@@ -237,7 +237,10 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_emit_kernel(View v, Band g,
 }
 
 // Where the walk is taken: images of few tiles, whose totals every block can scan, and up to this many tests of a rank against a bin.
-constexpr long long WALK_TESTS = 1LL << 21;
+// Binning behind the sort, us, the general distribution / the walk (tests): 64x64 over 2k splats 30.8 / 13.6, over 200k (0.2M) 65.5 / 31.3;
+// 200x150 over 40k (0.5M) 43.7 / 26.2, over 100k (1.2M) 55.1 / 46.7; 333x217 over 20k (0.5M) 43.8 / 24.1, over 60k (1.4M) 48.3 / 46.6;
+// 400x300 over 30k (1.1M) 45.6 / 40.3, over 60k (2.1M) 50.3 / 62.8; 512x512 over 8k (0.5M) 50.1 / 36.4, over 16k (1.0M) 50.2 / 52.6.
+constexpr long long WALK_TESTS = 1LL << 20;
 
 }  // namespace
 
