@@ -83,7 +83,7 @@ extern "C" int b2k_bin_sort(const B2kCtx* c, int32_t n, b2k_stream_t stream) {
   if (st) return st;
   mark(s);
   // 2. Hits to the tiles' lists, depth order surviving inside each tile; 3. the tile ids of the list.
-  st = launch_bins(c, n, nullptr, 0, 0, 256, nullptr, tables, s);
+  st = launch_bins(c, n, nullptr, 0, 0, 256, nullptr, nullptr, tables, s);
   if (st) return st;
   mark(s);
   if (!walks(c, n)) st = launch_fill_keys(c, s);
@@ -118,24 +118,25 @@ extern "C" int b2k_render_chunked(const B2kModel* m, const B2kCamera* cam, const
   }
   uint32_t* words = c->chunk_words;
   unsigned long long* alive = (unsigned long long*)(((uintptr_t)(words + CW_WORDS) + 7) & ~(uintptr_t)7);   // the caller's array may start at any word
+  const int bins = div_up(c->tiles_x, 8) * div_up(c->tiles_y, 8);
+  uint32_t* tiles = (uint32_t*)(alive + bins);
   if (n == 0) {
     B2K_CUDA(cudaMemsetAsync(c->tile_ranges, 0, sizeof(uint32_t) * 2 * (size_t)c->n_tiles * C, s));
     B2K_CUDA(cudaMemsetAsync(c->num_isect, 0, sizeof(uint32_t), s));
     B2K_CUDA(cudaMemsetAsync(words, 0, sizeof(uint32_t) * CW_WORDS, s));   // no tile of any chunk has a list
-    for (int ch = 0; ch < C; ch++) { st = launch_raster_fwd(c, o, ch, C, alive, s); if (st) return st; }
+    for (int ch = 0; ch < C; ch++) { st = launch_raster_fwd(c, o, ch, C, alive, lists_tiles(c, ch) ? tiles : nullptr, s); if (st) return st; }
     return B2K_OK;
   }
   if (c->sort_tmp_bytes < b2k_sort_tmp_bytes(c->n_cap, c->isect_cap) || c->isect_cap == 0 || c->isect_cap > 0x7FFFFFF0ull) return B2K_ERR_CAPACITY;
   uint32_t* tables = sort_tables_ptr(c);
   st = depth_sort(c, n, true, false, tables, s);
   if (st) return st;
-  const int bins = div_up(c->tiles_x, 8) * div_up(c->tiles_y, 8);
   launch_next(chunk_prepare_kernel, div_up(bins, 256), 256, 0, s, c->depth_keys_sorted, n, words, alive, bins);
   for (int ch = 0; ch < C; ch++) {
     const int lo = ch == 0 ? 0 : 256 >> (2 * (C - ch)), hi = 256 >> (2 * (C - 1 - ch));
-    st = launch_bins(c, n, words, ch, lo, hi, ch == 0 ? nullptr : alive, tables, s);   // the first chunk meets only live tiles
+    st = launch_bins(c, n, words, ch, lo, hi, ch == 0 ? nullptr : alive, lists_tiles(c, ch) ? tiles : nullptr, tables, s);   // the first chunk meets only live tiles
     if (st) return st;
-    st = launch_raster_fwd(c, o, ch, C, alive, s);
+    st = launch_raster_fwd(c, o, ch, C, alive, lists_tiles(c, ch) ? tiles : nullptr, s);
     if (st) return st;
   }
   return B2K_OK;

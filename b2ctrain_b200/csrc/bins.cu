@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(256) fill_keys_kernel(int n_tiles, const uint2
 
 // Bins the ranks of one depth chunk (words != nullptr) or of the whole view into vals_sorted and `ranges`. Level 1's pairs
 // take ctx->keys, the hit words (or more pairs) ctx->vals and ctx->keys_sorted, a chunk's live splats the scratch of the depth sort.
-int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, int hi_num, const unsigned long long* alive, uint32_t* tables, cudaStream_t s) {
+int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, int hi_num, const unsigned long long* alive, uint32_t* tiles_out, uint32_t* tables, cudaStream_t s) {
   const Tables t = bins_tables(tables);
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -714,7 +714,7 @@ int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, 
 #undef L
     if (bins >= 2 * sm_count()) launch_next(item_columns_kernel<4>, bins, 4 * BIN_TILES, 0, s, g, t, ranges);
     else launch_next(item_columns_kernel<16>, bins, 16 * BIN_TILES, 0, s, g, t, ranges);
-    launch_next(tile_scan_kernel, div_up(tiles, SCAN_TILES), SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect, alive ? (uint32_t*)(alive + (size_t)bins_x * bin_rows) : nullptr);
+    launch_next(tile_scan_kernel, div_up(tiles, SCAN_TILES), SCAN_TILES, 0, s, v, g, t, cap, ranges, c->num_isect, tiles_out);
     if (words) launch_next(item_emit_kernel<false>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
     else launch_next(item_emit_kernel<true>, item_blocks, L2_THREADS, 0, s, v, g, t, pr, ranges, c->vals_sorted);
   }

@@ -165,12 +165,51 @@ __device__ __forceinline__ bool stage_record(float4* pair, int k, const float4& 
   return strange;
 }
 
-template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
+// The pixels of the tiles without a list, by blocks of their own behind those that composite: a warp looks at 32 tiles at a time. In the
+// first chunk they get the background (a tile with a list that the backward's end has moved back to (0, 0) holds just these values);
+// in the last one their depths are finished, which a forward for a backward leaves to the compositing (it moves ranges).
+template <bool DEPTH>
+__device__ __forceinline__ void visit_unlisted(int block, int blocks, const uint2* __restrict__ tile_ranges, int n_tiles, int tiles_x, int W, int H, float3 bg, bool first,
+                                               float4* __restrict__ out_rgba, float4* __restrict__ out_feat, float* __restrict__ out_depth, uint32_t* __restrict__ last_idx) {
+  const int lane = threadIdx.x & 31, warps = blocks * FWD_WARPS;
+  for (int t0 = (block * FWD_WARPS + (threadIdx.x >> 5)) * 32; t0 < n_tiles; t0 += warps * 32) {
+    uint2 range = make_uint2(0u, 1u);
+    if (t0 + lane < n_tiles) range = tile_ranges[t0 + lane];
+    for (uint32_t todo = __ballot_sync(0xffffffffu, (range.x | range.y) == 0u); todo; todo &= todo - 1u) {
+      const int tile = t0 + __ffs(todo) - 1, tx = tile % tiles_x, ty = tile / tiles_x;
+      int pix[2];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int px = tx * RT_W + (lane & 7), py = ty * RT_W + (lane >> 3) + h * 4;
+        pix[h] = px < W && py < H ? py * W + px : -1;
+      }
+      if (first) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          if (pix[h] < 0) continue;
+          out_rgba[pix[h]] = make_float4(bg.x, bg.y, bg.z, 0.f);
+          out_feat[pix[h]] = make_float4(0.f, 0.f, 0.f, 1.f);
+          if constexpr (DEPTH) out_depth[pix[h]] = 0.f;   // a sum yet
+          last_idx[pix[h]] = 0u;                          // an empty range starts at 0
+        }
+      } else if constexpr (DEPTH) {
+        float zs[2], T[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) { zs[h] = pix[h] < 0 ? 0.f : out_depth[pix[h]]; T[h] = pix[h] < 0 ? 1.f : out_feat[pix[h]].w; }
+#pragma unroll
+        for (int h = 0; h < 2; h++) if (pix[h] >= 0) out_depth[pix[h]] = finished_depth(zs[h], T[h]);
+      }
+    }
+  }
+}
+
+template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT, bool LISTED>
 __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
-    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work) {
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work,
+    const uint32_t* __restrict__ words, const uint32_t* __restrict__ list, int fill_blocks) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
@@ -180,16 +219,23 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
   __shared__ float4 s_staged[FWD_TILES][2][FWD_BATCH / 2][RECORDS];   // [tile][buffer][pair]
   __shared__ uint32_t s_last[FWD_WARPS], s_odd[FWD_WARPS][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = warp & 1;
-  const int tile = blockIdx.x * FWD_TILES + (warp >> 1);
-  if (tile >= n_tiles) return;
+  const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
+  const int blocks = (int)gridDim.x - (LISTED ? fill_blocks : 0);
+  if (LISTED && (int)blockIdx.x >= blocks) {
+    if (CKPT == PER_SEGMENT && first && (int)blockIdx.x == blocks && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
+    visit_unlisted<DEPTH>(blockIdx.x - blocks, fill_blocks, tile_ranges, n_tiles, tiles_x, W, H, bg, first, out_rgba, out_feat, out_depth, last_idx);
+    return;
+  }
+  const TileList tiles = LISTED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
+  for (uint32_t w = blockIdx.x * FWD_TILES + (warp >> 1); w < tiles.count; w += blocks * FWD_TILES) {   // (once, unless LISTED)
+  const int tile = tiles.at(w);
   const int tx = tile % tiles_x, ty = tile / tiles_x, in_tile = half * 32 + lane;   // the lane's pixel in its tile
   const int px = tx * RT_W + (in_tile & 7), py = ty * RT_W + (in_tile >> 3), pix = py * W + px;
   const bool inside = px < W && py < H;
   const float2 pcx = make_float2((float)px + 0.5f, (float)px + 0.5f), pcy = make_float2((float)py + 0.5f, (float)py + 0.5f);
   const uint2 range = tile_ranges[tile];
-  const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
-  if (CKPT == PER_SEGMENT && first && tile == 0 && in_tile == 0) bwd_work[BWD_SUMMED] = 0u;
-  if (CHUNKED && !first && range.y <= range.x && !(final && FEAT)) {   // nothing of this chunk lands here: pixels, state and flag stay
+  if (CKPT == PER_SEGMENT && !LISTED && first && w == 0u && in_tile == 0) bwd_work[BWD_SUMMED] = 0u;
+  if (CHUNKED && !LISTED && !first && range.y <= range.x && !(final && FEAT)) {   // nothing of this chunk lands here: pixels, state and flag stay
     if (DEPTH && final && inside) out_depth[pix] = finished_depth(out_depth[pix], out_feat[pix].w);
     return;
   }
@@ -282,7 +328,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
       if constexpr (BWD) last_idx[pix] = P.last;
     }
   }
-  if constexpr (!BWD && !CHUNKED) return;
+  if constexpr (BWD || CHUNKED) {
   // What the tile's two warps settle together: whether any pixel is still open, and the last fragment any pixel used.
   const uint32_t mine = __reduce_max_sync(0xffffffffu, P.last);
   if (lane == 0) s_last[warp] = mine;
@@ -306,12 +352,14 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
       }
     }
   }
+  }
+  if (!LISTED) return;
+  }
 }
 
-// Eight warps to a tile, for whole views of so few tiles that all are in flight together (TEAM_PER_SM blocks fit an SM), where the GPU is
-// idle but for the lists' own length: four warps find the alphas of
-// a batch, two warps (a pixel per lane) carry the transmittances and the sums, two warps take turns to gather and stage the records of
-// the batches ahead. A batch passes from one to the next with one barrier of the block.
+// Eight warps to a tile, for views of so few tiles (TEAM_PER_SM to an SM) that the GPU is idle but for the lists' own length: four warps
+// find the alphas of a batch, two warps (a pixel per lane) carry the transmittances and the sums, two warps take turns to gather and stage
+// the records of the batches ahead. A batch passes from one to the next with one barrier of the block.
 constexpr int TEAM_BATCH = FWD_SEG, TEAM_PAIRS = TEAM_BATCH / 2, TEAM_PRODUCERS = 4, TEAM_THREADS = (2 + TEAM_PRODUCERS + 2) * 32, TEAM_PER_SM = 8;
 
 template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
@@ -460,7 +508,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
     const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work,
-    const uint32_t* __restrict__ words, const uint32_t* __restrict__ list) {
+    const uint32_t* __restrict__ words, const uint32_t* __restrict__ list, int fill_blocks) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   // FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
@@ -468,8 +516,15 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   static_assert(!(FEAT && BWD), "the chunked backward reads the colour sums from out_feat.xyz");
   __shared__ float4 s_staged[FWD_WARPS][FWD_SEG][FEAT ? 6 : 5];   // a fragment's constants, most of them twice, as operands of packed arithmetic
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool first = chunk == 0, final = chunk == n_chunks - 1;
+  const int blocks = (int)gridDim.x - (LISTED ? fill_blocks : 0);
+  if (LISTED && (int)blockIdx.x >= blocks) {
+    if (CKPT == PER_SEGMENT && first && (int)blockIdx.x == blocks && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
+    visit_unlisted<DEPTH>(blockIdx.x - blocks, fill_blocks, tile_ranges, n_tiles, tiles_x, W, H, bg, first, out_rgba, out_feat, out_depth, last_idx);
+    return;
+  }
   const TileList tiles = LISTED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
-  for (uint32_t w = blockIdx.x * FWD_WARPS + warp; w < tiles.count; w += gridDim.x * FWD_WARPS) {   // (once, unless LISTED)
+  for (uint32_t w = blockIdx.x * FWD_WARPS + warp; w < tiles.count; w += blocks * FWD_WARPS) {   // (once, unless LISTED)
   const int tile = tiles.at(w);
   float2 f0 = splat2(0.f), f1 = f0, f2 = f0;   // composited feature lanes (raster_fwd.cu:52)
   const int tx = tile % tiles_x, ty = tile / tiles_x;
@@ -477,8 +532,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
   const bool in0 = px0 < W && py < H, in1 = px0 + 1 < W && py < H;
   const float2 pcx = make_float2((float)px0 + 0.5f, (float)px0 + 1.5f), pcy = splat2((float)py + 0.5f);
   const uint2 range = tile_ranges[tile];
-  const bool first = chunk == 0, final = chunk == n_chunks - 1;
-  if (CKPT == PER_SEGMENT && first && tile == 0 && lane == 0) bwd_work[BWD_SUMMED] = 0u;
+  if (CKPT == PER_SEGMENT && !LISTED && first && w == 0u && lane == 0) bwd_work[BWD_SUMMED] = 0u;
   if (!LISTED && !first && range.y <= range.x && !(final && FEAT)) {   // nothing of this chunk lands here: pixels, state and flag stay
     if (DEPTH && final) {
 #pragma unroll
@@ -678,23 +732,28 @@ using namespace b2k;
 
 namespace b2k {
 // One chunk of a chunked view (n_chunks > 1), or the whole view (n_chunks <= 1).
-int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_chunks, unsigned long long* alive, cudaStream_t s) {
+int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_chunks, unsigned long long* alive, const uint32_t* tiles, cudaStream_t s) {
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
   uint2* ranges = (uint2*)c->tile_ranges + (n_chunks > 1 ? (size_t)chunk * c->n_tiles : 0);
   const bool chunked = n_chunks > 1, halves = n_chunks <= 2;   // (measured above)
   // Behind the first chunk only the tiles with a list are visited, but for the last one where it finishes depths or features.
-  const int bins = div_up(c->tiles_x, 8) * div_up(c->tiles_y, 8);
-  const uint32_t* list = chunked && chunk > 0 && !(chunk == n_chunks - 1 && (c->out_depth || o->feat_mode != 0)) ? (const uint32_t*)(alive + bins) : nullptr;
+  // Only the tiles with a list are composited; the others are filled by the first chunk, and by the last one finished where depths are
+  // wanted. Features travel by way of every pixel, and so do depths in a forward for a backward.
+  const bool depths = chunk == n_chunks - 1 && c->out_depth;
+  const uint32_t* list = chunked && o->feat_mode == 0 && !(depths && o->bwd_info) ? tiles : nullptr;
+  const int fill_blocks = list && (chunk == 0 || depths) ? min(div_up(c->n_tiles, 32 * FWD_WARPS), 8 * sm_count()) : 0, most = 24 * sm_count();   // (a few times what is resident: tiles differ)
 #define ARGS s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, \
     (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, \
     seg_shift_of(short_segments(c)), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr, bwd_work_ptr(c)
-#define HALF(B, D, C, F) launch_next(raster_fwd_half_kernel<B, D, C, F>, div_up(c->n_tiles, FWD_TILES), FWD_WARPS * 32, 0, ARGS)
+#define HALF(B, D, C, F, LISTED) launch_next(raster_fwd_half_kernel<B, D, C, F, LISTED>, (LISTED ? min(div_up(c->n_tiles, FWD_TILES), most) : div_up(c->n_tiles, FWD_TILES)) + fill_blocks, FWD_WARPS * 32, 0, ARGS, \
+    c->chunk_words, list, fill_blocks)
 #define TEAM(B, D, C, F) launch_next(raster_fwd_team_kernel<B, D, C, F>, C ? min(c->n_tiles, TEAM_PER_SM * sm_count()) : c->n_tiles, TEAM_THREADS, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, \
     (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, \
     (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c), c->chunk_words, list)
-#define WARP(B, D, F) do { if (list) launch_next(raster_fwd_kernel<B, D, F, true>, min(div_up(c->n_tiles, FWD_WARPS), 24 * sm_count()), FWD_WARPS * 32, 0, ARGS, c->chunk_words, list); \
-    else launch_next(raster_fwd_kernel<B, D, F, false>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS, c->chunk_words, list); } while (0)
-#define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_PER_SM * sm_count()) TEAM(B, D, false, F); else HALF(B, D, false, F); } else if (halves && list) TEAM(B, false, true, false); else if (halves) HALF(B, D, true, (F) && (B) == NONE); \
+#define WARP(B, D, F) do { if (list) launch_next(raster_fwd_kernel<B, D, false, true>, min(div_up(c->n_tiles, FWD_WARPS), most) + fill_blocks, FWD_WARPS * 32, 0, ARGS, c->chunk_words, list, fill_blocks); \
+    else launch_next(raster_fwd_kernel<B, D, F, false>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS, c->chunk_words, list, 0); } while (0)
+#define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_PER_SM * sm_count()) TEAM(B, D, false, F); else HALF(B, D, false, F, false); } else if (halves && list && chunk > 0 && !c->out_depth) TEAM(B, false, true, false); \
+    else if (halves && list) HALF(B, D, true, false, true); else if (halves) HALF(B, D, true, (F) && (B) == NONE, false); \
     else WARP(B, D, (F) && (B) == NONE); } while (0)
 #define LD(B, D) do { if (o->feat_mode != 0) L(B, D, true); else L(B, D, false); } while (0)   // a chunked view with features is forward only (checked by the caller)
 #define LB(B) do { if (c->out_depth) LD(B, true); else LD(B, false); } while (0)
@@ -718,5 +777,5 @@ extern "C" int b2k_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, b2k_strea
   B2K_REQUIRE(c->W > 0 && c->H > 0 && c->n_tiles == c->tiles_x * c->tiles_y);
   if (o->bwd_info && c->bwd_scratch_bytes < b2k_bwd_scratch_bytes(c->W, c->H, c->n_chunks, c->isect_cap)) return B2K_ERR_CAPACITY;
   B2K_REQUIRE(o->feat_mode >= 0 && o->feat_mode <= 2 && (o->feat_mode == 0 || c->proj3));
-  return launch_raster_fwd(c, o, 0, 1, nullptr, (cudaStream_t)stream);
+  return launch_raster_fwd(c, o, 0, 1, nullptr, nullptr, (cudaStream_t)stream);
 }

@@ -506,7 +506,6 @@ def test_accumulator_rows_are_the_gradients(degree, active, n):
     assert bool(got[0].any()) and torch.equal(got[0], got[1])
 
 
-
 @pytest.mark.parametrize("kind", ["uniform", "wide", "same", "culled", "any_bits"])
 @pytest.mark.parametrize("n", [8191, 16384, 16385, 24577, 32768, 32769])
 def test_depth_sort_in_one_cluster(n, kind):
@@ -514,8 +513,7 @@ def test_depth_sort_in_one_cluster(n, kind):
     test_depth_sort_is_stable_at_every_size(n, kind)
 
 
-
-@pytest.mark.parametrize("W,H", [(64, 64), (528, 520)])   # segments of 32 and of 128 fragments
+@pytest.mark.parametrize("W,H", [(64, 64), (528, 520), (1361, 900)])   # segments of 32 and of 128 fragments; tiles listed from the first chunk on
 @pytest.mark.parametrize("chunks", [2, 3, 5])
 @pytest.mark.parametrize("n", [1, 3, 40])
 def test_chunks_without_fragments(n, chunks, W, H):
@@ -537,3 +535,29 @@ def test_chunks_without_fragments(n, chunks, W, H):
             h.api.rasterize_backward(c, h.model, h.rp)
         assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
         assert torch.equal(ctx.vis_flag[:n], h.ctx.vis_flag[:n]) and rel_l2(ctx.v_splat[:n].cpu().numpy(), h.ctx.v_splat[:n].cpu().numpy()) <= 2e-5
+
+
+@pytest.mark.parametrize("bwd_info", [False, True])
+@pytest.mark.parametrize("W,H", [(333, 217), (1361, 900)])
+def test_depths_of_chunks(W, H, bwd_info):
+    """Depths finished by the compositing, by the blocks that visit tiles without fragments in the last chunk, and in a whole view."""
+    import torch
+    from b2ctrain_b200 import api
+    n = 3000
+    scene = scenes.make_splats(n, 1, 8, log_scale=(-3.0, 0.8))
+    cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 30.0, 10.0), W, H, float(H))
+    m = api.Model("cuda:0").upload(scenes.floor_for_cameras(scene, [cam]))
+    rp = api.RenderParams(cam, bg=(0.2, 0.1, 0.3), sh_degree=1, bwd_info=bwd_info)
+    got = []
+    for chunks in (1, 2, 3, 5):
+        ctx = api.RenderCtx("cuda:0")
+        ctx.want_depth = True
+        ctx.setup(W, H, m.cap, n_chunks=chunks)
+        for _ in range(2):
+            ctx.out_rgba.fill_(7.0); ctx.out_depth.fill_(7.0)
+            api.render_forward(ctx, m, rp)
+        got.append((ctx.out_rgba.clone(), ctx.out_depth.clone(), ctx.out_feat[:, 3].clone()))
+    assert bool(torch.isfinite(got[0][1]).any()) and bool(torch.isinf(got[0][1]).any())
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert torch.equal(a, b)
