@@ -33,10 +33,14 @@ namespace {
 
 constexpr int PROJ_BLOCK = 256;
 
-// Tile boxes of at most MASK_TILES tiles are remembered as a bit mask of the tiles hit. The tests of boxes of at most WARP_TILES tiles
-// are shared out over the splats' warp; larger ones are counted by a kernel of their own, a warp to each, so that no warp waits for a few of
-// them.
-constexpr int MASK_TILES = 64, WARP_TILES = 1024;
+// Tile boxes of at most MASK_TILES tiles are remembered as a bit mask of the tiles hit. The tests of boxes of at most warp_tiles() tiles are
+// shared out over the splats' warp; larger ones are counted by a kernel of their own, a warp to each. Few splats are few warps,
+// which wait for the one with the most tests: project_kernel and count_big_kernel at 1445x965 over 24k splats together 46 us with boxes of
+// up to 1,024 tiles in the warp, 41 up to 256, 31 up to 64; small images have few large boxes (333x217 over 20k: 13.5 us up to 128 and above,
+// 14.5 up to 64). Many splats fill the GPU, and the large boxes' kernel is then the more costly one: 1001x751 over 200k 46 us up to 1,024, 45 up
+// to 512, 47 up to 256, 54 up to 64; where a tenth are wide (801x603 over 90k) 114, 99, 95, 93.
+constexpr int MASK_TILES = 64;
+__device__ __forceinline__ int warp_tiles(int n, int n_tiles) { return n > 49152 ? 512 : n_tiles > 4096 ? MASK_TILES : 128; }
 
 // The tile tests of a warp's 32 splats, shared out in units of up to eight tiles of one row: boxes hold one to a thousand tiles, and with
 // a splat per lane most lanes wait for the largest.
@@ -86,9 +90,9 @@ __device__ __forceinline__ uint32_t shared_hits(TileShare& ts, const TileRec& re
 // What a splat's record says about its tiles: tiles hit, the words of hit_info, whether it goes to the list of large boxes. All lanes of
 // the warp call this; `drawn`: the splat has a record and its box is on the image.
 struct TileHits { uint32_t hits, w0, w1, box, height; bool big; };
-__device__ __forceinline__ TileHits decide_tiles(TileShare& ts, const TileRec& rec, const TileBox& b, bool drawn) {
+__device__ __forceinline__ TileHits decide_tiles(TileShare& ts, const TileRec& rec, const TileBox& b, bool drawn, int limit) {
   const int bw = drawn ? b.max_x - b.min_x : 0, bh = drawn ? b.max_y - b.min_y : 0, area = bw > 0 && bh > 0 ? bw * bh : 0;
-  TileHits t{0u, 0u, 0u, 0u, drawn ? (uint32_t)bh : 0u, area > WARP_TILES};
+  TileHits t{0u, 0u, 0u, 0u, drawn ? (uint32_t)bh : 0u, area > limit};
   t.hits = shared_hits(ts, rec, b, t.big ? 0 : area, t.w0, t.w1);
   if (area > MASK_TILES) {   // no mask: the box itself
     t.box = 0xFFFFFFFFu;
@@ -162,7 +166,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
       proj1[i] = make_float4(0.f, 0.f, 0.f, -1.f);   // no record
     }
   }
-  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn);
+  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn, warp_tiles(n, tiles_x * tiles_y));
   if (!valid) return;
   if (drawn && max_screen) {
     const float detc = pr.c00 * pr.c11 - pr.c01 * pr.c01;
@@ -247,7 +251,8 @@ __global__ void __launch_bounds__(PROJ_BLOCK, 4) project_lite_kernel(
   depth_keys[i] = area ? __float_as_uint(pr.mean_c.z) : 0xFFFFFFFFu;
 }
 
-// Boxes above WARP_TILES: a warp to each, its lanes sweep the box 32 tiles at a time. Warp w looks at every (number of warps)-th pair of
+// Boxes above warp_tiles: a warp to each, whose lanes take units of up to eight tiles of a row (562x569 over 4,303 wide splats: a tile
+// a lane, which divides for each, 33.7 us, units 19.9). Warp w looks at every (number of warps)-th pair of
 // splats from the w-th on (a pair is a sector of hit_info), so that large splats that follow each other go to different warps. (They used to
 // go to a list, whose counter took a launch of its own to clear: 64x64 over 2k splats 80.2 -> 78.9 us a step.)
 __global__ void __launch_bounds__(256) count_big_kernel(int n, const uint4* __restrict__ hit_info, const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H,
@@ -258,7 +263,7 @@ __global__ void __launch_bounds__(256) count_big_kernel(int n, const uint4* __re
     auto splat_of = [&](int l) { return 2 * (p0 + (long long)(l >> 1) * warps) + (l & 1); };
     const long long mine = splat_of(lane);
     const uint4 hi = mine < n ? hit_info[mine] : make_uint4(0u, 0u, 0u, 0u);
-    const bool big = hi.z == 0xFFFFFFFFu && (hi.y & 0xFFFFu) * (hi.y >> 16) > (uint32_t)WARP_TILES;
+    const bool big = hi.z == 0xFFFFFFFFu && (hi.y & 0xFFFFu) * (hi.y >> 16) > (uint32_t)warp_tiles(n, tiles_x * tiles_y);
     for (uint32_t todo = __ballot_sync(0xffffffffu, big); todo; todo &= todo - 1u) {
       const long long i = splat_of(__ffs(todo) - 1);
       const float4 a = proj0[i], b = proj1[i];
@@ -266,13 +271,16 @@ __global__ void __launch_bounds__(256) count_big_kernel(int n, const uint4* __re
       TileBox bb;
       uint32_t hits = 0;
       if (tile_box(rec, W, H, tiles_x, tiles_y, bb)) {
-        const int bw = bb.max_x - bb.min_x, area = bw * (bb.max_y - bb.min_y);
-        for (int t0 = 0; t0 < area; t0 += 32) {
-          const int t = t0 + lane;
-          const bool hit = t < area && tile_hit(bb.min_x + t % bw, bb.min_y + t / bw, rec);
-          hits += __popc(__ballot_sync(0xffffffffu, hit));
+        // units of up to eight tiles of one row, as in shared_hits
+        const int bw = bb.max_x - bb.min_x, per_row = (bw + 7) >> 3, units = (bb.max_y - bb.min_y) * per_row;
+        for (int u = lane; u < units; u += 32) {
+          const int y = u / per_row, x0 = (u - y * per_row) * 8;
+          const TileRow row = tile_row(bb.min_y + y, rec);
+#pragma unroll
+          for (int k = 0; k < 8; k++) hits += x0 + k < bw && tile_hit(bb.min_x + x0 + k, row, rec) ? 1u : 0u;
         }
       }
+      hits = __reduce_add_sync(0xffffffffu, hits);
       if (lane == 0) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
     }
   }
@@ -296,7 +304,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
     rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
     drawn = tile_box(rec, W, H, tiles_x, tiles_y, bb);
   }
-  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn);
+  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn, warp_tiles(n, tiles_x * tiles_y));
   if (!valid) return;
   hit_info[i] = make_uint4(t.w0, t.w1, t.box, t.height);
   order_in[i] = (uint32_t)i;

@@ -427,10 +427,12 @@ def test_chunks_of_wide_splats():
         assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
 
 
-def test_tile_boxes_of_every_size():
-    """The tile tests are shared out over a warp in units of eight tiles of a row: masks up to 64 tiles, counts up to 1,024, a list above."""
-    W, H, n = 1040, 720, 3001
-    scene = scenes.make_splats(n, 0, 11, log_scale=(-4.5, 1.6))
+@pytest.mark.parametrize("n,log_scale", [(3001, (-4.5, 1.6)), (49153, (-6.0, 1.0))])
+def test_tile_boxes_of_every_size(n, log_scale):
+    """The tile tests are shared out over a warp in units of eight tiles of a row: masks up to 64 tiles, counts of larger boxes there or by a
+    warp to each."""
+    W, H = 1040, 720
+    scene = scenes.make_splats(n, 0, 11, log_scale=log_scale)
     cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 25.0, 10.0), W, H, float(max(W, H)))
     scene = scenes.floor_for_cameras(scene, [cam])
     h = Harness(scene, cam, isect_cap=1 << 23)
@@ -439,7 +441,7 @@ def test_tile_boxes_of_every_size():
     info = h.u32(h.ctx.hit_info[:n]).reshape(-1, 4)
     large = info[:, 2] == 0xFFFFFFFF
     area = np.where(large, (info[:, 1] & 0xFFFF) * (info[:, 1] >> 16), (info[:, 2] >> 24) * info[:, 3])
-    assert (area[~large] == 64).any() and (area == 1).any() and ((area > 64) & (area <= 1024)).any() and (area > 1024).any()
+    assert (area[~large] == 64).any() and (area == 1).any() and ((area > 64) & (area <= 512)).any() and (area > 512).any()
     masks = np.array([bin(int(a)).count("1") + bin(int(b)).count("1") for a, b in info[:, :2]])
     for project in (False, True):
         assert np.array_equal(h.u32(h.ctx.tile_count, n), tc_o)
