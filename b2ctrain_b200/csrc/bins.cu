@@ -19,7 +19,7 @@
 // compositing kernel clears their bits in one 64-bit word per bin.
 //
 // Bound by instruction issue (ellipse tests, bit work) and by launch latency in small views. Against emission of expanded
-// pairs and two radix passes over them, sum of the stage's kernels per view: 4K, 6M splats, 37.5M hits 2,660 -> 960 us;
+// pairs and two radix passes over them, sum of the stage's kernels per view: 4K, 6M splats, 37.5M hits 2,660 -> 870 us;
 // 1080p, 500k splats, 4.4M hits 330 -> 150; 1024x1024, 1M splats of which a tenth cover hundreds of tiles 1,350 -> 390.
 // Inside that, the tests of a warp's 32 pairs shared out by tile row (not a pair per lane): 455 -> 286 us at 4K.
 #include "bins.cuh"

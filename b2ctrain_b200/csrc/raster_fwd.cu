@@ -9,8 +9,8 @@
 // Transmittances are multiplied up for a group of fragments first, and fragments are compared and selected one by one only where a
 // pixel of the warp closes inside the group (none_closes): 1024x1024 over 1M in four chunks 184 -> 172 us, 4K over 6M in five 681 -> 652.
 // Three kernels with the same arithmetic, bit for bit:
-//   raster_fwd_team_kernel  eight warps to a tile: some find alphas, two composite, two gather. For whole views of so few tiles that all
-//                           are in flight at once, whose time is that of the longest list.
+//   raster_fwd_team_kernel  eight warps to a tile: some find alphas, two composite, two gather. For whole views of few tiles and for the
+//                           few live tiles of the second of two chunks, whose time is that of the longest list.
 //   raster_fwd_half_kernel  two warps to a tile, a lane one pixel, two consecutive fragments to a packed operation: the chain of
 //                           one list is half as long. For whole views and two chunks, where a visit to a tile is a long list.
 //   raster_fwd_kernel       one warp to a tile, a lane two pixels that share packed operations: twice as many tiles in flight.
@@ -19,8 +19,8 @@
 // features 85 / 69 / 54, 1237x822 in two chunks 117 / 92 / 76, 1920x1080 in two 143 / 123 / 118; 1024x1024 over 1M in four
 // 231 / 187 / 206, 4K over 6M with depth in five 847 / 740 / 953, sixteen views of 3M in four on eight streams 20.6 / 21.6 ms.
 // Two warps / the team, us: 64x64 over 2k splats 21.3 / 15.1, 200x150 over 1k 11.7 / 9.9, 333x217 over 1k 11.8 / 10.0, over 20k 24.7 /
-// 18.7, over 150k 78 / 50 (1,176 tiles, a block each); 400x300 over 4k 12.9 / 16.1, over 40k 25.3 / 26.3 (1,900 tiles, the second
-// thousand waits), 512x512 over 10k 17.8 / 31.7, 1280x720 over 100k 40.7 / 70.7.
+// 18.7, over 150k 78 / 50 (1,176 tiles, a block each); 400x300 over 4k 12.9 / 16.1, over 40k 25.3 / 26.3 (1,900 tiles),
+// 512x512 over 10k 17.8 / 31.7, 1280x720 over 100k 40.7 / 70.7.
 #include "common.cuh"
 
 namespace b2k {
@@ -736,7 +736,6 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
   uint2* ranges = (uint2*)c->tile_ranges + (n_chunks > 1 ? (size_t)chunk * c->n_tiles : 0);
   const bool chunked = n_chunks > 1, halves = n_chunks <= 2;   // (measured above)
-  // Behind the first chunk only the tiles with a list are visited, but for the last one where it finishes depths or features.
   // Only the tiles with a list are composited; the others are filled by the first chunk, and by the last one finished where depths are
   // wanted. Features travel by way of every pixel, and so do depths in a forward for a backward.
   const bool depths = chunk == n_chunks - 1 && c->out_depth;
