@@ -56,8 +56,15 @@ constexpr uint32_t DONE_BIT = 0x80000000u;
 
 // A pixel carries its transmittance while it is open and zero once it has closed (the last value then waits in a variable of its own).
 // So a group of fragments multiplies up the transmittances first, one operation a fragment, and only if some pixel of the warp closes
-// inside the group (the product passes the cut-off: it never rises again) are fragments compared and selected one by one. Whether none does:
-__device__ __forceinline__ bool none_closes(float behind_group) { return __float_as_uint(behind_group) - 1u >= __float_as_uint(T_CUTOFF); }   // zero, or above the cut-off
+// inside the group (the product passes the cut-off: it never rises again) are fragments compared and selected one by one. Whether none does,
+// from the transmittances before and behind a group of N: what an open pixel has left behind eight fragments is at least 1e-4 * (1 - 0.999)^8, far from
+// zero, so that zero says "closed before". Behind sixteen fragments at the clamp it is below the smallest float, and the pixel itself is asked
+// (the team: 64x64 over 2k splats 15.0 us with either test, 333x217 over 20k 18.8 and 18.7).
+template <int N>
+__device__ __forceinline__ bool none_closes(float before, float behind) {
+  if constexpr (N <= 8) return __float_as_uint(behind) - 1u >= __float_as_uint(T_CUTOFF);   // zero, or above the cut-off
+  else return before == 0.f || behind > T_CUTOFF;
+}
 
 // Two fragments that follow each other in a list, the nearer in the first of each pair of lanes.
 constexpr int STAGED = 5;   // (-x, -y), (c00 / 2, c01), (c11 / 2, opacity), (power, r), (g, b); then (z, feature 0), (feature 1, 2)
@@ -128,7 +135,7 @@ struct Pixel {
       through[u] = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[u].x, -alpha[u].y));
       vis[u].x = alpha[u].x * ahead; ahead *= through[u].x; vis[u].y = alpha[u].y * ahead; ahead *= through[u].y;
     }
-    if (__all_sync(0xffffffffu, none_closes(ahead))) T = ahead;
+    if (__all_sync(0xffffffffu, none_closes<2 * PAIRS>(T, ahead))) T = ahead;
     else {
 #pragma unroll
       for (int u = 0; u < PAIRS; u++) { vis[u].x = weigh(alpha[u].x, through[u].x); vis[u].y = weigh(alpha[u].y, through[u].y); }
@@ -660,7 +667,7 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_kernel(
         float2 ahead = T;
 #pragma unroll
         for (int u = 0; u < FWD_GROUP; u++) { vis[u] = __fmul2_rn(alpha[u], ahead); ahead = __fmul2_rn(ahead, through[u]); }
-        if (__all_sync(0xffffffffu, none_closes(ahead.x) && none_closes(ahead.y))) T = ahead;
+        if (__all_sync(0xffffffffu, none_closes<FWD_GROUP>(T.x, ahead.x) && none_closes<FWD_GROUP>(T.y, ahead.y))) T = ahead;
         else {
 #pragma unroll
           for (int u = 0; u < FWD_GROUP; u++) vis[u] = make_float2(weigh(0, alpha[u].x, through[u].x), weigh(1, alpha[u].y, through[u].y));

@@ -563,3 +563,53 @@ def test_depths_of_chunks(W, H, bwd_info):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("W,H", [(64, 64), (65, 41)])            # and tiles of which one column, one row is on the image
+@pytest.mark.parametrize("front", ["none", "faint", "nearly_closed"])
+@pytest.mark.parametrize("n", [15, 16, 17, 31, 32, 33, 48])
+def test_stacks_of_opaque_splats(n, front, W, H):
+    """Splats at the alpha clamp one behind the other over the whole image: the product of a group's transmittances falls below the
+    smallest float, and the pixels close at the second one all the same. Whole views of few tiles, and two and three chunks."""
+    import torch
+    from b2ctrain_b200 import api
+    logits = {"none": [], "faint": [-3.0] * 3, "nearly_closed": [-0.277] * 16}[front]     # the last: 1.2e-4 is left in front of the stack
+    scene, cam = stack_scene(len(logits) + n, W, H, seed=n)
+    scene["pos_op"][:, :2] = 0.0
+    scene["pos_op"][:, 3] = logits + [9.5] * n
+    scene["lscale"][:, :3] = 4.5                                  # alpha above the clamp of 0.999 in every pixel
+    bg = (0.2, 0.1, 0.3)
+    h = Harness(scene, cam, bg=bg, want_depth=True)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    h.api.bin_and_sort(h.ctx, h.model)
+    ranges = h.u32(h.ctx.tile_ranges).reshape(-1, 2).copy()       # before the forward cuts them behind the last fragment taken
+    h.api.rasterize_forward(h.ctx, h.rp)
+    N, taken = scene["n"], min(len(logits) + 1, 16)
+    p0, p1, p2 = (t[:N].cpu().numpy().astype(np.float64) for t in (h.ctx.proj0, h.ctx.proj1, h.ctx.proj2))
+    geo, vals = np.concatenate([p0, p1], 1), h.u32(h.ctx.vals_sorted, h.ctx.num_isect)
+    assert len(vals) == N * h.ctx.n_tiles
+    rgba, T, last, _, zs = orc.raster_fwd(W, H, geo, p2[:, :3], vals, ranges, np.array(bg), want_depth=True)
+    assert np.all(last - ranges[:, 0][(np.arange(H) // 8)[:, None] * h.ctx.tiles_x + np.arange(W) // 8].reshape(-1) == taken)
+    # In fp32 the clamp lets 1 - 0.999f through, 4.7e-5 more than 0.001: half of that, 4.7e-8, is seen in an image of order one.
+    assert rel_l2(h.ctx.out_rgba.cpu().numpy(), rgba) <= 1e-6 and np.array_equal(h.u32(h.ctx.last_idx), last)
+    assert rel_l2(h.ctx.out_feat[:, 3].cpu().numpy(), T) <= 1e-4 and rel_l2(h.ctx.out_depth.cpu().numpy(), zs / (1.0 - T)) <= 1e-6
+    v_out = (np.random.Generator(np.random.PCG64(9)).standard_normal((W * H, 4)) * 1e-3).astype(np.float32)
+    h.ctx.v_out.copy_(torch.from_numpy(v_out))
+    h.api.rasterize_backward(h.ctx, h.model, h.rp)
+    want, vis, _ = orc.raster_bwd(N, W, H, geo, p2[:, :3], vals, ranges, np.array(bg), h.ctx.out_rgba.cpu().numpy(), h.ctx.out_feat.cpu().numpy()[:, 3], last, v_out)
+    assert np.array_equal(h.u32(h.ctx.vis_flag, N) != 0, vis != 0) and vis.sum() == taken
+    assert rel_l2(h.ctx.v_splat[:N, 5:8].cpu().numpy(), want[:, 5:8]) <= 1e-4           # colours: weights alone (again 4.7e-5)
+    got = []
+    for chunks in (1, 2, 3):
+        ctx = api.RenderCtx("cuda:0")
+        ctx.want_depth = True
+        ctx.setup(W, H, h.model.cap, n_chunks=chunks)
+        rp = api.RenderParams(cam, bg=bg, sh_degree=1, bwd_info=False)
+        api.render_forward(ctx, h.model, rp)
+        plain = [ctx.out_rgba.clone(), ctx.out_feat[:, 3].clone(), ctx.out_depth.clone()]
+        rp.feat = "Normals"
+        api.render_forward(ctx, h.model, rp)
+        got.append(plain + [ctx.out_rgba.clone(), ctx.out_feat.clone(), ctx.out_depth.clone()])
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert torch.equal(a, b)
