@@ -10,7 +10,7 @@
 // pixel of the warp closes inside the group (none_closes): 1024x1024 over 1M in four chunks 184 -> 172 us, 4K over 6M in five 681 -> 652.
 // Three kernels with the same arithmetic, bit for bit:
 //   raster_fwd_team_kernel  eight warps to a tile: some find alphas, two composite, two gather. For whole views of few tiles and for the
-//                           few live tiles of the second of two chunks, whose time is that of the longest list.
+//                           second of two chunks where few tiles are alive: the time is that of the longest list.
 //   raster_fwd_half_kernel  two warps to a tile, a lane one pixel, two consecutive fragments to a packed operation: the chain of
 //                           one list is half as long. For whole views and two chunks, where a visit to a tile is a long list.
 //   raster_fwd_kernel       one warp to a tile, a lane two pixels that share packed operations: twice as many tiles in flight.
@@ -210,31 +210,19 @@ __device__ __forceinline__ void visit_unlisted(int block, int blocks, const uint
   }
 }
 
-template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT, bool LISTED>
-__global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
+// Two warps to a tile, for a block of TILES pairs of warps: the pair of this thread takes every `step`-th tile from `begin` on.
+template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT, bool LISTED, int TILES, int RECORDS>
+__device__ __forceinline__ void composite_halves(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
     const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work,
-    const uint32_t* __restrict__ words, const uint32_t* __restrict__ list, int fill_blocks) {
-  after_previous();
+    const TileList& tiles, uint32_t begin, uint32_t step,
+    float4 (&s_staged)[TILES][2][FWD_BATCH / 2][RECORDS], uint32_t (&s_last)[TILES * 2], uint32_t (&s_odd)[TILES * 2][2]) {
   constexpr bool BWD = CKPT != NONE;
-  // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
-  // pixel travel in feat_acc and move into out_feat.xyz when the last chunk, which then visits every pixel, is done.
-  static_assert(!(FEAT && CHUNKED && BWD), "the chunked backward reads the colour sums from out_feat.xyz");
-  constexpr int RECORDS = FEAT ? STAGED + 2 : DEPTH ? STAGED + 1 : STAGED;
-  __shared__ float4 s_staged[FWD_TILES][2][FWD_BATCH / 2][RECORDS];   // [tile][buffer][pair]
-  __shared__ uint32_t s_last[FWD_WARPS], s_odd[FWD_WARPS][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = warp & 1;
   const bool first = !CHUNKED || chunk == 0, final = !CHUNKED || chunk == n_chunks - 1;
-  const int blocks = (int)gridDim.x - (LISTED ? fill_blocks : 0);
-  if (LISTED && (int)blockIdx.x >= blocks) {
-    if (CKPT == PER_SEGMENT && first && (int)blockIdx.x == blocks && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
-    visit_unlisted<DEPTH>(blockIdx.x - blocks, fill_blocks, tile_ranges, n_tiles, tiles_x, W, H, bg, first, out_rgba, out_feat, out_depth, last_idx);
-    return;
-  }
-  const TileList tiles = LISTED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
-  for (uint32_t w = blockIdx.x * FWD_TILES + (warp >> 1); w < tiles.count; w += blocks * FWD_TILES) {   // (once, unless LISTED)
+  for (uint32_t w = begin; w < tiles.count; w += step) {   // (once, unless LISTED)
   const int tile = tiles.at(w);
   const int tx = tile % tiles_x, ty = tile / tiles_x, in_tile = half * 32 + lane;   // the lane's pixel in its tile
   const int px = tx * RT_W + (in_tile & 7), py = ty * RT_W + (in_tile >> 3), pix = py * W + px;
@@ -364,17 +352,50 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
   }
 }
 
+template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT, bool LISTED>
+__global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
+    uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
+    const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
+    float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, float4* __restrict__ feat_acc, uint32_t* __restrict__ bwd_work,
+    const uint32_t* __restrict__ words, const uint32_t* __restrict__ list, int fill_blocks) {
+  after_previous();
+  // CHUNKED with FEAT (forward only): between chunks out_feat.xyz carries the colour sums, so the feature sums of a
+  // pixel travel in feat_acc and move into out_feat.xyz when the last chunk, which then visits every pixel, is done.
+  static_assert(!(FEAT && CHUNKED && CKPT != NONE), "the chunked backward reads the colour sums from out_feat.xyz");
+  constexpr int RECORDS = FEAT ? STAGED + 2 : DEPTH ? STAGED + 1 : STAGED;
+  __shared__ float4 s_staged[FWD_TILES][2][FWD_BATCH / 2][RECORDS];   // [tile][buffer][pair]
+  __shared__ uint32_t s_last[FWD_WARPS], s_odd[FWD_WARPS][2];
+  const bool first = !CHUNKED || chunk == 0;
+  const int blocks = (int)gridDim.x - (LISTED ? fill_blocks : 0);
+  if (LISTED && (int)blockIdx.x >= blocks) {
+    if (CKPT == PER_SEGMENT && first && (int)blockIdx.x == blocks && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
+    visit_unlisted<DEPTH>(blockIdx.x - blocks, fill_blocks, tile_ranges, n_tiles, tiles_x, W, H, bg, first, out_rgba, out_feat, out_depth, last_idx);
+    return;
+  }
+  const TileList tiles = LISTED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
+  composite_halves<CKPT, DEPTH, CHUNKED, FEAT, LISTED>(
+      tile_ranges, vals_sorted, proj0, proj1, proj2, W, H, tiles_x, n_tiles, bg, out_rgba, out_feat, out_depth, last_idx, chunk, n_chunks, alive, proj3, ckpt,
+      seg_shift, feat_acc, bwd_work, tiles, blockIdx.x * FWD_TILES + (threadIdx.x >> 6), blocks * FWD_TILES, s_staged, s_last, s_odd);
+}
+
 // Eight warps to a tile, for views of so few tiles (TEAM_PER_SM to an SM) that the GPU is idle but for the lists' own length: four warps
 // find the alphas of a batch, two warps (a pixel per lane) carry the transmittances and the sums, two warps take turns to gather and stage
 // the records of the batches ahead. A batch passes from one to the next with one barrier of the block.
 constexpr int TEAM_BATCH = FWD_SEG, TEAM_PAIRS = TEAM_BATCH / 2, TEAM_PRODUCERS = 4, TEAM_THREADS = (2 + TEAM_PRODUCERS + 2) * 32, TEAM_PER_SM = 8;
+// In the second of two chunks the device knows how many tiles have a list: the team takes up to CHUNK_TEAM_PER_SM to an SM, and above that
+// the same blocks take four tiles each at two warps. Visit, us, as two warps to a tile / the team (listed tiles, mean list; n = 300k to 500k): 821 of 190
+// 27.7 / 21.0, 1,047 of 112 21.5 / 17.1, 1,216 of 942 53.6 / 51.3, 1,256 of 605 31.6 / 32.5, 1,370 of 173 29.7 / 25.6, 1,407 of 872 55.7 / 55.8, 1,430 of 437
+// 24.9 / 27.9, 1,544 of 154 28.6 / 27.0, 1,662 of 53 15.9 / 18.5, 1,697 of 715 113 / 123, 4,544 of 458 155 / 193, 19,035 of 282 369 / 488, 24,983 of
+// 168 289 / 416 (faint splats leave nearly every tile alive). CHUNK_BLOCKS of them fit on an SM.
+constexpr int CHUNK_TEAM_PER_SM = 10, CHUNK_BLOCKS = 3, CHUNK_TILES = TEAM_THREADS / 64;
 
 template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
-__global__ void __launch_bounds__(TEAM_THREADS, CHUNKED ? 4 : 2) raster_fwd_team_kernel(
+__global__ void __launch_bounds__(TEAM_THREADS, CHUNKED ? CHUNK_BLOCKS : 2) raster_fwd_team_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
-    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, uint32_t* __restrict__ bwd_work, const uint32_t* __restrict__ words, const uint32_t* __restrict__ list) {
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, uint32_t* __restrict__ bwd_work, const uint32_t* __restrict__ words, const uint32_t* __restrict__ list, uint32_t sms) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   constexpr int RECORDS = FEAT ? STAGED + 2 : DEPTH ? STAGED + 1 : STAGED;
@@ -387,6 +408,21 @@ __global__ void __launch_bounds__(TEAM_THREADS, CHUNKED ? 4 : 2) raster_fwd_team
   const bool composites = warp < 2, weighs = !composites && warp < 2 + TEAM_PRODUCERS, final = !CHUNKED || chunk == n_chunks - 1;
   if (CKPT == PER_SEGMENT && !CHUNKED && blockIdx.x == 0 && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
   const TileList tiles = CHUNKED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
+  if constexpr (CHUNKED) {
+    if (tiles.count > CHUNK_TEAM_PER_SM * sms) {
+      __shared__ float4 s_pairs[CHUNK_TILES][2][FWD_BATCH / 2][STAGED];
+      __shared__ uint32_t s_ends[CHUNK_TILES * 2], s_strange[CHUNK_TILES * 2][2];
+      uint32_t begin = blockIdx.x * CHUNK_TILES + (threadIdx.x >> 6), step = gridDim.x * CHUNK_TILES;
+      const uint32_t resident = min(CHUNK_BLOCKS * sms, gridDim.x);
+      if (tiles.count <= resident * CHUNK_TILES) {   // no more than fit at once: evenly over the blocks (1,475 tiles: 118 -> 108 us)
+        if (blockIdx.x >= resident) return;
+        begin = (threadIdx.x >> 6) * resident + blockIdx.x; step = resident * CHUNK_TILES;
+      }
+      composite_halves<CKPT, DEPTH, CHUNKED, FEAT, true>(tile_ranges, vals_sorted, proj0, proj1, proj2, W, H, tiles_x, n_tiles, bg, out_rgba, out_feat, out_depth, last_idx, chunk, n_chunks,
+                                                         alive, proj3, ckpt, seg_shift, nullptr, bwd_work, tiles, begin, step, s_pairs, s_ends, s_strange);
+      return;
+    }
+  }
   for (uint32_t w = blockIdx.x; w < tiles.count; w += gridDim.x) {
   if (w != blockIdx.x) __syncthreads();   // the last tile's batches have been read
   const int tile = tiles.at(w), tx = tile % tiles_x, ty = tile / tiles_x;
@@ -755,7 +791,7 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
     c->chunk_words, list, fill_blocks)
 #define TEAM(B, D, C, F) launch_next(raster_fwd_team_kernel<B, D, C, F>, C ? min(c->n_tiles, TEAM_PER_SM * sm_count()) : c->n_tiles, TEAM_THREADS, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, \
     (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, \
-    (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c), c->chunk_words, list)
+    (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c), c->chunk_words, list, (uint32_t)sm_count())
 #define WARP(B, D, F) do { if (list) launch_next(raster_fwd_kernel<B, D, false, true>, min(div_up(c->n_tiles, FWD_WARPS), most) + fill_blocks, FWD_WARPS * 32, 0, ARGS, c->chunk_words, list, fill_blocks); \
     else launch_next(raster_fwd_kernel<B, D, F, false>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS, c->chunk_words, list, 0); } while (0)
 #define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_PER_SM * sm_count()) TEAM(B, D, false, F); else HALF(B, D, false, F, false); } else if (halves && list && chunk > 0 && !c->out_depth) TEAM(B, false, true, false); \

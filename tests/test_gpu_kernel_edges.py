@@ -613,3 +613,32 @@ def test_stacks_of_opaque_splats(n, front, W, H):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert torch.equal(a, b)
+
+
+# All tiles alive behind the first of two chunks: the team's most, evenly over the blocks, as many as fit at once, in several turns; segments of 128.
+@pytest.mark.parametrize("W,H", [(37 * 8, 40 * 8), (37 * 8 - 3, 41 * 8), (42 * 8, 42 * 8 - 5), (48 * 8, 37 * 8), (48 * 8, 38 * 8), (71 * 8 - 1, 65 * 8)])
+@pytest.mark.parametrize("logit", [-5.0, -1.0])                  # no pixel closes; most close, at different fragments
+def test_second_of_two_chunks(W, H, logit):
+    import torch
+    n = 400
+    scene = scenes.make_splats(n, 1, 12, log_scale=(1.5 if logit < -4.0 else -0.3, 0.3))
+    scene["pos_op"][:, 3] = logit
+    cam = scenes.look_at_camera((0.0, 0.0, 4.0), W, H, float(max(W, H)))
+    h = Harness(scenes.floor_for_cameras(scene, [cam]), cam, bg=(0.2, 0.1, 0.3), isect_cap=1 << 22)
+    ctx = h.api.RenderCtx("cuda:0")
+    ctx.setup(W, H, h.model.cap, n_chunks=2, isect_cap=1 << 22)
+    v_out = torch.from_numpy(np.random.Generator(np.random.PCG64(4)).standard_normal((W * H, 4)).astype(np.float32))
+    h.rp.bwd_info = False
+    for c in (ctx, h.ctx):
+        h.api.render_forward(c, h.model, h.rp)
+    assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
+    words = h.u32(ctx.chunk_words, 32)
+    assert logit > -5.0 or words[22 + 1] + words[27 + 1] == ctx.n_tiles          # listed, of the second chunk
+    h.rp.bwd_info = True
+    for c in (ctx, h.ctx):
+        h.api.render_forward(c, h.model, h.rp)
+        c.v_out.copy_(v_out)
+        c.v_splat.zero_(); c.vis_flag.zero_()
+        h.api.rasterize_backward(c, h.model, h.rp)
+    assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
+    assert torch.equal(ctx.vis_flag[:n], h.ctx.vis_flag[:n]) and rel_l2(ctx.v_splat[:n].cpu().numpy(), h.ctx.v_splat[:n].cpu().numpy()) <= 2e-5
