@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(256) chunk_prepare_kernel(const uint32_t* __re
   if (i != 0) return;
   words[CW_V] = (uint32_t)lo;
   words[CW_BASE] = 0u;
+  for (int k = CW_LONGEST; k < CW_COUNT; k++) words[k] = 0u;
   for (int k = CW_LONG; k < CW_WORDS; k++) words[k] = 0u;
 }
 
@@ -70,6 +71,7 @@ extern "C" int b2k_bin_sort(const B2kCtx* c, int32_t n, b2k_stream_t stream) {
   if (n == 0) {
     B2K_CUDA(cudaMemsetAsync(c->tile_ranges, 0, sizeof(uint32_t) * 2 * (size_t)c->n_tiles, s));
     B2K_CUDA(cudaMemsetAsync(c->num_isect, 0, sizeof(uint32_t), s));
+    B2K_CUDA(cudaMemsetAsync(c->num_isect + NI_LONGEST, 0, sizeof(uint32_t), s));
     return B2K_OK;
   }
   B2K_REQUIRE(c->proj0 && c->proj1 && c->tile_count && c->hit_info && c->depth_keys && c->depth_keys_sorted && c->order_in && c->order && c->tile_off);

@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
   if (!WHOLE) load_alive(v, g, s_alive);
   if (blockIdx.x == 0 && tid == 0) {    // this band's counters; the view's with its first band
     t.st[S_DONE_ROWS] = 0u; t.st[S_DONE_TILES] = 0u;
-    if (v.first_band) { t.st[S_SLOT] = v.words ? v.words[CW_BASE + v.chunk] : 0u; if (!v.words || v.chunk == 0) t.st[S_OVER] = 0u; }
+    if (v.first_band) { t.st[S_SLOT] = v.words ? v.words[CW_BASE + v.chunk] : 0u; if (!v.words || v.chunk == 0) t.st[S_OVER] = 0u; if (!v.words) *t.longest = 0u; }
   }
   __syncthreads();
   const bool some_dead = !WHOLE && v.alive;
@@ -567,12 +567,13 @@ __global__ void __launch_bounds__(COL_GROUPS * BIN_TILES) item_columns_kernel(Ba
 __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, Tables t, uint32_t cap, uint2* __restrict__ ranges, uint32_t* __restrict__ num_isect,
                                                                uint32_t* __restrict__ list) {
   after_previous();
-  __shared__ uint32_t s_warp[32], s_slot;
+  __shared__ uint32_t s_warp[32], s_longest[32], s_slot;
   const int tid = threadIdx.x, lane = tid & 31;
   const int tile0 = g.bin_row0 * BIN_W * g.tiles_x, tiles = (min((g.bin_row0 + g.bin_rows) * BIN_W, g.tiles_y) - g.bin_row0 * BIN_W) * g.tiles_x;
   const int mine = blockIdx.x * SCAN_TILES + tid;
   const uint32_t c = mine < tiles ? ranges[tile0 + mine].x : 0u;
   if (tid == 0) s_slot = t.st[S_SLOT];
+  { const uint32_t m = __reduce_max_sync(FULL, c); if (lane == 0) s_longest[tid >> 5] = m; }
   uint32_t all = 0, before = 0;   // hits of the band, and of the blocks before this one: every warp adds them up for itself
   {
     uint32_t seg[BINS_SEGMENTS / 32];
@@ -585,6 +586,7 @@ __global__ void __launch_bounds__(SCAN_TILES) tile_scan_kernel(View v, Band g, T
   uint32_t total;
   const uint32_t in_block = block_scan(c, s_warp, total) - c, slot = s_slot, start = slot + before + in_block;
   if (mine < tiles) ranges[tile0 + mine] = c ? make_uint2(min(start, cap), min(start + c, cap)) : make_uint2(0u, 0u);
+  if (tid < 32) { const uint32_t m = __reduce_max_sync(FULL, s_longest[lane]); if (lane == 0 && m) atomicMax(t.longest, m); }
   if (list) {   // the chunk's tiles with a list, for the compositing: long lists from the start, short ones from the end
     const uint32_t longs = __ballot_sync(FULL, c >= LONG_LIST), shorts = __ballot_sync(FULL, c > 0u && c < LONG_LIST), lane_lt = (1u << lane) - 1u;
     uint32_t at_long = 0u, at_short = 0u;
@@ -676,7 +678,7 @@ __global__ void __launch_bounds__(256) fill_keys_kernel(int n_tiles, const uint2
 // Bins the ranks of one depth chunk (words != nullptr) or of the whole view into vals_sorted and `ranges`. Level 1's pairs
 // take ctx->keys, the hit words (or more pairs) ctx->vals and ctx->keys_sorted, a chunk's live splats the scratch of the depth sort.
 int launch_bins(const B2kCtx* c, int n, uint32_t* words, int chunk, int lo_num, int hi_num, const unsigned long long* alive, uint32_t* tiles_out, uint32_t* tables, cudaStream_t s) {
-  const Tables t = bins_tables(tables);
+  const Tables t = bins_tables(tables, words ? words + CW_LONGEST + chunk : c->num_isect + NI_LONGEST);
   static bool attr_set[64] = {false};
   int dev = 0;
   constexpr int smem_max = MAX_BINS * ((L1_WARPS + 1) * (int)sizeof(uint32_t) + 8);

@@ -35,10 +35,12 @@ struct Tables {
   uint32_t* st;          // [16] see S_*
   uint32_t* tile_totals; // [WALK_TILES] hits per tile, of walk.cu
   uint32_t* live_counts; // [512][16] live splats of the parts of level 1's runs (a chunk)
+  uint32_t* longest;     // the longest list, for the compositing: of a whole view in ctx->num_isect, of a chunk in its words
 };
 constexpr int WALK_TILES = 4096;               // tiles of a view that walk.cu takes
-inline Tables bins_tables(uint32_t* tables) {
+inline Tables bins_tables(uint32_t* tables, uint32_t* longest) {
   Tables t;
+  t.longest = longest;
   t.cells = tables;
   t.totals = t.cells + BINS_TABLE_WORDS; t.base = t.totals + MAX_BINS; t.first_item = t.base + MAX_BINS + 1; t.item_bin = t.first_item + MAX_BINS + 1;
   t.block_sums = t.item_bin + MAX_ITEMS; t.segments = t.block_sums + 1024; t.st = t.segments + BINS_SEGMENTS; t.tile_totals = t.st + 16; t.live_counts = t.tile_totals + WALK_TILES;

@@ -9,8 +9,8 @@
 // Transmittances are multiplied up for a group of fragments first, and fragments are compared and selected one by one only where a
 // pixel of the warp closes inside the group (none_closes): 1024x1024 over 1M in four chunks 184 -> 172 us, 4K over 6M in five 681 -> 652.
 // Three kernels with the same arithmetic, bit for bit:
-//   raster_fwd_team_kernel  eight warps to a tile: some find alphas, two composite, two gather. For whole views of few tiles and for the
-//                           second of two chunks where few tiles are alive: the time is that of the longest list.
+//   raster_fwd_team_kernel  eight warps to a tile: some find alphas, two composite, two gather. For whole views of few tiles and the second of two
+//                           chunks, where the time is that of the longest list (team_pays).
 //   raster_fwd_half_kernel  two warps to a tile, a lane one pixel, two consecutive fragments to a packed operation: the chain of
 //                           one list is half as long. For whole views and two chunks, where a visit to a tile is a long list.
 //   raster_fwd_kernel       one warp to a tile, a lane two pixels that share packed operations: twice as many tiles in flight.
@@ -379,49 +379,67 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) raster_fwd_half_kernel(
       seg_shift, feat_acc, bwd_work, tiles, blockIdx.x * FWD_TILES + (threadIdx.x >> 6), blocks * FWD_TILES, s_staged, s_last, s_odd);
 }
 
-// Eight warps to a tile, for views of so few tiles (TEAM_PER_SM to an SM) that the GPU is idle but for the lists' own length: four warps
+// Eight warps to a tile, for views of so few tiles that the GPU is idle but for the longest lists: four warps
 // find the alphas of a batch, two warps (a pixel per lane) carry the transmittances and the sums, two warps take turns to gather and stage
 // the records of the batches ahead. A batch passes from one to the next with one barrier of the block.
 constexpr int TEAM_BATCH = FWD_SEG, TEAM_PAIRS = TEAM_BATCH / 2, TEAM_PRODUCERS = 4, TEAM_THREADS = (2 + TEAM_PRODUCERS + 2) * 32, TEAM_PER_SM = 8;
-// In the second of two chunks the device knows how many tiles have a list: the team takes up to CHUNK_TEAM_PER_SM to an SM, and above that
-// the same blocks take four tiles each at two warps. Visit, us, as two warps to a tile / the team (listed tiles, mean list; n = 300k to 500k): 821 of 190
-// 27.7 / 21.0, 1,047 of 112 21.5 / 17.1, 1,216 of 942 53.6 / 51.3, 1,256 of 605 31.6 / 32.5, 1,370 of 173 29.7 / 25.6, 1,407 of 872 55.7 / 55.8, 1,430 of 437
-// 24.9 / 27.9, 1,544 of 154 28.6 / 27.0, 1,662 of 53 15.9 / 18.5, 1,697 of 715 113 / 123, 4,544 of 458 155 / 193, 19,035 of 282 369 / 488, 24,983 of
-// 168 289 / 416 (faint splats leave nearly every tile alive). CHUNK_BLOCKS of them fit on an SM.
-constexpr int CHUNK_TEAM_PER_SM = 10, CHUNK_BLOCKS = 3, CHUNK_TILES = TEAM_THREADS / 64;
+// Up to TEAM_ALWAYS tiles to an SM there is a block for every tile at once. Above that (whole views of up to TEAM_PER_SM to an SM, and the
+// second of two chunks) the team pays where the time is that of the longest list, and loses where all tiles have much the same to do: its
+// blocks fill the GPU with fewer tiles. The binning leaves the number of hits and the longest list on the device, and the block asks them; where the
+// team does not pay, the same blocks take four tiles at two warps each. Forward, us, at two warps / the team, against hits over (SMs * longest list):
+//   whole views   200x150 over 20k splats 0.33: 28.5 / 19.1; 333x217 over 20k 0.66: 22.7 / 18.8; 256x192 over 8k 0.58: 30.1 / 23.0, over 20k 2.0: 13.1 /
+//                 15.6; 333x217 over 8k 2.2: 25.7 / 33.5, over 2k faint 3.9: 27.8 / 41.1, over 300 wide ones 6.7: 9.7 / 16.1; lists below 100: 2.8 / 4.5
+//   second chunk  1280x720 over 500k 0.50: 63.7 / 39.2, 1.07: 28.4 / 20.2; over 300k faint 2.35: 68.9 / 62.2, 4.1: 66.1 / 69.6; 1920x1080 over 500k 2.0: 24.1 /
+//                 27.2, 4.6: 22.6 / 38.9, faint and close (19,035 tiles with a list) 370 / 490. More than CHUNK_TEAM_PER_SM listed tiles to an SM do
+//                 not go to the team whatever their lists: 1,578 of up to 80 7.7 / 13.0, 1,970 of up to 745 24.1 / 27.2
+constexpr int TEAM_ALWAYS = 2, CHUNK_TEAM_PER_SM = 10, TEAM_BLOCKS = 2, CHUNK_BLOCKS = 3, TEAM_TILES = TEAM_THREADS / 64;   // blocks of whole views and of chunks that fit on an SM
+__device__ __forceinline__ bool team_pays(uint32_t hits, uint32_t longest, uint32_t sms, uint32_t blocks) {
+  return longest >= LONG_LIST && 2ull * hits <= (2ull * blocks - 1ull) * sms * longest;
+}
 
 template <int CKPT, bool DEPTH, bool CHUNKED, bool FEAT>
-__global__ void __launch_bounds__(TEAM_THREADS, CHUNKED ? CHUNK_BLOCKS : 2) raster_fwd_team_kernel(
+__global__ void __launch_bounds__(TEAM_THREADS, CHUNKED ? CHUNK_BLOCKS : TEAM_BLOCKS) raster_fwd_team_kernel(
     uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ vals_sorted, const float4* __restrict__ proj0, const float4* __restrict__ proj1,
     const float4* __restrict__ proj2, int W, int H, int tiles_x, int n_tiles, float3 bg, float4* __restrict__ out_rgba, float4* __restrict__ out_feat,
     float* __restrict__ out_depth, uint32_t* __restrict__ last_idx, int chunk, int n_chunks, unsigned long long* __restrict__ alive,
-    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, uint32_t* __restrict__ bwd_work, const uint32_t* __restrict__ words, const uint32_t* __restrict__ list, uint32_t sms) {
+    const float2* __restrict__ proj3, float4* __restrict__ ckpt, int seg_shift, uint32_t* __restrict__ bwd_work, const uint32_t* __restrict__ words, const uint32_t* __restrict__ list,
+    const uint32_t* __restrict__ hits, const uint32_t* __restrict__ longest, uint32_t sms) {
   after_previous();
   constexpr bool BWD = CKPT != NONE;
   constexpr int RECORDS = FEAT ? STAGED + 2 : DEPTH ? STAGED + 1 : STAGED;
-  __shared__ float4 s_staged[3][TEAM_PAIRS][RECORDS];   // of the batches that are staged, weighed and composited
-  __shared__ float2 s_alpha[2][TEAM_PAIRS][RT_PX];
-  __shared__ uint32_t s_odd[3], s_last[2];
+  union Shared {
+    struct {
+      float4 staged[3][TEAM_PAIRS][RECORDS];   // of the batches that are staged, weighed and composited
+      float2 alpha[2][TEAM_PAIRS][RT_PX];
+      uint32_t odd[3], last[2];
+    } team;
+    struct {
+      float4 staged[TEAM_TILES][2][FWD_BATCH / 2][RECORDS];
+      uint32_t last[TEAM_TILES * 2], odd[TEAM_TILES * 2][2];
+    } halves;
+  };
+  __shared__ __align__(16) unsigned char s_mem[sizeof(Shared)];
+  Shared& sh = *reinterpret_cast<Shared*>(s_mem);
+  auto &s_staged = sh.team.staged;
+  auto &s_alpha = sh.team.alpha;
+  auto &s_odd = sh.team.odd;
+  auto &s_last = sh.team.last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int TEAM_GROUP = CHUNKED ? 4 : 8;   // pairs whose sums are taken together: eight want registers for two blocks an SM, which is enough where tiles are few
   static_assert(!(CHUNKED && (DEPTH || FEAT)), "the last chunk finishes depths and features in every tile");
   const bool composites = warp < 2, weighs = !composites && warp < 2 + TEAM_PRODUCERS, final = !CHUNKED || chunk == n_chunks - 1;
   if (CKPT == PER_SEGMENT && !CHUNKED && blockIdx.x == 0 && threadIdx.x == 0) bwd_work[BWD_SUMMED] = 0u;
   const TileList tiles = CHUNKED ? tile_list(words, list, chunk, n_tiles) : TileList{nullptr, 0u, (uint32_t)n_tiles, n_tiles};
-  if constexpr (CHUNKED) {
-    if (tiles.count > CHUNK_TEAM_PER_SM * sms) {
-      __shared__ float4 s_pairs[CHUNK_TILES][2][FWD_BATCH / 2][STAGED];
-      __shared__ uint32_t s_ends[CHUNK_TILES * 2], s_strange[CHUNK_TILES * 2][2];
-      uint32_t begin = blockIdx.x * CHUNK_TILES + (threadIdx.x >> 6), step = gridDim.x * CHUNK_TILES;
-      const uint32_t resident = min(CHUNK_BLOCKS * sms, gridDim.x);
-      if (tiles.count <= resident * CHUNK_TILES) {   // no more than fit at once: evenly over the blocks (1,475 tiles: 118 -> 108 us)
-        if (blockIdx.x >= resident) return;
-        begin = (threadIdx.x >> 6) * resident + blockIdx.x; step = resident * CHUNK_TILES;
-      }
-      composite_halves<CKPT, DEPTH, CHUNKED, FEAT, true>(tile_ranges, vals_sorted, proj0, proj1, proj2, W, H, tiles_x, n_tiles, bg, out_rgba, out_feat, out_depth, last_idx, chunk, n_chunks,
-                                                         alive, proj3, ckpt, seg_shift, nullptr, bwd_work, tiles, begin, step, s_pairs, s_ends, s_strange);
-      return;
-    }
+  constexpr int BLOCKS = CHUNKED ? CHUNK_BLOCKS : TEAM_BLOCKS;
+  if (hits && ((CHUNKED && tiles.count > CHUNK_TEAM_PER_SM * sms) || !team_pays(*hits, *longest, sms, BLOCKS))) {
+    // Two neighbours, which share splats, to two pairs of warps and two far from them to the others, over as many blocks as fit at once or are
+    // needed (the 1,475 tiles of a faint scene, us: four neighbours to a block 122, none 108, this 99).
+    const uint32_t pair = threadIdx.x >> 6, used = min(max((uint32_t)BLOCKS * sms, (tiles.count + TEAM_TILES - 1u) / TEAM_TILES), gridDim.x);
+    if (blockIdx.x >= used) return;
+    const uint32_t begin = ((pair >> 1) * used + blockIdx.x) * 2u + (pair & 1u), step = used * TEAM_TILES;
+    composite_halves<CKPT, DEPTH, CHUNKED, FEAT, CHUNKED>(tile_ranges, vals_sorted, proj0, proj1, proj2, W, H, tiles_x, n_tiles, bg, out_rgba, out_feat, out_depth, last_idx, chunk, n_chunks,
+                                                          alive, proj3, ckpt, seg_shift, nullptr, bwd_work, tiles, begin, step, sh.halves.staged, sh.halves.last, sh.halves.odd);
+    return;
   }
   for (uint32_t w = blockIdx.x; w < tiles.count; w += gridDim.x) {
   if (w != blockIdx.x) __syncthreads();   // the last tile's batches have been read
@@ -789,12 +807,14 @@ int launch_raster_fwd(const B2kCtx* c, const B2kRenderOpts* o, int chunk, int n_
     seg_shift_of(short_segments(c)), (chunked && o->feat_mode != 0) ? (float4*)c->bwd_scratch : nullptr, bwd_work_ptr(c)
 #define HALF(B, D, C, F, LISTED) launch_next(raster_fwd_half_kernel<B, D, C, F, LISTED>, (LISTED ? min(div_up(c->n_tiles, FWD_TILES), most) : div_up(c->n_tiles, FWD_TILES)) + fill_blocks, FWD_WARPS * 32, 0, ARGS, \
     c->chunk_words, list, fill_blocks)
-#define TEAM(B, D, C, F) launch_next(raster_fwd_team_kernel<B, D, C, F>, C ? min(c->n_tiles, TEAM_PER_SM * sm_count()) : c->n_tiles, TEAM_THREADS, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, \
+#define TEAM(B, D, C, F, HITS, LONGEST) launch_next(raster_fwd_team_kernel<B, D, C, F>, C ? min(c->n_tiles, TEAM_PER_SM * sm_count()) : c->n_tiles, TEAM_THREADS, 0, s, ranges, c->vals_sorted, (const float4*)c->proj0, (const float4*)c->proj1, \
     (const float4*)c->proj2, c->W, c->H, c->tiles_x, c->n_tiles, bg, (float4*)c->out_rgba, (float4*)c->out_feat, c->out_depth, c->last_idx, chunk, n_chunks, alive, \
-    (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c), c->chunk_words, list, (uint32_t)sm_count())
+    (const float2*)c->proj3, o->bwd_info ? bwd_ckpt_ptr(c) : nullptr, seg_shift_of(short_segments(c)), bwd_work_ptr(c), c->chunk_words, list, HITS, LONGEST, (uint32_t)sm_count())
 #define WARP(B, D, F) do { if (list) launch_next(raster_fwd_kernel<B, D, false, true>, min(div_up(c->n_tiles, FWD_WARPS), most) + fill_blocks, FWD_WARPS * 32, 0, ARGS, c->chunk_words, list, fill_blocks); \
     else launch_next(raster_fwd_kernel<B, D, F, false>, div_up(c->n_tiles, FWD_WARPS), FWD_WARPS * 32, 0, ARGS, c->chunk_words, list, 0); } while (0)
-#define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_PER_SM * sm_count()) TEAM(B, D, false, F); else HALF(B, D, false, F, false); } else if (halves && list && chunk > 0 && !c->out_depth) TEAM(B, false, true, false); \
+#define L(B, D, F) do { if (!chunked) { if (c->n_tiles <= TEAM_ALWAYS * sm_count()) TEAM(B, D, false, F, nullptr, nullptr); \
+    else if (c->n_tiles <= TEAM_PER_SM * sm_count() && c->num_isect) TEAM(B, D, false, F, c->num_isect, c->num_isect + NI_LONGEST); else HALF(B, D, false, F, false); } \
+    else if (halves && list && chunk > 0 && !c->out_depth) TEAM(B, false, true, false, c->chunk_words + CW_COUNT + chunk, c->chunk_words + CW_LONGEST + chunk); \
     else if (halves && list) HALF(B, D, true, false, true); else if (halves) HALF(B, D, true, (F) && (B) == NONE, false); \
     else WARP(B, D, (F) && (B) == NONE); } while (0)
 #define LD(B, D) do { if (o->feat_mode != 0) L(B, D, true); else L(B, D, false); } while (0)   // a chunked view with features is forward only (checked by the caller)

@@ -504,7 +504,7 @@ int cluster_sort(const uint32_t* keys, const uint32_t* vals, int n, uint32_t* ko
 int depth_sort(const B2kCtx* c, int n, bool identity, bool for_walk, uint32_t* tables, cudaStream_t s) {
   const uint32_t* in = c->depth_keys_sorted;
   const uint32_t* index = identity ? nullptr : c->order;
-  uint32_t* cleared = for_walk ? bins_tables(tables).tile_totals : nullptr;
+  uint32_t* cleared = for_walk ? bins_tables(tables, nullptr).tile_totals : nullptr;
   uint32_t *k = c->depth_keys_sorted, *v = c->order;   // one block, or one cluster, reads everything before it writes: in place
   if (n <= SMALL_N) return small_sort(in, index, n, k, v, cleared, s);
   if (n <= CLUSTER_N) {

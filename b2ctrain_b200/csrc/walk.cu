@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_emit_kernel(View v, Band g,
   __shared__ EmitShare s_emit;
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_start[WALK_TILES + WALK_THREADS];
-  __shared__ uint32_t s_part[WALK_THREADS / BIN_TILES][BIN_TILES];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ uint32_t s_part[WALK_THREADS / BIN_TILES][BIN_TILES], s_longest[WALK_WARPS];
+  const int tid = threadIdx.x;
   if ((int)blockIdx.x < w.off_blocks) {
     uint32_t c[4], mine = 0, total;
     for (int k = tid; k < (int)blockIdx.x; k += WALK_THREADS) mine += w.off_sums[k];
@@ -209,15 +209,23 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_emit_kernel(View v, Band g,
   const int t0 = tid * per;
   for (int k = 0; k < per; k++) sum += t0 + k < n_tiles ? s_start[t0 + k + tid] : 0u;
   uint32_t start = block_scan(sum, s_warp, total) - sum;
+  uint32_t longest = 0u;
   for (int k = 0; k < per; k++) {
     if (t0 + k >= n_tiles) break;
     const uint32_t c = s_start[t0 + k + tid];
+    longest = max(longest, c);
     s_start[t0 + k + tid] = start;
     if (writes_ranges) ranges[t0 + k] = c ? make_uint2(min(start, cap), min(start + c, cap)) : make_uint2(0u, 0u);
     start += c;
   }
-  if (writes_ranges && tid == 0) *num_isect = total;
+  longest = __reduce_max_sync(FULL, longest);
+  if ((tid & 31) == 0) s_longest[tid >> 5] = longest;
   __syncthreads();
+  if (writes_ranges && tid == 0) {
+    num_isect[0] = total;
+    for (int k = 1; k < WALK_WARPS; k++) longest = max(longest, s_longest[k]);
+    num_isect[NI_LONGEST] = longest;
+  }
   if (!any) return;
   const int x0 = u.bx * BIN_W, y0 = u.by * BIN_W;
   if (tid < BIN_TILES) {
@@ -252,7 +260,7 @@ bool walks(const B2kCtx* c, int n) {
 }
 
 int launch_walk(const B2kCtx* c, const View& v, uint32_t* tables, cudaStream_t s) {
-  const Tables t = bins_tables(tables);
+  const Tables t = bins_tables(tables, c->num_isect + NI_LONGEST);
   const Band g{c->tiles_x, c->tiles_y, div_up(c->tiles_x, BIN_W), 0, div_up(c->tiles_y, BIN_W)};
   const int bins = g.bins_x * g.bin_rows;
   Walk w;

@@ -76,7 +76,8 @@ typedef struct {
   uint64_t isect_cap;
   uint32_t* num_isect;     /* [4] device words: [0] intersections of this view (may exceed isect_cap: overflow; also where the
                               binning would need more than 3 * isect_cap words of scratch, which it then reports instead);
-                              [1] entries of vis_list; [2] largest [0] since the caller cleared it (b2k_loss_accumulate) */
+                              [1] entries of vis_list; [2] largest [0] since the caller cleared it (b2k_loss_accumulate);
+                              [3] the longest tile list of the last whole view, by which b2k_raster_fwd chooses its kernel */
   void* sort_tmp;          /* scratch of b2k_sort_tmp_bytes() bytes */
   uint64_t sort_tmp_bytes;
   uint32_t* tile_ranges;   /* [n_tiles][2] start, end into vals_sorted; end shrunk by the forward when bwd_info

@@ -642,3 +642,43 @@ def test_second_of_two_chunks(W, H, logit):
         h.api.rasterize_backward(c, h.model, h.rp)
     assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
     assert torch.equal(ctx.vis_flag[:n], h.ctx.vis_flag[:n]) and rel_l2(ctx.v_splat[:n].cpu().numpy(), h.ctx.v_splat[:n].cpu().numpy()) <= 2e-5
+
+
+@pytest.mark.parametrize("W,H", [(168, 136), (200, 150), (333, 217), (296, 256)])     # 357 to 1,184 tiles: between two and eight to an SM of 148
+@pytest.mark.parametrize("n,log_scale,team", [(6000, -4.5, True), (3000, 0.5, False), (300, 0.5, False), (40, -5.0, False)])
+def test_forward_of_some_tiles_to_an_sm(W, H, n, log_scale, team):
+    """A few long lists go to the team, lists that are all alike or short to two warps a tile: the same image as in chunks, bit for bit, and
+    the same gradients. The binning leaves the longest list for the choice, by either route."""
+    import torch
+    from b2ctrain_b200 import api
+    scene = scenes.make_splats(n, 1, 21, log_scale=(log_scale, 0.3))
+    scene["pos_op"][:, :3] *= 0.3 if team else 1.0
+    cam = scenes.look_at_camera((0.0, 0.0, 4.0), W, H, float(H))
+    m = api.Model("cuda:0").upload(scenes.floor_for_cameras(scene, [cam]))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    v_out = torch.from_numpy(np.random.Generator(np.random.PCG64(4)).standard_normal((W * H, 4)).astype(np.float32)).cuda()
+    got = []
+    for chunks, cap in ((1, 1 << 22), (1, None), (3, 1 << 22)):
+        ctx = api.RenderCtx("cuda:0")
+        ctx.want_depth = True
+        ctx.setup(W, H, m.cap, n_chunks=chunks, isect_cap=got[0][0] if cap is None else cap)    # None: of the lists' size, which may take the general route
+        rp = api.RenderParams(cam, bg=(0.2, 0.1, 0.3), sh_degree=1, bwd_info=False)
+        api.render_forward(ctx, m, rp)
+        if chunks == 1:
+            r = ctx.tile_ranges.view(-1, 2).to(torch.int64)
+            hits, longest = int(ctx.d_num_isect[0].item()), int(ctx.d_num_isect[3].item())
+            assert longest == int((r[:, 1] - r[:, 0]).max()) and (longest >= 128 and 2 * hits <= 3 * sms * longest) == team
+        images = [ctx.out_rgba.clone(), ctx.out_feat[:, 3].clone(), ctx.out_depth.clone()]
+        rp.feat = "Normals"
+        api.render_forward(ctx, m, rp)
+        images += [ctx.out_rgba.clone(), ctx.out_feat.clone(), ctx.out_depth.clone()]
+        rp.feat, rp.bwd_info = "None", True
+        api.render_forward(ctx, m, rp)
+        images += [ctx.out_rgba.clone(), ctx.out_depth.clone()]
+        ctx.v_out.copy_(v_out)
+        ctx.v_splat.zero_(); ctx.vis_flag.zero_()
+        api.rasterize_backward(ctx, m, rp)
+        got.append((ctx.num_isect, images, ctx.vis_flag[:n].clone(), ctx.v_splat[:n].cpu().numpy()))
+    for _, images, flags, lanes in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0][1], images))
+        assert torch.equal(got[0][2], flags) and rel_l2(got[0][3], lanes) <= 5e-5
