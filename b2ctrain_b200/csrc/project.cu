@@ -33,14 +33,13 @@ namespace {
 
 constexpr int PROJ_BLOCK = 256;
 
-// Tile boxes of at most MASK_TILES tiles are remembered as a bit mask of the tiles hit. The tests of boxes of at most warp_tiles() tiles are
-// shared out over the splats' warp; larger ones are counted by a kernel of their own, a warp to each. Few splats are few warps,
-// which wait for the one with the most tests: project_kernel and count_big_kernel at 1445x965 over 24k splats together 46 us with boxes of
-// up to 1,024 tiles in the warp, 41 up to 256, 31 up to 64; small images have few large boxes (333x217 over 20k: 13.5 us up to 128 and above,
-// 14.5 up to 64). Many splats fill the GPU, and the large boxes' kernel is then the more costly one: 1001x751 over 200k 46 us up to 1,024, 45 up
-// to 512, 47 up to 256, 54 up to 64; where a tenth are wide (801x603 over 90k) 114, 99, 95, 93.
-constexpr int MASK_TILES = 64;
-__device__ __forceinline__ int warp_tiles(int n, int n_tiles) { return n > 49152 ? 512 : n_tiles > 4096 ? MASK_TILES : 128; }
+// Tile boxes of at most MASK_TILES tiles are remembered as a bit mask of the tiles hit. Their tests are shared out over the splats' warp, and so
+// are those of boxes of up to WARP_TILES where there are many splats, or where all such boxes of the warp make WARP_FEW tiles; the others are counted by
+// a kernel of their own, a warp to each. Few splats are few warps, which wait for the one with the most tests; project_kernel and count_big_kernel
+// together, us, WARP_FEW of 256 / 512 / 1,024: 256x192 over 2k splats over most of it 10.7 / 13.7 / 16.0, 333x217 over 45k wide ones 36.3 / 37.9 / 39.8; and
+// every box of up to 128 tiles in the warp 200x150 over 2k 26.3 against 15.8. Many splats fill the GPU, and the large boxes' kernel is then the
+// more costly one: 1001x751 over 200k 46 us up to 1,024, 45 up to 512, 47 up to 256, 54 up to 64; where a tenth are wide (801x603 over 90k) 114, 99, 95, 93.
+constexpr int MASK_TILES = 64, WARP_TILES = 512, WARP_FEW = 256, WARP_MANY_SPLATS = 49152, DIRECT_TILES = 16;
 
 // The tile tests of a warp's 32 splats, shared out in units of up to eight tiles of one row: boxes hold one to a thousand tiles, and with
 // a splat per lane most lanes wait for the largest.
@@ -49,13 +48,19 @@ struct TileShare { float4 rec[64]; uint32_t corner[32], width[32], end[32], mask
 __device__ __forceinline__ uint32_t shared_hits(TileShare& ts, const TileRec& rec, const TileBox& b, int area, uint32_t& mask_lo, uint32_t& mask_hi) {
   constexpr unsigned ALL = 0xffffffffu;
   const int lane = threadIdx.x & 31, bw = b.max_x - b.min_x;
+  mask_lo = mask_hi = 0u;
+  if (__reduce_max_sync(ALL, area) <= DIRECT_TILES) {   // each lane its own: 1920x1080 over 3M splats of one or two tiles 160 -> 144 us
+    for (int k = 0, tx = b.min_x, ty = b.min_y; k < area; k++) {
+      if (tile_hit(tx, ty, rec)) mask_lo |= 1u << k;
+      if (++tx == b.max_x) { tx = b.min_x; ty++; }
+    }
+    return (uint32_t)__popc(mask_lo);
+  }
   const int units = area > 0 ? (b.max_y - b.min_y) * ((bw + 7) >> 3) : 0;
   int end = units;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(ALL, end, o); if (lane >= o) end += u; }
   const int total = __shfl_sync(ALL, end, 31);
-  mask_lo = mask_hi = 0u;
-  if (total == 0) return 0u;
   ts.rec[lane * 2] = make_float4(rec.mx, rec.my, rec.c00, rec.c01);
   ts.rec[lane * 2 + 1] = make_float4(rec.c11, rec.power, rec.ia, rec.ib);
   ts.corner[lane] = (uint32_t)b.min_x | (uint32_t)b.min_y << 16; ts.width[lane] = (uint32_t)bw | (area <= MASK_TILES ? 0x80000000u : 0u); ts.end[lane] = (uint32_t)end;
@@ -87,11 +92,12 @@ __device__ __forceinline__ uint32_t shared_hits(TileShare& ts, const TileRec& re
   return ts.count[lane];
 }
 
-// What a splat's record says about its tiles: tiles hit, the words of hit_info, whether it goes to the list of large boxes. All lanes of
+// What a splat's record says about its tiles: tiles hit, the words of hit_info, whether its box is left to count_big_kernel. All lanes of
 // the warp call this; `drawn`: the splat has a record and its box is on the image.
 struct TileHits { uint32_t hits, w0, w1, box, height; bool big; };
-__device__ __forceinline__ TileHits decide_tiles(TileShare& ts, const TileRec& rec, const TileBox& b, bool drawn, int limit) {
+__device__ __forceinline__ TileHits decide_tiles(TileShare& ts, const TileRec& rec, const TileBox& b, bool drawn, int n) {
   const int bw = drawn ? b.max_x - b.min_x : 0, bh = drawn ? b.max_y - b.min_y : 0, area = bw > 0 && bh > 0 ? bw * bh : 0;
+  const int limit = n > WARP_MANY_SPLATS || __reduce_add_sync(0xffffffffu, area > MASK_TILES && area <= WARP_TILES ? area : 0) <= WARP_FEW ? WARP_TILES : MASK_TILES;
   TileHits t{0u, 0u, 0u, 0u, drawn ? (uint32_t)bh : 0u, area > limit};
   t.hits = shared_hits(ts, rec, b, t.big ? 0 : area, t.w0, t.w1);
   if (area > MASK_TILES) {   // no mask: the box itself
@@ -99,6 +105,12 @@ __device__ __forceinline__ TileHits decide_tiles(TileShare& ts, const TileRec& r
     t.w0 = (uint32_t)b.min_x | ((uint32_t)b.min_y << 16); t.w1 = (uint32_t)bw | ((uint32_t)bh << 16);
   } else if (area > 0) t.box = (uint32_t)b.min_x | ((uint32_t)b.min_y << 12) | ((uint32_t)bw << 24);
   return t;
+}
+
+// One bit a splat for count_big_kernel. All lanes call this.
+__device__ __forceinline__ void flag_big(uint32_t* __restrict__ big, int i, int n, bool is) {
+  const uint32_t word = __ballot_sync(0xffffffffu, is);
+  if ((i & 31) == 0 && i < n) big[i >> 5] = word;
 }
 
 // Feature lanes of a splat (src/gpu/project.cu:62-77). Mode 1: pseudo-normal = the local axis of the shortest scale,
@@ -145,7 +157,7 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
     const float* __restrict__ sh_dc, const float* __restrict__ sh_hi, CamDev cam, int active, int tiles_x, int tiles_y,
     float4* __restrict__ proj0, float4* __restrict__ proj1, float4* __restrict__ proj2, uint32_t* __restrict__ tile_count,
     uint4* __restrict__ hit_info, uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in, float* __restrict__ max_screen,
-    int feat_mode, const float* __restrict__ feat_in, float2* __restrict__ proj3) {
+    int feat_mode, const float* __restrict__ feat_in, float2* __restrict__ proj3, uint32_t* __restrict__ big) {
   after_previous();
   __shared__ TileShare s_share[PROJ_BLOCK / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -166,7 +178,8 @@ __global__ void __launch_bounds__(PROJ_BLOCK) project_kernel(
       proj1[i] = make_float4(0.f, 0.f, 0.f, -1.f);   // no record
     }
   }
-  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn, warp_tiles(n, tiles_x * tiles_y));
+  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn, n);
+  flag_big(big, i, n, t.big);
   if (!valid) return;
   if (drawn && max_screen) {
     const float detc = pr.c00 * pr.c11 - pr.c01 * pr.c01;
@@ -251,37 +264,48 @@ __global__ void __launch_bounds__(PROJ_BLOCK, 4) project_lite_kernel(
   depth_keys[i] = area ? __float_as_uint(pr.mean_c.z) : 0xFFFFFFFFu;
 }
 
-// Boxes above warp_tiles: a warp to each, whose lanes take units of up to eight tiles of a row (562x569 over 4,303 wide splats: a tile
-// a lane, which divides for each, 33.7 us, units 19.9). Warp w looks at every (number of warps)-th pair of
-// splats from the w-th on (a pair is a sector of hit_info), so that large splats that follow each other go to different warps. (They used to
-// go to a list, whose counter took a launch of its own to clear: 64x64 over 2k splats 80.2 -> 78.9 us a step.)
-__global__ void __launch_bounds__(256) count_big_kernel(int n, const uint4* __restrict__ hit_info, const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H,
-                                                        int tiles_x, int tiles_y, uint32_t* __restrict__ tile_count, uint32_t* __restrict__ depth_keys) {
+// Boxes that were not tested in their own warp: a warp to each, whose lanes take units of up to eight tiles of a row (562x569 over 4,303 wide splats: a tile
+// a lane, which divides for each, 33.7 us, units 19.9). The projection leaves a bit a splat; a warp's lanes look at 1 << shift neighbours each,
+// far from each other, so that large splats that follow each other go to different warps. (A list of them needs a counter that is
+// cleared, which took a launch of its own, 64x64 over 2k splats 80.2 -> 78.9 us a step; finding them in hit_info reads 16 bytes a splat, 3M
+// splats 16 us.)
+constexpr int BIG_WARPS = 8;             // of a block
+inline int big_shift(int n) { return n <= 32768 ? 0 : n <= 262144 ? 1 : 2; }
+// A warp for every unit of few, for two of more (blocks without a large box cost as much as the launch: 8k splats 1.9 us in 500 blocks, 2.6 in 1,000;
+// 256x192 over 1k splats over all of it 10.7 us with a warp to each, 13.8 with one to two).
+inline int big_blocks(int n) {
+  const int units = div_up(n, 1 << big_shift(n));
+  return min(max(min(div_up(units, BIG_WARPS), 512), div_up(units, 2 * BIG_WARPS)), sm_count() * 8);
+}
+__global__ void __launch_bounds__(BIG_WARPS * 32) count_big_kernel(int n, int shift, const uint32_t* __restrict__ big, const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H,
+                                                                   int tiles_x, int tiles_y, uint32_t* __restrict__ tile_count, uint32_t* __restrict__ depth_keys) {
   after_previous();
-  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5), first = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  for (long long p0 = first; 2 * p0 < n; p0 += 16ll * warps) {
-    auto splat_of = [&](int l) { return 2 * (p0 + (long long)(l >> 1) * warps) + (l & 1); };
-    const long long mine = splat_of(lane);
-    const uint4 hi = mine < n ? hit_info[mine] : make_uint4(0u, 0u, 0u, 0u);
-    const bool big = hi.z == 0xFFFFFFFFu && (hi.y & 0xFFFFu) * (hi.y >> 16) > (uint32_t)warp_tiles(n, tiles_x * tiles_y);
-    for (uint32_t todo = __ballot_sync(0xffffffffu, big); todo; todo &= todo - 1u) {
-      const long long i = splat_of(__ffs(todo) - 1);
-      const float4 a = proj0[i], b = proj1[i];
-      const TileRec rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
-      TileBox bb;
-      uint32_t hits = 0;
-      if (tile_box(rec, W, H, tiles_x, tiles_y, bb)) {
-        // units of up to eight tiles of one row, as in shared_hits
-        const int bw = bb.max_x - bb.min_x, per_row = (bw + 7) >> 3, units = (bb.max_y - bb.min_y) * per_row;
-        for (int u = lane; u < units; u += 32) {
-          const int y = u / per_row, x0 = (u - y * per_row) * 8;
-          const TileRow row = tile_row(bb.min_y + y, rec);
+  const int lane = threadIdx.x & 31, warps = gridDim.x * BIG_WARPS;
+  const long long units = ((long long)n + (1 << shift) - 1) >> shift;
+  for (long long u0 = blockIdx.x * BIG_WARPS + (threadIdx.x >> 5); u0 < units; u0 += 32ll * warps) {
+    const long long mine = (u0 + (long long)lane * warps) << shift;
+    const uint32_t flags = mine < n ? (big[mine >> 5] >> (mine & 31)) & ((1u << (1 << shift)) - 1u) : 0u;
+    for (uint32_t todo = __ballot_sync(0xffffffffu, flags != 0u); todo; todo &= todo - 1u) {
+      const int owner = __ffs(todo) - 1;
+      for (uint32_t left = __shfl_sync(0xffffffffu, flags, owner); left; left &= left - 1u) {
+        const long long i = ((u0 + (long long)owner * warps) << shift) + __ffs(left) - 1;
+        const float4 a = proj0[i], b = proj1[i];
+        const TileRec rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
+        TileBox bb;
+        uint32_t hits = 0;
+        if (tile_box(rec, W, H, tiles_x, tiles_y, bb)) {
+          // units of up to eight tiles of one row, as in shared_hits
+          const int bw = bb.max_x - bb.min_x, per_row = (bw + 7) >> 3, units = (bb.max_y - bb.min_y) * per_row;
+          for (int u = lane; u < units; u += 32) {
+            const int y = u / per_row, x0 = (u - y * per_row) * 8;
+            const TileRow row = tile_row(bb.min_y + y, rec);
 #pragma unroll
-          for (int k = 0; k < 8; k++) hits += x0 + k < bw && tile_hit(bb.min_x + x0 + k, row, rec) ? 1u : 0u;
+            for (int k = 0; k < 8; k++) hits += x0 + k < bw && tile_hit(bb.min_x + x0 + k, row, rec) ? 1u : 0u;
+          }
         }
+        hits = __reduce_add_sync(0xffffffffu, hits);
+        if (lane == 0) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
       }
-      hits = __reduce_add_sync(0xffffffffu, hits);
-      if (lane == 0) { tile_count[i] = hits; depth_keys[i] = hits ? __float_as_uint(b.z) : 0xFFFFFFFFu; }
     }
   }
 }
@@ -290,7 +314,7 @@ __global__ void __launch_bounds__(256) count_big_kernel(int n, const uint4* __re
 // already in proj0 / proj1 (power < -0.5 marks "no record").
 __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const float4* __restrict__ proj0, const float4* __restrict__ proj1, int W, int H,
                                                                  int tiles_x, int tiles_y, uint32_t* __restrict__ tile_count, uint4* __restrict__ hit_info,
-                                                                 uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in) {
+                                                                 uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ order_in, uint32_t* __restrict__ big) {
   after_previous();
   __shared__ TileShare s_share[PROJ_BLOCK / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -304,7 +328,8 @@ __global__ void __launch_bounds__(PROJ_BLOCK) count_tiles_kernel(int n, const fl
     rec = make_tile_rec(a.x, a.y, a.z, a.w, b.x, b.w);
     drawn = tile_box(rec, W, H, tiles_x, tiles_y, bb);
   }
-  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn, warp_tiles(n, tiles_x * tiles_y));
+  const TileHits t = decide_tiles(s_share[threadIdx.x >> 5], rec, bb, drawn, n);
+  flag_big(big, i, n, t.big);
   if (!valid) return;
   hit_info[i] = make_uint4(t.w0, t.w1, t.box, t.height);
   order_in[i] = (uint32_t)i;
@@ -327,8 +352,8 @@ int launch(const B2kModel* m, const CamDev& cam, const B2kRenderOpts* o, const B
   launch_next(project_kernel<DEG>, div_up(m->n, PROJ_BLOCK), PROJ_BLOCK, 0, s, 
       m->n, (size_t)m->cap, pos, quat, lscale, m->sh_dc, m->sh_hi, cam, active < 0 ? 0 : active, c->tiles_x, c->tiles_y,
       (float4*)c->proj0, (float4*)c->proj1, (float4*)c->proj2, c->tile_count, (uint4*)c->hit_info, c->depth_keys_sorted, c->order, m->max_screen,
-      o->feat_mode, o->feat_buffer, (float2*)c->proj3);
-  launch_next(count_big_kernel, min(div_up(m->n, 16), sm_count() * 8), 256, 0, s, m->n, (const uint4*)c->hit_info, (const float4*)c->proj0, (const float4*)c->proj1, cam.W, cam.H, c->tiles_x,
+      o->feat_mode, o->feat_buffer, (float2*)c->proj3, splat_words_ptr(c));
+  launch_next(count_big_kernel, big_blocks(m->n), BIG_WARPS * 32, 0, s, m->n, big_shift(m->n), splat_words_ptr(c), (const float4*)c->proj0, (const float4*)c->proj1, cam.W, cam.H, c->tiles_x,
                                                   c->tiles_y, c->tile_count, c->depth_keys_sorted);
   return check_launch();
 }
@@ -383,8 +408,8 @@ extern "C" int b2k_count_tiles(const B2kCtx* c, int32_t n, b2k_stream_t stream) 
   if (c->n_cap < n || c->sort_tmp_bytes < b2k_sort_tmp_bytes(c->n_cap, c->isect_cap)) return B2K_ERR_CAPACITY;
   cudaStream_t s = (cudaStream_t)stream;
   launch_next(count_tiles_kernel, div_up(n, 256), 256, 0, s, n, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y, c->tile_count,
-                                                   (uint4*)c->hit_info, c->depth_keys_sorted, c->order);
-  launch_next(count_big_kernel, min(div_up(n, 16), sm_count() * 8), 256, 0, s, n, (const uint4*)c->hit_info, (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y,
+                                                   (uint4*)c->hit_info, c->depth_keys_sorted, c->order, splat_words_ptr(c));
+  launch_next(count_big_kernel, big_blocks(n), BIG_WARPS * 32, 0, s, n, big_shift(n), splat_words_ptr(c), (const float4*)c->proj0, (const float4*)c->proj1, c->W, c->H, c->tiles_x, c->tiles_y,
                                                   c->tile_count, c->depth_keys_sorted);
   return check_launch();
 }

@@ -518,7 +518,7 @@ int depth_sort(const B2kCtx* c, int n, bool identity, bool for_walk, uint32_t* t
   const Shape sh = shape_of((uint32_t)n);
   const int range_blocks = std::min<int>(std::min(2 * sm_count(), MAX_BLOCKS), div_up(n, CNT_THREADS * 16));
   launch_next(key_range_kernel, range_blocks, CNT_THREADS, 0, s, in, (uint32_t)n, range, cleared);
-  // Three passes by way of two scratch pairs (the second: tile_off and the projection's list, both free here).
+  // Three passes by way of two scratch pairs (the second: tile_off and the words per splat, both free here).
   uint32_t* list = splat_words_ptr(c);
   const uint32_t* ki[3] = {in, c->depth_keys, c->tile_off};
   const uint32_t* vi[3] = {index, c->order_in, list};

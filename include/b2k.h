@@ -176,9 +176,9 @@ int b2k_read_num_isect(const B2kCtx* ctx, b2k_stream_t s, uint32_t* total);
  * the array's device address up (a synchronising runtime query): make that first call outside any stream capture.
  * All calls on a device share the one array, so two calls whose kernels overlap on the GPU (different streams or
  * threads) race; calls on one stream are safe. Nothing in it needs clearing by the caller.
- * Limits: only the binning scratch is covered. b2k_project and b2k_count_tiles ask for ctx->sort_tmp as before, so a host
- * that cannot allocate at all has to be handed a sort_tmp by whoever owns the memory, or feed this entry records it binned
- * elsewhere. The address
+ * Limits: only the binning scratch is covered. b2k_project and b2k_count_tiles keep a bit per splat (large tile box) in
+ * ctx->sort_tmp and still need that buffer from the caller, so a host that cannot allocate at all has to be handed a sort_tmp
+ * by whoever owns the memory, or feed this entry records it binned elsewhere. The address
  * looked up on the first call is cached per device ordinal: it is stale after cudaDeviceReset, and two host threads
  * making their first call on one device at once both look it up (harmless: they store the same value). */
 int b2k_bin_sort_static(const B2kCtx* ctx, int32_t n, b2k_stream_t s);

@@ -427,7 +427,7 @@ def test_chunks_of_wide_splats():
         assert torch.equal(ctx.out_rgba, h.ctx.out_rgba) and torch.equal(ctx.out_feat[:, 3], h.ctx.out_feat[:, 3])
 
 
-@pytest.mark.parametrize("n,log_scale", [(3001, (-4.5, 1.6)), (49153, (-6.0, 1.0))])
+@pytest.mark.parametrize("n,log_scale", [(3001, (-4.5, 1.6)), (32771, (-5.5, 1.0)), (49153, (-6.0, 1.0)), (262149, (-7.0, 1.1))])
 def test_tile_boxes_of_every_size(n, log_scale):
     """The tile tests are shared out over a warp in units of eight tiles of a row: masks up to 64 tiles, counts of larger boxes there or by a
     warp to each."""
@@ -450,6 +450,22 @@ def test_tile_boxes_of_every_size(n, log_scale):
             h.ctx.tile_count.zero_(); h.ctx.hit_info.zero_()
             h.api.count_tiles(h.ctx, h.model)
             assert np.array_equal(h.u32(h.ctx.hit_info[:n]).reshape(-1, 4)[tc_o > 0], info[tc_o > 0])
+
+
+@pytest.mark.parametrize("W,H", [(8, 8), (32, 32), (40, 24), (64, 64), (61, 43), (128, 33)])
+@pytest.mark.parametrize("n", [1, 33, 97])
+@pytest.mark.parametrize("log_scale", [(-4.0, 0.05), (0.5, 0.2), (-2.0, 1.0)])
+def test_tile_boxes_alike(n, W, H, log_scale):
+    """Boxes that are all small, or nearly all as large as the largest of the warp, are tested by their own lane."""
+    scene = scenes.make_splats(n, 0, n, log_scale=log_scale)
+    cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 25.0, 10.0), W, H, float(max(W, H)))
+    h = Harness(scenes.floor_for_cameras(scene, [cam]), cam)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    tc_o = orc.bin_sort(h.ctx.proj0[:n].cpu().numpy(), h.ctx.proj1[:n].cpu().numpy(), W, H)[0]
+    info = h.u32(h.ctx.hit_info[:n]).reshape(-1, 4)
+    masks = np.array([bin(int(a)).count("1") + bin(int(b)).count("1") for a, b in info[:, :2]])
+    large = info[:, 2] == 0xFFFFFFFF
+    assert np.array_equal(h.u32(h.ctx.tile_count, n), tc_o) and np.array_equal(masks[~large], tc_o[~large])
 
 
 @pytest.mark.parametrize("W,H", [(64, 64), (61, 43)])
