@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_count_kernel(View v, Band g
   const int p = u.run * RUN + tid, x0 = u.bx * BIN_W, y0 = u.by * BIN_W;
   uint32_t i = 0u;
   uint4 hi = make_uint4(0u, 0u, 0u, 0u);
-  if (p < v.n) { i = v.order[p]; hi = v.hit_info[i]; }
+  if (p < v.n) { i = v.order[p]; hi = v.hit_info[i]; if (v.tile_count[i] == 0u) hi = make_uint4(0u, 0u, 0u, 0u); }   // both loads at once
   const Box b = box_of(hi);
   const bool in = b.x0 < x0 + BIN_W && b.x1 > max(x0, b.x0) && b.y0 < y0 + BIN_W && b.y1 > max(y0, b.y0);
   const bool any = __syncthreads_or(in);

@@ -412,6 +412,52 @@ def test_small_views_walked(W, H, n, wide, room):
         assert np.array_equal(h.u32(h.ctx.tile_off, n), np.cumsum(tc[h.u32(h.ctx.order, n)], dtype=np.uint32))
 
 
+def walked(W, H, n, cap):
+    """Whether a whole view is binned by walking the ranks: few tiles, few tests, room for the hit words."""
+    tx, ty = -(-W // 8), -(-H // 8)
+    bins = -(-tx // 8) * -(-ty // 8)
+    units = bins * -(-n // 256)
+    return tx * ty <= 4096 and n * bins <= 1 << 20 and units * 65 <= 2048 * 320 and units * 256 <= cap
+
+
+def shown_lists(vals, ranges, hidden):
+    """The oracle's lists without some splats."""
+    keep = ~hidden[vals]
+    before = np.concatenate([[0], np.cumsum(keep)])
+    out = before[ranges]
+    out[out[:, 0] == out[:, 1]] = 0
+    return vals[keep], out.astype(np.uint32)
+
+
+@pytest.mark.parametrize("W,H,n,wide", [(8, 8, 40, 0), (64, 64, 300, 1), (65, 63, 300, 2), (1040, 72, 5000, 10), (333, 217, 3000, 5)])
+@pytest.mark.parametrize("walk", [True, False])
+def test_both_routes_to_small_views(W, H, n, wide, walk):
+    """One tile, one bin, ragged bins by the walk and, in buffers of just the lists' size, by the distribution over bins: the same lists, with all
+    splats and with some hidden by a tile count of zero."""
+    scene, cam = bin_scene(n, W, H, 0, seed=n)
+    scene["lscale"][:, :3] = np.log(1.5 / max(W, H))                # half a pixel
+    scene["pos_op"][np.arange(n) % 3 != 0, :3] = 2.0 * np.asarray(cam["pos"], np.float32)     # two of three behind the camera
+    if wide:
+        scene["lscale"][:: 3 * (n // 3 // wide), :3] = -0.7
+    h = Harness(scenes.floor_for_cameras(scene, [cam]), cam, isect_cap=1 << 22)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    tc_o, vals_o, keys_o, ranges_o = orc.bin_sort(h.ctx.proj0[:n].cpu().numpy(), h.ctx.proj1[:n].cpu().numpy(), W, H)
+    if not walk:
+        h.ctx._alloc_isect(len(vals_o))
+    assert walked(W, H, n, h.ctx.isect_cap) == walk
+    hidden = np.zeros(n, bool)
+    for _ in range(2):
+        h.api.bin_and_sort(h.ctx, h.model)
+        vals, ranges = shown_lists(vals_o, ranges_o, hidden)
+        tc = np.where(hidden, 0, tc_o)
+        assert h.ctx.num_isect == len(vals) > 0 and np.array_equal(h.u32(h.ctx.vals_sorted, len(vals)), vals)
+        assert np.array_equal(h.u32(h.ctx.keys_sorted, len(vals)), keys_o[~hidden[vals_o]])
+        assert np.array_equal(h.u32(h.ctx.tile_ranges).reshape(-1, 2), ranges)
+        assert np.array_equal(h.u32(h.ctx.tile_off, n), np.cumsum(tc[h.u32(h.ctx.order, n)], dtype=np.uint32))
+        hidden[::6] = True
+        h.ctx.tile_count[:n:6] = 0
+
+
 def test_chunks_of_wide_splats():
     """Hundreds of splats over most bins in one round of the distribution: shared out over the block's warps."""
     import torch
