@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) bin_count_kernel(View v, Band g
         const uint32_t i = rest ? s_splat[w][32 + lane] : 0u;
         const uint4 h = rest ? s_hit[w][32 + lane] : make_uint4(0u, 0u, 0u, 0u);
         if (rest) { s_splat[w][lane] = i; s_hit[w][lane] = h; }
+        __syncwarp();                   // the next to wait may be put where another lane has just read
       }
     }
   }
