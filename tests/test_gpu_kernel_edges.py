@@ -58,7 +58,7 @@ def bin_scene(n, W, H, wide, seed=5):
 @pytest.mark.parametrize("W,H,n,wide", [(8, 8, 40, 3),             # one tile
                                         (64, 64, 300, 3),          # one bin of 8x8 tiles
                                         (65, 63, 300, 3),          # a ragged second column of bins
-                                        (1040, 72, 5000, 200),     # 17x2 bins: splats over more bins than a lane walks alone
+                                        (1040, 72, 5000, 200),     # 17x2 bins: in chunks, splats over more bins than a lane walks alone
                                         (3848, 2312, 600, 40)])    # 61x37 bins: two bands of bin rows
 def test_binning_at_the_edges_of_bins_and_bands(W, H, n, wide):
     """Tile sets, list order and ranges are bit-exact functions of the records; a chunked view composites the same image."""
@@ -105,7 +105,7 @@ def test_binning_with_more_pairs_than_items_of_256_hold():
 
 
 @pytest.mark.parametrize("kind", ["uniform", "wide", "same", "culled", "all_culled", "any_bits"])
-@pytest.mark.parametrize("n", [1, 33, 2048, 2049, 8192, 8193, 100_003, 1_300_001])   # one block, then small, middle and large tiles
+@pytest.mark.parametrize("n", [1, 33, 2048, 2049, 8192, 8193, 100_003, 1_300_001])   # one block, one cluster, then many blocks of middle and large tiles
 def test_depth_sort_is_stable_at_every_size(n, kind):
     import ctypes as C
     import torch
@@ -336,7 +336,7 @@ def test_depth_sort_scratch_at_any_word(chunks):
     """The offsets' array, which the depth sort of many splats borrows, one word behind a 16-byte boundary."""
     import torch
     from b2ctrain_b200 import api
-    scene = scenes.make_splats(9001, 0, 4)
+    scene = scenes.make_splats(40001, 0, 4)                      # more than one cluster sorts
     cam = scenes.look_at_camera(scenes.orbit_eye(3.0, 30.0, 10.0), 320, 200, 200.0)
     m = api.Model("cuda:0").upload(scenes.floor_for_cameras(scene, [cam]))
     images = []
@@ -456,6 +456,39 @@ def test_both_routes_to_small_views(W, H, n, wide, walk):
         assert np.array_equal(h.u32(h.ctx.tile_off, n), np.cumsum(tc[h.u32(h.ctx.order, n)], dtype=np.uint32))
         hidden[::6] = True
         h.ctx.tile_count[:n:6] = 0
+
+
+@pytest.mark.parametrize("W,H,n", [(64, 64, 256), (64, 64, 300), (120, 64, 700)])
+@pytest.mark.parametrize("short", [0, 1, 5000])
+def test_walk_of_dense_runs_into_short_buffers(W, H, n, short):
+    """Runs whose splats cover their bin (more hits than fit in shared memory) before and behind sparse ones, in buffers of the lists' size and less:
+    the total is reported, the lists end with the buffers and nothing behind them is written; grown, they are whole."""
+    import ctypes as C
+    import torch
+    from b2ctrain_b200 import api
+    scene, cam = bin_scene(n, W, H, 0, seed=n)
+    scene["lscale"][:, :3] = -5.0
+    eye = np.asarray(cam["pos"], np.float32)
+    near = np.argsort(np.linalg.norm(scene["pos_op"][:, :3] - eye, axis=1))
+    scene["lscale"][near[-256:] if n == 300 else near[:400], :3] = -0.5
+    h = Harness(scenes.floor_for_cameras(scene, [cam]), cam, isect_cap=1 << 22)
+    h.api.project_splats(h.ctx, h.model, h.rp)
+    tc_o, vals_o, keys_o, ranges_o = orc.bin_sort(h.ctx.proj0[:n].cpu().numpy(), h.ctx.proj1[:n].cpu().numpy(), W, H)
+    cap = len(vals_o) - short
+    h.ctx._alloc_isect(cap)
+    backing = {k: torch.full((cap + 512,), 7, dtype=torch.int32, device="cuda:0") for k in ("keys", "vals", "keys_sorted", "vals_sorted")}
+    for k, t in backing.items():
+        setattr(h.ctx, k, t[:cap])
+    assert walked(W, H, n, cap) and len(vals_o) > 12_000
+    cs, total = h.ctx.struct(), C.c_uint32(0)
+    assert api.lib().b2k_bin_sort(C.byref(cs), n, api._stream(None)) == api.B2K_OK
+    assert api.lib().b2k_read_num_isect(C.byref(cs), api._stream(None), C.byref(total)) == (api.B2K_ERR_OVERFLOW if short else api.B2K_OK)
+    assert total.value == len(vals_o) and all(bool((t[cap:] == 7).all()) for t in backing.values())
+    assert np.array_equal(h.u32(h.ctx.vals_sorted), vals_o[:cap]) and np.array_equal(h.u32(h.ctx.keys_sorted), keys_o[:cap])
+    assert np.array_equal(h.u32(h.ctx.tile_ranges).reshape(-1, 2), np.minimum(ranges_o, cap))
+    h.api.bin_and_sort(h.ctx, h.model)
+    assert h.ctx.num_isect == len(vals_o) and np.array_equal(h.u32(h.ctx.vals_sorted, len(vals_o)), vals_o)
+    assert np.array_equal(h.u32(h.ctx.tile_ranges).reshape(-1, 2), ranges_o)
 
 
 def test_chunks_of_wide_splats():
