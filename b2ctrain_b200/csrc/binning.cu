@@ -1,6 +1,6 @@
 // Entry points of the binning stage and of the front-to-back chunked renderer. Reference semantics: bin_and_sort
-// (src/gpu/binning.cu:109-145). Depth order: sort.cu; from depth order to the tiles' lists: bins.cu. No host round trip: every
-// count stays on the device, so a view is one asynchronous chain.
+// (src/gpu/binning.cu:109-145). Depth order: sort.cu; from depth order to the tiles' lists: bins.cu, in small whole views walk.cu. No host round
+// trip: every count stays on the device, so a view is one asynchronous chain.
 #include "common.cuh"
 #include <algorithm>
 
@@ -177,7 +177,7 @@ extern "C" int b2k_read_num_isect(const B2kCtx* c, b2k_stream_t stream, uint32_t
 // cannot: a plugin loaded into a process whose memory pool is owned and fully reserved by the host application, a
 // render thread that must never take the allocator's lock, or a caller inside a region where the CUDA allocator is
 // off limits. For them the same scratch lives here, inside the library image, as a fixed device array. It is sized
-// for contexts of at most B2K_STATIC_MAX_SPLATS per-splat entries (about 3.7 MB, held by every GPU that loads the
+// for contexts of at most B2K_STATIC_MAX_SPLATS per-splat entries (about 3.8 MB, held by every GPU that loads the
 // library, until the process exits).
 // ---------------------------------------------------------------------------------------------------------------
 namespace b2k {

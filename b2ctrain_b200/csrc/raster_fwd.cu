@@ -80,7 +80,7 @@ __device__ __forceinline__ float2 pair_alpha(const float4& q0, const float4& q1,
                      __float_as_uint(sigma.y) <= __float_as_uint(power.y) ? fminf(ALPHA_MAX, al.y) : 0.f);
 }
 
-// The tiles of a chunk behind the first that have a list (tile_scan has written them down): those with long lists first.
+// The tiles of a chunk that have a list (tile_scan has written them down, see lists_tiles): those with long lists first.
 struct TileList {
   const uint32_t* list; uint32_t longs, count; int n_tiles;
   __device__ __forceinline__ int at(uint32_t w) const { return list ? (int)list[w < longs ? w : (uint32_t)n_tiles - 1u - (w - longs)] : (int)w; }

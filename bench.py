@@ -550,13 +550,17 @@ def stage_roofline(args, tr, cams, targets, mine, stats, clocks=None):
 
 
 def render_launches(n, W, H, chunks):
-    """Kernels of one render: the whole view (clear, projection, big boxes, depth sort, binning, tile ids, compositing) or depth
-    chunks (projection, depth sort, chunk words, per chunk binning and compositing). The binning takes seven kernels per band
-    of at most 2,048 bins of 8x8 tiles; the depth sort one up to 8,192 splats, ten above."""
+    """Kernels of one render: the whole view (projection, large boxes, depth sort, binning, compositing) or depth chunks (projection, depth
+    sort, chunk words, per chunk binning and compositing). The binning takes seven kernels per band of at most 2,048 bins of 8x8 tiles, and of a
+    whole view one more for the tile ids; a small whole view's takes two (given room for its hit words); the depth sort one up to 32,768 splats, ten above."""
+    tiles_x, tiles_y = -(-W // 8), -(-H // 8)
     bins_x, bin_rows = -(-W // 64), -(-H // 64)
     bands = -(-bin_rows // (2048 // bins_x))
-    sort = 1 if n <= 8192 else 10
-    return 1 + sort + 1 + chunks * (7 * bands + 1) if chunks > 1 else 3 + sort + 7 * bands + 2
+    sort = 1 if n <= 32768 else 10
+    if chunks > 1:
+        return 1 + sort + 1 + chunks * (7 * bands + 1)
+    walk = tiles_x * tiles_y <= 4096 and n * bins_x * bin_rows <= 1 << 20
+    return 2 + sort + (2 if walk else 7 * bands + 1) + 1
 
 
 def bench_render(args, scene, cams, device, rank, world, barrier, max_over_ranks, sampler):
